@@ -97,7 +97,8 @@ int qd_layout_workspace_bytes(const qd_layout* L, int64_t* bytes);
  * reference only has omp_get_wtime around whole runs, magnus_IMSRG.f90:30,159).
  * enable != 0 starts (and resets) it.  qd_layout_profile_read synchronises
  * and returns accumulated milliseconds and launch counts per stage:
- * 0 E0 (110+220), 1 commutator_111, 2 commutator_121, 3 commutator_221,
+ * 0 E0 (110+220), 1 commutator_111, 2 commutator_121, 3 commutator_221 (for
+ * operators that conserve (m_l, m_s) stages 0-2 run fused with it),
  * 4 commutator_122, 5 calc_cc, 6 ladder GEMMs (matrix_mult222),
  * 7 Pandya GEMMs (construct_cc_ints), 8 particle-hole gather, 9 BCH glue.  */
 #define QD_NSTAGE 10

@@ -75,7 +75,7 @@ int op_new(qd_layout* L, int herm, qd_op** out) {
   }
   ++L->children;
   QD_CUDA(cudaMemsetAsync(op->d, 0, sizeof(double) * L->neq, L->stream));
-  op->zero_mask = ALL_PARTS;
+  op->zero_mask = ALL_PARTS | CONSERVES;
   *out = op;
   return QD_OK;
 }
@@ -140,7 +140,19 @@ int scalar_out(qd_layout* L, const double* dslot, double* out) {
 int same_layout(const qd_op* a, const qd_op* b) {
   CHECK(a && b, QD_ERR_ARG, "null operator handle");
   CHECK(a->L == b->L, QD_ERR_ARG, "operators belong to different layouts");
+  // an operand whose raw pointer the caller holds may have been written since
+  for (const qd_op* o : {a, b})
+    if (o->exposed) const_cast<qd_op*>(o)->zero_mask &= ~CONSERVES;
   return QD_OK;
+}
+
+// Operators of one role pair (G/G0, HS/HS0, ETA/ETA0, INT2/AD) trade buffers
+// instead of copying: "G0 = G" becomes a swap after which G's buffer is
+// rewritten.
+void swap_ops(qd_op* a, qd_op* b) {
+  std::swap(a->d, b->d);
+  std::swap(a->zero_mask, b->zero_mask);
+  std::swap(a->exposed, b->exposed);
 }
 
 // zero mask of a host vector: parts that are identically zero
@@ -163,8 +175,21 @@ unsigned host_zero_mask(const qd_layout* L, const double* v) {
     }
     if (z) m |= 1u << (P_HHHH + p);
   }
+  const int n = L->n, mp = L->mp;
+  bool cons = true;
+  for (int j = 0; j < L->m && cons; ++j)
+    for (int i = 0; i < L->m && cons; ++i) {
+      if (L->gid[i] == L->gid[j] || (i < n && j >= n)) continue;
+      const i64 e = i < n ? L->o_fhh + i + (i64)j * n
+                          : (j < n ? L->o_fph + (i - n) + (i64)j * mp : L->o_fpp + (i - n) + (i64)(j - n) * mp);
+      cons = v[e] == 0.0;
+    }
+  if (cons) m |= CONSERVES;
   return m;
 }
+
+// CONSERVES of a commutator: both operands conserve (m_l, m_s)
+unsigned conserves(const qd_op* a, const qd_op* b) { return a->zero_mask & b->zero_mask & CONSERVES; }
 
 // RAII stage timer: records an event pair around a stage when profiling is on
 struct StageTimer {
@@ -174,6 +199,11 @@ struct StageTimer {
   StageTimer(qd_layout* l, int i) : L(l), id(i) {
     if (L->prof.on && cudaEventCreate(&a) == cudaSuccess && cudaEventCreate(&b) == cudaSuccess)
       cudaEventRecord(a, L->stream);
+  }
+  void cancel() {  // nothing was launched
+    if (a) cudaEventDestroy(a);
+    if (b) cudaEventDestroy(b);
+    a = b = nullptr;
   }
   ~StageTimer() {
     if (L->prof.on && a && b) {
@@ -211,7 +241,7 @@ int stage_111(qd_layout* L, const qd_op* A, const qd_op* B, qd_op* C) {
   StageTimer tm(L, S_111);
   const double* bufs[7] = {A->d, B->d, nullptr, nullptr, C->d, nullptr, nullptr};
   TRY(run_program(L, L->prog_111, bufs, (double)A->herm, (double)B->herm, A->zero_mask, B->zero_mask));
-  C->zero_mask &= ~((1u << P_FHH) | (1u << P_FPP) | (1u << P_FPH));
+  C->zero_mask = (C->zero_mask & ~(ONE_BODY | CONSERVES)) | conserves(A, B);
   return QD_OK;
 }
 
@@ -250,21 +280,38 @@ int stage_222(qd_layout* L, const qd_op* A, const qd_op* B, qd_op* C, const qd_c
   return QD_OK;
 }
 
-int commutator_seq(qd_layout* L, const qd_op* A, const qd_op* B, qd_op* C, qd_op* w1, qd_op* w2, qd_cc* ACC,
-                   qd_cc* BCC, bool pandya) {
-  TRY(build_programs(L));
+int white(qd_op* gen, const qd_op* H) {
+  TRY(launch_white(H->L, gen->d, H->d, H->herm));
+  gen->zero_mask &= ~((1u << P_FPH) | (1u << P_PPHH)) & (conserves(H, H) ? ~0u : ~CONSERVES);
+  return QD_OK;
+}
+
+// E0 and the one-body part of C = [A, B] (110, 220, 111, 121, 221): two
+// launches when both operands conserve (m_l, m_s), piece by piece otherwise.
+int stage_one_body(qd_layout* L, const qd_op* A, const qd_op* B, qd_op* C) {
+  bool done = false;
+  {
+    StageTimer tm(L, S_221);
+    TRY(launch_onebody(L, A, B, C->d, &done));
+    if (!done) tm.cancel();
+  }
+  if (done) return QD_OK;
   TRY(stage_e0(L, A, B, C->d, 0.0));
   TRY(stage_111(L, A, B, C));
   {
     StageTimer tm(L, S_121);
     TRY(launch_121(L, A, B, C->d));
   }
-  {  // w1, w2 are workspaces of the whole commutator: the fused 221 leaves them untouched
-    (void)w1;
-    (void)w2;
-    StageTimer tm(L, S_221);
-    TRY(launch_221_fused(L, A, B, C->d));
-  }
+  StageTimer tm(L, S_221);
+  return launch_221_fused(L, A, B, C->d);
+}
+
+int commutator_seq(qd_layout* L, const qd_op* A, const qd_op* B, qd_op* C, qd_op* w1, qd_op* w2, qd_cc* ACC,
+                   qd_cc* BCC, bool pandya) {
+  (void)w1;  // workspaces of the whole commutator: the fused 221 leaves them untouched
+  (void)w2;
+  TRY(build_programs(L));
+  TRY(stage_one_body(L, A, B, C));
   {
     StageTimer tm(L, S_122);
     TRY(launch_122(L, A, B, C->d));
@@ -279,7 +326,7 @@ int commutator_seq(qd_layout* L, const qd_op* A, const qd_op* B, qd_op* C, qd_op
     BCC->herm = B->herm;
   }
   TRY(stage_222(L, A, B, C, pandya ? BCC : nullptr, pandya ? ACC : nullptr));
-  C->zero_mask = 0;
+  C->zero_mask = conserves(A, B);
   return QD_OK;
 }
 
@@ -615,6 +662,7 @@ int qd_op_device_ptr(qd_op* op, double** dptr) {
   CHECK(op && dptr, QD_ERR_ARG, "null argument");
   *dptr = op->d;
   op->zero_mask = 0;  // the caller may write through the pointer
+  op->exposed = true;
   return QD_OK;
 }
 
@@ -632,7 +680,7 @@ int qd_add_arrays(const qd_op* r1, double s1, const qd_op* r2, double s2, qd_op*
   qd_layout* L = r1->L;
   TRY(use_device(L));
   TRY(launch_axpy(L, r1->d, s1, r2->d, s2, r3->d, L->neq));
-  unsigned m1 = s1 == 0.0 ? ALL_PARTS : r1->zero_mask, m2 = s2 == 0.0 ? ALL_PARTS : r2->zero_mask;
+  unsigned m1 = s1 == 0.0 ? ALL_PARTS | CONSERVES : r1->zero_mask, m2 = s2 == 0.0 ? ALL_PARTS | CONSERVES : r2->zero_mask;
   r3->zero_mask = m1 & m2;
   return QD_OK;
 }
@@ -650,7 +698,7 @@ int qd_set_to_zero(qd_op* r1) {
   CHECK(r1, QD_ERR_ARG, "null operator");
   TRY(use_device(r1->L));
   QD_CUDA(cudaMemsetAsync(r1->d, 0, sizeof(double) * r1->L->neq, r1->L->stream));
-  r1->zero_mask = ALL_PARTS;
+  r1->zero_mask = ALL_PARTS | CONSERVES;
   return QD_OK;
 }
 
@@ -694,7 +742,7 @@ int qd_commutator_121(const qd_op* r1, const qd_op* r2, qd_op* r3) {
   TRY(same_layout(r1, r3));
   TRY(use_device(r1->L));
   TRY(launch_121(r1->L, r1, r2, r3->d));
-  r3->zero_mask &= ~((1u << P_FHH) | (1u << P_FPP) | (1u << P_FPH));
+  r3->zero_mask &= ~ONE_BODY & (conserves(r1, r2) ? ~0u : ~CONSERVES);
   return QD_OK;
 }
 
@@ -706,7 +754,7 @@ int qd_commutator_221(const qd_op* r1, const qd_op* r2, qd_op* r3, qd_op* w1, qd
   TRY(use_device(r1->L));
   TRY(build_programs(r1->L));
   TRY(stage_221(r1->L, r1, r2, r3, w1, w2));
-  r3->zero_mask &= ~((1u << P_FHH) | (1u << P_FPP) | (1u << P_FPH));
+  r3->zero_mask &= ~ONE_BODY;
   return QD_OK;
 }
 
@@ -715,7 +763,7 @@ int qd_commutator_122(const qd_op* r1, const qd_op* r2, qd_op* r3) {
   TRY(same_layout(r1, r3));
   TRY(use_device(r1->L));
   TRY(launch_122(r1->L, r1, r2, r3->d));
-  r3->zero_mask &= (1u << P_FHH) | (1u << P_FPP) | (1u << P_FPH);
+  r3->zero_mask &= ONE_BODY | CONSERVES;
   return QD_OK;
 }
 
@@ -725,7 +773,7 @@ int qd_commutator_222(const qd_op* r1, const qd_op* r2, qd_op* r3, qd_op* w1, co
   TRY(same_layout(r1, r3));
   TRY(use_device(r1->L));
   TRY(build_programs(r1->L));
-  unsigned keep = r3->zero_mask & ((1u << P_FHH) | (1u << P_FPP) | (1u << P_FPH));
+  unsigned keep = r3->zero_mask & (ONE_BODY | CONSERVES);
   TRY(stage_222(r1->L, r1, r2, r3, HCC, ETACC));
   r3->zero_mask = keep;
   return QD_OK;
@@ -758,8 +806,8 @@ int qd_dgam(const qd_op* H, qd_op* DER, qd_cc* HCC, qd_cc* ETACC) {
   qd_op* eta = w->eta;
   eta->herm = -1;
   QD_CUDA(cudaMemsetAsync(eta->d, 0, sizeof(double) * L->neq, L->stream));
-  eta->zero_mask = ALL_PARTS;
-  TRY(qd_build_white(eta, H));
+  eta->zero_mask = ALL_PARTS | CONSERVES;
+  TRY(white(eta, H));
   TRY(commutator_seq(L, eta, H, DER, w->w1, w->w2, ETACC ? ETACC : w->ca, HCC ? HCC : w->cb, true));
   return QD_OK;
 }
@@ -785,7 +833,7 @@ int qd_eom_matvec(const qd_op* H, const qd_op* Q, qd_op* HQ) {
   qd_op* X = w->eomq;
   QD_CUDA(cudaMemcpyAsync(X->d, Q->d, sizeof(double) * L->neq, cudaMemcpyDeviceToDevice, L->stream));
   TRY(launch_keep_parts(L, X->d, exc));
-  X->zero_mask = (ALL_PARTS & ~exc) | (Q->zero_mask & exc);
+  X->zero_mask = (ALL_PARTS & ~exc) | (Q->zero_mask & (exc | CONSERVES));
   X->herm = 1;
   TRY(commutator_seq(L, H, X, HQ, w->w1, w->w2, w->cb, w->ca, true));
   X->herm = -1;
@@ -793,7 +841,7 @@ int qd_eom_matvec(const qd_op* H, const qd_op* Q, qd_op* HQ) {
   TRY(launch_axpy(L, HQ->d, 0.5, w->eomt->d, 0.5, HQ->d, L->neq));
   TRY(launch_keep_parts(L, HQ->d, exc));
   HQ->herm = 1;
-  HQ->zero_mask = ALL_PARTS & ~exc;
+  HQ->zero_mask = (ALL_PARTS & ~exc) | conserves(H, X);
   return QD_OK;
 }
 
@@ -846,9 +894,7 @@ int qd_cc_download(const qd_cc* cc, double* host, int64_t n, int64_t* needed) {
 int qd_build_white(qd_op* gen, const qd_op* H) {
   TRY(same_layout(gen, H));
   TRY(use_device(H->L));
-  TRY(launch_white(H->L, gen->d, H->d, H->herm));
-  gen->zero_mask &= ~((1u << P_FPH) | (1u << P_PPHH));
-  return QD_OK;
+  return white(gen, H);
 }
 
 int qd_mbpt2(const qd_op* H, double* out) {
@@ -939,7 +985,7 @@ static int bch_term_graph(qd_layout* L, const qd_op* G, qd_op* AD, qd_op* INT2, 
     QD_CUDA(cudaGraphLaunch(tg.exec, L->stream));
     L->nlaunch += tg.launches;
     ++L->graph_replays;
-    INT2->zero_mask = 0;  // what the captured commutator_seq leaves on the host side
+    INT2->zero_mask = conserves(G, AD);  // what the captured commutator_seq leaves on the host side
     if (pandya) {
       OCC->filled = true;
       OCC->herm = G->herm;
@@ -1037,6 +1083,7 @@ int capture_step(qd_layout* L, qd_op* HS, const qd_op* G, const qd_op* H, double
   cudaStream_t st = L->stream;
   qd_op ad = *H, out = *H;  // host views of the two buffers (herm +1, as BCH_EXPAND sets)
   ad.herm = out.herm = 1;
+  ad.exposed = out.exposed = false;
   cudaGraph_t g = nullptr;
   QD_CUDA(cudaGraphCreate(&g, 0));
   int rc = QD_OK;
@@ -1075,7 +1122,7 @@ int capture_step(qd_layout* L, qd_op* HS, const qd_op* G, const qd_op* H, double
     }
     const long long n1 = L->nlaunch;
     ad.d = P;
-    ad.zero_mask = 0;
+    ad.zero_mask = conserves(G, H);
     out.d = Q;
     r2 = bch_term(L, G, &ad, &out, HS, w1, w2, HCC, OCC, pandya, 0.0, k);
     if (!r2) r2 = launch_bch_decide(L, red_slot(L, 1), k, conv, hloop, hmore, 1);
@@ -1144,10 +1191,11 @@ int bch_step_graph(qd_layout* L, qd_op* HS, const qd_op* G, const qd_op* H, qd_o
     if (sg.failed || sg.seen++ == 0) return QD_OK;  // eager (first sight builds plans for H's masks)
     // plans and task lists of the later terms ([G, X] with X a full operator)
     qd_op full = *H;  // H as a full operator: the masks of AD in the later terms
-    full.zero_mask = 0;
-    TRY(prepare_program(L, L->prog_ladder, G->zero_mask, 0u));
-    TRY(prepare_program(L, L->prog_111, G->zero_mask, 0u));
+    full.zero_mask = conserves(G, H);
+    TRY(prepare_program(L, L->prog_ladder, G->zero_mask, full.zero_mask));
+    TRY(prepare_program(L, L->prog_111, G->zero_mask, full.zero_mask));
     TRY(prepare_program(L, L->prog_pandya, 0u, 0u));
+    TRY(prepare_onebody(L));
     TRY(prepare_122(L, G, &full));
     TRY(prepare_program(L, L->prog_ladder, G->zero_mask, H->zero_mask));
     TRY(prepare_program(L, L->prog_111, G->zero_mask, H->zero_mask));
@@ -1169,9 +1217,7 @@ int bch_step_graph(qd_layout* L, qd_op* HS, const qd_op* G, const qd_op* H, qd_o
   ++L->graph_replays;
   // host-side state the eager loop leaves: HS and the workspaces hold full
   // operators; the two workspace buffers keep their handles
-  HS->zero_mask = 0;
-  INT2->zero_mask = 0;
-  AD->zero_mask = 0;
+  HS->zero_mask = INT2->zero_mask = AD->zero_mask = conserves(G, H);
   if (pandya) {
     OCC->filled = true;
     OCC->herm = G->herm;
@@ -1219,11 +1265,10 @@ int bch_eager(qd_layout* L, qd_op* HS, const qd_op* G, const qd_op* H, qd_op* IN
   const double conv = (double)1e-5f;  // "conv = 1e-5" is a real(4) literal in the reference
   double* const p0 = INT2->d;
   TRY(qd_copy_arrays(H, HS));
-  TRY(qd_copy_arrays(HS, INT2));
+  TRY(qd_copy_arrays(H, INT2));
   int count = 0;
   for (int i = 2; i <= 12; ++i) {
-    std::swap(INT2->d, AD->d);  // AD = previous term; INT2 becomes the output buffer
-    std::swap(INT2->zero_mask, AD->zero_mask);
+    swap_ops(INT2, AD);  // AD = previous term; INT2 becomes the output buffer
     const double cof = kCof[i - 2];
     TRY(bch_term_graph(L, G, AD, INT2, HS, w1, w2, HCC, OCC, pandya, i, cof));
     ++count;
@@ -1233,8 +1278,7 @@ int bch_eager(qd_layout* L, qd_op* HS, const qd_op* G, const qd_op* H, qd_op* IN
     if (n2 * cof / n1 < conv) break;
   }
   if (INT2->d != p0) {  // the workspaces keep their buffers (contents unspecified)
-    std::swap(INT2->d, AD->d);
-    std::swap(INT2->zero_mask, AD->zero_mask);
+    swap_ops(INT2, AD);
   }
   if (nterms) *nterms = count;
   return QD_OK;
@@ -1275,13 +1319,6 @@ namespace {
 const double kConvCriteria = (double)1e-9f;  // real(4) literal in the reference
 
 int flow_eta_norm(qd_flow* f, const qd_op* op, double* out) { return qd_mat_2_norm(op, out); }
-
-// Operators of one role pair (G/G0, HS/HS0, ETA/ETA0) trade buffers instead
-// of copying: "G0 = G" becomes a swap after which G's buffer is rewritten.
-void swap_ops(qd_op* a, qd_op* b) {
-  std::swap(a->d, b->d);
-  std::swap(a->zero_mask, b->zero_mask);
-}
 
 // Give the caller's HS its own buffer back (copying the current contents).
 int flow_home_hs(qd_flow* f) {
@@ -1343,11 +1380,11 @@ int qd_flow_create(const qd_op* HAM, qd_op* HS, unsigned flags, qd_flow** out) {
   // and Vpphh
   for (qd_op* z : {f->ETA, f->ETA0, f->G}) {
     if (cudaMemsetAsync(z->d, 0, sizeof(double) * L->neq, L->stream) != cudaSuccess) rc = QD_ERR_CUDA;
-    z->zero_mask = ALL_PARTS;
+    z->zero_mask = ALL_PARTS | CONSERVES;
   }
   if (!rc) rc = qd_copy_arrays(HAM, HS);
   HS->herm = 1;
-  if (!rc) rc = qd_build_white(f->ETA, HS);
+  if (!rc) rc = white(f->ETA, HS);
   if (!rc) rc = flow_eta_norm(f, f->ETA, &f->nrm1);
   if (!rc) rc = qd_mbpt2(HAM, &f->crit);
   if (!rc) rc = flow_e0(f, &f->E0);
@@ -1371,7 +1408,7 @@ int qd_flow_warm_start(qd_flow* f, const qd_op* G, double s) {
   int terms = 0;
   TRY(qd_bch_expand(f->HS, f->G, f->HAM, f->INT1, f->INT2, f->AD, f->w1, f->w2, f->HCC, f->OCC, f->flags, &terms));
   f->comms += terms;
-  TRY(qd_build_white(f->ETA, f->HS));
+  TRY(white(f->ETA, f->HS));
   double mb;
   TRY(qd_mbpt2(f->HS, &mb));
   f->crit = std::fabs(mb);
@@ -1410,7 +1447,7 @@ int flow_begin(qd_flow* f, qd_flow_step_info* inf, bool* converged) {
 int flow_end(qd_flow* f, int terms, qd_flow_step_info* inf) {
   f->comms += terms;
   swap_ops(f->ETA, f->ETA0);  // ETA0 = ETA: build_white rewrites fph and Vpphh, the rest stays 0
-  TRY(qd_build_white(f->ETA, f->HS));
+  TRY(white(f->ETA, f->HS));
   double nrm2, E0;
   TRY(flow_eta_norm(f, f->ETA, &nrm2));
   TRY(flow_e0(f, &E0));
@@ -1562,10 +1599,7 @@ int commutator_batch(BatchCtx& bc, std::vector<CommItem>& items, bool pandya) {
     qd_layout* L = it.L;
     Ls.push_back(L);
     TRY(build_programs(L));
-    TRY(stage_e0(L, it.A, it.B, it.C->d, 0.0));
-    TRY(stage_111(L, it.A, it.B, it.C));
-    TRY(launch_121(L, it.A, it.B, it.C->d));
-    TRY(launch_221_fused(L, it.A, it.B, it.C->d));
+    TRY(stage_one_body(L, it.A, it.B, it.C));
     if (pandya) {
       TRY(launch_calc_cc(L, it.A, it.ACC->d));
       it.ACC->filled = true;
@@ -1598,7 +1632,7 @@ int commutator_batch(BatchCtx& bc, std::vector<CommItem>& items, bool pandya) {
       TRY(run_program(L, L->prog_pandya, zb, it.ACC->herm, it.BCC->herm, 0u, 0u));
       TRY(launch_pandya_tiles(L, L->d_z, it.C->d));
     }
-    it.C->zero_mask = 0;
+    it.C->zero_mask = conserves(it.A, it.B);
   }
   return QD_OK;
 }
@@ -1616,7 +1650,7 @@ int bch_batch(BatchCtx& bc, const std::vector<qd_flow*>& fl, std::vector<int>& t
     f->INT2->herm = 1;
     f->AD->herm = 1;
     TRY(qd_copy_arrays(f->HAM, f->HS));
-    TRY(qd_copy_arrays(f->HS, f->INT2));
+    TRY(qd_copy_arrays(f->HAM, f->INT2));
     p0[j] = f->INT2->d;
     terms[j] = 0;
     live.push_back((int)j);
@@ -1626,8 +1660,7 @@ int bch_batch(BatchCtx& bc, const std::vector<qd_flow*>& fl, std::vector<int>& t
     std::vector<CommItem> items;
     for (int j : live) {
       qd_flow* f = fl[j];
-      std::swap(f->INT2->d, f->AD->d);
-      std::swap(f->INT2->zero_mask, f->AD->zero_mask);
+      swap_ops(f->INT2, f->AD);
       items.push_back(CommItem{f->L, f->G, f->AD, f->INT2, f->OCC, f->HCC});
     }
     TRY(commutator_batch(bc, items, pandya));
@@ -1650,8 +1683,7 @@ int bch_batch(BatchCtx& bc, const std::vector<qd_flow*>& fl, std::vector<int>& t
   }
   for (size_t j = 0; j < fl.size(); ++j)  // the workspaces keep their buffers
     if (fl[j]->INT2->d != p0[j]) {
-      std::swap(fl[j]->INT2->d, fl[j]->AD->d);
-      std::swap(fl[j]->INT2->zero_mask, fl[j]->AD->zero_mask);
+      swap_ops(fl[j]->INT2, fl[j]->AD);
     }
   return QD_OK;
 }

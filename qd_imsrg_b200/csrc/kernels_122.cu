@@ -438,7 +438,7 @@ __global__ void __launch_bounds__(T122, 1024 / T122) k_122_tile(DevLayout L, con
 //            B_pppp column with coefficient -s fA(t, h); kind 1 an hh column
 //            (h, t) of B_pphh and A_pphh.
 __host__ __device__ __forceinline__ bool gen_like(unsigned zmask) {
-  return (zmask | (1u << P_FPH) | (1u << P_PPHH)) == ALL_PARTS;
+  return ((zmask | (1u << P_FPH) | (1u << P_PPHH)) & ALL_PARTS) == ALL_PARTS;
 }
 
 constexpr int SP_T = 256, SP_B = 64, SP_LD = SP_B + 1;

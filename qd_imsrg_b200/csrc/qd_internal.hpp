@@ -30,6 +30,10 @@ typedef long long i64;
 // qd_op::zero_mask)
 enum Part { P_FHH = 0, P_FPP, P_FPH, P_HHHH, P_PPPP, P_PPHH, P_PHPH, P_PPPH, P_PHHH, P_COUNT };
 constexpr unsigned ALL_PARTS = (1u << P_COUNT) - 1;
+// Further bit of qd_op::zero_mask: no one-body entry couples states of
+// different (m_l, m_s) (such entries are all known to be zero).
+constexpr unsigned CONSERVES = 1u << (P_COUNT + 1);
+constexpr unsigned ONE_BODY = (1u << P_FHH) | (1u << P_FPP) | (1u << P_FPH);
 
 // pair-table packing: idx (13 bits) | block (10 bits) | class-1 (2 bits) | swap (1 bit)
 __host__ __device__ inline int pt_idx(int e) { return e & 0x1FFF; }
@@ -123,6 +127,7 @@ struct GemmProgram {
 
 namespace qd {
 // stages timed by the optional per-stage CUDA-event profiler
+struct OneBody;  // tables of the fused one-body stage (onebody.cu)
 enum Stage { S_E0 = 0, S_111, S_121, S_221, S_122, S_CALC_CC, S_LADDER, S_PANDYA_GEMM, S_PANDYA_GATHER, S_GLUE,
              S_COUNT };
 struct StageProf {
@@ -171,6 +176,7 @@ struct qd_layout {
   int* d_ccflag = nullptr;        // per cross-coupled block: fph of A or B non-zero (121)
   const int* d_tgt221 = nullptr;  // one-body targets whose states share (m_l, m_s) (fused 221)
   int ntgt221 = -1;
+  qd::OneBody* onebody = nullptr;
   qd::i64 ws_bytes = 0;
   // GEMM programs
   qd::GemmProgram prog_ladder, prog_221, prog_111, prog_pandya;
@@ -190,6 +196,7 @@ struct qd_op {
   int herm = 1;
   double* d = nullptr;
   unsigned zero_mask = 0;  // parts known to be identically zero
+  bool exposed = false;    // a raw pointer to d was handed out: the caller may write between calls
 };
 
 struct qd_cc {
@@ -260,6 +267,9 @@ int launch_white(qd_layout* L, double* gen, const double* h, int herm);
 int launch_keep_parts(qd_layout* L, double* op, unsigned keep);
 int launch_121(qd_layout* L, const qd_op* A, const qd_op* B, double* C);
 int launch_221_trace(qd_layout* L, const qd_op* A, const qd_op* B, const qd_op* w1, const qd_op* w2, double* C);
+int prepare_onebody(qd_layout* L);
+int launch_onebody(qd_layout* L, const qd_op* A, const qd_op* B, double* C, bool* done);
+void onebody_free(qd_layout* L);
 int launch_221_fused(qd_layout* L, const qd_op* A, const qd_op* B, double* C);
 int launch_122(qd_layout* L, const qd_op* A, const qd_op* B, double* C);
 int launch_calc_cc(qd_layout* L, const qd_op* H, double* X);
