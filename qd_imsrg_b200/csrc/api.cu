@@ -82,8 +82,6 @@ int op_new(qd_layout* L, int herm, qd_op** out) {
 
 // Tear down a layout's device state and the layout itself.
 void layout_finish(qd_layout* L) {
-  drop_merged_gemm(L);
-  drop_merged_122(L);
   drop_122_plan(L);
   drop_eom_plans(L);
   layout_free_device(L);
@@ -258,11 +256,27 @@ int stage_221(qd_layout* L, const qd_op* A, const qd_op* B, qd_op* C, qd_op* w1,
   return QD_OK;
 }
 
-int stage_222(qd_layout* L, const qd_op* A, const qd_op* B, qd_op* C, const qd_cc* HCC, const qd_cc* ETACC) {
+// Whether a whole commutator takes its ladders with 122 (a split-form layout
+// keeps every ladder in the split form), and the ladders left then.
+bool ladder_in_122(const qd_layout* L, const qd_op* A) { return gen_like(A->zero_mask) && L->split_slices == 0; }
+GemmProgram& ladder_program(qd_layout* L, const qd_op* A) {
+  return ladder_in_122(L, A) ? L->prog_ladder_gen : L->prog_ladder;
+}
+
+constexpr i64 SPLIT_UPDATE_ENTRIES = 4000000;
+// Whether a BCH term's update of HS runs where C_pppp is made: C_pppp must be
+// final there (no ladder left to the grouped GEMM; the particle-hole channel
+// adds nothing to it, see launch_pandya_tiles).
+bool splits_update(qd_layout* L, const qd_op* G) {
+  return L->neq >= SPLIT_UPDATE_ENTRIES && ladder_in_122(L, G) && L->prog_ladder_gen.probs.empty();
+}
+
+int stage_222(qd_layout* L, const qd_op* A, const qd_op* B, qd_op* C, const qd_cc* HCC, const qd_cc* ETACC,
+              GemmProgram& ladders) {
   const double* bufs[7] = {A->d, B->d, nullptr, nullptr, C->d, nullptr, nullptr};
   {
     StageTimer tm(L, S_LADDER);
-    TRY(run_program(L, L->prog_ladder, bufs, (double)A->herm, (double)B->herm, A->zero_mask, B->zero_mask));
+    TRY(run_program(L, ladders, bufs, (double)A->herm, (double)B->herm, A->zero_mask, B->zero_mask));
   }
   if (HCC && ETACC && HCC->filled && ETACC->filled && L->zsize > 0) {
     CHECK(std::fabs(HCC->herm) == 1.0 && std::fabs(ETACC->herm) == 1.0, QD_ERR_ARG,
@@ -306,15 +320,80 @@ int stage_one_body(qd_layout* L, const qd_op* A, const qd_op* B, qd_op* C) {
   return launch_221_fused(L, A, B, C->d);
 }
 
+// Branches of one commutator beside the layout's stream.  E0 and the
+// one-body part, and for a generator-like A the parts other than C_pppp,
+// depend on nothing else of the commutator; their kernels leave much of the
+// chip idle (latency-bound, or a last wave of few CTAs), which the other
+// branches fill.  Small bases launched one by one are bound by the host's
+// launches, to which the events would only add; in a captured step they cost
+// nothing.  FORK_ENTRIES: where the gain and the events' cost meet (both
+// sides' times stand beside it).
+constexpr i64 FORK_ENTRIES = 1000000;
+
+struct Branches {
+  qd_layout* L = nullptr;
+  bool on = false;
+  int fork(qd_layout* l) {
+    L = l;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    QD_CUDA(cudaStreamIsCapturing(L->stream, &cs));
+    const bool cap = cs != cudaStreamCaptureStatusNone;
+    if (L->prof.on || (!cap && L->neq < FORK_ENTRIES)) return QD_OK;
+    if (!L->ev_fork) {
+      if (cap) return QD_OK;  // no stream or event is created inside a capture
+      TRY(make_branches(L));
+    }
+    QD_CUDA(cudaEventRecord(L->ev_fork, L->stream));
+    for (int k = 0; k < 2; ++k) QD_CUDA(cudaStreamWaitEvent(L->side[k], L->ev_fork, 0));
+    on = true;
+    return QD_OK;
+  }
+  cudaStream_t side(int k) const { return on ? L->side[k] : L->stream; }
+  int join() {
+    if (!on) return QD_OK;
+    on = false;
+    for (int k = 0; k < 2; ++k) {
+      QD_CUDA(cudaEventRecord(L->ev_side[k], L->side[k]));
+      QD_CUDA(cudaStreamWaitEvent(L->stream, L->ev_side[k], 0));
+    }
+    return QD_OK;
+  }
+  // an error path: the main stream still waits for what was launched
+  ~Branches() {
+    if (on) join();
+  }
+  static int make_branches(qd_layout* L) {
+    for (int k = 0; k < 2; ++k) {
+      QD_CUDA(cudaStreamCreateWithFlags(&L->side[k], cudaStreamNonBlocking));
+      QD_CUDA(cudaEventCreateWithFlags(&L->ev_side[k], cudaEventDisableTiming));
+    }
+    QD_CUDA(cudaEventCreateWithFlags(&L->ev_fork, cudaEventDisableTiming));
+    return QD_OK;
+  }
+};
+
+// The layout's launches go to another stream while this lives.
+struct OnStream {
+  qd_layout* L;
+  cudaStream_t keep;
+  OnStream(qd_layout* l, cudaStream_t s) : L(l), keep(l->stream) { L->stream = s; }
+  ~OnStream() { L->stream = keep; }
+};
+
 int commutator_seq(qd_layout* L, const qd_op* A, const qd_op* B, qd_op* C, qd_op* w1, qd_op* w2, qd_cc* ACC,
-                   qd_cc* BCC, bool pandya) {
+                   qd_cc* BCC, bool pandya, const HsUpdate* upd = nullptr) {
   (void)w1;  // workspaces of the whole commutator: the fused 221 leaves them untouched
   (void)w2;
   TRY(build_programs(L));
-  TRY(stage_one_body(L, A, B, C));
+  Branches br;
+  TRY(br.fork(L));
+  {
+    OnStream os(L, br.side(0));
+    TRY(stage_one_body(L, A, B, C));
+  }
   {
     StageTimer tm(L, S_122);
-    TRY(launch_122(L, A, B, C->d));
+    TRY(launch_122(L, A, B, C->d, ladder_in_122(L, A), br.side(1), upd));
   }
   if (pandya) {
     StageTimer tm(L, S_CALC_CC);
@@ -325,7 +404,13 @@ int commutator_seq(qd_layout* L, const qd_op* A, const qd_op* B, qd_op* C, qd_op
     BCC->filled = true;
     BCC->herm = B->herm;
   }
-  TRY(stage_222(L, A, B, C, pandya ? BCC : nullptr, pandya ? ACC : nullptr));
+  if (!pandya && ladder_program(L, A).probs.empty()) {  // no ladder is left
+    TRY(br.join());
+    C->zero_mask = conserves(A, B);
+    return QD_OK;
+  }
+  TRY(br.join());  // what follows adds to the parts that the branches write
+  TRY(stage_222(L, A, B, C, pandya ? BCC : nullptr, pandya ? ACC : nullptr, ladder_program(L, A)));
   C->zero_mask = conserves(A, B);
   return QD_OK;
 }
@@ -379,9 +464,7 @@ double* qd::scratch_operator(qd_layout* L) {
 
 namespace {
 
-const double kCof[11] = {1.0, 0.5, 0.166666666666666666, 0.04166666666666666, 0.0083333333333333333,
-                         .001388888888888, 1.984126984e-4, 2.48015873e-5, 2.755731922e-6, 2.755731922e-7,
-                         2.505210839e-8};
+const double kCof[11] = QD_BCH_COF;
 
 }  // namespace
 
@@ -679,7 +762,11 @@ int qd_add_arrays(const qd_op* r1, double s1, const qd_op* r2, double s2, qd_op*
   TRY(same_layout(r1, r3));
   qd_layout* L = r1->L;
   TRY(use_device(L));
-  TRY(launch_axpy(L, r1->d, s1, r2->d, s2, r3->d, L->neq));
+  // two generators into one that already holds zeros elsewhere (euler_step)
+  if (std::isfinite(s1) && std::isfinite(s2) && gen_like(r1->zero_mask & r2->zero_mask & r3->zero_mask) && !r1->exposed && !r2->exposed && !r3->exposed)
+    TRY(launch_axpy_gen(L, r1->d, s1, r2->d, s2, r3->d));
+  else
+    TRY(launch_axpy(L, r1->d, s1, r2->d, s2, r3->d, L->neq));
   unsigned m1 = s1 == 0.0 ? ALL_PARTS | CONSERVES : r1->zero_mask, m2 = s2 == 0.0 ? ALL_PARTS | CONSERVES : r2->zero_mask;
   r3->zero_mask = m1 & m2;
   return QD_OK;
@@ -706,7 +793,7 @@ int qd_mat_2_norm(const qd_op* r, double* out) {
   CHECK(r && out, QD_ERR_ARG, "null argument");
   qd_layout* L = r->L;
   TRY(use_device(L));
-  TRY(reduce_norm(L, r->d, red_slot(L, 0)));
+  TRY(reduce_norm(L, r->d, r->exposed ? 0u : r->zero_mask, red_slot(L, 0)));
   return scalar_out(L, red_slot(L, 0), out);
 }
 
@@ -762,7 +849,7 @@ int qd_commutator_122(const qd_op* r1, const qd_op* r2, qd_op* r3) {
   TRY(same_layout(r1, r2));
   TRY(same_layout(r1, r3));
   TRY(use_device(r1->L));
-  TRY(launch_122(r1->L, r1, r2, r3->d));
+  TRY(launch_122(r1->L, r1, r2, r3->d, false));
   r3->zero_mask &= ONE_BODY | CONSERVES;
   return QD_OK;
 }
@@ -774,7 +861,7 @@ int qd_commutator_222(const qd_op* r1, const qd_op* r2, qd_op* r3, qd_op* w1, co
   TRY(use_device(r1->L));
   TRY(build_programs(r1->L));
   unsigned keep = r3->zero_mask & (ONE_BODY | CONSERVES);
-  TRY(stage_222(r1->L, r1, r2, r3, HCC, ETACC));
+  TRY(stage_222(r1->L, r1, r2, r3, HCC, ETACC, r1->L->prog_ladder));
   r3->zero_mask = keep;
   return QD_OK;
 }
@@ -929,7 +1016,7 @@ int qd_hf_e2(qd_op* H, double* out) {
 // with one cudaGraphLaunch.  A capture that fails leaves the key eager.
 namespace {
 struct TermKey {
-  const void* p[8];  // G, AD, INT2, HS, w1, w2, OCC, HCC data
+  const void* p[9];  // G, AD, INT2, HS, w1, w2, OCC, HCC, source of HS
   unsigned mg, mad, mhs;
   int gh, term, flags, split;
   bool operator<(const TermKey& o) const { return std::memcmp(this, &o, sizeof(TermKey)) < 0; }
@@ -942,16 +1029,20 @@ struct TermGraph {
 };
 using TermGraphs = std::map<TermKey, TermGraph>;
 
-int bch_term(qd_layout* L, const qd_op* G, qd_op* AD, qd_op* INT2, qd_op* HS, qd_op* w1, qd_op* w2, qd_cc* HCC,
-             qd_cc* OCC, bool pandya, double cof, const int* kidx = nullptr) {
-  if (pandya) {
-    TRY(commutator_seq(L, G, AD, INT2, w1, w2, OCC, HCC, true));
-  } else {
-    TRY(commutator_seq(L, G, AD, INT2, w1, w2, nullptr, nullptr, false));
-  }
+// HS = src + cof [G, AD]: src is HS, or for the first term H (= AD)
+int bch_term(qd_layout* L, const qd_op* G, const qd_op* AD, qd_op* INT2, const qd_op* src, qd_op* HS, qd_op* w1,
+             qd_op* w2, qd_cc* HCC, qd_cc* OCC, bool pandya, double cof, int* kidx = nullptr, const BchDecide& dec = BchDecide{}) {
+  HsUpdate upd;
+  const bool split = splits_update(L, G);
+  if (split) TRY(hs_update_begin(L, src->d, HS->d, cof, kidx, &upd));
+  TRY(commutator_seq(L, G, AD, INT2, w1, w2, pandya ? OCC : nullptr, pandya ? HCC : nullptr, pandya,
+                     split ? &upd : nullptr));
   {
     StageTimer tm(L, S_GLUE);
-    TRY(launch_axpy_norms(L, HS->d, 1.0, INT2->d, cof, HS->d, red_slot(L, 1), kidx));
+    if (split)
+      TRY(launch_axpy_norms_rest(L, INT2->d, upd, red_slot(L, 1), dec));
+    else
+      TRY(launch_axpy_norms(L, src->d, 1.0, INT2->d, cof, HS->d, red_slot(L, 1), kidx, dec));
   }
   if (!kidx)  // host decides: copy both norms back
     QD_CUDA(cudaMemcpyAsync(L->h_red + 1, red_slot(L, 1), 2 * sizeof(double), cudaMemcpyDeviceToHost, L->stream));
@@ -959,9 +1050,9 @@ int bch_term(qd_layout* L, const qd_op* G, qd_op* AD, qd_op* INT2, qd_op* HS, qd
 }
 }  // namespace
 
-static int bch_term_graph(qd_layout* L, const qd_op* G, qd_op* AD, qd_op* INT2, qd_op* HS, qd_op* w1, qd_op* w2,
-                          qd_cc* HCC, qd_cc* OCC, bool pandya, int term, double cof) {
-  if (!L->use_graphs || L->prof.on) return bch_term(L, G, AD, INT2, HS, w1, w2, HCC, OCC, pandya, cof);
+static int bch_term_graph(qd_layout* L, const qd_op* G, const qd_op* AD, qd_op* INT2, const qd_op* src, qd_op* HS,
+                          qd_op* w1, qd_op* w2, qd_cc* HCC, qd_cc* OCC, bool pandya, int term, double cof) {
+  if (!L->use_graphs || L->prof.on) return bch_term(L, G, AD, INT2, src, HS, w1, w2, HCC, OCC, pandya, cof);
   if (!L->graphs) L->graphs = new TermGraphs();
   TermKey k;
   std::memset(&k, 0, sizeof(k));
@@ -973,6 +1064,7 @@ static int bch_term_graph(qd_layout* L, const qd_op* G, qd_op* AD, qd_op* INT2, 
   k.p[5] = w2->d;
   k.p[6] = OCC ? OCC->d : nullptr;
   k.p[7] = HCC ? HCC->d : nullptr;
+  k.p[8] = src->d;
   k.mg = G->zero_mask;
   k.mad = AD->zero_mask;
   k.mhs = HS->zero_mask;
@@ -996,7 +1088,7 @@ static int bch_term_graph(qd_layout* L, const qd_op* G, qd_op* AD, qd_op* INT2, 
   }
   if (tg.failed || tg.seen == 0) {
     ++tg.seen;
-    return bch_term(L, G, AD, INT2, HS, w1, w2, HCC, OCC, pandya, cof);
+    return bch_term(L, G, AD, INT2, src, HS, w1, w2, HCC, OCC, pandya, cof);
   }
   // second sight: capture, instantiate, launch
   const long long n0 = L->nlaunch;
@@ -1004,7 +1096,7 @@ static int bch_term_graph(qd_layout* L, const qd_op* G, qd_op* AD, qd_op* INT2, 
   int rc = QD_OK;
   cudaError_t e = cudaStreamBeginCapture(L->stream, cudaStreamCaptureModeThreadLocal);
   if (e == cudaSuccess) {
-    rc = bch_term(L, G, AD, INT2, HS, w1, w2, HCC, OCC, pandya, cof);
+    rc = bch_term(L, G, AD, INT2, src, HS, w1, w2, HCC, OCC, pandya, cof);
     e = cudaStreamEndCapture(L->stream, &graph);
   }
   if (e == cudaSuccess && rc == QD_OK && graph) e = cudaGraphInstantiate(&tg.exec, graph, 0);
@@ -1015,7 +1107,7 @@ static int bch_term_graph(qd_layout* L, const qd_op* G, qd_op* AD, qd_op* INT2, 
     tg.exec = nullptr;
     tg.failed = true;
     L->nlaunch = n0;
-    return bch_term(L, G, AD, INT2, HS, w1, w2, HCC, OCC, pandya, cof);
+    return bch_term(L, G, AD, INT2, src, HS, w1, w2, HCC, OCC, pandya, cof);
   }
   tg.launches = L->nlaunch - n0;
   ++L->graphs_captured;
@@ -1030,7 +1122,7 @@ namespace {
 // The exit test runs on the device (k_bch_decide), so the term loop is a
 // graph "while" node and a BCH step needs one host synchronisation (for the
 // term count) instead of one per term.  Layout of the graph:
-//   prologue: HS = H; AD = H; INT2 = [G, AD]; HS += cof(1) INT2; decide
+//   prologue: INT2 = [G, H]; HS = H + cof(1) INT2; decide
 //   while (go): INT2' = [G, INT2]; HS += cof INT2'; decide (sets go, more)
 //               if (more): INT2 = [G, INT2']; HS += cof INT2; decide (sets go)
 // The two buffers of INT2 and AD alternate between the two halves of the
@@ -1052,6 +1144,12 @@ struct StepGraph {
   long long first = 0, per_term = 0;  // launches of the prologue and of one later term
 };
 using StepGraphs = std::map<StepKey, StepGraph>;
+
+// Whether the first term can read H in place of copies in AD and HS: H is
+// none of the buffers written, and Hermitian as BCH_EXPAND takes AD to be.
+bool reads_h(const qd_op* H, const qd_op* HS, const double* P, const double* Q) {
+  return H->herm == 1 && H->d != HS->d && H->d != P && H->d != Q;
+}
 
 int* bch_counter(qd_layout* L) { return reinterpret_cast<int*>(red_slot(L, 16)); }
 
@@ -1096,18 +1194,20 @@ int capture_step(qd_layout* L, qd_op* HS, const qd_op* G, const qd_op* H, double
       rc = QD_ERR_CUDA;
       break;
     }
-    // prologue: HS = H, AD = H (Q), term 1 into P
+    // prologue: term 1 into P, of H itself unless that is one of the buffers
+    const bool direct = reads_h(H, HS, P, Q);
     int r2 = QD_OK;
     if (cudaMemsetAsync(k, 0, sizeof(int), st) != cudaSuccess ||
-        cudaMemcpyAsync(HS->d, H->d, sizeof(double) * L->neq, cudaMemcpyDeviceToDevice, st) != cudaSuccess ||
-        cudaMemcpyAsync(Q, H->d, sizeof(double) * L->neq, cudaMemcpyDeviceToDevice, st) != cudaSuccess)
+        (!direct && (cudaMemcpyAsync(HS->d, H->d, sizeof(double) * L->neq, cudaMemcpyDeviceToDevice, st) != cudaSuccess ||
+                     cudaMemcpyAsync(Q, H->d, sizeof(double) * L->neq, cudaMemcpyDeviceToDevice, st) != cudaSuccess)))
       r2 = QD_ERR_CUDA;
-    ad.d = Q;
+    ad.d = direct ? H->d : Q;
     ad.zero_mask = H->zero_mask;
     out.d = P;
     HS->zero_mask = H->zero_mask;
-    if (!r2) r2 = bch_term(L, G, &ad, &out, HS, w1, w2, HCC, OCC, pandya, 0.0, k);
-    if (!r2) r2 = launch_bch_decide(L, red_slot(L, 1), k, conv, hloop, hloop, 0);
+    if (!r2)
+      r2 = bch_term(L, G, &ad, &out, direct ? &ad : HS, HS, w1, w2, HCC, OCC, pandya, 0.0, k,
+                    BchDecide{hloop, hloop, 1, 0, conv});
     *first = L->nlaunch - n0;
     if (!r2) r2 = add_conditional(st, g, hloop, cudaGraphCondTypeWhile, &body);
     if (cudaStreamEndCapture(st, &cap) != cudaSuccess || r2) {
@@ -1124,8 +1224,7 @@ int capture_step(qd_layout* L, qd_op* HS, const qd_op* G, const qd_op* H, double
     ad.d = P;
     ad.zero_mask = conserves(G, H);
     out.d = Q;
-    r2 = bch_term(L, G, &ad, &out, HS, w1, w2, HCC, OCC, pandya, 0.0, k);
-    if (!r2) r2 = launch_bch_decide(L, red_slot(L, 1), k, conv, hloop, hmore, 1);
+    r2 = bch_term(L, G, &ad, &out, HS, HS, w1, w2, HCC, OCC, pandya, 0.0, k, BchDecide{hloop, hmore, 1, 1, conv});
     *per_term = L->nlaunch - n1;
     if (!r2) r2 = add_conditional(st, body, hmore, cudaGraphCondTypeIf, &body2);
     if (cudaStreamEndCapture(st, &cap) != cudaSuccess || r2) {
@@ -1140,8 +1239,7 @@ int capture_step(qd_layout* L, qd_op* HS, const qd_op* G, const qd_op* H, double
     }
     ad.d = Q;
     out.d = P;
-    r2 = bch_term(L, G, &ad, &out, HS, w1, w2, HCC, OCC, pandya, 0.0, k);
-    if (!r2) r2 = launch_bch_decide(L, red_slot(L, 1), k, conv, hloop, hloop, 0);
+    r2 = bch_term(L, G, &ad, &out, HS, HS, w1, w2, HCC, OCC, pandya, 0.0, k, BchDecide{hloop, hloop, 1, 0, conv});
     if (cudaStreamEndCapture(st, &cap) != cudaSuccess || r2) {
       rc = r2 ? r2 : QD_ERR_CUDA;
       break;
@@ -1167,10 +1265,11 @@ int capture_step(qd_layout* L, qd_op* HS, const qd_op* G, const qd_op* H, double
 int bch_eager(qd_layout* L, qd_op* HS, const qd_op* G, const qd_op* H, qd_op* INT2, qd_op* AD, qd_op* w1, qd_op* w2,
               qd_cc* HCC, qd_cc* OCC, bool pandya, int* nterms);
 
-// Whole step as a graph when possible; *done = false leaves it to the caller.
-int bch_step_graph(qd_layout* L, qd_op* HS, const qd_op* G, const qd_op* H, qd_op* INT2, qd_op* AD, qd_op* w1,
-                   qd_op* w2, qd_cc* HCC, qd_cc* OCC, bool pandya, int* nterms, bool* done) {
-  *done = false;
+// Launch the whole step as a graph when possible (bch_step_finish waits for
+// it); *launched = false leaves it to the caller.
+int bch_step_launch(qd_layout* L, qd_op* HS, const qd_op* G, const qd_op* H, qd_op* INT2, qd_op* AD, qd_op* w1,
+                    qd_op* w2, qd_cc* HCC, qd_cc* OCC, bool pandya, bool* launched) {
+  *launched = false;
   if (!L->use_graphs || L->prof.on || L->split_slices > 0) return QD_OK;
   if (!L->step_graphs) L->step_graphs = new StepGraphs();
   StepKey key;
@@ -1192,12 +1291,14 @@ int bch_step_graph(qd_layout* L, qd_op* HS, const qd_op* G, const qd_op* H, qd_o
     // plans and task lists of the later terms ([G, X] with X a full operator)
     qd_op full = *H;  // H as a full operator: the masks of AD in the later terms
     full.zero_mask = conserves(G, H);
-    TRY(prepare_program(L, L->prog_ladder, G->zero_mask, full.zero_mask));
+    TRY(prepare_program(L, ladder_program(L, G), G->zero_mask, full.zero_mask));
     TRY(prepare_program(L, L->prog_111, G->zero_mask, full.zero_mask));
     TRY(prepare_program(L, L->prog_pandya, 0u, 0u));
     TRY(prepare_onebody(L));
+    TRY(prepare_hs_update(L));
+    if (!L->ev_fork) TRY(Branches::make_branches(L));
     TRY(prepare_122(L, G, &full));
-    TRY(prepare_program(L, L->prog_ladder, G->zero_mask, H->zero_mask));
+    TRY(prepare_program(L, ladder_program(L, G), G->zero_mask, H->zero_mask));
     TRY(prepare_program(L, L->prog_111, G->zero_mask, H->zero_mask));
     TRY(prepare_122(L, G, H));
     if (pandya) TRY(ensure_z(L));
@@ -1211,12 +1312,21 @@ int bch_step_graph(qd_layout* L, qd_op* HS, const qd_op* G, const qd_op* H, qd_o
   QD_CUDA(cudaGraphLaunch(sg.exec, L->stream));
   int* hk = reinterpret_cast<int*>(L->h_red + 16);
   QD_CUDA(cudaMemcpyAsync(hk, bch_counter(L), sizeof(int), cudaMemcpyDeviceToHost, L->stream));
+  L->step_first = sg.first;
+  L->step_per_term = sg.per_term;
+  *launched = true;
+  return QD_OK;
+}
+
+// Wait for a launched step and leave the host-side state of the eager loop:
+// HS and the workspaces hold full operators, the two workspace buffers keep
+// their handles.
+int bch_step_finish(qd_layout* L, qd_op* HS, const qd_op* G, const qd_op* H, qd_op* INT2, qd_op* AD, qd_cc* HCC,
+                    qd_cc* OCC, bool pandya, int* nterms) {
   QD_CUDA(cudaStreamSynchronize(L->stream));
-  const int terms = *hk;
-  L->nlaunch += sg.first + sg.per_term * (terms - 1);
+  const int terms = *reinterpret_cast<int*>(L->h_red + 16);
+  L->nlaunch += L->step_first + L->step_per_term * (terms - 1);
   ++L->graph_replays;
-  // host-side state the eager loop leaves: HS and the workspaces hold full
-  // operators; the two workspace buffers keep their handles
   HS->zero_mask = INT2->zero_mask = AD->zero_mask = conserves(G, H);
   if (pandya) {
     OCC->filled = true;
@@ -1225,7 +1335,6 @@ int bch_step_graph(qd_layout* L, qd_op* HS, const qd_op* G, const qd_op* H, qd_o
     HCC->herm = 1;
   }
   *nterms = terms;
-  *done = true;
   return QD_OK;
 }
 
@@ -1251,8 +1360,11 @@ int qd_bch_expand(qd_op* HS, const qd_op* G, const qd_op* H, qd_op* INT1, qd_op*
   AD->herm = 1;
   bool done = false;
   int count = 0;
-  TRY(bch_step_graph(L, HS, G, H, INT2, AD, w1, w2, HCC, OCC, pandya, &count, &done));
-  if (!done) TRY(bch_eager(L, HS, G, H, INT2, AD, w1, w2, HCC, OCC, pandya, &count));
+  TRY(bch_step_launch(L, HS, G, H, INT2, AD, w1, w2, HCC, OCC, pandya, &done));
+  if (done)
+    TRY(bch_step_finish(L, HS, G, H, INT2, AD, HCC, OCC, pandya, &count));
+  else
+    TRY(bch_eager(L, HS, G, H, INT2, AD, w1, w2, HCC, OCC, pandya, &count));
   if (nterms) *nterms = count;
   return QD_OK;
 }
@@ -1264,13 +1376,18 @@ int bch_eager(qd_layout* L, qd_op* HS, const qd_op* G, const qd_op* H, qd_op* IN
               qd_cc* HCC, qd_cc* OCC, bool pandya, int* nterms) {
   const double conv = (double)1e-5f;  // "conv = 1e-5" is a real(4) literal in the reference
   double* const p0 = INT2->d;
-  TRY(qd_copy_arrays(H, HS));
-  TRY(qd_copy_arrays(H, INT2));
+  const bool direct = reads_h(H, HS, INT2->d, AD->d);
+  if (!direct) {
+    TRY(qd_copy_arrays(H, HS));
+    TRY(qd_copy_arrays(H, INT2));
+  }
+  HS->zero_mask = H->zero_mask;
   int count = 0;
   for (int i = 2; i <= 12; ++i) {
     swap_ops(INT2, AD);  // AD = previous term; INT2 becomes the output buffer
     const double cof = kCof[i - 2];
-    TRY(bch_term_graph(L, G, AD, INT2, HS, w1, w2, HCC, OCC, pandya, i, cof));
+    const bool first = direct && i == 2;
+    TRY(bch_term_graph(L, G, first ? H : AD, INT2, first ? H : HS, HS, w1, w2, HCC, OCC, pandya, i, cof));
     ++count;
     HS->zero_mask &= INT2->zero_mask;
     QD_CUDA(cudaStreamSynchronize(L->stream));
@@ -1444,13 +1561,23 @@ int flow_begin(qd_flow* f, qd_flow_step_info* inf, bool* converged) {
   return QD_OK;
 }
 
-int flow_end(qd_flow* f, int terms, qd_flow_step_info* inf) {
-  f->comms += terms;
+int flow_end_launch(qd_flow* f) {
   swap_ops(f->ETA, f->ETA0);  // ETA0 = ETA: build_white rewrites fph and Vpphh, the rest stays 0
   TRY(white(f->ETA, f->HS));
-  double nrm2, E0;
-  TRY(flow_eta_norm(f, f->ETA, &nrm2));
-  TRY(flow_e0(f, &E0));
+  // |ETA|, MBPT2 (used if the step is accepted) and E0 in one synchronisation
+  qd_layout* L = f->L;
+  TRY(reduce_norm(L, f->ETA->d, f->ETA->exposed ? 0u : f->ETA->zero_mask, red_slot(L, 4)));
+  TRY(reduce_mbpt2(L, f->HS->d, red_slot(L, 5)));
+  QD_CUDA(cudaMemcpyAsync(L->h_red + 4, red_slot(L, 4), 2 * sizeof(double), cudaMemcpyDeviceToHost, L->stream));
+  QD_CUDA(cudaMemcpyAsync(L->h_red + 8, f->HS->d, sizeof(double), cudaMemcpyDeviceToHost, L->stream));
+  return QD_OK;
+}
+
+int flow_end_finish(qd_flow* f, int terms, qd_flow_step_info* inf) {
+  qd_layout* L = f->L;
+  f->comms += terms;
+  QD_CUDA(cudaStreamSynchronize(L->stream));
+  const double nrm2 = L->h_red[4], mb = L->h_red[5], E0 = L->h_red[8];
   CHECK(std::isfinite(E0) && std::isfinite(nrm2), QD_ERR_NAN,
         "qd_flow_step: non-finite energy or generator norm at s = %g", f->s);
   inf->s = f->s;
@@ -1469,8 +1596,6 @@ int flow_end(qd_flow* f, int terms, qd_flow_step_info* inf) {
     f->stp = f->stp / 2.0 + (double)1e-3f;
     inf->accepted = 0;
   } else {
-    double mb;
-    TRY(qd_mbpt2(f->HS, &mb));
     f->crit = std::fabs(mb);
     f->E0 = E0;
     f->iteration += 1;
@@ -1493,7 +1618,8 @@ int qd_flow_step(qd_flow* f, qd_flow_step_info* info) {
     int terms = 0;
     TRY(qd_bch_expand(f->HS, f->G, f->HAM, f->INT1, f->INT2, f->AD, f->w1, f->w2, f->HCC, f->OCC, f->flags,
                       &terms));
-    TRY(flow_end(f, terms, &inf));
+    TRY(flow_end_launch(f));
+    TRY(flow_end_finish(f, terms, &inf));
   }
   if (info) *info = inf;
   return QD_OK;
@@ -1556,141 +1682,71 @@ int qd_magnus_flow(const qd_op* HAM, qd_op* HS, unsigned flags, int max_iter, do
 }  // extern "C"
 
 namespace {
-// ---- batched flows: several instances in lockstep, one launch per stage ---
-// One commutator C = [A, B] per item, every item's layout on the same stream:
-// the small stages (E0, 111, 121, 221, Pandya re-coupling) per item, the
-// 122 tiles and the ladder GEMM tasks of all items in one launch each.
-struct CommItem {
-  qd_layout* L;
-  const qd_op *A, *B;
-  qd_op* C;
-  qd_cc *ACC, *BCC;
-};
-
-// Streams of a lockstep batch: each instance's small stages run on its own
-// layout's stream; the merged launches run on `st` after a join (events) and
-// the instances' streams wait for them before going on.
-struct BatchCtx {
-  cudaStream_t st = nullptr;
-  cudaEvent_t ev_st = nullptr;
-  std::map<const qd_layout*, cudaEvent_t> ev;
-};
-
-int join_to(cudaStream_t st, const std::vector<qd_layout*>& Ls, BatchCtx& bc) {
-  for (qd_layout* L : Ls) {
-    cudaEvent_t e = bc.ev[L];
-    QD_CUDA(cudaEventRecord(e, L->stream));
-    QD_CUDA(cudaStreamWaitEvent(st, e, 0));
-  }
-  return QD_OK;
-}
-
-int fork_from(cudaStream_t st, const std::vector<qd_layout*>& Ls, BatchCtx& bc) {
-  QD_CUDA(cudaEventRecord(bc.ev_st, st));
-  for (qd_layout* L : Ls) QD_CUDA(cudaStreamWaitEvent(L->stream, bc.ev_st, 0));
-  return QD_OK;
-}
-
-int commutator_batch(BatchCtx& bc, std::vector<CommItem>& items, bool pandya) {
-  std::vector<Item122> i122;
-  std::vector<GemmItem> gl;
-  std::vector<qd_layout*> Ls;
-  for (CommItem& it : items) {
-    qd_layout* L = it.L;
-    Ls.push_back(L);
-    TRY(build_programs(L));
-    TRY(stage_one_body(L, it.A, it.B, it.C));
-    if (pandya) {
-      TRY(launch_calc_cc(L, it.A, it.ACC->d));
-      it.ACC->filled = true;
-      it.ACC->herm = it.A->herm;
-      TRY(launch_calc_cc(L, it.B, it.BCC->d));
-      it.BCC->filled = true;
-      it.BCC->herm = it.B->herm;
-    }
-    i122.push_back(Item122{L, it.A, it.B, it.C->d});
-    GemmItem g;
-    g.L = L;
-    g.P = &L->prog_ladder;
-    const double* bufs[NBUF] = {it.A->d, it.B->d, nullptr, nullptr, it.C->d, nullptr, nullptr};
-    for (int k = 0; k < NBUF; ++k) g.bufs[k] = bufs[k];
-    g.hv0 = (double)it.A->herm;
-    g.hv1 = (double)it.B->herm;
-    g.maskA = it.A->zero_mask;
-    g.maskB = it.B->zero_mask;
-    gl.push_back(g);
-  }
-  TRY(join_to(bc.st, Ls, bc));
-  TRY(launch_122_batched(bc.st, i122));
-  TRY(run_programs_batched(bc.st, gl));
-  TRY(fork_from(bc.st, Ls, bc));
-  for (CommItem& it : items) {
-    qd_layout* L = it.L;
-    if (pandya && L->zsize > 0) {  // the particle-hole channel, as stage_222 after its ladders
-      TRY(ensure_z(L));
-      const double* zb[7] = {nullptr, nullptr, it.ACC->d, it.BCC->d, nullptr, nullptr, L->d_z};
-      TRY(run_program(L, L->prog_pandya, zb, it.ACC->herm, it.BCC->herm, 0u, 0u));
-      TRY(launch_pandya_tiles(L, L->d_z, it.C->d));
-    }
-    it.C->zero_mask = conserves(it.A, it.B);
-  }
-  return QD_OK;
-}
-
-// BCH_EXPAND of several flows in lockstep: every term is one batched
-// commutator over the instances whose series is still running; the host
-// reads all norms once per term and applies each instance's exit test.
-int bch_batch(BatchCtx& bc, const std::vector<qd_flow*>& fl, std::vector<int>& terms) {
+// ---- batched flows: several instances in lockstep -------------------------
+// Every instance runs on its own layout's stream with the kernels and graphs
+// of a separate flow (a generator-like Omega leaves no work that a launch
+// merged over the instances would share), so that the results are those of
+// separate flows; the host launches a step of all of them before it waits
+// for any, and the instances' kernels fill the chip together.
+//
+// BCH_EXPAND of several flows: a step seen before is one graph launch per
+// flow; the others go term by term together.
+int bch_batch(const std::vector<qd_flow*>& fl, std::vector<int>& terms) {
   const double conv = (double)1e-5f;
-  const bool pandya = fl.empty() ? false : (fl[0]->flags & QD_PANDYA) != 0;
+  std::vector<char> graph(fl.size(), 0), direct(fl.size(), 0);
   std::vector<double*> p0(fl.size());
   std::vector<int> live;
+  auto pandya = [&](const qd_flow* f) { return (f->flags & QD_PANDYA) != 0; };
   for (size_t j = 0; j < fl.size(); ++j) {
     qd_flow* f = fl[j];
+    TRY(build_programs(f->L));
     f->INT2->herm = 1;
     f->AD->herm = 1;
-    TRY(qd_copy_arrays(f->HAM, f->HS));
-    TRY(qd_copy_arrays(f->HAM, f->INT2));
-    p0[j] = f->INT2->d;
     terms[j] = 0;
+    bool launched = false;
+    TRY(bch_step_launch(f->L, f->HS, f->G, f->HAM, f->INT2, f->AD, f->w1, f->w2, f->HCC, f->OCC, pandya(f), &launched));
+    graph[j] = launched;
+    if (launched) continue;
+    direct[j] = reads_h(f->HAM, f->HS, f->INT2->d, f->AD->d);
+    if (!direct[j]) {
+      TRY(qd_copy_arrays(f->HAM, f->HS));
+      TRY(qd_copy_arrays(f->HAM, f->INT2));
+    }
+    f->HS->zero_mask = f->HAM->zero_mask;
+    p0[j] = f->INT2->d;
     live.push_back((int)j);
   }
   for (int i = 2; i <= 12 && !live.empty(); ++i) {
     const double cof = kCof[i - 2];
-    std::vector<CommItem> items;
     for (int j : live) {
       qd_flow* f = fl[j];
       swap_ops(f->INT2, f->AD);
-      items.push_back(CommItem{f->L, f->G, f->AD, f->INT2, f->OCC, f->HCC});
-    }
-    TRY(commutator_batch(bc, items, pandya));
-    for (int j : live) {
-      qd_flow* f = fl[j];
-      qd_layout* L = f->L;
-      TRY(launch_axpy_norms(L, f->HS->d, 1.0, f->INT2->d, cof, f->HS->d, red_slot(L, 1)));
-      QD_CUDA(cudaMemcpyAsync(L->h_red + 1, red_slot(L, 1), 2 * sizeof(double), cudaMemcpyDeviceToHost,
-                              L->stream));
+      const bool first = direct[j] && i == 2;
+      TRY(bch_term(f->L, f->G, first ? f->HAM : f->AD, f->INT2, first ? f->HAM : f->HS, f->HS, f->w1, f->w2, f->HCC,
+                   f->OCC, pandya(f), cof));
       f->HS->zero_mask &= f->INT2->zero_mask;
       ++terms[j];
     }
-    for (int j : live) QD_CUDA(cudaStreamSynchronize(fl[j]->L->stream));
     std::vector<int> next;
     for (int j : live) {
+      QD_CUDA(cudaStreamSynchronize(fl[j]->L->stream));
       const double n1 = fl[j]->L->h_red[1], n2 = fl[j]->L->h_red[2];
       if (!(n2 * cof / n1 < conv)) next.push_back(j);
     }
     live.swap(next);
   }
-  for (size_t j = 0; j < fl.size(); ++j)  // the workspaces keep their buffers
-    if (fl[j]->INT2->d != p0[j]) {
-      swap_ops(fl[j]->INT2, fl[j]->AD);
-    }
+  for (size_t j = 0; j < fl.size(); ++j) {
+    qd_flow* f = fl[j];
+    if (graph[j])
+      TRY(bch_step_finish(f->L, f->HS, f->G, f->HAM, f->INT2, f->AD, f->HCC, f->OCC, pandya(f), &terms[j]));
+    else if (f->INT2->d != p0[j])  // the workspaces keep their buffers
+      swap_ops(f->INT2, f->AD);
+  }
   return QD_OK;
 }
 
-// The lockstep batch: every layout on one stream (restored afterwards); per
-// flow step the instances not yet converged run their step halves and one
-// batched BCH_EXPAND.  An instance that fails or exceeds max_iter leaves the
+// The lockstep batch: per flow step the instances not yet converged run their
+// step halves and one BCH_EXPAND, launched for all before any is waited for.  An instance that fails or exceeds max_iter leaves the
 // batch with its own status.
 int flow_batch_lockstep(int count, const qd_op* const* HAM, qd_op* const* HS, unsigned flags, int max_iter,
                         qd_flow_result* results, int* status, std::vector<std::string>& msg) {
@@ -1698,14 +1754,6 @@ int flow_batch_lockstep(int count, const qd_op* const* HAM, qd_op* const* HS, un
   for (int i = 0; i < count; ++i) {
     Ls[i] = HAM[i]->L;
     TRY(use_device(Ls[i]));
-  }
-  BatchCtx bc;
-  QD_CUDA(cudaStreamCreateWithFlags(&bc.st, cudaStreamNonBlocking));
-  QD_CUDA(cudaEventCreateWithFlags(&bc.ev_st, cudaEventDisableTiming));
-  for (qd_layout* L : Ls) {
-    cudaEvent_t e;
-    QD_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    bc.ev[L] = e;
   }
   std::vector<qd_flow*> fl(count, nullptr);
   std::vector<int> loops(count, 0);
@@ -1739,13 +1787,15 @@ int flow_batch_lockstep(int count, const qd_op* const* HAM, qd_op* const* HS, un
     }
     if (act.empty()) break;
     std::vector<int> terms(act.size(), 0);
-    rc = bch_batch(bc, act, terms);
+    rc = bch_batch(act, terms);
     if (rc) break;
-    for (size_t k = 0; k < act.size(); ++k) {
-      const int i = idx[k];
-      status[i] = flow_end(act[k], terms[k], &inf[i]);
-      if (status[i] != QD_OK) msg[i] = qd::last_error();
-    }
+    for (int half = 0; half < 2; ++half)
+      for (size_t k = 0; k < act.size(); ++k) {
+        const int i = idx[k];
+        if (status[i] != QD_OK) continue;
+        status[i] = half == 0 ? flow_end_launch(act[k]) : flow_end_finish(act[k], terms[k], &inf[i]);
+        if (status[i] != QD_OK) msg[i] = qd::last_error();
+      }
   }
   const std::string batch_err = rc ? qd::last_error() : std::string();
   for (int i = 0; i < count; ++i) {
@@ -1758,10 +1808,6 @@ int flow_batch_lockstep(int count, const qd_op* const* HAM, qd_op* const* HS, un
       msg[i] = batch_err;
     }
   }
-  cudaStreamSynchronize(bc.st);
-  for (auto& kv : bc.ev) cudaEventDestroy(kv.second);
-  cudaEventDestroy(bc.ev_st);
-  cudaStreamDestroy(bc.st);
   return QD_OK;
 }
 }  // namespace

@@ -8,6 +8,11 @@ namespace qd {
 constexpr int RED_BLOCKS = 296;  // 2 x 148 SMs: partial sums of the deterministic reductions
 constexpr int RED_THREADS = 256;
 
+// BCH_EXPAND's truncated coefficients cof(1..11) (magnus_IMSRG.f90:265-267)
+#define QD_BCH_COF                                                                                             \
+  {1.0, 0.5, 0.166666666666666666, 0.04166666666666666, 0.0083333333333333333, .001388888888888, 1.984126984e-4, \
+   2.48015873e-5, 2.755731922e-6, 2.755731922e-7, 2.505210839e-8}
+
 // v_elem (src/ME_general.f90:1557-1680) on a device operator, 0-based states.
 // Energy order equals states order (convertF sets eh(i)=i, ep(a)=n+a).
 __device__ __forceinline__ double dv_elem(const DevLayout& L, const double* __restrict__ op, double herm, int a,

@@ -25,12 +25,6 @@
 #include <mutex>
 #include <vector>
 
-#define TRY_GEMM(x)      \
-  do {                   \
-    int rc_ = (x);       \
-    if (rc_) return rc_; \
-  } while (0)
-
 #include "dev_common.cuh"
 
 namespace qd {
@@ -225,20 +219,8 @@ __device__ __forceinline__ void stash(double* T, const double acc[4][4][2]) {
 __global__ void __launch_bounds__(GEMM_THREADS) k_grouped_gemm(const GTask* __restrict__ tasks,
                                                                const GProb* __restrict__ probs,
                                                                const GSeg* __restrict__ segs, Bufs bufs, double hv0,
-                                                               double hv1, unsigned maskA, unsigned maskB,
-                                                               const int* __restrict__ tinst,
-                                                               const GInst* __restrict__ insts) {
+                                                               double hv1, unsigned maskA, unsigned maskB) {
   extern __shared__ double smem[];
-  if (tinst) {  // a task of several instances' programs: this instance's operands
-    const GInst& I = insts[tinst[blockIdx.x]];
-    probs = I.probs;
-    segs = I.segs;
-    bufs = I.bufs;
-    hv0 = I.hv0;
-    hv1 = I.hv1;
-    maskA = I.maskA;
-    maskB = I.maskB;
-  }
   const GTask t = tasks[blockIdx.x];
   const GProb P = probs[t.prob];
   double* out = const_cast<double*>(bufs.p[P.outbuf]) + P.offC;
@@ -411,21 +393,9 @@ __device__ __forceinline__ void ks_stash(double* T, const double acc[4][2][2]) {
 __global__ void __launch_bounds__(KS_THREADS, 3) k_gemm_kshort(const GTask* __restrict__ tasks,
                                                             const GProb* __restrict__ probs,
                                                             const GSeg* __restrict__ segs, Bufs bufs, double hv0,
-                                                            double hv1, unsigned maskA, unsigned maskB,
-                                                            const int* __restrict__ tinst,
-                                                            const GInst* __restrict__ insts) {
+                                                            double hv1, unsigned maskA, unsigned maskB) {
   extern __shared__ double smem[];
   __shared__ SegList sl;
-  if (tinst) {  // a task of several instances' programs: this instance's operands
-    const GInst& I = insts[tinst[blockIdx.x]];
-    probs = I.probs;
-    segs = I.segs;
-    bufs = I.bufs;
-    hv0 = I.hv0;
-    hv1 = I.hv1;
-    maskA = I.maskA;
-    maskB = I.maskB;
-  }
   const GTask t = tasks[blockIdx.x];
   const GProb P = probs[t.prob];
   double* out = const_cast<double*>(bufs.p[P.outbuf]) + P.offC;
@@ -594,12 +564,13 @@ int build_programs(qd_layout* L) {
   if (L->programs_built) return QD_OK;
   const int n = L->n, mp = L->mp;
   // ---- matrix_mult222 ladders (ACC into C) ----
-  {
-    GemmProgram& P = L->prog_ladder;
+  for (int gen = 0; gen < 2; ++gen) {
+    GemmProgram& P = gen ? L->prog_ladder_gen : L->prog_ladder;
     Builder b(P);
     for (int q = 0; q < L->nblock; ++q) {
       const int nh = L->blk[q].x, nb = L->blk[q].y, np = L->blk[q].z;
       const i64* o = &L->boff[6 * q];
+      if (gen && (nh == 0 || gen_ladder_fused(L, q))) continue;  // no hh pairs: no ladder has a live factor
       const i64 hhhh = o[0], pppp = o[1], pphh = o[2], phph = o[3], ppph = o[4], phhh = o[5];
       if (nh > 0) {  // V = -hB Bpphh^T Apphh - Ahhhh Bhhhh ; C += V + s V^T
         b.prob(nh, nh, hhhh, nh, GM_ACC_PAIR, BO0, -1.0, 1, 1);
@@ -719,7 +690,7 @@ int build_programs(qd_layout* L) {
     }
   }
   // upload
-  for (GemmProgram* P : {&L->prog_ladder, &L->prog_221, &L->prog_111, &L->prog_pandya}) {
+  for (GemmProgram* P : {&L->prog_ladder, &L->prog_ladder_gen, &L->prog_221, &L->prog_111, &L->prog_pandya}) {
     size_t pb = std::max<size_t>(1, P->probs.size()) * sizeof(GProb);
     size_t sb = std::max<size_t>(1, P->segs.size()) * sizeof(GSeg);
     QD_CUDA(cudaMalloc(&P->d_probs, pb));
@@ -871,134 +842,15 @@ int run_program_f64(qd_layout* L, GemmProgram& P, const double* const* bufs, dou
   for (int i = 0; i < NBUF; ++i) b.p[i] = bufs[i];
   if (nt > 0) {
     k_grouped_gemm<<<nt, GEMM_THREADS, GEMM_SMEM, L->stream>>>(d_tasks, P.d_probs, P.d_segs, b, hv0, hv1, maskA,
-                                                                maskB, nullptr, nullptr);
+                                                                maskB);
     ++L->nlaunch;
   }
   if (ns > 0) {
-    k_gemm_kshort<<<ns, KS_THREADS, KS_SMEM, L->stream>>>(d_short, P.d_probs, P.d_segs, b, hv0, hv1, maskA, maskB,
-                                                          nullptr, nullptr);
+    k_gemm_kshort<<<ns, KS_THREADS, KS_SMEM, L->stream>>>(d_short, P.d_probs, P.d_segs, b, hv0, hv1, maskA, maskB);
     ++L->nlaunch;
   }
   QD_CUDA(cudaGetLastError());
   return QD_OK;
-}
-
-// ---- one launch over several instances' programs (batched flows) ---------
-namespace {
-struct MergedGemm {
-  GTask* d_task[2] = {nullptr, nullptr};  // long-K, K-short
-  int* d_tinst[2] = {nullptr, nullptr};
-  int n[2] = {0, 0};
-  GInst* d_inst = nullptr;
-  GInst* h_inst = nullptr;  // pinned staging of the per-call instance table
-  std::vector<const qd_layout*> layouts;
-};
-std::map<std::vector<uintptr_t>, MergedGemm>& merged_gemm() {
-  static std::map<std::vector<uintptr_t>, MergedGemm> m;
-  return m;
-}
-std::mutex g_merged_gemm_mutex;
-
-void free_merged(MergedGemm& m) {
-  for (int w = 0; w < 2; ++w) {
-    if (m.d_task[w]) cudaFree(m.d_task[w]);
-    if (m.d_tinst[w]) cudaFree(m.d_tinst[w]);
-  }
-  if (m.d_inst) cudaFree(m.d_inst);
-  if (m.h_inst) cudaFreeHost(m.h_inst);
-}
-}  // namespace
-
-// Every item's program P on its operands, as one launch per kernel (long-K
-// and K-short tasks of all items interleaved, longest first); the items'
-// layouts share `st`.  The task lists are cached per (layout, program,
-// masks) tuple; the instance table is uploaded per call from pinned memory,
-// which the caller rewrites only after synchronising the stream.
-int run_programs_batched(cudaStream_t st, const std::vector<GemmItem>& items) {
-  if (items.empty()) return QD_OK;
-  std::vector<uintptr_t> key;
-  for (const GemmItem& it : items) {
-    TRY_GEMM(build_programs(it.L));
-    key.push_back((uintptr_t)it.L);
-    key.push_back((uintptr_t)it.P);
-    key.push_back(((uintptr_t)it.maskA << 16) | it.maskB);
-  }
-  MergedGemm* m;
-  {
-    std::lock_guard<std::mutex> lock(g_merged_gemm_mutex);
-    auto f = merged_gemm().find(key);
-    if (f == merged_gemm().end()) {
-      MergedGemm mg;
-      std::vector<std::pair<double, std::pair<GTask, int>>> all[2];
-      for (size_t i = 0; i < items.size(); ++i) {
-        std::vector<std::pair<double, GTask>> v[2];
-        task_vectors(*items[i].P, items[i].maskA, items[i].maskB, v);
-        for (int w = 0; w < 2; ++w)
-          for (auto& x : v[w]) all[w].push_back({x.first, {x.second, (int)i}});
-        mg.layouts.push_back(items[i].L);
-      }
-      for (int w = 0; w < 2; ++w) {
-        std::stable_sort(all[w].begin(), all[w].end(), [](const auto& a, const auto& b) { return a.first > b.first; });
-        std::vector<GTask> ht(all[w].size());
-        std::vector<int> hi(all[w].size());
-        for (size_t k = 0; k < all[w].size(); ++k) {
-          ht[k] = all[w][k].second.first;
-          hi[k] = all[w][k].second.second;
-        }
-        mg.n[w] = (int)ht.size();
-        if (!ht.empty()) {
-          QD_CUDA(cudaMalloc(&mg.d_task[w], ht.size() * sizeof(GTask)));
-          QD_CUDA(cudaMemcpy(mg.d_task[w], ht.data(), ht.size() * sizeof(GTask), cudaMemcpyHostToDevice));
-          QD_CUDA(cudaMalloc(&mg.d_tinst[w], hi.size() * sizeof(int)));
-          QD_CUDA(cudaMemcpy(mg.d_tinst[w], hi.data(), hi.size() * sizeof(int), cudaMemcpyHostToDevice));
-        }
-      }
-      QD_CUDA(cudaMalloc(&mg.d_inst, items.size() * sizeof(GInst)));
-      QD_CUDA(cudaMallocHost(&mg.h_inst, items.size() * sizeof(GInst)));
-      f = merged_gemm().emplace(key, mg).first;
-    }
-    m = &f->second;
-  }
-  for (size_t i = 0; i < items.size(); ++i) {
-    const GemmItem& it = items[i];
-    GInst& g = m->h_inst[i];
-    g.probs = it.P->d_probs;
-    g.segs = it.P->d_segs;
-    for (int b = 0; b < NBUF; ++b) g.bufs.p[b] = it.bufs[b];
-    g.hv0 = it.hv0;
-    g.hv1 = it.hv1;
-    g.maskA = it.maskA;
-    g.maskB = it.maskB;
-  }
-  QD_CUDA(cudaMemcpyAsync(m->d_inst, m->h_inst, items.size() * sizeof(GInst), cudaMemcpyHostToDevice, st));
-  Bufs none;
-  for (int b = 0; b < NBUF; ++b) none.p[b] = nullptr;
-  if (m->n[0] > 0) {
-    k_grouped_gemm<<<m->n[0], GEMM_THREADS, GEMM_SMEM, st>>>(m->d_task[0], nullptr, nullptr, none, 0.0, 0.0, 0u, 0u,
-                                                             m->d_tinst[0], m->d_inst);
-    ++items[0].L->nlaunch;
-  }
-  if (m->n[1] > 0) {
-    k_gemm_kshort<<<m->n[1], KS_THREADS, KS_SMEM, st>>>(m->d_task[1], nullptr, nullptr, none, 0.0, 0.0, 0u, 0u,
-                                                        m->d_tinst[1], m->d_inst);
-    ++items[0].L->nlaunch;
-  }
-  QD_CUDA(cudaGetLastError());
-  return QD_OK;
-}
-
-// Drop every merged task list that involves layout L (called when L goes).
-void drop_merged_gemm(const qd_layout* L) {
-  std::lock_guard<std::mutex> lock(g_merged_gemm_mutex);
-  auto& mm = merged_gemm();
-  for (auto it = mm.begin(); it != mm.end();) {
-    if (std::find(it->second.layouts.begin(), it->second.layouts.end(), L) != it->second.layouts.end()) {
-      free_merged(it->second);
-      it = mm.erase(it);
-    } else {
-      ++it;
-    }
-  }
 }
 
 }  // namespace qd

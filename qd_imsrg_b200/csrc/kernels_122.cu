@@ -164,7 +164,7 @@ constexpr unsigned LEG_SPARSE = 1u << 31;
 // (0,0) (1,0) (1,1) (2,0) (2,1) (2,2) -> 0..5; bit r of an output mask.
 __host__ __device__ __forceinline__ int out_region(int c1, int c2) { return (c1 * (c1 + 1)) / 2 + c2; }
 constexpr unsigned OUT_ALL = 0x3Fu;
-// none: k_122_pppp and k_122_gen write every part for a generator-like A
+// none: k_gen_pppp and k_122_gen write every part for a generator-like A
 constexpr unsigned OUT_NONE = 0u;
 
 // Regions (c1 * 3 + c2) of the staged operand that the legs of a tile read
@@ -198,63 +198,19 @@ __device__ __forceinline__ double leg_sum(const double2* __restrict__ Frow, int 
   return y;
 }
 
-// One instance of a launch that covers several layouts (batched flows): its
-// layout view, plan tables, F table and operands.
-struct Inst122 {
-  DevLayout L;
-  const int2* tiles;
-  const int4* gpd;
-  const int2* gpp;
-  const double2* F;
-  int nfent;
-  const double* A;
-  double hA;
-  unsigned zA;
-  unsigned legA;
-  const double* B;
-  double hB;
-  unsigned zB;
-  unsigned legB;
-  double* C;
-  unsigned outmask;
-};
-
 // Task: {tile, op}; op bit 0: the B term (FA x TB), bit 1: the A term
 // (-FB x TA), bit 2: accumulate into C instead of setting it.  op & 3 == 0
 // writes zeros.  TW = doubles per staged cell: 1 (one operand), 2 (A and B);
 // T122 = threads per CTA (picked per launch bucket by the autotuner below).
-// MULTI: the tasks come from several layouts and each names its instance in
-// tinst (a separate instantiation: the single-layout kernel keeps its
-// arguments in the parameter bank instead of registers).
-template <int TW, int T122, bool MULTI>
+template <int TW, int T122>
 __global__ void __launch_bounds__(T122, 1024 / T122) k_122_tile(DevLayout L, const int2* __restrict__ tasks,
                                                    const int2* __restrict__ tiles, const int4* __restrict__ gpd,
                                                    const int2* __restrict__ gpp,
                                                    const double2* __restrict__ F, int nfent,
                                                    const double* __restrict__ A, double hA, unsigned zA, unsigned legA,
                                                    const double* __restrict__ B, double hB, unsigned zB, unsigned legB,
-                                                   double* __restrict__ C, unsigned outmask,
-                                                   const int* __restrict__ tinst, const Inst122* __restrict__ insts) {
+                                                   double* __restrict__ C, unsigned outmask) {
   extern __shared__ __align__(16) double sm122[];
-  if constexpr (MULTI) {  // a task of several layouts' task lists: this instance's tables and operands
-    const Inst122& I = insts[tinst[blockIdx.x]];
-    L = I.L;
-    tiles = I.tiles;
-    gpd = I.gpd;
-    gpp = I.gpp;
-    F = I.F;
-    nfent = I.nfent;
-    A = I.A;
-    hA = I.hA;
-    zA = I.zA;
-    legA = I.legA;
-    B = I.B;
-    hB = I.hB;
-    zB = I.zB;
-    legB = I.legB;
-    C = I.C;
-    outmask = I.outmask;
-  }
   const int2 task = tasks[blockIdx.x];
   const int2 tl = __ldg(&tiles[task.x]);
   const int op = task.y;
@@ -437,13 +393,7 @@ __global__ void __launch_bounds__(T122, 1024 / T122) k_122_tile(DevLayout L, con
 //   ph pair: {column, hole | (particle - n) << 8 | neg << 20, kind}: kind 0 a
 //            B_pppp column with coefficient -s fA(t, h); kind 1 an hh column
 //            (h, t) of B_pphh and A_pphh.
-__host__ __device__ __forceinline__ bool gen_like(unsigned zmask) {
-  return ((zmask | (1u << P_FPH) | (1u << P_PPHH)) & ALL_PARTS) == ALL_PARTS;
-}
-
-constexpr int SP_T = 256, SP_B = 64, SP_LD = SP_B + 1;
-// k_122_pppp tiles: 32 x 32 (two W tiles of 8.4 KB per CTA: seven CTAs per SM)
-constexpr int PP_B = 32, PP_LD = PP_B + 1;
+constexpr int SP_T = 256, SP_B = 64;
 
 __device__ __forceinline__ double sp_coef(const DevLayout& L, const double* __restrict__ f, int code) {
   const double v = __ldg(&f[L.o_fph + ((code >> 8) & 0xFFF) + (i64)(code & 0xFF) * L.mp]);
@@ -458,69 +408,321 @@ struct StagedTerm {
 };
 constexpr int MULT_MASK = 0x3FFFFFFF;
 
-// One task = the tile pair (I, J), (J, I) of a block's C_pppp (32 x 32 each).
-// The W terms of the tile's columns (J, then I) are staged in shared memory
-// first, with their coefficients resolved; each W element then reads only
-// its B_ppph entries.
-__global__ void __launch_bounds__(SP_T) k_122_pppp(DevLayout L, const int4* __restrict__ tasks,
-                                                  const int* __restrict__ ppbase, const int* __restrict__ ppstart,
-                                                  const int2* __restrict__ ppterm, const double* __restrict__ A,
-                                                  double hA, const double* __restrict__ B, double hB, unsigned zB,
-                                                  double* __restrict__ C) {
-  extern __shared__ __align__(16) double spw[];  // W1[c][r] = W(I0 + r, J0 + c), W2[c][r] = W(J0 + r, I0 + c), terms
-  __shared__ int sst[2][PP_B + 1];               // per pass: each column's first staged term
-  const int4 t = tasks[blockIdx.x];
-  const int q = t.x, I0 = t.y * PP_B, J0 = t.z * PP_B;
-  const int4 bd = __ldg(&L.blk[q]);
-  const int np = bd.z;
-  const i64* boff = L.boff + 6 * q;
-  const bool live = !((zB >> P_PPPH) & 1u);
-  const double* X = B + __ldg(boff + 4);  // B_ppph, np x nph
-  const int pb = __ldg(&ppbase[q]);
-  const int tid = threadIdx.x, r = tid & (PP_B - 1), cg = tid >> 5;
-  const bool diag = t.y == t.z;
-  const int npass = diag ? 1 : 2;
-  StagedTerm* T = reinterpret_cast<StagedTerm*>(spw + 2 * PP_B * PP_LD);
-  int base = 0;
-  for (int pass = 0; pass < npass; ++pass) {
-    const int C0 = pass == 0 ? J0 : I0, nc = live ? min(PP_B, np - C0) : 0;
-    const int e0 = __ldg(&ppstart[pb + C0]);
-    for (int i = tid; i <= PP_B; i += SP_T) sst[pass][i] = base + (i <= nc ? __ldg(&ppstart[pb + C0 + i]) : __ldg(&ppstart[pb + C0 + nc])) - e0;
-    const int ne = nc > 0 ? __ldg(&ppstart[pb + C0 + nc]) - e0 : 0;
-    for (int i = tid; i < ne; i += SP_T) {
-      const int2 tm = __ldg(&ppterm[e0 + i]);
-      T[base + i] = StagedTerm{sp_coef(L, A, tm.y), tm.x * np, 0};
-    }
-    base += ne;
+// C_pppp of a block for a generator-like A, and with it the pppp ladder of
+// commutator_222 (matrix_mult222, src/commutators.f90:1010-1032), which for
+// such an A is the rank-n_h update D = -hB A_pphh B_pphh^T, C += D + s D^T,
+// s = -hA hB.  One task = the 64 x 64 tile pair (I, J), (J, I):
+//   C(I,J)[r,c] = hB W(J,I)[c,r] - hA W(I,J)[r,c]
+//                 - hB sum_k (A_I[r,k] B_J[c,k] + s A_J[c,k] B_I[r,k]),
+// and C(J,I) = s C(I,J)^T (both terms change by that sign).
+//   phase 0  the W terms of the columns of J and I (coefficients resolved)
+//            and the n_h-column panels of A_pphh, B_pphh go to shared memory
+//   phase 1  the ladder's two products on the FP64 tensor pipe; the tile then
+//            takes the panels' place in shared memory
+//   phase 2  hB W(J,I)^T is added, lanes along W's rows
+//   phase 3  W(I,J) in registers, lanes along its rows; C(I,J) is written and
+//            s C(I,J) stored in the tile
+//   phase 4  C(J,I) is written from there
+// Bound: writing C once (437 MB at N=20, R=20).  The tile is 64 x 64 because
+// a CTA's chain of dependent table reads (~4 us) is the same for any size:
+// the 32 x 32 tiles used before paid it four times as often, and the ladder
+// as a separate read-modify-write of C_pppp moved its half that has hh pairs
+// twice more.  Times of both forms stand at launch_122_gen.
+constexpr int GP_B = 64, GP_LD = GP_B + 1, GP_T = 256, GP_KMAX = 16;
+
+// A warp takes one column at a time, its lanes the rows l and l + 32: a staged
+// term is read from shared memory once for 64 rows.  Four of the warp's
+// columns (c = wid + 8 (j + jj)): sums over their terms of coef * X[row + off].
+// Neighbouring columns are pairs (a, b), (a, b') with b, b' of one group, so
+// they mostly have the same number of terms (0 to 4).
+__device__ __forceinline__ void gp_cols(const StagedTerm* T, const int* st, const double* __restrict__ X, bool ok0,
+                                        bool ok1, int wid, int j, double w[4][2]) {
+  int s[4], n[4], most = 0;
+#pragma unroll
+  for (int jj = 0; jj < 4; ++jj) {
+    const int c = wid + 8 * (j + jj);
+    s[jj] = st[c];
+    n[jj] = st[c + 1] - s[jj];
+    most = max(most, n[jj]);
+    w[jj][0] = w[jj][1] = 0.0;
   }
-  __syncthreads();
-  for (int pass = 0; pass < npass; ++pass) {
-    const int R0 = pass == 0 ? I0 : J0;
-    double* W = spw + pass * PP_B * PP_LD;
-    const int row = R0 + r;
-    for (int cc = cg; cc < PP_B; cc += SP_T / PP_B) {
-      double w = 0.0;
-      if (row < np)
-        for (int e = sst[pass][cc]; e < sst[pass][cc + 1]; ++e) w += T[e].c * X[row + (i64)T[e].off];
-      W[cc * PP_LD + r] = w;
-    }
-  }
-  __syncthreads();
-  const double* W1 = spw;
-  const double* W2 = diag ? spw : spw + PP_B * PP_LD;
-  double* out = C + __ldg(boff + 1);
-  for (int idx = tid; idx < PP_B * PP_B; idx += SP_T) {
-    const int rr = idx & (PP_B - 1), c = idx >> 5;
-    if (I0 + rr < np && J0 + c < np)  // C(I0 + rr, J0 + c) = hB W(J0 + c, I0 + rr) - hA W(I0 + rr, J0 + c)
-      out[(I0 + rr) + (i64)(J0 + c) * np] = hB * W2[rr * PP_LD + c] - hA * W1[c * PP_LD + rr];
-  }
-  if (diag) return;
-  for (int idx = tid; idx < PP_B * PP_B; idx += SP_T) {
-    const int rr = idx & (PP_B - 1), c = idx >> 5;
-    if (J0 + rr < np && I0 + c < np)  // C(J0 + rr, I0 + c) = hB W(I0 + c, J0 + rr) - hA W(J0 + rr, I0 + c)
-      out[(J0 + rr) + (i64)(I0 + c) * np] = hB * W1[rr * PP_LD + c] - hA * W2[c * PP_LD + rr];
+  for (int i = 0; i < most; ++i) {
+#pragma unroll
+    for (int jj = 0; jj < 4; ++jj)
+      if (i < n[jj]) {
+        const StagedTerm t = T[s[jj] + i];
+        const double* p = X + t.off;
+        if (ok0) w[jj][0] += t.c * __ldg(p);
+        if (ok1) w[jj][1] += t.c * __ldg(p + 32);
+      }
   }
 }
+
+__constant__ double c_gp_cof[11] = QD_BCH_COF;
+
+// Panels are [k][64] with the column swizzled by k, so that a DMMA fragment
+// (4 k x 8 columns) touches every bank once.
+__device__ __forceinline__ int gp_pos(int k, int m) { return k * GP_B + (m ^ ((k & 3) << 2)); }
+
+__device__ __forceinline__ void gp_dmma(double& d0, double& d1, double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+               : "+d"(d0), "+d"(d1)
+               : "d"(a), "d"(b));
+}
+
+template <bool UPD>
+__global__ void __launch_bounds__(GP_T, UPD ? 3 : 4) k_gen_pppp(DevLayout L, const int4* __restrict__ tasks,
+                                                     const int* __restrict__ ppbase, const int* __restrict__ ppstart,
+                                                     const int2* __restrict__ ppterm, const double* __restrict__ A,
+                                                     double hA, const double* __restrict__ B, double hB, unsigned zB,
+                                                     int ladder, double* __restrict__ C, HsUpdate U) {
+  extern __shared__ __align__(16) double gsm[];  // tile [64][65], before it the panels A_I, s B_I, A_J, B_J | terms
+  __shared__ int sst[2][GP_B + 1];               // each column's first staged term, of J and of I
+  const int4 t = tasks[blockIdx.x];
+  const int q = t.x, I0 = t.y * GP_B, J0 = t.z * GP_B;
+  const int4 bd = __ldg(&L.blk[q]);
+  const int np = bd.z, nI = min(GP_B, np - I0), nJ = min(GP_B, np - J0);
+  const i64* boff = L.boff + 6 * q;
+  const bool diag = t.y == t.z;
+  const int K = ladder && bd.x <= GP_KMAX ? bd.x : 0;  // as gen_ladder_fused
+  double* Tt = gsm;
+  StagedTerm* T = reinterpret_cast<StagedTerm*>(gsm + GP_B * GP_LD);
+  const int tid = threadIdx.x, r = tid & (GP_B - 1), cq = tid >> 6;
+  const bool live = !((zB >> P_PPPH) & 1u);
+  const int pb = __ldg(&ppbase[q]);
+  const int j0 = __ldg(&ppstart[pb + J0]), jn = live ? __ldg(&ppstart[pb + J0 + nJ]) - j0 : 0;
+  const int i0 = __ldg(&ppstart[pb + I0]), in = live ? __ldg(&ppstart[pb + I0 + nI]) - i0 : 0;
+  double* out = C + __ldg(boff + 1);
+  // UPD: HS += cof C and the sums of squares of both
+  const double* hs = UPD ? U.src + __ldg(boff + 1) : nullptr;
+  const i64 hsd = UPD ? U.HS - U.src : 0;  // from an entry read to the entry written
+  double an = 0.0, bn = 0.0;
+  auto sums = [&]() {  // the CTA's two sums, in a fixed order
+    if (!UPD) return;
+    __shared__ double red[GP_T / 32];
+    const double a = block_sum<GP_T>(an, red), b = block_sum<GP_T>(bn, red);
+    if (threadIdx.x == 0) {
+      U.partial[2 * blockIdx.x] = a;
+      U.partial[2 * blockIdx.x + 1] = b;
+    }
+  };
+  if (jn == 0 && in == 0 && K == 0) {  // nothing reaches the tile pair: C = 0, HS = src
+    for (int side = 0; side < (diag ? 1 : 2); ++side) {
+      const int R0 = side ? J0 : I0, C0 = side ? I0 : J0, nr = side ? nJ : nI, nc = side ? nI : nJ;
+      if (r < nr)
+#pragma unroll 4
+        for (int c = cq; c < nc; c += 4) {
+          const i64 e = (R0 + r) + (i64)(C0 + c) * np;
+          out[e] = 0.0;
+          if (UPD) {
+            const double x = hs[e];
+            an += x * x;
+            if (hsd) U.HS[__ldg(boff + 1) + e] = x;
+          }
+        }
+    }
+    sums();
+    return;
+  }
+  double cof = 0.0;
+  if (UPD) {
+    cof = U.kidx ? c_gp_cof[*U.kidx] : U.cof;
+    // HS of both tiles on its way to L2 while the tables are read: a column's
+    // 64 rows are 512 bytes, five sectors' starts 128 bytes apart
+    for (int i = tid; i < 5 * (nJ + (diag ? 0 : nI)); i += GP_T) {
+      const int c = i / 5, s = i - 5 * c, side = c >= nJ;
+      const int R0 = side ? J0 : I0, nr = side ? nJ : nI, col = side ? I0 + c - nJ : J0 + c;
+      const double* p = hs + R0 + min(16 * s, nr - 1) + (i64)col * np;
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+    }
+  }
+  const double sg = -hA * hB;
+  const int ib = diag ? 0 : jn;  // first staged term of I's columns
+  for (int i = tid; i <= GP_B; i += GP_T) {
+    sst[0][i] = live ? __ldg(&ppstart[pb + J0 + min(i, nJ)]) - j0 : 0;
+    sst[1][i] = ib + (live ? __ldg(&ppstart[pb + I0 + min(i, nI)]) - i0 : 0);
+  }
+  const int K4 = (K + 3) & ~3;
+  double *PAI = gsm, *PBI = PAI + GP_KMAX * GP_B, *PAJ = PBI + GP_KMAX * GP_B, *PBJ = PAJ + GP_KMAX * GP_B;
+  if (K > 0) {
+    const double* pA = A + __ldg(boff + 2);
+    const double* pB = B + __ldg(boff + 2);
+    for (int k = cq; k < K4; k += 4) {
+      const i64 o = (i64)k * np;
+      const bool oi = k < K && r < nI, oj = k < K && r < nJ;
+      const double ai = oi ? __ldg(pA + I0 + r + o) : 0.0, bi = oi ? __ldg(pB + I0 + r + o) : 0.0;
+      const double aj = oj ? __ldg(pA + J0 + r + o) : 0.0, bj = oj ? __ldg(pB + J0 + r + o) : 0.0;
+      const int p = gp_pos(k, r);
+      PAI[p] = ai;
+      PBI[p] = sg * bi;
+      PAJ[p] = aj;
+      PBJ[p] = bj;
+    }
+  }
+  for (int i = tid; i < jn; i += GP_T) {
+    const int2 tm = __ldg(&ppterm[j0 + i]);
+    T[i] = StagedTerm{sp_coef(L, A, tm.y), tm.x * np, 0};
+  }
+  if (!diag)
+    for (int i = tid; i < in; i += GP_T) {
+      const int2 tm = __ldg(&ppterm[i0 + i]);
+      T[ib + i] = StagedTerm{sp_coef(L, A, tm.y), tm.x * np, 0};
+    }
+  __syncthreads();
+  if (K > 0) {
+    const int lane = tid & 31, wm = (tid >> 5) & 1, wn = tid >> 6;  // warp tile 32 x 16
+    double acc[4][2][2];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 2; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+    for (int kk = 0; kk < K4; kk += 4) {
+      const int kr = kk + (lane & 3);
+#pragma unroll
+      for (int side = 0; side < 2; ++side) {  // A_I B_J^T, then (s B_I) A_J^T
+        const double *pa = side ? PBI : PAI, *pb2 = side ? PAJ : PBJ;
+        double af[4], bf[2];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) af[i] = pa[gp_pos(kr, wm * 32 + i * 8 + (lane >> 2))];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) bf[j] = pb2[gp_pos(kr, wn * 16 + j * 8 + (lane >> 2))];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 2; ++j) gp_dmma(acc[i][j][0], acc[i][j][1], af[i], bf[j]);
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        double* p = Tt + (wm * 32 + i * 8 + (lane >> 2)) * GP_LD + wn * 16 + j * 8 + 2 * (lane & 3);
+        p[0] = -hB * acc[i][j][0];
+        p[1] = -hB * acc[i][j][1];
+      }
+    if (in > 0) __syncthreads();
+  }
+  const double* X = B + __ldg(boff + 4);  // B_ppph, np x nph
+  const int l = tid & 31, wid = tid >> 5;
+  if (in > 0) {
+#pragma unroll 1
+    for (int j = 0; j < GP_B / 8; j += 4) {
+      double w[4][2];
+      gp_cols(T, sst[1], X + J0 + l, l < nJ, l + 32 < nJ, wid, j, w);
+#pragma unroll
+      for (int jj = 0; jj < 4; ++jj) {
+        double* p = Tt + (wid + 8 * (j + jj)) * GP_LD + l;
+        p[0] = K > 0 ? p[0] + hB * w[jj][0] : hB * w[jj][0];
+        p[32] = K > 0 ? p[32] + hB * w[jj][1] : hB * w[jj][1];
+      }
+    }
+  }
+  __syncthreads();
+  const bool have = in > 0 || K > 0;
+  const i64 step = (i64)8 * np;
+  {
+    double* o = out + (I0 + l) + (i64)(J0 + wid) * np;
+    const double* ho = UPD ? hs + (I0 + l) + (i64)(J0 + wid) * np : nullptr;
+    const bool ok0 = l < nI, ok1 = l + 32 < nI;
+#pragma unroll 1
+    for (int j = 0; j < GP_B / 8; j += 4) {
+      double w[4][2] = {{0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}};
+      double g[4][2];
+      double* hw = UPD ? const_cast<double*>(ho) + hsd : nullptr;
+      if (UPD)
+#pragma unroll
+        for (int jj = 0; jj < 4; ++jj) {  // in flight while W is summed
+          const bool in = wid + 8 * (j + jj) < nJ;
+          g[jj][0] = in && ok0 ? ho[jj * step] : 0.0;
+          g[jj][1] = in && ok1 ? ho[jj * step + 32] : 0.0;
+        }
+      if (jn > 0) gp_cols(T, sst[0], X + I0 + l, ok0, ok1, wid, j, w);
+#pragma unroll
+      for (int jj = 0; jj < 4; ++jj) {
+        const int c = wid + 8 * (j + jj);
+        double *p0 = Tt + l * GP_LD + c, *p1 = p0 + 32 * GP_LD;
+        const double v0 = (have ? *p0 : 0.0) - hA * w[jj][0], v1 = (have ? *p1 : 0.0) - hA * w[jj][1];
+        if (c < nJ) {
+          if (ok0) {
+            o[0] = v0;
+            if (UPD) {
+              hw[jj * step] = __dadd_rn(g[jj][0], __dmul_rn(cof, v0));
+              an += g[jj][0] * g[jj][0];
+              bn += v0 * v0;
+            }
+          }
+          if (ok1) {
+            o[32] = v1;
+            if (UPD) {
+              hw[jj * step + 32] = __dadd_rn(g[jj][1], __dmul_rn(cof, v1));
+              an += g[jj][1] * g[jj][1];
+              bn += v1 * v1;
+            }
+          }
+        }
+        o += step;
+        *p0 = sg * v0;
+        *p1 = sg * v1;
+      }
+      if (UPD) ho += 4 * step;
+    }
+  }
+  if (!diag) {
+    __syncthreads();
+    const bool ok0 = l < nJ, ok1 = l + 32 < nJ;
+    double* o = out + (J0 + l) + (i64)(I0 + wid) * np;
+    const double* ho = UPD ? hs + (J0 + l) + (i64)(I0 + wid) * np : nullptr;
+#pragma unroll 1
+    for (int j = 0; j < GP_B / 8; j += 4) {
+      double g[4][2];
+      double* hw = UPD ? const_cast<double*>(ho) + hsd : nullptr;
+      if (UPD)
+#pragma unroll
+        for (int jj = 0; jj < 4; ++jj) {
+          const bool in = wid + 8 * (j + jj) < nI;
+          g[jj][0] = in && ok0 ? ho[jj * step] : 0.0;
+          g[jj][1] = in && ok1 ? ho[jj * step + 32] : 0.0;
+        }
+#pragma unroll
+      for (int jj = 0; jj < 4; ++jj) {
+        const int c = wid + 8 * (j + jj);
+        if (c < nI) {
+          const double v0 = Tt[c * GP_LD + l], v1 = Tt[c * GP_LD + l + 32];
+          if (ok0) {
+            o[0] = v0;
+            if (UPD) {
+              hw[jj * step] = __dadd_rn(g[jj][0], __dmul_rn(cof, v0));
+              an += g[jj][0] * g[jj][0];
+              bn += v0 * v0;
+            }
+          }
+          if (ok1) {
+            o[32] = v1;
+            if (UPD) {
+              hw[jj * step + 32] = __dadd_rn(g[jj][1], __dmul_rn(cof, v1));
+              an += g[jj][1] * g[jj][1];
+              bn += v1 * v1;
+            }
+          }
+        }
+        o += step;
+      }
+      if (UPD) ho += 4 * step;
+    }
+  }
+  sums();
+}
+
+// Whether k_gen_pppp takes block q's pppp ladder with it: up to 16 hh pairs
+// fit its panels (N <= 20 has at most 16); blocks with more keep the grouped
+// GEMM, whose read-modify-write of C is then a smaller part of the work.
+bool gen_ladder_fused(const qd_layout* L, int q) { return L->blk[q].x > 0 && L->blk[q].x <= GP_KMAX; }
+
+// one term more than any tile stages: an empty last column reads (and drops) it
+size_t gp_smem(int terms) { return sizeof(double) * GP_B * GP_LD + sizeof(StagedTerm) * (size_t)(terms + 1); }
+size_t gen_smem(int terms) { return sizeof(StagedTerm) * (size_t)(terms + 1); }
+static_assert(4 * GP_KMAX * GP_B <= GP_B * GP_LD, "the panels share the tile's shared memory");
 
 // The other five parts of a block for a generator-like A, one 64 x 64 tile
 // of one part per task {q, part, ti, tj}: every output element (R, c) is
@@ -576,11 +778,115 @@ __device__ __forceinline__ StagedTerm stage_term(const DevLayout& L, const int4&
   return st;
 }
 
+// Sums over a lane's row terms for four columns: coef * M[c * m], two terms
+// at a time (eight loads in flight).
+__device__ __forceinline__ void gen_rows(const StagedTerm* T, int e, int e1, const double* __restrict__ A,
+                                         const double* __restrict__ B, const i64 cj[4], double y[4]) {
+  for (; e + 1 < e1; e += 2) {
+    const StagedTerm ta = T[e], tb = T[e + 1];
+    const i64 ma = ta.m & MULT_MASK, mb = tb.m & MULT_MASK;
+    const double *pa = ((ta.m >> 30) ? B : A) + ta.off, *pb = ((tb.m >> 30) ? B : A) + tb.off;
+    double va[4], vb[4];
+#pragma unroll
+    for (int jj = 0; jj < 4; ++jj) {
+      va[jj] = __ldg(pa + cj[jj] * ma);
+      vb[jj] = __ldg(pb + cj[jj] * mb);
+    }
+#pragma unroll
+    for (int jj = 0; jj < 4; ++jj) {
+      y[jj] += ta.c * va[jj];
+      y[jj] += tb.c * vb[jj];
+    }
+  }
+  if (e < e1) {
+    const StagedTerm tm = T[e];
+    const i64 m = tm.m & MULT_MASK;
+    const double* p = ((tm.m >> 30) ? B : A) + tm.off;
+#pragma unroll
+    for (int jj = 0; jj < 4; ++jj) y[jj] += tm.c * __ldg(p + cj[jj] * m);
+  }
+}
+
+// Columns k, k + 8, k + 16, k + 24 of a tile of n columns, past its end the last one.
+__device__ __forceinline__ void gen_columns(int J0, int k, int n, i64 cj[4]) {
+#pragma unroll
+  for (int jj = 0; jj < 4; ++jj) cj[jj] = J0 + min(k + 8 * jj, n - 1);
+}
+
+// C_phph of the tile pair (I, J), (J, I), I <= J: the column terms of phph are
+// s = -hA hB times the transposed row terms, so C(I,J) = V(I,J) + s V(J,I)^T
+// with V the row terms alone (half the loads, and all along rows: a column
+// term reads B_ppph across its columns), and C(J,I) = s C(I,J)^T.
+__global__ void __launch_bounds__(SP_T) k_gen_phph(DevLayout L, const int4* __restrict__ tasks, GenTables G,
+                                                  const double* __restrict__ A, double hA,
+                                                  const double* __restrict__ B, double hB, double* __restrict__ C) {
+  extern __shared__ __align__(16) double sm[];
+  __shared__ int si[SP_B + 1], sj[SP_B + 1];
+  const int4 t = tasks[blockIdx.x];
+  const int4 bd = __ldg(&L.blk[t.x]);
+  const int q = t.x, n = bd.y, I0 = t.z * SP_B, J0 = t.w * SP_B, nI = min(SP_B, n - I0), nJ = min(SP_B, n - J0);
+  const bool diag = t.z == t.w;
+  constexpr int LD = SP_B + 1;
+  double* Tt = sm;  // V(J,I)^T, then s C(I,J)
+  StagedTerm* T = reinterpret_cast<StagedTerm*>(sm + SP_B * LD);
+  const int* rs = G.rstart + G.rso[3] + __ldg(&G.gbase[L.nblock + q]);
+  const int i0 = __ldg(&rs[I0]), ni = __ldg(&rs[I0 + nI]) - i0;
+  const int j0 = __ldg(&rs[J0]), nj = diag ? 0 : __ldg(&rs[J0 + nJ]) - j0;
+  const int tid = threadIdx.x, l = tid & 31, wid = tid >> 5;
+  for (int i = tid; i <= SP_B; i += SP_T) {
+    si[i] = __ldg(&rs[I0 + min(i, nI)]) - i0;
+    sj[i] = (diag ? 0 : ni) + __ldg(&rs[J0 + min(i, nJ)]) - j0;
+  }
+  for (int i = tid; i < ni; i += SP_T) T[i] = stage_term(L, __ldg(&G.rterm[i0 + i]), q, bd, true, A, hA, B, hB);
+  for (int i = tid; i < nj; i += SP_T) T[ni + i] = stage_term(L, __ldg(&G.rterm[j0 + i]), q, bd, true, A, hA, B, hB);
+  __syncthreads();
+  for (int k = wid; k < nI; k += 32) {  // V(J,I): lanes along the rows of J
+    i64 cj[4];
+    gen_columns(I0, k, nI, cj);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int r = l + 32 * h;
+      if (r >= nJ) continue;
+      double y[4] = {0.0, 0.0, 0.0, 0.0};
+      gen_rows(T, sj[r], sj[r + 1], A, B, cj, y);
+#pragma unroll
+      for (int jj = 0; jj < 4; ++jj)
+        if (k + 8 * jj < nI) Tt[(k + 8 * jj) * LD + r] = y[jj];
+    }
+  }
+  __syncthreads();
+  const double sg = -hA * hB;
+  double* out = C + __ldg(L.boff + 6 * q + 3);
+  for (int k = wid; k < nJ; k += 32) {
+    i64 cj[4];
+    gen_columns(J0, k, nJ, cj);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int r = l + 32 * h;
+      if (r >= nI) continue;
+      double y[4] = {0.0, 0.0, 0.0, 0.0};
+      gen_rows(T, si[r], si[r + 1], A, B, cj, y);
+#pragma unroll
+      for (int jj = 0; jj < 4; ++jj) {
+        const int c = k + 8 * jj;
+        if (c >= nJ) continue;
+        const double v = y[jj] + sg * Tt[r * LD + c];
+        out[(I0 + r) + (i64)(J0 + c) * n] = v;
+        if (!diag) Tt[r * LD + c] = sg * v;  // this thread's own element
+      }
+    }
+  }
+  if (diag) return;
+  __syncthreads();
+  for (int c = wid; c < nI; c += 8)
+    for (int r = l; r < nJ; r += 32) out[(J0 + r) + (i64)(I0 + c) * n] = Tt[c * LD + r];
+}
+
 // The tile's column terms, then its row terms, are staged once per CTA in
 // shared memory (dynamic size: the most terms of any tile of the launch).
 __global__ void __launch_bounds__(SP_T) k_122_gen(DevLayout L, const int4* __restrict__ tasks, GenTables G,
                                                  const double* __restrict__ A, double hA,
-                                                 const double* __restrict__ B, double hB,
+                                                 const double* __restrict__ B, double hB, int ladder,
                                                  double* __restrict__ C) {
   extern __shared__ __align__(16) double sgt[];
   StagedTerm* T = reinterpret_cast<StagedTerm*>(sgt);
@@ -604,23 +910,226 @@ __global__ void __launch_bounds__(SP_T) k_122_gen(DevLayout L, const int4* __res
   for (int i = tid; i < nce; i += SP_T) T[i] = stage_term(L, __ldg(&G.cterm[c0 + i]), q, bd, false, A, hA, B, hB);
   for (int i = tid; i < nre; i += SP_T) T[nce + i] = stage_term(L, __ldg(&G.rterm[r0 + i]), q, bd, true, A, hA, B, hB);
   __syncthreads();
-  const int r = tid & (SP_B - 1), cg = tid >> 6;
-  if (r >= nrt) return;  // after the only barrier
-  const int row = I0 + r;
-  const int er0 = srs[r], er1 = srs[r + 1];
-  double* out = C + __ldg(L.boff + 6 * q + slot);
-  for (int k = cg; k < nct; k += SP_T / SP_B) {
-    const int col = J0 + k;
-    double y = 0.0;
-    for (int e = scs[k]; e < scs[k + 1]; ++e) {
-      const StagedTerm s = T[e];
-      y += s.c * ((s.m >> 30) ? B : A)[s.off + (i64)row * (s.m & MULT_MASK)];
+  // a warp takes four columns at a time, its lanes the rows l and l + 32: a
+  // term is read from shared memory once for the loads it feeds, and eight
+  // (column terms) or four (row terms) loads are in flight together
+  const int l = tid & 31, wid = tid >> 5;
+  const bool ok0 = l < nrt, ok1 = l + 32 < nrt;
+  const int row = I0 + l;
+  double* out = C + __ldg(L.boff + 6 * q + slot) + row + (i64)J0 * nrow;
+  // the ppph ladder that a generator-like A leaves: -hB A_pphh B_phhh^T
+  const int K = slot == 4 && ladder && bd.x <= GP_KMAX ? bd.x : 0;
+  const double* LA = A + __ldg(L.boff + 6 * q + 2) + row;
+  const double* LB = B + __ldg(L.boff + 6 * q + 5) + J0;
+  for (int k = wid; k < nct; k += 4 * (SP_T / 32)) {
+    double y[4][2];
+    int s[4], n[4], most = 0;
+#pragma unroll
+    for (int jj = 0; jj < 4; ++jj) {
+      const int c = min(k + 8 * jj, nct);
+      s[jj] = scs[c];
+      n[jj] = scs[min(c + 1, nct)] - s[jj];
+      most = max(most, n[jj]);
+      y[jj][0] = y[jj][1] = 0.0;
     }
-    for (int e = er0; e < er1; ++e) {
-      const StagedTerm s = T[e];
-      y += s.c * ((s.m >> 30) ? B : A)[s.off + (i64)col * (s.m & MULT_MASK)];
+    for (int i = 0; i < most; ++i) {
+#pragma unroll
+      for (int jj = 0; jj < 4; ++jj)
+        if (i < n[jj]) {
+          const StagedTerm tm = T[s[jj] + i];
+          const int m = tm.m & MULT_MASK;
+          const double* p = ((tm.m >> 30) ? B : A) + tm.off + (i64)row * m;
+          if (ok0) y[jj][0] += tm.c * __ldg(p);
+          if (ok1) y[jj][1] += tm.c * __ldg(p + 32 * m);
+        }
     }
-    out[row + (i64)col * nrow] = y;
+    i64 cj[4];
+    gen_columns(J0, k, nct, cj);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      if (!(h ? ok1 : ok0)) continue;
+      double z[4] = {0.0, 0.0, 0.0, 0.0};
+      gen_rows(T, srs[l + 32 * h], srs[l + 32 * h + 1], A, B, cj, z);
+#pragma unroll
+      for (int jj = 0; jj < 4; ++jj) y[jj][h] += z[jj];
+    }
+#pragma unroll 2
+    for (int h = 0; h < K; ++h) {
+      const double a0 = ok0 ? -hB * __ldg(LA + (i64)h * nrow) : 0.0, a1 = ok1 ? -hB * __ldg(LA + (i64)h * nrow + 32) : 0.0;
+#pragma unroll
+      for (int jj = 0; jj < 4; ++jj) {
+        const double b = k + 8 * jj < nct ? __ldg(LB + k + 8 * jj + (i64)h * ncol) : 0.0;
+        y[jj][0] += a0 * b;
+        y[jj][1] += a1 * b;
+      }
+    }
+#pragma unroll
+    for (int jj = 0; jj < 4; ++jj)
+      if (k + 8 * jj < nct) {
+        double* o = out + (i64)(k + 8 * jj) * nrow;
+        if (ok0) o[0] = y[jj][0];
+        if (ok1) o[32] = y[jj][1];
+      }
+  }
+}
+
+// ---- the ladders with a long K that a generator-like A leaves --------------
+// (matrix_mult222, src/commutators.f90:996-1130, blocks with n_h <= 16 hh pairs)
+//   pphh += -B_pppp A_pphh - A_pphh B_hhhh
+//   phhh += -hB B_ppph^T A_pphh
+//   hhhh += V + s V^T, V = -hB B_pphh^T A_pphh, s = -hA hB
+// All multiply by the n_p x n_h panel A_pphh: n_h <= 16 columns, so a 64 x 64
+// tile of the grouped GEMM was three quarters padding.  Bound: reading B_pppp
+// of the blocks with hh pairs once (218 MB at N=20, R=20).  Roles (task.y):
+//   0  64 rows of pphh on the FP64 tensor pipe: a warp multiplies every eighth
+//      group of four columns of B_pppp (a fragment is four runs of eight rows,
+//      straight from global memory, sixteen fragments in flight) with the
+//      panel's fragment; the eight warps' sums are added in warp order
+//   1  16 rows of phhh, 2 all of hhhh: a warp per two rows, lanes along the
+//      contracted index (contiguous), one warp sum per output at the end
+constexpr int GL_T = 256;
+
+// sums of v[16] over a warp: lanes 2 i and 2 i + 1 return that of v[i]
+__device__ __forceinline__ double gl_sum16(double* v, int lane) {
+#pragma unroll
+  for (int s = 0; s < 4; ++s) {
+    const int half = 8 >> s, d = 16 >> s;
+    const bool up = lane & d;
+#pragma unroll
+    for (int i = 0; i < half; ++i) {
+      const double send = up ? v[i] : v[i + half], keep = up ? v[i + half] : v[i];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, d);
+    }
+  }
+  return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
+}
+
+template <int NB>  // groups of eight hh pairs
+__device__ void gl_pphh(int np, int nh, int I0, const double* __restrict__ Bpp, const double* __restrict__ Ap,
+                        const double* __restrict__ Bhh, double* __restrict__ out, double* sm) {
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, lr = lane >> 2, lk = lane & 3;
+  const int nr = min(64, np - I0);
+  double acc[8][NB][2];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int n = 0; n < NB; ++n) acc[i][n][0] = acc[i][n][1] = 0.0;
+  if (Bpp) {
+    int ro[8];  // rows past the block repeat its last one: their sums are not used
+#pragma unroll
+    for (int i = 0; i < 8; ++i) ro[i] = I0 + min(8 * i + lr, nr - 1);
+    const double* pb[NB];
+#pragma unroll
+    for (int n = 0; n < NB; ++n) pb[n] = Ap + (i64)min(8 * n + lr, nh - 1) * np;
+    constexpr int U = NB == 1 ? 2 : 1;
+    auto step = [&](int k, auto tail) {  // columns k .. k + 3 and, U = 2, k + 32 .. k + 35
+      double a[U][8], b[U][NB];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int kk = k + 32 * u + lk;
+        const bool in = !decltype(tail)::value || kk < np;
+        const double* p = Bpp + (i64)kk * np;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) a[u][i] = in ? __ldg(p + ro[i]) : 0.0;
+#pragma unroll
+        for (int n = 0; n < NB; ++n) b[u][n] = in && 8 * n + lr < nh ? __ldg(pb[n] + kk) : 0.0;
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+          for (int n = 0; n < NB; ++n) gp_dmma(acc[i][n][0], acc[i][n][1], a[u][i], b[u][n]);
+    };
+    int k = 4 * w;
+#pragma unroll 1
+    for (; k + 32 * (U - 1) + 4 <= np; k += 32 * U) step(k, std::false_type());
+    if (k < np) step(k, std::true_type());
+  }
+  // the eight warps' sums, added in warp order through shared memory
+  for (int turn = 0; turn < GL_T / 32; ++turn) {
+    __syncthreads();
+    if (w == turn) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int n = 0; n < NB; ++n)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            double* p = sm + (8 * n + 2 * lk + e) * 64 + 8 * i + lr;
+            *p = turn == 0 ? acc[i][n][e] : *p + acc[i][n][e];
+          }
+    }
+  }
+  __syncthreads();
+  for (int i = tid; i < 64 * nh; i += GL_T) {
+    const int r = i & 63, h = i >> 6;
+    if (r >= nr) continue;
+    double s = sm[h * 64 + r];
+    if (Bhh)
+      for (int k = 0; k < nh; ++k) s += __ldg(Ap + I0 + r + (i64)k * np) * __ldg(Bhh + k + h * nh);
+    out[(I0 + r) + (i64)h * np] -= s;
+  }
+}
+
+__global__ void __launch_bounds__(GL_T, 2) k_gen_ladder(DevLayout L, const int4* __restrict__ tasks,
+                                                       const double* __restrict__ A, double hA,
+                                                       const double* __restrict__ B, double hB, unsigned zB,
+                                                       double* __restrict__ C) {
+  __shared__ double sm[64 * GP_KMAX];
+  const int4 t = tasks[blockIdx.x];
+  const int q = t.x;
+  const int4 bd = __ldg(&L.blk[q]);
+  const int nh = bd.x, nb = bd.y, np = bd.z;
+  const i64* o = L.boff + 6 * q;
+  const double* Ap = A + __ldg(o + 2);
+  if (t.y == 0) {
+    const double* Bpp = (zB >> P_PPPP) & 1u ? nullptr : B + __ldg(o + 1);
+    const double* Bhh = (zB >> P_HHHH) & 1u ? nullptr : B + __ldg(o + 0);
+    double* out = C + __ldg(o + 2);
+    if (nh <= 8)
+      gl_pphh<1>(np, nh, t.z, Bpp, Ap, Bhh, out, sm);
+    else
+      gl_pphh<2>(np, nh, t.z, Bpp, Ap, Bhh, out, sm);
+    return;
+  }
+  const bool hh = t.y == 2;
+  if ((zB >> (hh ? P_PPHH : P_PPPH)) & 1u) return;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int rows = hh ? nh : nb, r0 = t.z + 2 * w;  // at most 16 hh pairs: one CTA holds all of hhhh
+  const double* x0 = B + __ldg(o + (hh ? 2 : 4)) + (i64)min(r0, rows - 1) * np;
+  const double* x1 = r0 + 1 < rows ? x0 + np : x0;
+  for (int half = 0; half < 2 && 8 * half < nh; ++half) {
+    double v[16];  // rows r0, r0 + 1 times eight columns
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = 0.0;
+    const double* a = Ap + (i64)8 * half * np;
+#pragma unroll 2
+    for (int k = lane; k < np; k += 32) {
+      const double b0 = __ldg(x0 + k), b1 = __ldg(x1 + k);
+#pragma unroll
+      for (int h = 0; h < 8; ++h)
+        if (8 * half + h < nh) {
+          const double c = __ldg(a + k + (i64)h * np);
+          v[h] += b0 * c;
+          v[8 + h] += b1 * c;
+        }
+    }
+    const double s = -hB * gl_sum16(v, lane);
+    const int r = r0 + (lane >> 4), h = 8 * half + ((lane >> 1) & 7);
+    if (!(lane & 1) && r < rows && h < nh) {
+      if (hh)
+        sm[r * 16 + h] = s;
+      else
+        C[__ldg(o + 5) + r + (i64)h * nb] += s;
+    }
+  }
+  if (!hh) return;
+  __syncthreads();
+  const double sg = -hA * hB;
+  for (int i = threadIdx.x; i < nh * nh; i += GL_T) {
+    const int r = i % nh, h = i / nh;
+    C[__ldg(o + 0) + r + (i64)h * nh] += sm[r * 16 + h] + sg * sm[h * 16 + r];
   }
 }
 
@@ -862,7 +1371,6 @@ struct Bucket122 {
 };
 struct TaskSet {
   int2* d_task = nullptr;
-  std::vector<int2> h_task;  // host copy (merged launches of several layouts)
   std::vector<Bucket122> buckets;
   bool tuned = false;
   unsigned outmask = OUT_ALL;  // output regions the tiles write (OUT_NONE: A generator-like)
@@ -886,7 +1394,7 @@ struct Plan122 {
   int ng = 0;
   int* d_ptask = nullptr;
   std::vector<PdBucket> pbuckets;
-  // generator-like A: term tables of k_122_pppp / k_122_gen and their tasks
+  // generator-like A: term tables of k_gen_pppp / k_122_gen and their tasks
   int* d_ppbase = nullptr;   // per block: first pp pair
   int* d_ppstart = nullptr;  // per pp pair: first term (one more entry at the end)
   int2* d_ppterm = nullptr;
@@ -896,9 +1404,13 @@ struct Plan122 {
   int4* d_rterm = nullptr;
   int4* d_cterm = nullptr;
   int gen_rso[6] = {0}, gen_cso[6] = {0};
-  int4* d_sptask = nullptr;  // C_pppp tile pairs, then the k_122_gen tiles
+  int4* d_sptask = nullptr;  // C_pppp tile pairs, then the k_122_gen tiles, then the C_phph tile pairs
+  int4* d_ltask = nullptr;   // k_gen_ladder: {block, role, first row}, longest first
+  int nsp_ladder = 0;
   int nsp_pppp = 0, nsp_gen = 0;
-  int pppp_terms = 0, gen_terms = 0;  // the most terms one task of each kernel stages
+  int pppp_terms = 0;    // the most terms one task of k_gen_pppp stages
+  size_t gen_bytes = 0, phph_bytes = 0;  // the most shared memory a task of k_122_gen, k_gen_phph needs
+  int nsp_phph = 0;
 };
 std::map<const qd_layout*, Plan122>& plans() {
   static std::map<const qd_layout*, Plan122> m;
@@ -1066,7 +1578,7 @@ static int plan_122(qd_layout* L, Plan122** out) {
       (rc = upload_vec(L, th, &p.d_tiles)) ||
       (rc = upload_vec(L, sbase, &p.d_sbase)))
     return rc;
-  // generator-like A: the pp pairs' W terms (k_122_pppp) and the row and
+  // generator-like A: the pp pairs' W terms (k_gen_pppp) and the row and
   // column terms of the other five parts (k_122_gen), per block
   {
     const int n = L->n, mp = L->mp;
@@ -1076,7 +1588,7 @@ static int plan_122(qd_layout* L, Plan122** out) {
     // per slot: its terms and, per pair of its classes (block order), their starts
     std::vector<int> rst[6], cst[6];
     std::vector<int4> rterm_s[6], cterm_s[6];
-    std::vector<int4> ptask, gtask;
+    std::vector<int4> ptask, gtask, htask;
     int cnt[3] = {0, 0, 0};
     enum { NEG = 1, MA = 2, MB = 4, CB = 8 };
     auto fA = [&](int pt, int h) { return ofph + (pt - n) + h * mp; };  // A's or B's fph(p, h)
@@ -1185,14 +1697,7 @@ static int plan_122(qd_layout* L, Plan122** out) {
             T.push_back(int4{idx, fA(pt, t), MA | (sg > 0 ? NEG : 0), src(1, 2, 0)});
             T.push_back(int4{idx, fA(pt, t), MB | CB | (sg < 0 ? NEG : 0), src(0, 2, 0)});
           });
-        } else if (slot == 3) {  // columns ph (k1, k2)
-          const int k1 = php(k).x, k2 = php(k).y;
-          each(k1, false, k2, [&](int t) {
-            if (srt(ipp, t, k2, &idx, &sg)) T.push_back(int4{idx, fA(t, k1), MB | (sg > 0 ? NEG : 0), src(1, 4, 1)});
-          });
-          each(k2, true, k1, [&](int t) {
-            if (srt(ihh, k1, t, &idx, &sg)) T.push_back(int4{idx, fA(k2, t), MA | (sg > 0 ? NEG : 0), src(1, 5, 0)});
-          });
+        } else if (slot == 3) {  // none: k_gen_phph transposes the row terms
         } else {  // columns hh (k1, k2): slots 2, 5, 0
           const int k1 = hhp(k).x, k2 = hhp(k).y;
           for (int side = 0; side < 2; ++side) {
@@ -1228,9 +1733,10 @@ static int plan_122(qd_layout* L, Plan122** out) {
         }
         if (rows_n[slot] > 0 && cols_n[slot] > 0)
           for (int i = 0; i < (rows_n[slot] + SP_B - 1) / SP_B; ++i)
-            for (int j = 0; j < (cols_n[slot] + SP_B - 1) / SP_B; ++j) gtask.push_back(int4{q, slot, i, j});
+            for (int j = slot == 3 ? i : 0; j < (cols_n[slot] + SP_B - 1) / SP_B; ++j)
+              (slot == 3 ? htask : gtask).push_back(int4{q, slot, i, j});
       }
-      const int tr = (np + PP_B - 1) / PP_B;
+      const int tr = (np + GP_B - 1) / GP_B;
       for (int i = 0; i < tr; ++i)
         for (int j = i; j < tr; ++j) ptask.push_back(int4{q, i, j, 0});
     }
@@ -1252,36 +1758,63 @@ static int plan_122(qd_layout* L, Plan122** out) {
     }
     p.nsp_pppp = (int)ptask.size();
     p.nsp_gen = (int)gtask.size();
+    // the parts with many terms per element first (their CTAs run longest),
+    // then ppph, whose many CTAs fill the rest
+    std::stable_sort(gtask.begin(), gtask.end(), [](const int4& x, const int4& y) {
+      const auto rank = [](int slot) { return slot == 5 ? 0 : (slot == 2 ? 1 : (slot == 0 ? 2 : 3)); };
+      return rank(x.y) < rank(y.y);
+    });
     // the most terms one task stages (its shared memory)
     p.pppp_terms = 0;
     for (const int4& tk : ptask) {
       const int q = tk.x, np = L->blk[q].z, pbq = gbase[2 * L->nblock + q];
       int ne = 0;
       for (int pass = 0; pass < (tk.y == tk.z ? 1 : 2); ++pass) {
-        const int c0 = (pass == 0 ? tk.z : tk.y) * PP_B, nc = std::min(PP_B, np - c0);
+        const int c0 = (pass == 0 ? tk.z : tk.y) * GP_B, nc = std::min(GP_B, np - c0);
         ne += ppstart[pbq + c0 + nc] - ppstart[pbq + c0];
       }
       p.pppp_terms = std::max(p.pppp_terms, ne);
     }
-    p.gen_terms = 0;
-    for (const int4& tk : gtask) {
-      const int q = tk.x, slot = tk.y;
-      int cr, cc;
-      part_classes(P_HHHH + slot, cr, cc);
-      const int4 bd = L->blk[q];
-      const int nr = cr == 0 ? bd.x : (cr == 1 ? bd.y : bd.z), nc = cc == 0 ? bd.x : (cc == 1 ? bd.y : bd.z);
-      const int i0 = tk.z * SP_B, j0 = tk.w * SP_B, nrt = std::min(SP_B, nr - i0), nct = std::min(SP_B, nc - j0);
-      const int* rr = rall.data() + p.gen_rso[slot] + gbase[cr * L->nblock + q] + i0;
-      const int* cs = call.data() + p.gen_cso[slot] + gbase[cc * L->nblock + q] + j0;
-      p.gen_terms = std::max(p.gen_terms, (rr[nrt] - rr[0]) + (cs[nct] - cs[0]));
-    }
-    if (2 * PP_B * PP_LD * sizeof(double) + (size_t)p.pppp_terms * sizeof(StagedTerm) > SMEM_MAX_122 - 1024 ||
-        (size_t)p.gen_terms * sizeof(StagedTerm) > SMEM_MAX_122 - 1024) {
-      set_error("commutator_122: %d / %d terms of one tile exceed shared memory", p.pppp_terms, p.gen_terms);
+    p.gen_bytes = p.phph_bytes = 0;
+    for (const std::vector<int4>* v : {&gtask, &htask})
+      for (const int4& tk : *v) {
+        const int q = tk.x, slot = tk.y;
+        int cr, cc;
+        part_classes(P_HHHH + slot, cr, cc);
+        const int4 bd = L->blk[q];
+        const int nr = cr == 0 ? bd.x : (cr == 1 ? bd.y : bd.z), nc = cc == 0 ? bd.x : (cc == 1 ? bd.y : bd.z);
+        const int i0 = tk.z * SP_B, j0 = tk.w * SP_B, nrt = std::min(SP_B, nr - i0), nct = std::min(SP_B, nc - j0);
+        const int* rr = rall.data() + p.gen_rso[slot] + gbase[cr * L->nblock + q];
+        const int* cs = call.data() + p.gen_cso[slot] + gbase[cc * L->nblock + q];
+        const int rows = rr[i0 + nrt] - rr[i0];
+        if (slot == 3)  // the pair's row terms beside its transposed tile
+          p.phph_bytes = std::max(p.phph_bytes, sizeof(double) * SP_B * (SP_B + 1) +
+                                                    gen_smem(rows + (i0 == j0 ? 0 : rr[j0 + nct] - rr[j0])));
+        else
+          p.gen_bytes = std::max(p.gen_bytes, gen_smem(rows + cs[j0 + nct] - cs[j0]));
+      }
+    if (gp_smem(p.pppp_terms) > SMEM_MAX_122 - 1024 ||
+        std::max(p.gen_bytes, p.phph_bytes) > SMEM_MAX_122 - 1024) {
+      set_error("commutator_122: the terms of one tile exceed shared memory");
       return QD_ERR_ARG;
     }
     std::vector<int4> all = ptask;
     all.insert(all.end(), gtask.begin(), gtask.end());
+    all.insert(all.end(), htask.begin(), htask.end());
+    p.nsp_phph = (int)htask.size();
+    std::vector<std::pair<i64, int4>> lt;
+    for (int q = 0; q < L->nblock; ++q) {
+      if (!gen_ladder_fused(L, q) || L->blk[q].z == 0) continue;
+      const int4 bd = L->blk[q];
+      for (int r = 0; r < bd.z; r += 64) lt.push_back({(i64)bd.z * 64, int4{q, 0, r, 0}});
+      for (int r = 0; r < bd.y; r += 16) lt.push_back({(i64)bd.z * 16, int4{q, 1, r, 0}});
+      lt.push_back({(i64)bd.z * 16, int4{q, 2, 0, 0}});
+    }
+    std::stable_sort(lt.begin(), lt.end(), [](const auto& x, const auto& y) { return x.first > y.first; });
+    std::vector<int4> ltask;
+    for (const auto& x : lt) ltask.push_back(x.second);
+    p.nsp_ladder = (int)ltask.size();
+    if ((rc = upload_vec(L, ltask, &p.d_ltask))) return rc;
     std::vector<int> ppbase(L->nblock);
     for (int q = 0; q < L->nblock; ++q) ppbase[q] = gbase[2 * L->nblock + q];
     if ((rc = upload_vec(L, ppbase, &p.d_ppbase)) || (rc = upload_vec(L, ppstart, &p.d_ppstart)) ||
@@ -1346,13 +1879,12 @@ static int plan_122(qd_layout* L, Plan122** out) {
   }
   QD_CUDA(cudaMalloc(&p.d_ftab, sizeof(double2) * 2 * (size_t)std::max(1, p.nfent)));
   L->ws_bytes += (i64)sizeof(double2) * 2 * p.nfent;
-  for (const void* fn : {(const void*)k_122_tile<1, 64, false>, (const void*)k_122_tile<2, 64, false>,
-                         (const void*)k_122_tile<1, 128, false>, (const void*)k_122_tile<2, 128, false>,
-                         (const void*)k_122_tile<1, 256, false>, (const void*)k_122_tile<2, 256, false>,
-                         (const void*)k_122_tile<1, 256, true>, (const void*)k_122_tile<2, 256, true>,
+  for (const void* fn : {(const void*)k_122_tile<1, 64>, (const void*)k_122_tile<2, 64>,
+                         (const void*)k_122_tile<1, 128>, (const void*)k_122_tile<2, 128>,
+                         (const void*)k_122_tile<1, 256>, (const void*)k_122_tile<2, 256>,
                          (const void*)k_pandya_tile<PD_ALL4>, (const void*)k_pandya_tile<PD_PAIRS>,
                          (const void*)k_pandya_tile<PD_SINGLE>, (const void*)k_pandya_tile<PD_DIRECT>,
-                         (const void*)k_122_pppp, (const void*)k_122_gen}) {
+                         (const void*)k_gen_pppp<false>, (const void*)k_gen_pppp<true>, (const void*)k_122_gen, (const void*)k_gen_phph}) {
     cudaFuncAttributes fa;
     QD_CUDA(cudaFuncGetAttributes(&fa, fn));
     QD_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1414,7 +1946,6 @@ static int build_variant(qd_layout* L, const Plan122* p, std::vector<std::pair<s
     });
   int rc = upload_vec(L, all, &ts.d_task);
   if (rc) return rc;
-  ts.h_task = all;
   return QD_OK;
 }
 
@@ -1439,7 +1970,7 @@ static int task_set(qd_layout* L, Plan122* p, unsigned zA, unsigned zB, TaskSet*
   const unsigned outmask = gen_like(zA) ? OUT_NONE : OUT_ALL;
   for (size_t i = 0; i < p->tiles.size(); ++i) {
     const TileInfo& t = p->tiles[i];
-    if (!(t.outs & outmask)) continue;  // every output of the tile comes from k_122_pppp / k_122_gen
+    if (!(t.outs & outmask)) continue;  // every output of the tile comes from k_gen_pppp / k_122_gen
     const bool nb = !fa0 && (t.parts & ~zb2) && !(spa && t.holefree);
     const bool na = !fb0 && (t.parts & ~za2) && !(spb && t.holefree);
     const int op = (nb ? 1 : 0) | (na ? 2 : 0);
@@ -1472,7 +2003,7 @@ void drop_122_plan(const qd_layout* L) {
   if (it == plans().end()) return;
   Plan122& p = it->second;
   for (void* ptr : {(void*)p.d_gpd, (void*)p.d_gpp, (void*)p.d_tiles, (void*)p.d_sbase,
-                    (void*)p.d_ftab, (void*)p.d_gpg, (void*)p.d_zrow, (void*)p.d_ptask, (void*)p.d_ppbase,
+                    (void*)p.d_ftab, (void*)p.d_ltask, (void*)p.d_gpg, (void*)p.d_zrow, (void*)p.d_ptask, (void*)p.d_ppbase,
                     (void*)p.d_ppstart, (void*)p.d_ppterm, (void*)p.d_gbase, (void*)p.d_rstart,
                     (void*)p.d_cstart, (void*)p.d_rterm, (void*)p.d_cterm, (void*)p.d_sptask})
     if (ptr) cudaFree(ptr);
@@ -1514,11 +2045,10 @@ static int launch_bucket(qd_layout* L, const Plan122* p, const TaskSet* ts, cons
   // the B term (FA x TB) and the A term (-FB x TA)
   const unsigned legB = leg_masks(spA, B->zero_mask), legA = leg_masks(spB, A->zero_mask);
 #define QD_122_LAUNCH(TW, NT)                                                                                   \
-  k_122_tile<TW, NT, false><<<b.count, NT, b.smem, L->stream>>>(L->dev, ts->d_task + b.first, p->d_tiles, p->d_gpd,   \
+  k_122_tile<TW, NT><<<b.count, NT, b.smem, L->stream>>>(L->dev, ts->d_task + b.first, p->d_tiles, p->d_gpd,   \
                                                          p->d_gpp, p->d_ftab, p->nfent, A->d,                   \
                                                          (double)A->herm, A->zero_mask, legA, B->d,             \
-                                                         (double)B->herm, B->zero_mask, legB, C, ts->outmask,   \
-                                                         nullptr, nullptr)
+                                                         (double)B->herm, B->zero_mask, legB, C, ts->outmask)
   if (b.tw == 2) {
     if (threads == 64) QD_122_LAUNCH(2, 64); else if (threads == 128) QD_122_LAUNCH(2, 128); else QD_122_LAUNCH(2, 256);
   } else {
@@ -1604,7 +2134,6 @@ static int tune_122(qd_layout* L, Plan122* p, TaskSet* ts, const qd_op* A, const
   for (TaskSet& t : others) {
     if (t.d_task) cudaFree(t.d_task);
     t.d_task = nullptr;
-    t.h_task.clear();
     ts->alts.push_back(t);
   }
   cudaEventDestroy(e0);
@@ -1671,36 +2200,63 @@ int prepare_122(qd_layout* L, const qd_op* A, const qd_op* B) {
   return QD_OK;
 }
 
-// Every two-body part of C for a generator-like A (k_122_pppp, k_122_gen)
-// on stream st.
-static int launch_122_gen(qd_layout* L, const Plan122* p, const qd_op* A, const qd_op* B, double* C,
-                          cudaStream_t st) {
-  if (p->nsp_pppp > 0) {
-    k_122_pppp<<<p->nsp_pppp, SP_T, 2 * PP_B * PP_LD * sizeof(double) + p->pppp_terms * sizeof(StagedTerm), st>>>(
-        L->dev, p->d_sptask, p->d_ppbase, p->d_ppstart, p->d_ppterm, A->d, (double)A->herm, B->d, (double)B->herm,
-        B->zero_mask, C);
-    ++L->nlaunch;
+// Every two-body part of C for a generator-like A, and with `ladder` the
+// ladders of the blocks that gen_ladder_fused names: C_pppp on stream st, the
+// other parts (which no kernel of C_pppp touches) on stream st2.
+static int launch_122_gen(qd_layout* L, const Plan122* p, const qd_op* A, const qd_op* B, double* C, bool ladder,
+                          cudaStream_t st, cudaStream_t st2, const HsUpdate* upd) {
+  const bool lad = ladder && !((A->zero_mask >> P_PPHH) & 1u);  // every ladder left has the factor A_pphh
+  const double hA = (double)A->herm, hB = (double)B->herm;
+  GenTables G;
+  G.gbase = p->d_gbase;
+  G.rstart = p->d_rstart;
+  G.cstart = p->d_cstart;
+  G.rterm = p->d_rterm;
+  G.cterm = p->d_cterm;
+  for (int k = 0; k < 6; ++k) {
+    G.rso[k] = p->gen_rso[k];
+    G.cso[k] = p->gen_cso[k];
   }
   if (p->nsp_gen > 0) {
-    GenTables G;
-    G.gbase = p->d_gbase;
-    G.rstart = p->d_rstart;
-    G.cstart = p->d_cstart;
-    G.rterm = p->d_rterm;
-    G.cterm = p->d_cterm;
-    for (int k = 0; k < 6; ++k) {
-      G.rso[k] = p->gen_rso[k];
-      G.cso[k] = p->gen_cso[k];
-    }
-    k_122_gen<<<p->nsp_gen, SP_T, p->gen_terms * sizeof(StagedTerm), st>>>(
-        L->dev, p->d_sptask + p->nsp_pppp, G, A->d, (double)A->herm, B->d, (double)B->herm, C);
+    k_122_gen<<<p->nsp_gen, SP_T, p->gen_bytes, st2>>>(L->dev, p->d_sptask + p->nsp_pppp, G, A->d, hA, B->d, hB,
+                                                       lad && !((B->zero_mask >> P_PHHH) & 1u), C);
+    ++L->nlaunch;
+  }
+  if (lad && p->nsp_ladder > 0) {
+    k_gen_ladder<<<p->nsp_ladder, GL_T, 0, st2>>>(L->dev, p->d_ltask, A->d, hA, B->d, hB, B->zero_mask, C);
+    ++L->nlaunch;
+  }
+  if (p->nsp_phph > 0) {
+    k_gen_phph<<<p->nsp_phph, SP_T, p->phph_bytes, st2>>>(L->dev, p->d_sptask + p->nsp_pppp + p->nsp_gen, G, A->d, hA,
+                                                          B->d, hB, C);
+    ++L->nlaunch;
+  }
+  if (p->nsp_pppp > 0) {
+    const int plad = lad && !((B->zero_mask >> P_PPHH) & 1u);
+    if (upd)
+      k_gen_pppp<true><<<p->nsp_pppp, GP_T, gp_smem(p->pppp_terms), st>>>(L->dev, p->d_sptask, p->d_ppbase, p->d_ppstart,
+                                                                        p->d_ppterm, A->d, hA, B->d, hB, B->zero_mask,
+                                                                        plad, C, *upd);
+    else
+      k_gen_pppp<false><<<p->nsp_pppp, GP_T, gp_smem(p->pppp_terms), st>>>(
+          L->dev, p->d_sptask, p->d_ppbase, p->d_ppstart, p->d_ppterm, A->d, hA, B->d, hB, B->zero_mask, plad, C,
+          HsUpdate{});
     ++L->nlaunch;
   }
   QD_CUDA(cudaGetLastError());
   return QD_OK;
 }
 
-int launch_122(qd_layout* L, const qd_op* A, const qd_op* B, double* C) {
+int gen_pppp_ctas(qd_layout* L, int* n) {
+  Plan122* p;
+  int rc = plan_122(L, &p);
+  if (rc) return rc;
+  *n = p->nsp_pppp;
+  return QD_OK;
+}
+
+int launch_122(qd_layout* L, const qd_op* A, const qd_op* B, double* C, bool ladder, cudaStream_t st2,
+               const HsUpdate* upd) {
   Plan122* p;
   int rc = plan_122(L, &p);
   if (rc) return rc;
@@ -1708,7 +2264,7 @@ int launch_122(qd_layout* L, const qd_op* A, const qd_op* B, double* C) {
   TaskSet* ts;
   if ((rc = task_set(L, p, A->zero_mask, B->zero_mask, &ts))) return rc;
   const int spA = spars(A), spB = spars(B);
-  if (ts->outmask != OUT_ALL) TRY(launch_122_gen(L, p, A, B, C, L->stream));
+  if (ts->outmask != OUT_ALL) TRY(launch_122_gen(L, p, A, B, C, ladder, L->stream, st2 ? st2 : L->stream, upd));
   if (ts->buckets.empty()) return QD_OK;  // no group-pair tiles: their F tables are not needed
   const int nf = L->m * p->gmax;
   k_ftab<<<(nf + 127) / 128, 128, 0, L->stream>>>(L->dev, p->d_sbase, A->d, (double)A->herm, B->d,
@@ -1745,176 +2301,6 @@ int launch_pandya_tiles(qd_layout* L, const double* Z, double* C) {
   }
   QD_CUDA(cudaGetLastError());
   return QD_OK;
-}
-
-// ---- one launch over several layouts' tiles (batched flows) ---------------
-namespace {
-struct Merged122 {
-  int2* d_task = nullptr;
-  int* d_tinst = nullptr;
-  std::vector<Bucket122> buckets;
-  Inst122* d_inst = nullptr;
-  Inst122* h_inst = nullptr;  // pinned staging of the per-call instance table
-  std::vector<const qd_layout*> layouts;
-};
-std::map<std::vector<uintptr_t>, Merged122>& merged122() {
-  static std::map<std::vector<uintptr_t>, Merged122> m;
-  return m;
-}
-std::mutex g_m122_mutex;
-}  // namespace
-
-// commutator_122 of every item in one set of launches: the items' tiles are
-// merged per list (set with one operand, set with both, accumulate) and per
-// shared-memory bucket, largest first, each task carrying its instance; the
-// items' layouts share `st`.  Merged lists are cached per (layout, masks)
-// tuple; the instance table is uploaded per call from pinned memory, which
-// the caller rewrites only after synchronising the stream.
-int launch_122_batched(cudaStream_t st, const std::vector<Item122>& items) {
-  if (items.empty()) return QD_OK;
-  const size_t n = items.size();
-  std::vector<Plan122*> pl(n);
-  std::vector<TaskSet*> tsv(n);
-  std::vector<uintptr_t> key;
-  for (size_t i = 0; i < n; ++i) {
-    qd_layout* L = items[i].L;
-    TRY(plan_122(L, &pl[i]));
-    TRY(task_set(L, pl[i], items[i].A->zero_mask, items[i].B->zero_mask, &tsv[i]));
-    key.push_back((uintptr_t)L);
-    key.push_back(((uintptr_t)items[i].A->zero_mask << 16) | items[i].B->zero_mask);
-  }
-  Merged122* m;
-  {
-    std::lock_guard<std::mutex> lock(g_m122_mutex);
-    auto f = merged122().find(key);
-    if (f == merged122().end()) {
-      Merged122 mg;
-      std::vector<std::pair<size_t, std::pair<int2, int>>> lists[3];
-      for (size_t i = 0; i < n; ++i) {
-        mg.layouts.push_back(items[i].L);
-        for (const Bucket122& b : tsv[i]->buckets)
-          for (int k = b.first; k < b.first + b.count; ++k) {
-            const int2 t = tsv[i]->h_task[k];
-            const TileInfo& ti = pl[i]->tiles[t.x];
-            lists[b.list].push_back({t.y == 0 ? zero_smem(ti) : tile_smem(ti, b.tw), {t, (int)i}});
-          }
-      }
-      std::vector<int2> ht;
-      std::vector<int> hi;
-      const size_t bounds[4] = {24 * 1024, 56 * 1024, 112 * 1024, SMEM_MAX_122};
-      for (int l = 0; l < 3; ++l) {
-        auto& v = lists[l];
-        std::stable_sort(v.begin(), v.end(), [](const auto& x, const auto& y) { return x.first > y.first; });
-        size_t k = 0;
-        while (k < v.size()) {
-          const size_t top = v[k].first;
-          size_t lower = 0;
-          for (size_t bnd : bounds)
-            if (bnd < top) lower = bnd;
-          Bucket122 b;
-          b.tw = l == 1 ? 2 : 1;
-          b.list = l;
-          b.first = (int)ht.size();
-          b.smem = top;
-          while (k < v.size() && v[k].first > lower) {
-            ht.push_back(v[k].second.first);
-            hi.push_back(v[k].second.second);
-            ++k;
-          }
-          b.count = (int)ht.size() - b.first;
-          mg.buckets.push_back(b);
-          {  // column strips together within the bucket (see task_set)
-            std::vector<size_t> ord(b.count);
-            for (int x = 0; x < b.count; ++x) ord[x] = b.first + x;
-            std::stable_sort(ord.begin(), ord.end(), [&](size_t x, size_t y) {
-              const TileInfo &tx = pl[hi[x]]->tiles[ht[x].x], &ty = pl[hi[y]]->tiles[ht[y].x];
-              if (hi[x] != hi[y]) return hi[x] < hi[y];
-              return tx.b != ty.b ? tx.b < ty.b : tx.a < ty.a;
-            });
-            std::vector<int2> t2(b.count);
-            std::vector<int> i2(b.count);
-            for (int x = 0; x < b.count; ++x) {
-              t2[x] = ht[ord[x]];
-              i2[x] = hi[ord[x]];
-            }
-            std::copy(t2.begin(), t2.end(), ht.begin() + b.first);
-            std::copy(i2.begin(), i2.end(), hi.begin() + b.first);
-          }
-        }
-      }
-      QD_CUDA(cudaMalloc(&mg.d_task, std::max<size_t>(1, ht.size()) * sizeof(int2)));
-      QD_CUDA(cudaMalloc(&mg.d_tinst, std::max<size_t>(1, hi.size()) * sizeof(int)));
-      if (!ht.empty()) {
-        QD_CUDA(cudaMemcpy(mg.d_task, ht.data(), ht.size() * sizeof(int2), cudaMemcpyHostToDevice));
-        QD_CUDA(cudaMemcpy(mg.d_tinst, hi.data(), hi.size() * sizeof(int), cudaMemcpyHostToDevice));
-      }
-      QD_CUDA(cudaMalloc(&mg.d_inst, n * sizeof(Inst122)));
-      QD_CUDA(cudaMallocHost(&mg.h_inst, n * sizeof(Inst122)));
-      f = merged122().emplace(key, mg).first;
-    }
-    m = &f->second;
-  }
-  for (size_t i = 0; i < n; ++i) {
-    const Item122& it = items[i];
-    const Plan122* p = pl[i];
-    if (!tsv[i]->buckets.empty()) {  // F tables for the group-pair tiles
-      const int nf = it.L->m * p->gmax;
-      k_ftab<<<(nf + 127) / 128, 128, 0, st>>>(it.L->dev, p->d_sbase, it.A->d, (double)it.A->herm, it.B->d,
-                                               (double)it.B->herm, p->d_ftab, p->gmax, p->nfent);
-      ++it.L->nlaunch;
-    }
-    Inst122& I = m->h_inst[i];
-    I.L = it.L->dev;
-    I.tiles = p->d_tiles;
-    I.gpd = p->d_gpd;
-    I.gpp = p->d_gpp;
-    I.F = p->d_ftab;
-    I.nfent = p->nfent;
-    I.A = it.A->d;
-    I.hA = (double)it.A->herm;
-    I.zA = it.A->zero_mask;
-    I.legA = leg_masks(spars(it.B), it.A->zero_mask);
-    I.B = it.B->d;
-    I.hB = (double)it.B->herm;
-    I.zB = it.B->zero_mask;
-    I.legB = leg_masks(spars(it.A), it.B->zero_mask);
-    I.C = it.C;
-    I.outmask = tsv[i]->outmask;
-    if (I.outmask != OUT_ALL) TRY(launch_122_gen(it.L, p, it.A, it.B, it.C, st));
-  }
-  QD_CUDA(cudaMemcpyAsync(m->d_inst, m->h_inst, n * sizeof(Inst122), cudaMemcpyHostToDevice, st));
-  const DevLayout& L0 = items[0].L->dev;
-  for (const Bucket122& b : m->buckets) {
-    if (b.tw == 2)
-      k_122_tile<2, 256, true><<<b.count, 256, b.smem, st>>>(L0, m->d_task + b.first, nullptr, nullptr, nullptr, nullptr, 0,
-                                                       nullptr, 0.0, 0u, 0u, nullptr, 0.0, 0u, 0u, nullptr, 0u,
-                                                       m->d_tinst + b.first, m->d_inst);
-    else
-      k_122_tile<1, 256, true><<<b.count, 256, b.smem, st>>>(L0, m->d_task + b.first, nullptr, nullptr, nullptr, nullptr, 0,
-                                                       nullptr, 0.0, 0u, 0u, nullptr, 0.0, 0u, 0u, nullptr, 0u,
-                                                       m->d_tinst + b.first, m->d_inst);
-    ++items[0].L->nlaunch;
-  }
-  QD_CUDA(cudaGetLastError());
-  return QD_OK;
-}
-
-// Drop every merged list that involves layout L (called when L goes).
-void drop_merged_122(const qd_layout* L) {
-  std::lock_guard<std::mutex> lock(g_m122_mutex);
-  auto& mm = merged122();
-  for (auto it = mm.begin(); it != mm.end();) {
-    auto& ls = it->second.layouts;
-    if (std::find(ls.begin(), ls.end(), L) != ls.end()) {
-      if (it->second.d_task) cudaFree(it->second.d_task);
-      if (it->second.d_tinst) cudaFree(it->second.d_tinst);
-      if (it->second.d_inst) cudaFree(it->second.d_inst);
-      if (it->second.h_inst) cudaFreeHost(it->second.h_inst);
-      it = mm.erase(it);
-    } else {
-      ++it;
-    }
-  }
 }
 
 }  // namespace qd

@@ -2,6 +2,9 @@
 // axpy (add_arrays), deterministic FP64 reductions (commutator_110/220 traces,
 // mat_2_norm, MBPT2, HF_E2), the White generator, the Pandya re-coupling
 // (calc_cc) and the particle-hole gather of commutator_222.
+#include <algorithm>
+#include <vector>
+
 #include "dev_common.cuh"
 
 namespace qd {
@@ -9,9 +12,7 @@ namespace qd {
 // BCH_EXPAND's truncated coefficients cof(1..11) (magnus_IMSRG.f90:265-267),
 // for terms whose coefficient is picked on the device (whole BCH step in one
 // graph): term k (0-based) adds cof[k] * INT2.
-__constant__ double c_bch_cof[11] = {1.0, 0.5, 0.166666666666666666, 0.04166666666666666,
-                                     0.0083333333333333333, .001388888888888, 1.984126984e-4, 2.48015873e-5,
-                                     2.755731922e-6, 2.755731922e-7, 2.505210839e-8};
+__constant__ double c_bch_cof[11] = QD_BCH_COF;
 
 // ---------------------------------------------------------------------------
 // add_arrays (src/ME_general.f90:592-618): c = sa*a + sb*b over the whole
@@ -56,6 +57,28 @@ __global__ void k_keep_parts(DevLayout L, double* __restrict__ op, unsigned keep
 
 int launch_keep_parts(qd_layout* L, double* op, unsigned keep) {
   if (L->neq > 0) k_keep_parts<<<(unsigned)((L->neq + 255) / 256), 256, 0, L->stream>>>(L->dev, op, keep);
+  ++L->nlaunch;
+  QD_CUDA(cudaGetLastError());
+  return QD_OK;
+}
+
+__global__ void __launch_bounds__(256) k_axpy_gen(DevLayout L, const double* a, double sa, const double* b, double sb,
+                                                  double* c) {
+  const i64 n1 = (i64)L.mp * L.n, n = 1 + n1 + L.pcnt[P_PPHH - P_HHHH];
+  const i64 stride = (i64)gridDim.x * blockDim.x;
+  for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
+    i64 pos = i == 0 ? 0 : L.o_fph + i - 1;
+    if (i > n1) {
+      int q, row, col;
+      part_elem(L, P_PPHH - P_HHHH, i - 1 - n1, q, pos, row, col);
+    }
+    c[pos] = __dadd_rn(__dmul_rn(sa, a[pos]), __dmul_rn(sb, b[pos]));
+  }
+}
+
+int launch_axpy_gen(qd_layout* L, const double* a, double sa, const double* b, double sb, double* c) {
+  const i64 n = 1 + (i64)L->mp * L->n + L->dev.pcnt[P_PPHH - P_HHHH];
+  k_axpy_gen<<<(unsigned)std::min<i64>(148 * 8, (n + 255) / 256), 256, 0, L->stream>>>(L->dev, a, sa, b, sb, c);
   ++L->nlaunch;
   QD_CUDA(cudaGetLastError());
   return QD_OK;
@@ -124,6 +147,20 @@ struct RedMBPT2 {
   }
 };
 
+struct RedGenSquares {  // squares of fph, then of Vpphh
+  DevLayout L;
+  const double* a;
+  i64 n1;
+  __device__ double operator()(i64 e) const {
+    i64 pos = L.o_fph + e;
+    if (e >= n1) {
+      int q, row, col;
+      part_elem(L, P_PPHH - P_HHHH, e - n1, q, pos, row, col);
+    }
+    return a[pos] * a[pos];
+  }
+};
+
 // HF_E2 trace: sum over blocks of Vhhhh(j,j)
 struct RedHHTrace {
   DevLayout L;
@@ -146,17 +183,18 @@ __global__ void __launch_bounds__(RED_THREADS) k_reduce(F f, i64 n, double* __re
   if (threadIdx.x == 0) partial[blockIdx.x] = s;
 }
 
-// out = scale * sum(partial) + add * (*out)
-__global__ void k_reduce_final(const double* __restrict__ partial, int np, double scale, double add,
+// out = scale * sum(partial) + add * (*out), or its square root
+__global__ void k_reduce_final(const double* __restrict__ partial, int np, double scale, double add, bool root,
                                double* __restrict__ out) {
   __shared__ double sh[RED_THREADS / 32];
   double s = 0.0;
   for (int i = threadIdx.x; i < np; i += blockDim.x) s += partial[i];
   s = block_sum<RED_THREADS>(s, sh);
-  if (threadIdx.x == 0) *out = scale * s + (add != 0.0 ? add * (*out) : 0.0);
+  if (threadIdx.x == 0) {
+    const double v = scale * s + (add != 0.0 ? add * (*out) : 0.0);
+    *out = root ? sqrt(v) : v;
+  }
 }
-
-__global__ void k_sqrt(double* x) { *x = sqrt(*x); }
 
 int ensure_reduction(qd_layout* L) {
   if (!L->d_red) {
@@ -168,15 +206,16 @@ int ensure_reduction(qd_layout* L) {
 }
 
 template <class F>
-static int reduce_to(qd_layout* L, const F& f, i64 n, double scale, double add, double* dout) {
+static int reduce_to(qd_layout* L, const F& f, i64 n, double scale, double add, double* dout, bool root = false) {
   int rc = ensure_reduction(L);
   if (rc) return rc;
   if (n > 0) {
-    k_reduce<F><<<RED_BLOCKS, RED_THREADS, 0, L->stream>>>(f, n, L->d_red);
-    k_reduce_final<<<1, RED_THREADS, 0, L->stream>>>(L->d_red, RED_BLOCKS, scale, add, dout);
+    const int blocks = (int)std::min<i64>(RED_BLOCKS, (n + RED_THREADS - 1) / RED_THREADS);
+    k_reduce<F><<<blocks, RED_THREADS, 0, L->stream>>>(f, n, L->d_red);
+    k_reduce_final<<<1, RED_THREADS, 0, L->stream>>>(L->d_red, blocks, scale, add, root, dout);
     L->nlaunch += 2;
   } else {
-    k_reduce_final<<<1, RED_THREADS, 0, L->stream>>>(L->d_red, 0, scale, add, dout);
+    k_reduce_final<<<1, RED_THREADS, 0, L->stream>>>(L->d_red, 0, scale, add, root, dout);
     ++L->nlaunch;
   }
   QD_CUDA(cudaGetLastError());
@@ -200,42 +239,16 @@ int reduce_mbpt2(qd_layout* L, const double* h, double* dout) {
 int reduce_hhtrace(qd_layout* L, const double* h, double* dout) {
   return reduce_to(L, RedHHTrace{L->dev, h}, L->dev.pcnt[0], 1.0, 0.0, dout);
 }
-// BCH_EXPAND's exit test on the device (magnus_IMSRG.f90:316): after the
-// term whose coefficient index is *kidx, continue while
-// |INT2| cof / |INT1| >= conv and fewer than 11 terms ran; the answer sets the
-// graph's loop condition (and, for the first term of a two-term loop body,
-// the condition of the second).  *kidx advances by one.
-__global__ void k_bch_decide(const double* __restrict__ norms, int* __restrict__ kidx, double conv,
-                             cudaGraphConditionalHandle hloop, cudaGraphConditionalHandle hnext, int set_next) {
-  const int k = *kidx;
-  const double cof = c_bch_cof[k];
-  const bool stop = norms[1] * cof / norms[0] < conv;  // NaN continues, as the host test does
-  const unsigned go = (!stop && k + 1 < 11) ? 1u : 0u;
-  *kidx = k + 1;
-  cudaGraphSetConditional(hloop, go);
-  if (set_next) cudaGraphSetConditional(hnext, go);
-}
-
-int launch_bch_decide(qd_layout* L, const double* norms, int* kidx, double conv, cudaGraphConditionalHandle hloop,
-                      cudaGraphConditionalHandle hnext, int set_next) {
-  k_bch_decide<<<1, 1, 0, L->stream>>>(norms, kidx, conv, hloop, hnext, set_next);
-  ++L->nlaunch;
-  QD_CUDA(cudaGetLastError());
-  return QD_OK;
-}
-
 // mat_2_norm (src/ME_general.f90:2112-2138): sqrt of the sum of squares of
 // every stored one- and two-body entry (E0 excluded), sqrt on the device.
 // The entries are summed in vectorize order by the fixed two-stage tree; the
 // reference's order (fph, fpp, fhh, then per block hhhh, pppp, pphh, phph,
 // phhh, ppph) differs only in rounding.
-int reduce_norm(qd_layout* L, const double* a, double* dout) {
-  int rc = reduce_to(L, RedDotRange{a, nullptr, L->o_fhh}, L->neq - L->o_fhh, 1.0, 0.0, dout);
-  if (rc) return rc;
-  k_sqrt<<<1, 1, 0, L->stream>>>(dout);
-  ++L->nlaunch;
-  QD_CUDA(cudaGetLastError());
-  return QD_OK;
+int reduce_norm(qd_layout* L, const double* a, unsigned zmask, double* dout) {
+  if (gen_like(zmask))  // a generator: its other parts add exact zeros
+    return reduce_to(L, RedGenSquares{L->dev, a, (i64)L->mp * L->n}, (i64)L->mp * L->n + L->dev.pcnt[P_PPHH - P_HHHH],
+                     1.0, 0.0, dout, true);
+  return reduce_to(L, RedDotRange{a, nullptr, L->o_fhh}, L->neq - L->o_fhh, 1.0, 0.0, dout, true);
 }
 
 // ---------------------------------------------------------------------------
@@ -249,14 +262,54 @@ int reduce_norm(qd_layout* L, const double* a, double* dout) {
 constexpr int AXN_BLOCKS = 4 * 148, AXN_THREADS = 256;
 
 
+// The last CTA of an update to finish adds the np pairs of partial sums in a
+// fixed order, writes out[0] = |a|, out[1] = |b| and, inside a step graph,
+// BCH_EXPAND's exit test (magnus_IMSRG.f90:316): after the term whose
+// coefficient index is *kidx, continue while |INT2| cof / |INT1| >= conv and
+// fewer than 11 terms ran; the answer sets the graph's loop condition (and,
+// for the first term of a two-term loop body, the condition of the second),
+// and *kidx advances by one.  (As two more launches, a final sum and the
+// test, a term of a small flow took 6 us more.)  Every CTA calls this after
+// its partial sums are written; count returns to zero for the next launch.
+__device__ __forceinline__ void axn_finish(const double2* partial, int np, unsigned* count, double* out, int* kidx,
+                                           const BchDecide& D) {
+  __shared__ double sh[AXN_THREADS / 32];
+  __shared__ bool last;
+  __threadfence();
+  if (threadIdx.x == 0) last = atomicAdd(count, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  double a = 0.0, b = 0.0;
+#pragma unroll 8
+  for (int i = threadIdx.x; i < np; i += AXN_THREADS) {
+    const double2 v = __ldcg(partial + i);
+    a += v.x;
+    b += v.y;
+  }
+  a = block_sum<AXN_THREADS>(a, sh);
+  b = block_sum<AXN_THREADS>(b, sh);
+  if (threadIdx.x != 0) return;
+  *count = 0;
+  const double n1 = sqrt(a), n2 = sqrt(b);
+  out[0] = n1;
+  out[1] = n2;
+  if (!D.on) return;
+  const int k = *kidx;
+  const bool stop = n2 * c_bch_cof[k] / n1 < D.conv;  // NaN continues, as the host test does
+  const unsigned go = (!stop && k + 1 < 11) ? 1u : 0u;
+  *kidx = k + 1;
+  cudaGraphSetConditional(D.hloop, go);
+  if (D.set_next) cudaGraphSetConditional(D.hnext, go);
+}
+
 // 16-byte accesses: the arrays are 16-byte aligned (cudaMalloc) and walked
 // as pairs of entries; entry 0 (E0) is left out of the norms, an odd last
 // entry is handled by thread 0.
-__global__ void __launch_bounds__(AXN_THREADS) k_axpy_norms(const double* __restrict__ a, double sa,
+__global__ void __launch_bounds__(AXN_THREADS) k_axpy_norms(const double* a, double sa,
                                                             const double* __restrict__ b, double sb,
-                                                            double* __restrict__ c, i64 n, i64 o1,
-                                                            double* __restrict__ partial,
-                                                            const int* __restrict__ kidx) {
+                                                            double* c, i64 n, i64 o1, double2* partial,
+                                                            int* kidx, unsigned* count, double* out, BchDecide D) {
   __shared__ double sh[AXN_THREADS / 32];
   if (kidx) sb = c_bch_cof[*kidx];  // coefficient of the term the device counter names
   double an = 0.0, bn = 0.0;
@@ -288,40 +341,110 @@ __global__ void __launch_bounds__(AXN_THREADS) k_axpy_norms(const double* __rest
   }
   an = block_sum<AXN_THREADS>(an, sh);
   bn = block_sum<AXN_THREADS>(bn, sh);
-  if (threadIdx.x == 0) {
-    partial[blockIdx.x] = an;
-    partial[gridDim.x + blockIdx.x] = bn;
-  }
+  if (threadIdx.x == 0) partial[blockIdx.x] = make_double2(an, bn);
+  axn_finish(partial, gridDim.x, count, out, kidx, D);
 }
 
-// out[0] = |a|, out[1] = |b|
-__global__ void k_axpy_norms_final(const double* __restrict__ partial, int np, double* __restrict__ out) {
-  __shared__ double sh[RED_THREADS / 32];
-  double v[2];
-  for (int k = 0; k < 2; ++k) {
-    double s = 0.0;
-    for (int i = threadIdx.x; i < np; i += blockDim.x) s += partial[k * np + i];
-    v[k] = block_sum<RED_THREADS>(s, sh);
-  }
-  if (threadIdx.x == 0) {
-    out[0] = sqrt(v[0]);
-    out[1] = sqrt(v[1]);
-  }
+// {sums of one-pass updates | their CTA counter}
+static int ensure_axn(qd_layout* L) {
+  if (L->d_axn) return QD_OK;
+  const size_t bytes = sizeof(double2) * (AXN_BLOCKS + 1);
+  QD_CUDA(cudaMalloc(&L->d_axn, bytes));
+  QD_CUDA(cudaMemsetAsync(L->d_axn, 0, bytes, L->stream));
+  L->ws_bytes += (i64)bytes;
+  return QD_OK;
 }
+static unsigned* axn_count(qd_layout* L) { return reinterpret_cast<unsigned*>(L->d_axn + 2 * AXN_BLOCKS); }
 
 int launch_axpy_norms(qd_layout* L, const double* a, double sa, const double* b, double sb, double* c,
-                      double* dout2, const int* kidx) {
-  if (!L->d_axn) {
-    QD_CUDA(cudaMalloc(&L->d_axn, sizeof(double) * 2 * AXN_BLOCKS));
-    L->ws_bytes += sizeof(double) * 2 * AXN_BLOCKS;
-  }
+                      double* dout2, int* kidx, const BchDecide& D) {
+  int rc = ensure_axn(L);
+  if (rc) return rc;
   if ((((uintptr_t)a | (uintptr_t)b | (uintptr_t)c) & 15) != 0) {
     set_error("launch_axpy_norms: operator arrays must be 16-byte aligned");
     return QD_ERR_ARG;
   }
-  k_axpy_norms<<<AXN_BLOCKS, AXN_THREADS, 0, L->stream>>>(a, sa, b, sb, c, L->neq, L->o_fhh, L->d_axn, kidx);
-  k_axpy_norms_final<<<1, RED_THREADS, 0, L->stream>>>(L->d_axn, AXN_BLOCKS, dout2);
-  L->nlaunch += 2;
+  // a CTA per two rounds of its threads at least: small bases need few
+  const int blocks = (int)std::max<i64>(1, std::min<i64>(AXN_BLOCKS, L->neq / (4 * AXN_THREADS)));
+  k_axpy_norms<<<blocks, AXN_THREADS, 0, L->stream>>>(a, sa, b, sb, c, L->neq, L->o_fhh, (double2*)L->d_axn, kidx,
+                                                      axn_count(L), dout2, D);
+  ++L->nlaunch;
+  QD_CUDA(cudaGetLastError());
+  return QD_OK;
+}
+
+// The update outside Vpppp, whose entries k_gen_pppp updates where it makes
+// them (reading C_pppp back costs as much as writing it): one CTA per piece
+// of at most AXR_PIECE entries.  Bound: HBM, 24 bytes an entry.  At N=20,
+// R=20 the one-pass update of all 61.9 M entries takes 230 us; Vpppp is 88%
+// of them.
+constexpr int AXR_PIECE = 4096;
+__global__ void __launch_bounds__(AXN_THREADS) k_axpy_norms_rest(const longlong2* __restrict__ piece,
+                                                                 const double* src, double* hs,
+                                                                 const double* __restrict__ b, double sb, int* kidx, i64 o1, double2* partial,
+                                                                 int first, unsigned* count, double* out,
+                                                                 BchDecide D) {
+  __shared__ double sh[AXN_THREADS / 32];
+  if (kidx) sb = c_bch_cof[*kidx];
+  const longlong2 p = piece[blockIdx.x];
+  double an = 0.0, bn = 0.0;
+#pragma unroll 4
+  for (int i = threadIdx.x; i < (int)p.y; i += AXN_THREADS) {
+    const i64 e = p.x + i;
+    const double x = src[e], y = b[e];
+    hs[e] = __dadd_rn(x, __dmul_rn(sb, y));
+    if (e >= o1) {
+      an += x * x;
+      bn += y * y;
+    }
+  }
+  an = block_sum<AXN_THREADS>(an, sh);
+  bn = block_sum<AXN_THREADS>(bn, sh);
+  if (threadIdx.x == 0) partial[first + blockIdx.x] = make_double2(an, bn);
+  axn_finish(partial, first + gridDim.x, count, out, kidx, D);  // the first sums are k_gen_pppp's
+}
+
+int prepare_hs_update(qd_layout* L) {
+  int rc = ensure_axn(L);
+  if (rc || L->d_axp) return rc;
+  if ((rc = gen_pppp_ctas(L, &L->naxp))) return rc;
+  std::vector<longlong2> v;
+  auto add = [&](i64 o, i64 e) {
+    for (; o < e; o += AXR_PIECE) v.push_back(longlong2{o, std::min<i64>(AXR_PIECE, e - o)});
+  };
+  i64 o = 0;
+  for (int q = 0; q < L->nblock; ++q) {
+    add(o, L->boff[6 * q + 1]);
+    o = L->boff[6 * q + 2];
+  }
+  add(o, L->neq);
+  void* p = nullptr;
+  QD_CUDA(cudaMalloc(&p, sizeof(longlong2) * std::max<size_t>(1, v.size())));
+  L->dev_allocs.push_back(p);
+  QD_CUDA(cudaMemcpy(p, v.data(), sizeof(longlong2) * v.size(), cudaMemcpyHostToDevice));
+  L->d_axrest = (const longlong2*)p;
+  L->naxrest = (int)v.size();
+  const size_t bytes = sizeof(double) * 2 * (size_t)std::max(1, L->naxp + L->naxrest);
+  QD_CUDA(cudaMalloc(&L->d_axp, bytes));
+  L->ws_bytes += (i64)(bytes + sizeof(longlong2) * v.size());
+  return QD_OK;
+}
+
+int hs_update_begin(qd_layout* L, const double* src, double* HS, double cof, int* kidx, HsUpdate* upd) {
+  int rc = prepare_hs_update(L);
+  if (rc) return rc;
+  upd->src = src;
+  upd->HS = HS;
+  upd->cof = cof;
+  upd->kidx = kidx;
+  upd->partial = L->d_axp;
+  return QD_OK;
+}
+
+int launch_axpy_norms_rest(qd_layout* L, const double* b, const HsUpdate& u, double* dout2, const BchDecide& D) {
+  k_axpy_norms_rest<<<L->naxrest, AXN_THREADS, 0, L->stream>>>(L->d_axrest, u.src, u.HS, b, u.cof, u.kidx, L->o_fhh,
+                                                               (double2*)u.partial, L->naxp, axn_count(L), dout2, D);
+  ++L->nlaunch;
   QD_CUDA(cudaGetLastError());
   return QD_OK;
 }

@@ -314,6 +314,7 @@ void layout_free_device(qd_layout* L) {
   for (void* p : L->dev_allocs) cudaFree(p);
   L->dev_allocs.clear();
   L->prog_ladder.clear_device();
+  L->prog_ladder_gen.clear_device();
   L->prog_221.clear_device();
   L->prog_111.clear_device();
   L->prog_pandya.clear_device();
@@ -324,6 +325,9 @@ void layout_free_device(qd_layout* L) {
   if (L->d_red) cudaFree(L->d_red);
   if (L->d_axn) cudaFree(L->d_axn);
   L->d_axn = nullptr;
+  if (L->d_axp) cudaFree(L->d_axp);
+  L->d_axp = nullptr;
+  L->d_axrest = nullptr;  // in dev_allocs
   if (L->h_red) cudaFreeHost(L->h_red);
   L->d_z = nullptr;
   L->d_red = nullptr;
@@ -331,6 +335,14 @@ void layout_free_device(qd_layout* L) {
   L->d_ccflag = nullptr;  // in dev_allocs
   L->d_tgt221 = nullptr;
   L->ntgt221 = -1;
+  for (int k = 0; k < 2; ++k) {
+    if (L->side[k]) cudaStreamDestroy(L->side[k]);
+    if (L->ev_side[k]) cudaEventDestroy(L->ev_side[k]);
+    L->side[k] = nullptr;
+    L->ev_side[k] = nullptr;
+  }
+  if (L->ev_fork) cudaEventDestroy(L->ev_fork);
+  L->ev_fork = nullptr;
   if (L->own_stream && L->stream) cudaStreamDestroy(L->stream);
   L->stream = nullptr;
 }

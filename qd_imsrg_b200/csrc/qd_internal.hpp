@@ -33,6 +33,10 @@ constexpr unsigned ALL_PARTS = (1u << P_COUNT) - 1;
 // Further bit of qd_op::zero_mask: no one-body entry couples states of
 // different (m_l, m_s) (such entries are all known to be zero).
 constexpr unsigned CONSERVES = 1u << (P_COUNT + 1);
+// A holds only fph and Vpphh (the Magnus generator, the White generator).
+inline bool gen_like(unsigned zmask) {
+  return ((zmask | (1u << P_FPH) | (1u << P_PPHH)) & ALL_PARTS) == ALL_PARTS;
+}
 constexpr unsigned ONE_BODY = (1u << P_FHH) | (1u << P_FPP) | (1u << P_FPH);
 
 // pair-table packing: idx (13 bits) | block (10 bits) | class-1 (2 bits) | swap (1 bit)
@@ -102,16 +106,6 @@ constexpr int NBUF = 7;
 struct Bufs {
   const double* p[NBUF];
 };
-// One instance of a launch that covers several layouts' programs (batched
-// flows): its program tables, operand buffers, herm factors and masks.
-struct GInst {
-  const GProb* probs;
-  const GSeg* segs;
-  Bufs bufs;
-  double hv0, hv1;
-  unsigned maskA, maskB;
-};
-
 struct GemmProgram {
   std::vector<GProb> probs;
   std::vector<GSeg> segs;
@@ -173,13 +167,20 @@ struct qd_layout {
   double* d_red = nullptr;        // reduction partials
   double* h_red = nullptr;        // pinned scalar results
   double* d_axn = nullptr;        // partial sums of the fused BCH update (axpy + norms)
+  double* d_axp = nullptr;        // the same for the update split between k_gen_pppp and the rest
+  const longlong2* d_axrest = nullptr;  // {offset, entries} of the pieces outside Vpppp
+  int naxrest = 0, naxp = 0;            // pieces; CTAs of k_gen_pppp
   int* d_ccflag = nullptr;        // per cross-coupled block: fph of A or B non-zero (121)
   const int* d_tgt221 = nullptr;  // one-body targets whose states share (m_l, m_s) (fused 221)
   int ntgt221 = -1;
   qd::OneBody* onebody = nullptr;
+  // branches of one commutator that run beside the main stream's (api.cu)
+  cudaStream_t side[2] = {nullptr, nullptr};
+  cudaEvent_t ev_fork = nullptr, ev_side[2] = {nullptr, nullptr};
   qd::i64 ws_bytes = 0;
   // GEMM programs
   qd::GemmProgram prog_ladder, prog_221, prog_111, prog_pandya;
+  qd::GemmProgram prog_ladder_gen;  // the blocks of prog_ladder that gen_ladder_fused leaves out
   bool programs_built = false;
   // split form of the GEMM programs: slices per operand (0 = plain FP64)
   int split_slices = 0;
@@ -189,6 +190,7 @@ struct qd_layout {
   void* graphs = nullptr;       // per-term graphs
   void* step_graphs = nullptr;  // whole BCH steps with the truncation decided on the device
   long long graphs_captured = 0, graph_replays = 0;
+  long long step_first = 0, step_per_term = 0;  // launches of the step graph in flight
 };
 
 struct qd_op {
@@ -227,32 +229,37 @@ int build_programs(qd_layout* L);
 // part helpers
 i64 part_count(const qd_layout* L, int part);  // total elements of a part over all blocks
 
+// BCH update of one term, HS = src + cof C with |src| and |C| (src: HS itself,
+// or the series' first operator), for the
+// C_pppp entries where they are produced (k_gen_pppp); partial receives two
+// sums of squares per CTA.  kidx: a device counter that picks the coefficient.
+struct HsUpdate {
+  const double* src = nullptr;
+  double* HS = nullptr;
+  double cof = 0.0;
+  int* kidx = nullptr;
+  double* partial = nullptr;
+};
+// BCH_EXPAND's exit test on the device, taken with a term's update
+struct BchDecide {
+  cudaGraphConditionalHandle hloop = 0, hnext = 0;
+  int on = 0, set_next = 0;
+  double conv = 0.0;
+};
 // kernels (kernels_*.cu)
 int launch_axpy(qd_layout* L, const double* a, double sa, const double* b, double sb, double* c, i64 n);
+// the same on E0, fph and Vpphh alone (every other part zero in a, b and c)
+int launch_axpy_gen(qd_layout* L, const double* a, double sa, const double* b, double sb, double* c);
 int launch_axpy_norms(qd_layout* L, const double* a, double sa, const double* b, double sb, double* c,
-                      double* dout2, const int* kidx = nullptr);
-int launch_bch_decide(qd_layout* L, const double* norms, int* kidx, double conv, cudaGraphConditionalHandle hloop,
-                      cudaGraphConditionalHandle hnext, int set_next);
+                      double* dout2, int* kidx = nullptr, const BchDecide& D = BchDecide{});
+// The same for every entry outside Vpppp, with the CTAs' sums of k_gen_pppp
+// (HsUpdate::partial) added; *upd is filled by hs_update_begin, which also
+// makes the tables and buffers (ahead of a stream capture: prepare_hs_update).
+int prepare_hs_update(qd_layout* L);
+int hs_update_begin(qd_layout* L, const double* src, double* HS, double cof, int* kidx, HsUpdate* upd);
+int launch_axpy_norms_rest(qd_layout* L, const double* b, const HsUpdate& upd, double* dout2,
+                           const BchDecide& D = BchDecide{});
 int prepare_program(qd_layout* L, GemmProgram& P, unsigned maskA, unsigned maskB);
-// one program of one instance in a batched launch
-struct GemmItem {
-  qd_layout* L;
-  GemmProgram* P;
-  const double* bufs[NBUF];
-  double hv0, hv1;
-  unsigned maskA, maskB;
-};
-int run_programs_batched(cudaStream_t st, const std::vector<GemmItem>& items);
-void drop_merged_gemm(const qd_layout* L);
-// commutator_122 of one instance in a batched launch
-struct Item122 {
-  qd_layout* L;
-  const qd_op* A;
-  const qd_op* B;
-  double* C;
-};
-int launch_122_batched(cudaStream_t st, const std::vector<Item122>& items);
-void drop_merged_122(const qd_layout* L);
 int prepare_122(qd_layout* L, const qd_op* A, const qd_op* B);
 std::string tuning_report_122(const qd_layout* L);
 double* scratch_operator(qd_layout* L);
@@ -261,7 +268,8 @@ int reduce_dot_range(qd_layout* L, const double* a, const double* b, i64 o, i64 
 int reduce_dot_part(qd_layout* L, const double* a, const double* b, int part, double scale, double add, double* dout);
 int reduce_mbpt2(qd_layout* L, const double* h, double* dout);
 int reduce_hhtrace(qd_layout* L, const double* h, double* dout);
-int reduce_norm(qd_layout* L, const double* a, double* dout);
+// zmask: parts known to be zero (fph and Vpphh alone are read if the rest is)
+int reduce_norm(qd_layout* L, const double* a, unsigned zmask, double* dout);
 double* red_slot(qd_layout* L, int k);
 int launch_white(qd_layout* L, double* gen, const double* h, int herm);
 int launch_keep_parts(qd_layout* L, double* op, unsigned keep);
@@ -271,7 +279,15 @@ int prepare_onebody(qd_layout* L);
 int launch_onebody(qd_layout* L, const qd_op* A, const qd_op* B, double* C, bool* done);
 void onebody_free(qd_layout* L);
 int launch_221_fused(qd_layout* L, const qd_op* A, const qd_op* B, double* C);
-int launch_122(qd_layout* L, const qd_op* A, const qd_op* B, double* C);
+// CTAs of k_gen_pppp for L (each writes two partial sums), 0 if it is not used
+int gen_pppp_ctas(qd_layout* L, int* n);
+// ladder: for a generator-like A also the ladders of the blocks for which
+// gen_ladder_fused holds (the caller then runs prog_ladder_gen, not prog_ladder)
+// st2: stream for the parts other than C_pppp of a generator-like A (null:
+// the layout's); upd: update HS with C_pppp (generator-like A only)
+int launch_122(qd_layout* L, const qd_op* A, const qd_op* B, double* C, bool ladder, cudaStream_t st2 = nullptr,
+               const HsUpdate* upd = nullptr);
+bool gen_ladder_fused(const qd_layout* L, int q);
 int launch_calc_cc(qd_layout* L, const qd_op* H, double* X);
 // Particle-hole channel (commutators.f90:716-980): C += the four re-coupled
 // Z terms, over the commutator_122 tiles (kernels_122.cu).
