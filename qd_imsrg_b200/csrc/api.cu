@@ -263,7 +263,11 @@ GemmProgram& ladder_program(qd_layout* L, const qd_op* A) {
   return ladder_in_122(L, A) ? L->prog_ladder_gen : L->prog_ladder;
 }
 
-constexpr i64 SPLIT_UPDATE_ENTRIES = 4000000;
+// From here on a BCH term's update of HS runs where C_pppp is made: reading
+// C_pppp back then costs more than the slower kernel does.  Whole flows with
+// the update split and in one pass (ms): N=12 R=12 6.7 and 6.3, N=12 R=14
+// (5.4 M entries) 10.9 and 10.6, N=20 R=16 (13 M) 19.0 and 19.5.
+constexpr i64 SPLIT_UPDATE_ENTRIES = 8000000;
 // Whether a BCH term's update of HS runs where C_pppp is made: C_pppp must be
 // final there (no ladder left to the grouped GEMM; the particle-hole channel
 // adds nothing to it, see launch_pandya_tiles).
@@ -271,24 +275,31 @@ bool splits_update(qd_layout* L, const qd_op* G) {
   return L->neq >= SPLIT_UPDATE_ENTRIES && ladder_in_122(L, G) && L->prog_ladder_gen.probs.empty();
 }
 
-int stage_222(qd_layout* L, const qd_op* A, const qd_op* B, qd_op* C, const qd_cc* HCC, const qd_cc* ETACC,
-              GemmProgram& ladders) {
+int stage_ladders(qd_layout* L, const qd_op* A, const qd_op* B, qd_op* C, GemmProgram& ladders) {
   const double* bufs[7] = {A->d, B->d, nullptr, nullptr, C->d, nullptr, nullptr};
-  {
-    StageTimer tm(L, S_LADDER);
-    TRY(run_program(L, ladders, bufs, (double)A->herm, (double)B->herm, A->zero_mask, B->zero_mask));
-  }
+  StageTimer tm(L, S_LADDER);
+  return run_program(L, ladders, bufs, (double)A->herm, (double)B->herm, A->zero_mask, B->zero_mask);
+}
+
+// construct_cc_ints: Z of the cross-coupled matrices, and its re-coupling into C
+int stage_ph_product(qd_layout* L, const qd_cc* HCC, const qd_cc* ETACC) {
+  TRY(ensure_z(L));
+  const double* zb[7] = {nullptr, nullptr, ETACC->d, HCC->d, nullptr, nullptr, L->d_z};
+  StageTimer tm(L, S_PANDYA_GEMM);
+  return run_program(L, L->prog_pandya, zb, ETACC->herm, HCC->herm, 0u, 0u);
+}
+int stage_ph_recouple(qd_layout* L, qd_op* C) {
+  StageTimer tm(L, S_PANDYA_GATHER);
+  return launch_pandya_tiles(L, L->d_z, C->d);
+}
+
+int stage_222(qd_layout* L, const qd_op* A, const qd_op* B, qd_op* C, const qd_cc* HCC, const qd_cc* ETACC) {
+  TRY(stage_ladders(L, A, B, C, L->prog_ladder));
   if (HCC && ETACC && HCC->filled && ETACC->filled && L->zsize > 0) {
     CHECK(std::fabs(HCC->herm) == 1.0 && std::fabs(ETACC->herm) == 1.0, QD_ERR_ARG,
           "cross-coupled herm must be +1 or -1");
-    TRY(ensure_z(L));
-    const double* zb[7] = {nullptr, nullptr, ETACC->d, HCC->d, nullptr, nullptr, L->d_z};
-    {
-      StageTimer tm(L, S_PANDYA_GEMM);
-      TRY(run_program(L, L->prog_pandya, zb, ETACC->herm, HCC->herm, 0u, 0u));
-    }
-    StageTimer tm(L, S_PANDYA_GATHER);
-    TRY(launch_pandya_tiles(L, L->d_z, C->d));
+    TRY(stage_ph_product(L, HCC, ETACC));
+    TRY(stage_ph_recouple(L, C));
   }
   C->zero_mask = 0;
   return QD_OK;
@@ -324,35 +335,45 @@ int stage_one_body(qd_layout* L, const qd_op* A, const qd_op* B, qd_op* C) {
 // one-body part, and for a generator-like A the parts other than C_pppp,
 // depend on nothing else of the commutator; their kernels leave much of the
 // chip idle (latency-bound, or a last wave of few CTAs), which the other
-// branches fill.  Small bases launched one by one are bound by the host's
-// launches, to which the events would only add; in a captured step they cost
-// nothing.  FORK_ENTRIES: where the gain and the events' cost meet (both
-// sides' times stand beside it).
-constexpr i64 FORK_ENTRIES = 1000000;
+// branches fill.  Measured with and without branches (us): generator-like A
+// N=6 R=8 27 and 48, N=12 R=12 62 and 83, N=20 R=16 176 and 222; two dense
+// operators N=6 R=8 151 and 163, N=12 R=14 (5.4 M entries) 1215 and 1235,
+// N=20 R=16 (13 M) 3158 and 3109: there the tiles of 122 fill the chip and
+// the one-body kernels only disturb them.
+constexpr i64 FORK_ENTRIES = 8000000;
 
 struct Branches {
   qd_layout* L = nullptr;
   bool on = false;
-  int fork(qd_layout* l) {
+  int used = 0;  // bit k: branch k has work
+  int fork(qd_layout* l, const qd_op* A) {
     L = l;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     QD_CUDA(cudaStreamIsCapturing(L->stream, &cs));
     const bool cap = cs != cudaStreamCaptureStatusNone;
-    if (L->prof.on || (!cap && L->neq < FORK_ENTRIES)) return QD_OK;
+    if (L->prof.on || (!gen_like(A->zero_mask) && L->neq >= FORK_ENTRIES)) return QD_OK;
     if (!L->ev_fork) {
       if (cap) return QD_OK;  // no stream or event is created inside a capture
       TRY(make_branches(L));
     }
     QD_CUDA(cudaEventRecord(L->ev_fork, L->stream));
-    for (int k = 0; k < 2; ++k) QD_CUDA(cudaStreamWaitEvent(L->side[k], L->ev_fork, 0));
     on = true;
     return QD_OK;
   }
-  cudaStream_t side(int k) const { return on ? L->side[k] : L->stream; }
+  // stream of branch k (the main one without branches)
+  int side(int k, cudaStream_t* st) {
+    *st = on ? L->side[k] : L->stream;
+    if (on && !((used >> k) & 1)) {
+      QD_CUDA(cudaStreamWaitEvent(*st, L->ev_fork, 0));
+      used |= 1 << k;
+    }
+    return QD_OK;
+  }
   int join() {
     if (!on) return QD_OK;
     on = false;
-    for (int k = 0; k < 2; ++k) {
+    for (int k = 0; k < qd_layout::NSIDE; ++k) {
+      if (!((used >> k) & 1)) continue;
       QD_CUDA(cudaEventRecord(L->ev_side[k], L->side[k]));
       QD_CUDA(cudaStreamWaitEvent(L->stream, L->ev_side[k], 0));
     }
@@ -363,7 +384,7 @@ struct Branches {
     if (on) join();
   }
   static int make_branches(qd_layout* L) {
-    for (int k = 0; k < 2; ++k) {
+    for (int k = 0; k < qd_layout::NSIDE; ++k) {
       QD_CUDA(cudaStreamCreateWithFlags(&L->side[k], cudaStreamNonBlocking));
       QD_CUDA(cudaEventCreateWithFlags(&L->ev_side[k], cudaEventDisableTiming));
     }
@@ -380,37 +401,59 @@ struct OnStream {
   ~OnStream() { L->stream = keep; }
 };
 
+// upd: also the BCH update of HS.  fill_acc: the caller can see ACC, which a
+// generator-like A's particle-hole channel does not need (see ph_gen.cu).
 int commutator_seq(qd_layout* L, const qd_op* A, const qd_op* B, qd_op* C, qd_op* w1, qd_op* w2, qd_cc* ACC,
-                   qd_cc* BCC, bool pandya, const HsUpdate* upd = nullptr) {
+                   qd_cc* BCC, bool pandya, const HsUpdate* upd = nullptr, bool fill_acc = true) {
   (void)w1;  // workspaces of the whole commutator: the fused 221 leaves them untouched
   (void)w2;
   TRY(build_programs(L));
+  const bool gen = gen_like(A->zero_mask);
+  const bool ph_short = pandya && gen && L->split_slices == 0 && L->ncc > 0;
   Branches br;
-  TRY(br.fork(L));
-  {
-    OnStream os(L, br.side(0));
-    TRY(stage_one_body(L, A, B, C));
-  }
-  {
-    StageTimer tm(L, S_122);
-    TRY(launch_122(L, A, B, C->d, ladder_in_122(L, A), br.side(1), upd));
-  }
+  cudaStream_t side;
+  TRY(br.fork(L, A));
   if (pandya) {
+    TRY(br.side(2, &side));
+    OnStream os(L, side);
     StageTimer tm(L, S_CALC_CC);
-    TRY(launch_calc_cc(L, A, ACC->d));
+    if (!ph_short || fill_acc) TRY(launch_calc_cc(L, A, ACC->d));
     ACC->filled = true;
     ACC->herm = A->herm;
     TRY(launch_calc_cc(L, B, BCC->d));
     BCC->filled = true;
     BCC->herm = B->herm;
   }
-  if (!pandya && ladder_program(L, A).probs.empty()) {  // no ladder is left
-    TRY(br.join());
-    C->zero_mask = conserves(A, B);
-    return QD_OK;
+  const bool ph_full = pandya && !ph_short && L->zsize > 0;
+  if (ph_short || ph_full) {
+    TRY(br.side(2, &side));
+    OnStream os(L, side);
+    if (ph_short) {
+      StageTimer tm(L, S_PANDYA_GEMM);
+      TRY(launch_ph_gen_products(L, A, BCC->d, (double)B->herm));
+    } else {
+      TRY(stage_ph_product(L, BCC, ACC));
+    }
   }
-  TRY(br.join());  // what follows adds to the parts that the branches write
-  TRY(stage_222(L, A, B, C, pandya ? BCC : nullptr, pandya ? ACC : nullptr, ladder_program(L, A)));
+  {
+    TRY(br.side(0, &side));
+    OnStream os(L, side);
+    TRY(stage_one_body(L, A, B, C));
+  }
+  {
+    if (gen) TRY(br.side(1, &side));
+    StageTimer tm(L, S_122);
+    TRY(launch_122(L, A, B, C->d, ladder_in_122(L, A), gen ? side : nullptr, upd));
+  }
+  GemmProgram& ladders = ladder_program(L, A);
+  if (gen) TRY(br.join());  // the branches write parts that the rest adds to
+  if (!ladders.probs.empty()) TRY(stage_ladders(L, A, B, C, ladders));
+  TRY(br.join());
+  if (ph_short) {
+    StageTimer tm(L, S_PANDYA_GATHER);
+    TRY(launch_ph_gen(L, (double)A->herm, (double)B->herm, C->d));
+  }
+  if (ph_full) TRY(stage_ph_recouple(L, C));
   C->zero_mask = conserves(A, B);
   return QD_OK;
 }
@@ -861,7 +904,7 @@ int qd_commutator_222(const qd_op* r1, const qd_op* r2, qd_op* r3, qd_op* w1, co
   TRY(use_device(r1->L));
   TRY(build_programs(r1->L));
   unsigned keep = r3->zero_mask & (ONE_BODY | CONSERVES);
-  TRY(stage_222(r1->L, r1, r2, r3, HCC, ETACC, r1->L->prog_ladder));
+  TRY(stage_222(r1->L, r1, r2, r3, HCC, ETACC));
   r3->zero_mask = keep;
   return QD_OK;
 }
@@ -874,7 +917,7 @@ int qd_commutator(const qd_op* A, const qd_op* B, qd_op* C, unsigned flags) {
   TRY(use_device(L));
   Workspace* w;
   TRY(get_ws(L, &w));
-  return commutator_seq(L, A, B, C, w->w1, w->w2, w->ca, w->cb, (flags & QD_PANDYA) != 0);
+  return commutator_seq(L, A, B, C, w->w1, w->w2, w->ca, w->cb, (flags & QD_PANDYA) != 0, nullptr, false);
 }
 
 // dGam (src/gs_IMSRG.f90:223-273): ETA = build_white(H) on a zeroed
@@ -895,7 +938,8 @@ int qd_dgam(const qd_op* H, qd_op* DER, qd_cc* HCC, qd_cc* ETACC) {
   QD_CUDA(cudaMemsetAsync(eta->d, 0, sizeof(double) * L->neq, L->stream));
   eta->zero_mask = ALL_PARTS | CONSERVES;
   TRY(white(eta, H));
-  TRY(commutator_seq(L, eta, H, DER, w->w1, w->w2, ETACC ? ETACC : w->ca, HCC ? HCC : w->cb, true));
+  TRY(commutator_seq(L, eta, H, DER, w->w1, w->w2, ETACC ? ETACC : w->ca, HCC ? HCC : w->cb, true, nullptr,
+                     ETACC != nullptr));
   return QD_OK;
 }
 
@@ -922,9 +966,9 @@ int qd_eom_matvec(const qd_op* H, const qd_op* Q, qd_op* HQ) {
   TRY(launch_keep_parts(L, X->d, exc));
   X->zero_mask = (ALL_PARTS & ~exc) | (Q->zero_mask & (exc | CONSERVES));
   X->herm = 1;
-  TRY(commutator_seq(L, H, X, HQ, w->w1, w->w2, w->cb, w->ca, true));
+  TRY(commutator_seq(L, H, X, HQ, w->w1, w->w2, w->cb, w->ca, true, nullptr, false));
   X->herm = -1;
-  TRY(commutator_seq(L, H, X, w->eomt, w->w1, w->w2, w->cb, w->ca, true));
+  TRY(commutator_seq(L, H, X, w->eomt, w->w1, w->w2, w->cb, w->ca, true, nullptr, false));
   TRY(launch_axpy(L, HQ->d, 0.5, w->eomt->d, 0.5, HQ->d, L->neq));
   TRY(launch_keep_parts(L, HQ->d, exc));
   HQ->herm = 1;
@@ -1029,14 +1073,14 @@ struct TermGraph {
 };
 using TermGraphs = std::map<TermKey, TermGraph>;
 
-// HS = src + cof [G, AD]: src is HS, or for the first term H (= AD)
+// HS = src + cof [G, AD]: src is HS, or for the first term H (= AD).
 int bch_term(qd_layout* L, const qd_op* G, const qd_op* AD, qd_op* INT2, const qd_op* src, qd_op* HS, qd_op* w1,
-             qd_op* w2, qd_cc* HCC, qd_cc* OCC, bool pandya, double cof, int* kidx = nullptr, const BchDecide& dec = BchDecide{}) {
+             qd_op* w2, qd_cc* HCC, qd_cc* OCC, bool pandya, bool first, double cof, int* kidx = nullptr, const BchDecide& dec = BchDecide{}) {
   HsUpdate upd;
   const bool split = splits_update(L, G);
   if (split) TRY(hs_update_begin(L, src->d, HS->d, cof, kidx, &upd));
   TRY(commutator_seq(L, G, AD, INT2, w1, w2, pandya ? OCC : nullptr, pandya ? HCC : nullptr, pandya,
-                     split ? &upd : nullptr));
+                     split ? &upd : nullptr, first));  // Omega's matrices once a series
   {
     StageTimer tm(L, S_GLUE);
     if (split)
@@ -1052,7 +1096,7 @@ int bch_term(qd_layout* L, const qd_op* G, const qd_op* AD, qd_op* INT2, const q
 
 static int bch_term_graph(qd_layout* L, const qd_op* G, const qd_op* AD, qd_op* INT2, const qd_op* src, qd_op* HS,
                           qd_op* w1, qd_op* w2, qd_cc* HCC, qd_cc* OCC, bool pandya, int term, double cof) {
-  if (!L->use_graphs || L->prof.on) return bch_term(L, G, AD, INT2, src, HS, w1, w2, HCC, OCC, pandya, cof);
+  if (!L->use_graphs || L->prof.on) return bch_term(L, G, AD, INT2, src, HS, w1, w2, HCC, OCC, pandya, term == 2, cof);
   if (!L->graphs) L->graphs = new TermGraphs();
   TermKey k;
   std::memset(&k, 0, sizeof(k));
@@ -1088,7 +1132,7 @@ static int bch_term_graph(qd_layout* L, const qd_op* G, const qd_op* AD, qd_op* 
   }
   if (tg.failed || tg.seen == 0) {
     ++tg.seen;
-    return bch_term(L, G, AD, INT2, src, HS, w1, w2, HCC, OCC, pandya, cof);
+    return bch_term(L, G, AD, INT2, src, HS, w1, w2, HCC, OCC, pandya, term == 2, cof);
   }
   // second sight: capture, instantiate, launch
   const long long n0 = L->nlaunch;
@@ -1096,7 +1140,7 @@ static int bch_term_graph(qd_layout* L, const qd_op* G, const qd_op* AD, qd_op* 
   int rc = QD_OK;
   cudaError_t e = cudaStreamBeginCapture(L->stream, cudaStreamCaptureModeThreadLocal);
   if (e == cudaSuccess) {
-    rc = bch_term(L, G, AD, INT2, src, HS, w1, w2, HCC, OCC, pandya, cof);
+    rc = bch_term(L, G, AD, INT2, src, HS, w1, w2, HCC, OCC, pandya, term == 2, cof);
     e = cudaStreamEndCapture(L->stream, &graph);
   }
   if (e == cudaSuccess && rc == QD_OK && graph) e = cudaGraphInstantiate(&tg.exec, graph, 0);
@@ -1107,7 +1151,7 @@ static int bch_term_graph(qd_layout* L, const qd_op* G, const qd_op* AD, qd_op* 
     tg.exec = nullptr;
     tg.failed = true;
     L->nlaunch = n0;
-    return bch_term(L, G, AD, INT2, src, HS, w1, w2, HCC, OCC, pandya, cof);
+    return bch_term(L, G, AD, INT2, src, HS, w1, w2, HCC, OCC, pandya, term == 2, cof);
   }
   tg.launches = L->nlaunch - n0;
   ++L->graphs_captured;
@@ -1206,7 +1250,7 @@ int capture_step(qd_layout* L, qd_op* HS, const qd_op* G, const qd_op* H, double
     out.d = P;
     HS->zero_mask = H->zero_mask;
     if (!r2)
-      r2 = bch_term(L, G, &ad, &out, direct ? &ad : HS, HS, w1, w2, HCC, OCC, pandya, 0.0, k,
+      r2 = bch_term(L, G, &ad, &out, direct ? &ad : HS, HS, w1, w2, HCC, OCC, pandya, true, 0.0, k,
                     BchDecide{hloop, hloop, 1, 0, conv});
     *first = L->nlaunch - n0;
     if (!r2) r2 = add_conditional(st, g, hloop, cudaGraphCondTypeWhile, &body);
@@ -1224,7 +1268,7 @@ int capture_step(qd_layout* L, qd_op* HS, const qd_op* G, const qd_op* H, double
     ad.d = P;
     ad.zero_mask = conserves(G, H);
     out.d = Q;
-    r2 = bch_term(L, G, &ad, &out, HS, HS, w1, w2, HCC, OCC, pandya, 0.0, k, BchDecide{hloop, hmore, 1, 1, conv});
+    r2 = bch_term(L, G, &ad, &out, HS, HS, w1, w2, HCC, OCC, pandya, false, 0.0, k, BchDecide{hloop, hmore, 1, 1, conv});
     *per_term = L->nlaunch - n1;
     if (!r2) r2 = add_conditional(st, body, hmore, cudaGraphCondTypeIf, &body2);
     if (cudaStreamEndCapture(st, &cap) != cudaSuccess || r2) {
@@ -1239,7 +1283,7 @@ int capture_step(qd_layout* L, qd_op* HS, const qd_op* G, const qd_op* H, double
     }
     ad.d = Q;
     out.d = P;
-    r2 = bch_term(L, G, &ad, &out, HS, HS, w1, w2, HCC, OCC, pandya, 0.0, k, BchDecide{hloop, hloop, 1, 0, conv});
+    r2 = bch_term(L, G, &ad, &out, HS, HS, w1, w2, HCC, OCC, pandya, false, 0.0, k, BchDecide{hloop, hloop, 1, 0, conv});
     if (cudaStreamEndCapture(st, &cap) != cudaSuccess || r2) {
       rc = r2 ? r2 : QD_ERR_CUDA;
       break;
@@ -1301,7 +1345,7 @@ int bch_step_launch(qd_layout* L, qd_op* HS, const qd_op* G, const qd_op* H, qd_
     TRY(prepare_program(L, ladder_program(L, G), G->zero_mask, H->zero_mask));
     TRY(prepare_program(L, L->prog_111, G->zero_mask, H->zero_mask));
     TRY(prepare_122(L, G, H));
-    if (pandya) TRY(ensure_z(L));
+    if (pandya) TRY(gen_like(G->zero_mask) ? prepare_ph_gen(L) : ensure_z(L));
     QD_CUDA(cudaStreamSynchronize(L->stream));
     if (capture_step(L, HS, G, H, P, Q, w1, w2, HCC, OCC, pandya, &sg.exec, &sg.first, &sg.per_term)) {
       sg.failed = true;
@@ -1723,7 +1767,7 @@ int bch_batch(const std::vector<qd_flow*>& fl, std::vector<int>& terms) {
       swap_ops(f->INT2, f->AD);
       const bool first = direct[j] && i == 2;
       TRY(bch_term(f->L, f->G, first ? f->HAM : f->AD, f->INT2, first ? f->HAM : f->HS, f->HS, f->w1, f->w2, f->HCC,
-                   f->OCC, pandya(f), cof));
+                   f->OCC, pandya(f), i == 2, cof));
       f->HS->zero_mask &= f->INT2->zero_mask;
       ++terms[j];
     }

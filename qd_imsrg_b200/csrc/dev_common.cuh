@@ -41,6 +41,36 @@ __device__ __forceinline__ double dv_elem(const DevLayout& L, const double* __re
   return sgn * v;
 }
 
+// Where dv_elem finds the element of the pair entries e1 = ptab(a,b), e2 =
+// ptab(c,d) (-1 where a == b or c == d): its position, sign (0: an exact zero,
+// position 0) and whether it is stored transposed (then times herm).  Without
+// a branch, so that several reads of one thread overlap.
+struct PairPos {
+  i64 pos;
+  double sgn;
+  bool up;
+};
+__device__ __forceinline__ PairPos dv_pos(const DevLayout& L, int e1, int e2) {
+  const int q = pt_blk(e1);
+  const bool ok = (e1 | e2) >= 0 && q == pt_blk(e2);
+  const int c1 = pt_cls(e1), c2 = pt_cls(e2);
+  PairPos p;
+  p.up = c1 < c2;
+  const int ch = p.up ? c2 : c1, cl = p.up ? c1 : c2, row = pt_idx(p.up ? e2 : e1), col = pt_idx(p.up ? e1 : e2);
+  const int qq = ok ? q : 0;
+  // vectorize slot of (row class, column class): hhhh 0, phhh 5, phph 3, pphh 2, ppph 4, pppp 1
+  const int slot = ok ? (int)((0x142035000ull >> (4 * (3 * ch + cl))) & 7) : 0;
+  const int4 bd = __ldg(&L.blk[qq]);
+  const int ld = ch == 0 ? bd.x : (ch == 1 ? bd.y : bd.z);
+  p.pos = ok ? __ldg(L.boff + 6 * qq + slot) + row + (i64)col * ld : 0;
+  p.sgn = ok ? ((pt_swap(e1) ^ pt_swap(e2)) ? -1.0 : 1.0) : 0.0;
+  return p;
+}
+__device__ __forceinline__ double dv_at(const PairPos& p, const double* __restrict__ op, double herm) {
+  const double v = __ldg(op + p.pos) * (p.up ? herm : 1.0);
+  return p.sgn == 0.0 ? 0.0 : p.sgn * v;
+}
+
 // One-body reads exactly as commutator_122 makes them:
 //   hole-loop read f(x,i):      fhh(x,i) (x hole) or fph(x-n,i) (x particle)
 //   particle-loop read f'(a,x): fph(a-n,x) (x hole) or fpp(a-n,x-n) (x particle)

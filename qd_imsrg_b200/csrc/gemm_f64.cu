@@ -706,6 +706,29 @@ int build_programs(qd_layout* L) {
   return QD_OK;
 }
 
+static int upload_program(GemmProgram& P) {
+  size_t pb = std::max<size_t>(1, P.probs.size()) * sizeof(GProb);
+  size_t sb = std::max<size_t>(1, P.segs.size()) * sizeof(GSeg);
+  QD_CUDA(cudaMalloc(&P.d_probs, pb));
+  QD_CUDA(cudaMalloc(&P.d_segs, sb));
+  if (!P.probs.empty())
+    QD_CUDA(cudaMemcpy(P.d_probs, P.probs.data(), P.probs.size() * sizeof(GProb), cudaMemcpyHostToDevice));
+  if (!P.segs.empty())
+    QD_CUDA(cudaMemcpy(P.d_segs, P.segs.data(), P.segs.size() * sizeof(GSeg), cudaMemcpyHostToDevice));
+  return QD_OK;
+}
+
+// The products of the particle-hole channel of a generator-like A (ph_gen.cu)
+int build_ph_products(qd_layout* L, const std::vector<PhProduct>& v, GemmProgram& P) {
+  (void)L;
+  Builder b(P);
+  for (const PhProduct& x : v) {
+    b.prob(x.r, x.rows, x.offY, x.r, GM_SET, BZ);  // nb == 0 writes zeros
+    b.seg(BXB, x.offB, x.r, N_, -1, BXA, x.offA, x.rows, T_, -1, x.nb, 1.0);
+  }
+  return upload_program(P);
+}
+
 // Ladder sums of the EOM product for a non-scalar target (eom.cu): per bra
 // block q with ket block partner[q] (pairs of M_q minus the target), the
 // npp(q) x nhh(partner[q]) output Wb[q] = Vpppp[q] Qb[q] + Qb[q] Vhhhh[partner[q]]
@@ -722,15 +745,7 @@ int build_eom_ladders(qd_layout* L, const std::vector<int>& partner, const std::
     b.seg(BA, L->boff[6 * q + 1], np, N_, P_PPPP, BB, qoff[q], np, N_, -1, np, 1.0);
     b.seg(BB, qoff[q], np, N_, -1, BA, L->boff[6 * q2 + 0], nh2, N_, P_HHHH, nh2, 1.0);
   }
-  size_t pb = std::max<size_t>(1, P.probs.size()) * sizeof(GProb);
-  size_t sb = std::max<size_t>(1, P.segs.size()) * sizeof(GSeg);
-  QD_CUDA(cudaMalloc(&P.d_probs, pb));
-  QD_CUDA(cudaMalloc(&P.d_segs, sb));
-  if (!P.probs.empty())
-    QD_CUDA(cudaMemcpy(P.d_probs, P.probs.data(), P.probs.size() * sizeof(GProb), cudaMemcpyHostToDevice));
-  if (!P.segs.empty())
-    QD_CUDA(cudaMemcpy(P.d_segs, P.segs.data(), P.segs.size() * sizeof(GSeg), cudaMemcpyHostToDevice));
-  return QD_OK;
+  return upload_program(P);
 }
 
 static bool seg_active_host(const GSeg& s, unsigned mA, unsigned mB) {

@@ -320,6 +320,7 @@ void layout_free_device(qd_layout* L) {
   L->prog_pandya.clear_device();
   split_free(L);
   onebody_free(L);
+  ph_gen_free(L);
   graphs_free(L);
   if (L->d_z) cudaFree(L->d_z);
   if (L->d_red) cudaFree(L->d_red);
@@ -334,8 +335,9 @@ void layout_free_device(qd_layout* L) {
   L->h_red = nullptr;
   L->d_ccflag = nullptr;  // in dev_allocs
   L->d_tgt221 = nullptr;
+  L->d_cctask = nullptr;
   L->ntgt221 = -1;
-  for (int k = 0; k < 2; ++k) {
+  for (int k = 0; k < qd_layout::NSIDE; ++k) {
     if (L->side[k]) cudaStreamDestroy(L->side[k]);
     if (L->ev_side[k]) cudaEventDestroy(L->ev_side[k]);
     L->side[k] = nullptr;

@@ -343,10 +343,12 @@ __global__ void __launch_bounds__(OB_T) k_one_final(DevLayout L, OneTab T, const
       const int i = ia.x, a = ia.y;
       const i64 f = L.o_fph + (a - n) + (i64)i * mp;
       const double fa = A[f], fb = B[f];
-      const double t1 = b1 ? fa * hA * dv_elem(L, B, hB, a, x, i, y) : 0.0;
-      const double t2 = a1 ? fb * hB * dv_elem(L, A, hA, a, x, i, y) : 0.0;
-      const double t3 = b2 ? -fa * dv_elem(L, B, hB, i, x, a, y) : 0.0;
-      const double t4 = a2 ? fb * dv_elem(L, A, hA, i, x, a, y) : 0.0;
+      const PairPos p1 = dv_pos(L, __ldg(&L.ptab[a * L.m + x]), __ldg(&L.ptab[i * L.m + y]));  // <a x|i y>
+      const PairPos p2 = dv_pos(L, __ldg(&L.ptab[i * L.m + x]), __ldg(&L.ptab[a * L.m + y]));  // <i x|a y>
+      const double t1 = b1 ? fa * hA * dv_at(p1, B, hB) : 0.0;
+      const double t2 = a1 ? fb * hB * dv_at(p1, A, hA) : 0.0;
+      const double t3 = b2 ? -fa * dv_at(p2, B, hB) : 0.0;
+      const double t4 = a2 ? fb * dv_at(p2, A, hA) : 0.0;
       s += (t1 - t2) + (t3 + t4);
     }
   }

@@ -122,6 +122,7 @@ struct GemmProgram {
 namespace qd {
 // stages timed by the optional per-stage CUDA-event profiler
 struct OneBody;  // tables of the fused one-body stage (onebody.cu)
+struct PhGen;    // tables and buffers of the particle-hole channel of a generator-like A (ph_gen.cu)
 enum Stage { S_E0 = 0, S_111, S_121, S_221, S_122, S_CALC_CC, S_LADDER, S_PANDYA_GEMM, S_PANDYA_GATHER, S_GLUE,
              S_COUNT };
 struct StageProf {
@@ -171,12 +172,16 @@ struct qd_layout {
   const longlong2* d_axrest = nullptr;  // {offset, entries} of the pieces outside Vpppp
   int naxrest = 0, naxp = 0;            // pieces; CTAs of k_gen_pppp
   int* d_ccflag = nullptr;        // per cross-coupled block: fph of A or B non-zero (121)
+  const int4* d_cctask = nullptr;  // calc_cc: {cross-coupled block, first row, first column}
+  int ncctask = 0;
   const int* d_tgt221 = nullptr;  // one-body targets whose states share (m_l, m_s) (fused 221)
   int ntgt221 = -1;
   qd::OneBody* onebody = nullptr;
+  qd::PhGen* ph_gen = nullptr;
   // branches of one commutator that run beside the main stream's (api.cu)
-  cudaStream_t side[2] = {nullptr, nullptr};
-  cudaEvent_t ev_fork = nullptr, ev_side[2] = {nullptr, nullptr};
+  static constexpr int NSIDE = 3;
+  cudaStream_t side[NSIDE] = {nullptr};
+  cudaEvent_t ev_fork = nullptr, ev_side[NSIDE] = {nullptr};
   qd::i64 ws_bytes = 0;
   // GEMM programs
   qd::GemmProgram prog_ladder, prog_221, prog_111, prog_pandya;
@@ -275,6 +280,16 @@ int launch_white(qd_layout* L, double* gen, const double* h, int herm);
 int launch_keep_parts(qd_layout* L, double* op, unsigned keep);
 int launch_121(qd_layout* L, const qd_op* A, const qd_op* B, double* C);
 int launch_221_trace(qd_layout* L, const qd_op* A, const qd_op* B, const qd_op* w1, const qd_op* w2, double* C);
+// One product of ph_gen: Y (r x rows, at offY) = X_B (r x nb, at offB) X'_A^T (rows x nb, at offA)
+struct PhProduct {
+  int r, rows, nb;
+  i64 offY, offB, offA;
+};
+int build_ph_products(qd_layout* L, const std::vector<PhProduct>& v, GemmProgram& P);
+int prepare_ph_gen(qd_layout* L);
+int launch_ph_gen_products(qd_layout* L, const qd_op* A, const double* XB, double hB);
+int launch_ph_gen(qd_layout* L, double hA, double hB, double* C);
+void ph_gen_free(qd_layout* L);
 int prepare_onebody(qd_layout* L);
 int launch_onebody(qd_layout* L, const qd_op* A, const qd_op* B, double* C, bool* done);
 void onebody_free(qd_layout* L);
