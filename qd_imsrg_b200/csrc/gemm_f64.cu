@@ -13,12 +13,20 @@
 //   SET       C  = V
 //   ACC_PAIR  C += V + sigma V^T      (M == N; the CTA computes the tile pair
 //   SET_PAIR  C  = V + sigma V^T       (I,J),(J,I) so V^T is at hand)
-// The pair modes carry the "hA*W^T - hB*W" transpose-adds of the reference
+// (sigma = +-1).  The pair modes carry the "hA*W^T - hB*W" transpose-adds of the reference
 // (src/commutators.f90:1002-1127, :154-169) without a second GEMM.
 //
 // Tile 64x64x16, 4 warps (2x2), each warp 32x32 = 4x4 DMMA m8n8k4 fragments;
 // 3-stage cp.async (8-byte, zero-fill) pipeline; FP64 accumulate.
-// tcgen05 has no f64 kind, so mma.sync DMMA is the FP64 tensor path here.
+// tcgen05 has no f64 kind, so mma.sync DMMA is the FP64 tensor path here (the
+// shapes m8n8k4 to m16n8k16 all reach 36 to 37 TFLOP/s from registers).
+// Bound: keeping the tensor pipe fed.  A tile pair (I,J), (J,I) is one product
+// of twice the K -- V(J,I)^T is the product of the transposed operands in the
+// other order, so C(I,J) = V(I,J) + sigma V(J,I)^T accumulates in one set of
+// registers and C(J,I) = sigma C(I,J)^T -- and the panels are swizzled instead
+// of padded: 48 KB of shared memory and 128 registers, four CTAs on an SM.
+// (With V(I,J) kept in shared memory while V(J,I) was formed: 85.5 KB, two
+// CTAs, the tensor pipe 59% active; times of both stand at run_program_f64.)
 #include <algorithm>
 #include <cstring>
 #include <map>
@@ -29,11 +37,16 @@
 
 namespace qd {
 
-constexpr int BM = 64, BN = 64, BK = 16, LDS = 68, NSTAGE = 3, TLD = 65;
+constexpr int BM = 64, BN = 64, BK = 16, NSTAGE = 3, TLD = 65;
 constexpr int GEMM_THREADS = 128;
-constexpr int SMEM_PIPE = 2 * NSTAGE * BK * LDS;  // doubles
-constexpr int SMEM_TILE = BN * TLD;               // doubles
-constexpr size_t GEMM_SMEM = sizeof(double) * (SMEM_PIPE + SMEM_TILE);
+constexpr int PANEL = BK * BM;  // doubles of one panel [k][m]
+constexpr size_t GEMM_SMEM = sizeof(double) * 2 * NSTAGE * PANEL;
+static_assert(BN * TLD <= 2 * NSTAGE * PANEL, "the epilogue's tile uses the pipeline's buffers");
+
+// Position of (k, m) in a panel: m is permuted within 16 by k, so that every
+// access touches each bank once -- stores along m, stores along k (16 k of
+// one m), and a DMMA fragment (4 k x 8 m).
+__device__ __forceinline__ int panel_pos(int k, int m) { return k * BM + (m ^ (((k & 3) << 2) | ((k >> 2) & 3))); }
 
 __device__ __forceinline__ void cp_async8(double* s, const double* g, bool pred) {
   unsigned sa = (unsigned)__cvta_generic_to_shared(s);
@@ -77,7 +90,7 @@ __device__ __forceinline__ void load_stage(const GSeg& s, const double* A, const
     for (int it = 0; it < IT; ++it) {
       const int kk = kk0 + 2 * it;
       const bool ok = rok && (k0 + kk < s.K);
-      cp_async8(sA + kk * LDS + mm, ok ? g : A, ok);
+      cp_async8(sA + panel_pos(kk, mm), ok ? g : A, ok);
       g += step;
     }
   } else {  // op(A)(m,k) = A[k + m*lda]: threads along k
@@ -89,7 +102,7 @@ __device__ __forceinline__ void load_stage(const GSeg& s, const double* A, const
     for (int it = 0; it < IT; ++it) {
       const int mm = mm0 + 8 * it;
       const bool ok = kok && (row0 + mm < M);
-      cp_async8(sA + kk * LDS + mm, ok ? g : A, ok);
+      cp_async8(sA + panel_pos(kk, mm), ok ? g : A, ok);
       g += step;
     }
   }
@@ -102,7 +115,7 @@ __device__ __forceinline__ void load_stage(const GSeg& s, const double* A, const
     for (int it = 0; it < IT; ++it) {
       const int nn = nn0 + 8 * it;
       const bool ok = kok && (col0 + nn < N);
-      cp_async8(sB + kk * LDS + nn, ok ? g : B, ok);
+      cp_async8(sB + panel_pos(kk, nn), ok ? g : B, ok);
       g += step;
     }
   } else {  // op(B)(k,n) = B[n + k*ldb]: threads along n
@@ -114,18 +127,19 @@ __device__ __forceinline__ void load_stage(const GSeg& s, const double* A, const
     for (int it = 0; it < IT; ++it) {
       const int kk = kk0 + 2 * it;
       const bool ok = nok && (k0 + kk < s.K);
-      cp_async8(sB + kk * LDS + nn, ok ? g : B, ok);
+      cp_async8(sB + panel_pos(kk, nn), ok ? g : B, ok);
       g += step;
     }
   }
 }
 
 // Active segments of the CTA's problem, kept in shared memory.
+constexpr int SEG_MAX = 8;  // problems have up to four segments, pair problems up to two (a tile pair doubles them)
 struct SegList {
-  GSeg seg[8];
-  const double* A[8];  // operand bases (buffer + offset)
-  const double* B[8];
-  double alpha[8];
+  GSeg seg[SEG_MAX];
+  const double* A[SEG_MAX];  // operand bases (buffer + offset)
+  const double* B[SEG_MAX];
+  double alpha[SEG_MAX];
   int nact;
   int total;  // k-tiles over all active segments
 };
@@ -139,7 +153,7 @@ __device__ __forceinline__ void cursor_next(const SegList& sl, int& si, int& k0)
   }
 }
 
-// Accumulate the tile (row0, col0) of problem P into acc[4][4][2].
+// Accumulate the tile (row0, col0) of problem P over the listed segments.
 __device__ void tile_mainloop(const GProb& P, const SegList& sl, int row0, int col0, double* smem,
                               double acc[4][4][2]) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -151,14 +165,13 @@ __device__ void tile_mainloop(const GProb& P, const SegList& sl, int row0, int c
   const int total = sl.total;
   if (total == 0) return;
   double* sA = smem;
-  double* sB = smem + NSTAGE * BK * LDS;
+  double* sB = smem + NSTAGE * PANEL;
   int ls = 0, lk = 0;  // load cursor
   int cs = 0, ck = 0;  // compute cursor
 #pragma unroll
   for (int st = 0; st < NSTAGE - 1; ++st) {
     if (st < total) {
-      load_stage(sl.seg[ls], sl.A[ls], sl.B[ls], P.M, P.N, row0, col0, lk, sA + st * BK * LDS,
-                 sB + st * BK * LDS);
+      load_stage(sl.seg[ls], sl.A[ls], sl.B[ls], P.M, P.N, row0, col0, lk, sA + st * PANEL, sB + st * PANEL);
       cursor_next(sl, ls, lk);
     }
     cp_commit();
@@ -167,25 +180,27 @@ __device__ void tile_mainloop(const GProb& P, const SegList& sl, int row0, int c
     const int gl = g + NSTAGE - 1;
     if (gl < total) {
       const int b = gl % NSTAGE;
-      load_stage(sl.seg[ls], sl.A[ls], sl.B[ls], P.M, P.N, row0, col0, lk, sA + b * BK * LDS,
-                 sB + b * BK * LDS);
+      load_stage(sl.seg[ls], sl.A[ls], sl.B[ls], P.M, P.N, row0, col0, lk, sA + b * PANEL, sB + b * PANEL);
       cursor_next(sl, ls, lk);
     }
     cp_commit();
     cp_wait<NSTAGE - 1>();
     __syncthreads();
     const double alpha = sl.alpha[cs];
-    const double* a_s = sA + (g % NSTAGE) * BK * LDS;
-    const double* b_s = sB + (g % NSTAGE) * BK * LDS;
+    const double* a_s = sA + (g % NSTAGE) * PANEL;
+    const double* b_s = sB + (g % NSTAGE) * PANEL;
 #pragma unroll
     for (int kk = 0; kk < BK; kk += 4) {
       double af[4], bf[4];
       const int kr = kk + (lane & 3);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) af[i] = a_s[kr * LDS + wm * 32 + i * 8 + (lane >> 2)];
+      for (int i = 0; i < 4; ++i) af[i] = a_s[panel_pos(kr, wm * 32 + i * 8 + (lane >> 2))];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) bf[j] = b_s[kr * LDS + wn * 32 + j * 8 + (lane >> 2)];
-      if (alpha != 1.0) {
+      for (int j = 0; j < 4; ++j) bf[j] = b_s[panel_pos(kr, wn * 32 + j * 8 + (lane >> 2))];
+      if (alpha == -1.0) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) af[i] = -af[i];
+      } else if (alpha != 1.0) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) af[i] *= alpha;
       }
@@ -216,95 +231,85 @@ __device__ __forceinline__ void stash(double* T, const double acc[4][4][2]) {
     }
 }
 
-__global__ void __launch_bounds__(GEMM_THREADS) k_grouped_gemm(const GTask* __restrict__ tasks,
-                                                               const GProb* __restrict__ probs,
-                                                               const GSeg* __restrict__ segs, Bufs bufs, double hv0,
-                                                               double hv1, unsigned maskA, unsigned maskB) {
+// Rows r < mr and columns c < nc of a tile at out (leading dimension ld) from
+// val(r, c): set or added; the reads of eight entries go out together.
+template <class F>
+__device__ __forceinline__ void write_tile(double* __restrict__ out, int ld, int mr, int nc, bool acc, F val) {
+  constexpr int PER = BM * BN / GEMM_THREADS, CH = 8;
+#pragma unroll 1
+  for (int k0 = 0; k0 < PER; k0 += CH) {
+    double cv[CH];
+#pragma unroll
+    for (int k = 0; k < CH; ++k) {
+      const int idx = threadIdx.x + (k0 + k) * GEMM_THREADS, r = idx & (BM - 1), c = idx >> 6;
+      cv[k] = acc && r < mr && c < nc ? out[r + (i64)c * ld] : 0.0;
+    }
+#pragma unroll
+    for (int k = 0; k < CH; ++k) {
+      const int idx = threadIdx.x + (k0 + k) * GEMM_THREADS, r = idx & (BM - 1), c = idx >> 6;
+      if (r < mr && c < nc) out[r + (i64)c * ld] = acc ? cv[k] + val(r, c) : val(r, c);
+    }
+  }
+}
+
+__global__ void __launch_bounds__(GEMM_THREADS, 4) k_grouped_gemm(const GTask* __restrict__ tasks,
+                                                                  const GProb* __restrict__ probs,
+                                                                  const GSeg* __restrict__ segs, Bufs bufs, double hv0,
+                                                                  double hv1, unsigned maskA, unsigned maskB) {
   extern __shared__ double smem[];
   const GTask t = tasks[blockIdx.x];
   const GProb P = probs[t.prob];
   double* out = const_cast<double*>(bufs.p[P.outbuf]) + P.offC;
+  const bool pair = P.mode == GM_ACC_PAIR || P.mode == GM_SET_PAIR;
+  const bool acc_mode = P.mode == GM_ACC || P.mode == GM_ACC_PAIR;
+  const bool twin = pair && t.ti != t.tj;  // with the tile (J,I)
+  const double sigma = pair ? P.sc * (P.spa ? hv0 : 1.0) * (P.spb ? hv1 : 1.0) : 0.0;
 
   __shared__ SegList sl;
   if (threadIdx.x == 0) {
     int na = 0, tot = 0;
-    for (int k = 0; k < P.nseg && na < 8; ++k) {
+    for (int k = 0; k < P.nseg && na < SEG_MAX; ++k) {
       const GSeg sg = segs[P.seg0 + k];
       if (!seg_active(sg, maskA, maskB) || sg.K <= 0) continue;
+      const double alpha = sg.c * (sg.pa ? hv0 : 1.0) * (sg.pb ? hv1 : 1.0);
       sl.seg[na] = sg;
       sl.A[na] = bufs.p[sg.srcA] + sg.offA;
       sl.B[na] = bufs.p[sg.srcB] + sg.offB;
-      sl.alpha[na] = sg.c * (sg.pa ? hv0 : 1.0) * (sg.pb ? hv1 : 1.0);
+      sl.alpha[na] = alpha;
       tot += (sg.K + BK - 1) / BK;
       ++na;
+      if (twin) {  // sigma (op(A) op(B))^T = sigma op(B)^T op(A)^T
+        GSeg sw = sg;
+        sw.lda = sg.ldb;
+        sw.ldb = sg.lda;
+        sw.tA = !sg.tB;
+        sw.tB = !sg.tA;
+        sl.seg[na] = sw;
+        sl.A[na] = sl.B[na - 1];
+        sl.B[na] = sl.A[na - 1];
+        sl.alpha[na] = sigma * alpha;
+        tot += (sg.K + BK - 1) / BK;
+        ++na;
+      }
     }
     sl.nact = na;
     sl.total = tot;
   }
   __syncthreads();
-  const bool pair = P.mode == GM_ACC_PAIR || P.mode == GM_SET_PAIR;
-  const bool acc_mode = P.mode == GM_ACC || P.mode == GM_ACC_PAIR;
-  double* T1 = smem + SMEM_PIPE;  // first tile stash (pair mode)
-  double* T2 = smem;              // aliases the pipeline buffers after the main loop
+  double* T = smem;  // the pipeline's buffers, free after the main loop
   double acc[4][4][2];
-
   const int r0 = t.ti * BM, c0 = t.tj * BN;
   tile_mainloop(P, sl, r0, c0, smem, acc);
-
-  if (!pair) {
-    stash(T2, acc);
-    __syncthreads();
-    const int mr = min(BM, P.M - r0), nc = min(BN, P.N - c0);
-    for (int idx = threadIdx.x; idx < BM * BN; idx += GEMM_THREADS) {
-      int r = idx & (BM - 1), c = idx >> 6;
-      if (r < mr && c < nc) {
-        double* p = out + (r0 + r) + (i64)(c0 + c) * P.ldc;
-        double v = T2[c * TLD + r];
-        *p = acc_mode ? *p + v : v;
-      }
-    }
-    return;
-  }
-  const double sigma = P.sc * (P.spa ? hv0 : 1.0) * (P.spb ? hv1 : 1.0);
-  if (t.ti == t.tj) {
-    stash(T1, acc);
-    __syncthreads();
-    const int mr = min(BM, P.M - r0);
-    for (int idx = threadIdx.x; idx < BM * BN; idx += GEMM_THREADS) {
-      int r = idx & (BM - 1), c = idx >> 6;
-      if (r < mr && c < mr) {
-        double* p = out + (r0 + r) + (i64)(r0 + c) * P.ldc;
-        double v = T1[c * TLD + r] + sigma * T1[r * TLD + c];
-        *p = acc_mode ? *p + v : v;
-      }
-    }
-    return;
-  }
-  // off-diagonal tile pair: V(I,J) -> T1, then V(J,I) -> T2
-  stash(T1, acc);
+  stash(T, acc);
   __syncthreads();
-  tile_mainloop(P, sl, c0, r0, smem, acc);
-  stash(T2, acc);
-  __syncthreads();
-  const int mI = min(BM, P.M - r0), mJ = min(BM, P.M - c0);
-  // C(I,J) (rows r0.., cols c0..) = T1 + sigma * T2^T
-  for (int idx = threadIdx.x; idx < BM * BN; idx += GEMM_THREADS) {
-    int r = idx & (BM - 1), c = idx >> 6;
-    if (r < mI && c < mJ) {
-      double* p = out + (r0 + r) + (i64)(c0 + c) * P.ldc;
-      double v = T1[c * TLD + r] + sigma * T2[r * TLD + c];
-      *p = acc_mode ? *p + v : v;
-    }
-  }
-  // C(J,I) (rows c0.., cols r0..) = T2 + sigma * T1^T
-  for (int idx = threadIdx.x; idx < BM * BN; idx += GEMM_THREADS) {
-    int r = idx & (BM - 1), c = idx >> 6;
-    if (r < mJ && c < mI) {
-      double* p = out + (c0 + r) + (i64)(r0 + c) * P.ldc;
-      double v = T2[c * TLD + r] + sigma * T1[r * TLD + c];
-      *p = acc_mode ? *p + v : v;
-    }
-  }
+  const int mr = min(BM, P.M - r0), nc = min(BN, P.N - c0);
+  double* o = out + r0 + (i64)c0 * P.ldc;
+  if (pair && !twin)
+    write_tile(o, P.ldc, mr, nc, acc_mode, [&](int r, int c) { return T[c * TLD + r] + sigma * T[r * TLD + c]; });
+  else
+    write_tile(o, P.ldc, mr, nc, acc_mode, [&](int r, int c) { return T[c * TLD + r]; });
+  if (twin)
+    write_tile(out + c0 + (i64)r0 * P.ldc, P.ldc, nc, mr, acc_mode, [&](int r, int c) { return sigma * T[r * TLD + c]; });
 }
 
 // ---------------------------------------------------------------------------
@@ -401,7 +406,7 @@ __global__ void __launch_bounds__(KS_THREADS, 3) k_gemm_kshort(const GTask* __re
   double* out = const_cast<double*>(bufs.p[P.outbuf]) + P.offC;
   if (threadIdx.x == 0) {
     int na = 0, tot = 0;
-    for (int k = 0; k < P.nseg && na < 8; ++k) {
+    for (int k = 0; k < P.nseg && na < SEG_MAX; ++k) {
       const GSeg sg = segs[P.seg0 + k];
       if (!seg_active(sg, maskA, maskB) || sg.K <= 0) continue;
       sl.seg[na] = sg;
