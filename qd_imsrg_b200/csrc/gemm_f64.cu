@@ -16,7 +16,10 @@
 // (sigma = +-1).  The pair modes carry the "hA*W^T - hB*W" transpose-adds of the reference
 // (src/commutators.f90:1002-1127, :154-169) without a second GEMM.
 //
-// Tile 64x64x16, 4 warps (2x2), each warp 32x32 = 4x4 DMMA m8n8k4 fragments;
+// Tiles of 64 or 32 rows by 64, 32 or 16 columns and 16 k (64 x 64: 4 warps,
+// each 32 x 32 = 4 x 4 DMMA m8n8k4 fragments); the rows and columns of a
+// problem are cut into full tiles and one narrower rest (see cuts), 32 x 32
+// throughout where a program has too few tiles to fill the chip;
 // 3-stage cp.async (8-byte, zero-fill) pipeline; FP64 accumulate.
 // tcgen05 has no f64 kind, so mma.sync DMMA is the FP64 tensor path here (the
 // shapes m8n8k4 to m16n8k16 all reach 36 to 37 TFLOP/s from registers).
@@ -37,8 +40,10 @@
 
 namespace qd {
 
-constexpr int BM = 64, BN = 64, BK = 16, NSTAGE = 3, TLD = 65;
+constexpr int BM = 64, BN = 64, BK = 16, NSTAGE = 3, TLD = 65;  // the largest tile
 constexpr int GEMM_THREADS = 128;
+// tile shapes of k_grouped_gemm as a task names them
+__host__ __device__ constexpr int tile_shape(int tm, int tn) { return tm * 128 + tn; }
 constexpr int PANEL = BK * BM;  // doubles of one panel [k][m]
 constexpr size_t GEMM_SMEM = sizeof(double) * 2 * NSTAGE * PANEL;
 static_assert(BN * TLD <= 2 * NSTAGE * PANEL, "the epilogue's tile uses the pipeline's buffers");
@@ -74,60 +79,37 @@ __device__ __forceinline__ bool seg_active(const GSeg& s, unsigned mA, unsigned 
   return !dead(s.srcA, s.depA) && !dead(s.srcB, s.depB);
 }
 
-// Load the (row0, col0) tile's k-slab [k0, k0+BK) of segment s (operands at
-// A, B) into stage buffers sA[k][m], sB[k][n].  Each thread walks a fixed
-// column (or row) with a pointer stride; out-of-range elements are zero-filled.
-__device__ __forceinline__ void load_stage(const GSeg& s, const double* A, const double* B, int M, int N, int row0,
-                                           int col0, int k0, double* sA, double* sB) {
+// k-slab [k0, k0 + BK) of W rows (columns) from x0 on of one operand, into a
+// panel [k][x].  contig: x is the contiguous index in memory (threads along
+// x), else k is (threads along k).  Out-of-range elements are zero-filled.
+template <int W>
+__device__ __forceinline__ void load_panel(const double* G, bool contig, int ld, int X, int K, int x0, int k0,
+                                           double* s) {
   const int tid = threadIdx.x;
-  constexpr int IT = (BM * BK) / GEMM_THREADS;  // 8
-  if (!s.tA) {  // A(m,k) at A[m + k*lda]: threads along m
-    const int mm = tid & (BM - 1), kk0 = tid >> 6;
-    const bool rok = row0 + mm < M;
-    const double* g = A + (row0 + mm) + (i64)(k0 + kk0) * s.lda;
-    const i64 step = (i64)2 * s.lda;
+  constexpr int IT = (W * BK) / GEMM_THREADS;
+  if (contig) {  // element (x, k) at G[x + k ld]
+    constexpr int KP = GEMM_THREADS / W;  // k per pass
+    const int x = tid & (W - 1), kk0 = tid / W;
+    const bool xok = x0 + x < X;
+    const double* g = G + (x0 + x) + (i64)(k0 + kk0) * ld;
+    const i64 step = (i64)KP * ld;
 #pragma unroll
     for (int it = 0; it < IT; ++it) {
-      const int kk = kk0 + 2 * it;
-      const bool ok = rok && (k0 + kk < s.K);
-      cp_async8(sA + panel_pos(kk, mm), ok ? g : A, ok);
+      const int kk = kk0 + KP * it;
+      const bool ok = xok && (k0 + kk < K);
+      cp_async8(s + panel_pos(kk, x), ok ? g : G, ok);
       g += step;
     }
-  } else {  // op(A)(m,k) = A[k + m*lda]: threads along k
-    const int kk = tid & (BK - 1), mm0 = tid >> 4;
-    const bool kok = k0 + kk < s.K;
-    const double* g = A + (k0 + kk) + (i64)(row0 + mm0) * s.lda;
-    const i64 step = (i64)8 * s.lda;
+  } else {  // at G[k + x ld]
+    const int kk = tid & (BK - 1), xx0 = tid >> 4;
+    const bool kok = k0 + kk < K;
+    const double* g = G + (k0 + kk) + (i64)(x0 + xx0) * ld;
+    const i64 step = (i64)8 * ld;
 #pragma unroll
     for (int it = 0; it < IT; ++it) {
-      const int mm = mm0 + 8 * it;
-      const bool ok = kok && (row0 + mm < M);
-      cp_async8(sA + panel_pos(kk, mm), ok ? g : A, ok);
-      g += step;
-    }
-  }
-  if (!s.tB) {  // B(k,n) at B[k + n*ldb]: threads along k
-    const int kk = tid & (BK - 1), nn0 = tid >> 4;
-    const bool kok = k0 + kk < s.K;
-    const double* g = B + (k0 + kk) + (i64)(col0 + nn0) * s.ldb;
-    const i64 step = (i64)8 * s.ldb;
-#pragma unroll
-    for (int it = 0; it < IT; ++it) {
-      const int nn = nn0 + 8 * it;
-      const bool ok = kok && (col0 + nn < N);
-      cp_async8(sB + panel_pos(kk, nn), ok ? g : B, ok);
-      g += step;
-    }
-  } else {  // op(B)(k,n) = B[n + k*ldb]: threads along n
-    const int nn = tid & (BN - 1), kk0 = tid >> 6;
-    const bool nok = col0 + nn < N;
-    const double* g = B + (col0 + nn) + (i64)(k0 + kk0) * s.ldb;
-    const i64 step = (i64)2 * s.ldb;
-#pragma unroll
-    for (int it = 0; it < IT; ++it) {
-      const int kk = kk0 + 2 * it;
-      const bool ok = nok && (k0 + kk < s.K);
-      cp_async8(sB + panel_pos(kk, nn), ok ? g : B, ok);
+      const int x = xx0 + 8 * it;
+      const bool ok = kok && (x0 + x < X);
+      cp_async8(s + panel_pos(kk, x), ok ? g : G, ok);
       g += step;
     }
   }
@@ -153,103 +135,129 @@ __device__ __forceinline__ void cursor_next(const SegList& sl, int& si, int& k0)
   }
 }
 
-// Accumulate the tile (row0, col0) of problem P over the listed segments.
-__device__ void tile_mainloop(const GProb& P, const SegList& sl, int row0, int col0, double* smem,
-                              double acc[4][4][2]) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int wm = warp & 1, wn = warp >> 1;
+// One TM x TN tile, WM x (4 / WM) warps.
+template <int TM, int TN, int WM>
+struct Tile {
+  static constexpr int WN = 4 / WM, MI = TM / WM / 8, NJ = TN / WN / 8;  // DMMA fragments of a warp
+  double acc[MI][NJ][2];
+
+  // Accumulate the tile (row0, col0) of problem P over the listed segments.
+  __device__ __forceinline__ void mainloop(const GProb& P, const SegList& sl, int row0, int col0, double* smem) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int wm = warp % WM, wn = warp / WM;
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < MI; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
-  const int total = sl.total;
-  if (total == 0) return;
-  double* sA = smem;
-  double* sB = smem + NSTAGE * PANEL;
-  int ls = 0, lk = 0;  // load cursor
-  int cs = 0, ck = 0;  // compute cursor
-#pragma unroll
-  for (int st = 0; st < NSTAGE - 1; ++st) {
-    if (st < total) {
-      load_stage(sl.seg[ls], sl.A[ls], sl.B[ls], P.M, P.N, row0, col0, lk, sA + st * PANEL, sB + st * PANEL);
+      for (int j = 0; j < NJ; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+    const int total = sl.total;
+    if (total == 0) return;
+    double* sA = smem;
+    double* sB = smem + NSTAGE * PANEL;
+    int ls = 0, lk = 0;  // load cursor
+    int cs = 0, ck = 0;  // compute cursor
+    auto load = [&](int st) {
+      const GSeg& g = sl.seg[ls];
+      load_panel<TM>(sl.A[ls], !g.tA, g.lda, P.M, g.K, row0, lk, sA + st * PANEL);
+      load_panel<TN>(sl.B[ls], g.tB, g.ldb, P.N, g.K, col0, lk, sB + st * PANEL);
       cursor_next(sl, ls, lk);
+    };
+#pragma unroll
+    for (int st = 0; st < NSTAGE - 1; ++st) {
+      if (st < total) load(st);
+      cp_commit();
     }
-    cp_commit();
-  }
-  for (int g = 0; g < total; ++g) {
-    const int gl = g + NSTAGE - 1;
-    if (gl < total) {
-      const int b = gl % NSTAGE;
-      load_stage(sl.seg[ls], sl.A[ls], sl.B[ls], P.M, P.N, row0, col0, lk, sA + b * PANEL, sB + b * PANEL);
-      cursor_next(sl, ls, lk);
-    }
-    cp_commit();
-    cp_wait<NSTAGE - 1>();
-    __syncthreads();
-    const double alpha = sl.alpha[cs];
-    const double* a_s = sA + (g % NSTAGE) * PANEL;
-    const double* b_s = sB + (g % NSTAGE) * PANEL;
+    for (int g = 0; g < total; ++g) {
+      const int gl = g + NSTAGE - 1;
+      if (gl < total) load(gl % NSTAGE);
+      cp_commit();
+      cp_wait<NSTAGE - 1>();
+      __syncthreads();
+      const double alpha = sl.alpha[cs];
+      const double* a_s = sA + (g % NSTAGE) * PANEL;
+      const double* b_s = sB + (g % NSTAGE) * PANEL;
 #pragma unroll
-    for (int kk = 0; kk < BK; kk += 4) {
-      double af[4], bf[4];
-      const int kr = kk + (lane & 3);
+      for (int kk = 0; kk < BK; kk += 4) {
+        double af[MI], bf[NJ];
+        const int kr = kk + (lane & 3);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) af[i] = a_s[panel_pos(kr, wm * 32 + i * 8 + (lane >> 2))];
+        for (int i = 0; i < MI; ++i) af[i] = a_s[panel_pos(kr, (wm * MI + i) * 8 + (lane >> 2))];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) bf[j] = b_s[panel_pos(kr, wn * 32 + j * 8 + (lane >> 2))];
-      if (alpha == -1.0) {
+        for (int j = 0; j < NJ; ++j) bf[j] = b_s[panel_pos(kr, (wn * NJ + j) * 8 + (lane >> 2))];
+        if (alpha == -1.0) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) af[i] = -af[i];
-      } else if (alpha != 1.0) {
+          for (int i = 0; i < MI; ++i) af[i] = -af[i];
+        } else if (alpha != 1.0) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) af[i] *= alpha;
+          for (int i = 0; i < MI; ++i) af[i] *= alpha;
+        }
+#pragma unroll
+        for (int i = 0; i < MI; ++i)
+#pragma unroll
+          for (int j = 0; j < NJ; ++j) dmma(acc[i][j][0], acc[i][j][1], af[i], bf[j]);
       }
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) dmma(acc[i][j][0], acc[i][j][1], af[i], bf[j]);
+      cursor_next(sl, cs, ck);
+      __syncthreads();
     }
-    cursor_next(sl, cs, ck);
+    cp_wait<0>();
     __syncthreads();
   }
-  cp_wait<0>();
-  __syncthreads();
-}
 
-// accumulator fragments -> smem tile T[col*TLD + row]
-__device__ __forceinline__ void stash(double* T, const double acc[4][4][2]) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int wm = warp & 1, wn = warp >> 1;
+  // accumulator fragments -> smem tile T[col * TLD + row]
+  __device__ __forceinline__ void stash(double* T) const {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int wm = warp % WM, wn = warp / WM;
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < MI; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      int r = wm * 32 + i * 8 + (lane >> 2);
-      int c = wn * 32 + j * 8 + 2 * (lane & 3);
-      T[c * TLD + r] = acc[i][j][0];
-      T[(c + 1) * TLD + r] = acc[i][j][1];
-    }
-}
+      for (int j = 0; j < NJ; ++j) {
+        const int r = (wm * MI + i) * 8 + (lane >> 2), c = (wn * NJ + j) * 8 + 2 * (lane & 3);
+        T[c * TLD + r] = acc[i][j][0];
+        T[(c + 1) * TLD + r] = acc[i][j][1];
+      }
+  }
+};
 
-// Rows r < mr and columns c < nc of a tile at out (leading dimension ld) from
-// val(r, c): set or added; the reads of eight entries go out together.
-template <class F>
+// Rows r < mr and columns c < nc of an R x C tile at out (leading dimension
+// ld) from val(r, c): set or added; the reads of up to eight entries go out
+// together.
+template <int R, int CO, class F>
 __device__ __forceinline__ void write_tile(double* __restrict__ out, int ld, int mr, int nc, bool acc, F val) {
-  constexpr int PER = BM * BN / GEMM_THREADS, CH = 8;
+  constexpr int PER = R * CO / GEMM_THREADS, CH = PER < 8 ? PER : 8;
 #pragma unroll 1
   for (int k0 = 0; k0 < PER; k0 += CH) {
     double cv[CH];
 #pragma unroll
     for (int k = 0; k < CH; ++k) {
-      const int idx = threadIdx.x + (k0 + k) * GEMM_THREADS, r = idx & (BM - 1), c = idx >> 6;
+      const int idx = threadIdx.x + (k0 + k) * GEMM_THREADS, r = idx % R, c = idx / R;
       cv[k] = acc && r < mr && c < nc ? out[r + (i64)c * ld] : 0.0;
     }
 #pragma unroll
     for (int k = 0; k < CH; ++k) {
-      const int idx = threadIdx.x + (k0 + k) * GEMM_THREADS, r = idx & (BM - 1), c = idx >> 6;
+      const int idx = threadIdx.x + (k0 + k) * GEMM_THREADS, r = idx % R, c = idx / R;
       if (r < mr && c < nc) out[r + (i64)c * ld] = acc ? cv[k] + val(r, c) : val(r, c);
     }
   }
+}
+
+// One task of problem P; twin: with the transposed tile.
+template <int TM, int TN, int WM>
+__device__ __forceinline__ void run_tile(const GProb& P, const SegList& sl, int r0, int c0, bool pair, bool twin,
+                                         bool acc_mode, double sigma, double* out, double* smem) {
+  Tile<TM, TN, WM> t;
+  double* T = smem;  // the pipeline's buffers, free after the main loop
+  t.mainloop(P, sl, r0, c0, smem);
+  t.stash(T);
+  __syncthreads();
+  const int mr = min(TM, P.M - r0), nc = min(TN, P.N - c0);
+  double* o = out + r0 + (i64)c0 * P.ldc;
+  if (pair && !twin)
+    write_tile<TM, TN>(o, P.ldc, mr, nc, acc_mode,
+                       [&](int r, int c) { return T[c * TLD + r] + sigma * T[r * TLD + c]; });
+  else
+    write_tile<TM, TN>(o, P.ldc, mr, nc, acc_mode, [&](int r, int c) { return T[c * TLD + r]; });
+  if (twin)
+    write_tile<TN, TM>(out + c0 + (i64)r0 * P.ldc, P.ldc, nc, mr, acc_mode,
+                       [&](int r, int c) { return sigma * T[r * TLD + c]; });
 }
 
 __global__ void __launch_bounds__(GEMM_THREADS, 4) k_grouped_gemm(const GTask* __restrict__ tasks,
@@ -262,7 +270,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 4) k_grouped_gemm(const GTask* _
   double* out = const_cast<double*>(bufs.p[P.outbuf]) + P.offC;
   const bool pair = P.mode == GM_ACC_PAIR || P.mode == GM_SET_PAIR;
   const bool acc_mode = P.mode == GM_ACC || P.mode == GM_ACC_PAIR;
-  const bool twin = pair && t.ti != t.tj;  // with the tile (J,I)
+  const int r0 = t.r0, c0 = t.c0;
+  const bool twin = pair && r0 != c0;  // with the tile (J,I)
   const double sigma = pair ? P.sc * (P.spa ? hv0 : 1.0) * (P.spb ? hv1 : 1.0) : 0.0;
 
   __shared__ SegList sl;
@@ -296,20 +305,16 @@ __global__ void __launch_bounds__(GEMM_THREADS, 4) k_grouped_gemm(const GTask* _
     sl.total = tot;
   }
   __syncthreads();
-  double* T = smem;  // the pipeline's buffers, free after the main loop
-  double acc[4][4][2];
-  const int r0 = t.ti * BM, c0 = t.tj * BN;
-  tile_mainloop(P, sl, r0, c0, smem, acc);
-  stash(T, acc);
-  __syncthreads();
-  const int mr = min(BM, P.M - r0), nc = min(BN, P.N - c0);
-  double* o = out + r0 + (i64)c0 * P.ldc;
-  if (pair && !twin)
-    write_tile(o, P.ldc, mr, nc, acc_mode, [&](int r, int c) { return T[c * TLD + r] + sigma * T[r * TLD + c]; });
-  else
-    write_tile(o, P.ldc, mr, nc, acc_mode, [&](int r, int c) { return T[c * TLD + r]; });
-  if (twin)
-    write_tile(out + c0 + (i64)r0 * P.ldc, P.ldc, nc, mr, acc_mode, [&](int r, int c) { return sigma * T[r * TLD + c]; });
+#define QD_TILE(TM, TN, WM) run_tile<TM, TN, WM>(P, sl, r0, c0, pair, twin, acc_mode, sigma, out, smem)
+  switch (t.shape) {
+    case tile_shape(64, 64): QD_TILE(64, 64, 2); break;
+    case tile_shape(64, 32): QD_TILE(64, 32, 2); break;
+    case tile_shape(64, 16): QD_TILE(64, 16, 4); break;
+    case tile_shape(32, 64): QD_TILE(32, 64, 2); break;
+    case tile_shape(32, 32): QD_TILE(32, 32, 2); break;
+    default: QD_TILE(32, 16, 4); break;
+  }
+#undef QD_TILE
 }
 
 // ---------------------------------------------------------------------------
@@ -422,12 +427,12 @@ __global__ void __launch_bounds__(KS_THREADS, 3) k_gemm_kshort(const GTask* __re
   __syncthreads();
   const bool pair = P.mode == GM_ACC_PAIR || P.mode == GM_SET_PAIR;
   const bool acc_mode = P.mode == GM_ACC || P.mode == GM_ACC_PAIR;
-  const int r0 = t.ti * BM, c0 = t.tj * BN;
+  const int r0 = t.r0, c0 = t.c0;
   double* pA1 = smem + KS_PANEL0;
   double* pB1 = pA1 + KS_PANEL;
   double* T = smem;  // stash 1: below the panels
   double v1[4][2][2];
-  if (!pair || t.ti == t.tj) {
+  if (!pair || r0 == c0) {
     ks_panels(sl, P.M, P.N, r0, c0, pA1, pB1);
     ks_mma(pA1, pB1, v1);
     __syncthreads();
@@ -762,38 +767,63 @@ static bool seg_active_host(const GSeg& s, unsigned mA, unsigned mB) {
   return !dead(s.srcA, s.depA) && !dead(s.srcB, s.depB);
 }
 
+// Starts and widths of the tiles along n entries: full tiles of `w` and one
+// rest of the narrowest width that holds it (of 64, 32 and, where `least` is
+// 16, 16): n_h-column outputs are mostly padding in 64-wide tiles.  At N=20,
+// R=20 the ladders' padded work falls from 1.22 to 1.11 times the real one.
+static std::vector<std::pair<int, int>> cuts(int n, int w, int least) {
+  std::vector<std::pair<int, int>> v;
+  for (int x = 0; x < n; x += w) {
+    int c = w;
+    while (c > least && n - x <= c / 2) c /= 2;
+    v.push_back({x, c});
+  }
+  return v;
+}
+
 // Host task lists of P for (mA, mB): [0] long-K problems, [1] K-short ones,
 // each as (cost, task), longest first.  Every tile (tile pair in the pair
 // modes) of every problem that has an active segment (SET problems always:
 // they must write); problems whose active segments span K <= KS_K (at most
-// 8 of them) go to the K-short kernel.
+// 8 of them) go to the K-short kernel.  Tiles are 64 wide; where these are
+// fewer than FEW_TILES (the chip holds 592 CTAs), 32: a tile's products take
+// the same time on one SM however many SMs are idle.
+constexpr size_t FEW_TILES = 1184;
 static void task_vectors(const GemmProgram& P, unsigned mA, unsigned mB, std::vector<std::pair<double, GTask>> v[2]) {
-  for (size_t pi = 0; pi < P.probs.size(); ++pi) {
-    const GProb& g = P.probs[pi];
-    double kt = 0.0;
-    int ksum = 0, nact = 0;
-    for (int k = 0; k < g.nseg; ++k) {
-      const GSeg& s = P.segs[g.seg0 + k];
-      if (seg_active_host(s, mA, mB) && s.K > 0) {
-        kt += (s.K + BK - 1) / BK;
-        ksum += s.K;
-        ++nact;
+  for (int w : {64, 32}) {
+    v[0].clear();
+    v[1].clear();
+    for (size_t pi = 0; pi < P.probs.size(); ++pi) {
+      const GProb& g = P.probs[pi];
+      double kt = 0.0;
+      int ksum = 0, nact = 0;
+      for (int k = 0; k < g.nseg; ++k) {
+        const GSeg& s = P.segs[g.seg0 + k];
+        if (seg_active_host(s, mA, mB) && s.K > 0) {
+          kt += (s.K + BK - 1) / BK;
+          ksum += s.K;
+          ++nact;
+        }
       }
+      const bool set = g.mode == GM_SET || g.mode == GM_SET_PAIR;
+      if (kt == 0.0 && !set) continue;
+      const int which = (ksum <= KS_K && nact <= 8) ? 1 : 0;
+      const bool pair = g.mode == GM_ACC_PAIR || g.mode == GM_SET_PAIR;
+      // the K-short kernel has 64 x 64 tiles only; a pair's rows and columns are cut alike
+      const auto rows = which ? cuts(g.M, 64, 64) : cuts(g.M, w, 32);
+      const auto cols = which ? cuts(g.N, 64, 64) : cuts(g.N, w, pair ? 32 : 16);
+      for (size_t i = 0; i < rows.size(); ++i)
+        for (size_t j = pair ? i : 0; j < cols.size(); ++j) {
+          GTask t;
+          t.prob = (int)pi;
+          t.r0 = rows[i].first;
+          t.c0 = cols[j].first;
+          t.shape = tile_shape(rows[i].second, cols[j].second);
+          const double area = rows[i].second * cols[j].second / 4096.0;
+          v[which].push_back({(kt + 1.0) * ((pair && i != j) ? 2.0 : 1.0) * (which ? 1.0 : area + 0.1), t});
+        }
     }
-    bool set = g.mode == GM_SET || g.mode == GM_SET_PAIR;
-    if (kt == 0.0 && !set) continue;
-    const int which = (ksum <= KS_K && nact <= 8) ? 1 : 0;
-    int tm = (g.M + BM - 1) / BM, tn = (g.N + BN - 1) / BN;
-    bool pair = g.mode == GM_ACC_PAIR || g.mode == GM_SET_PAIR;
-    for (int i = 0; i < tm; ++i)
-      for (int j = pair ? i : 0; j < tn; ++j) {
-        GTask t;
-        t.prob = (int)pi;
-        t.ti = (short)i;
-        t.tj = (short)j;
-        double cost = (kt + 1.0) * ((pair && i != j) ? 2.0 : 1.0);
-        v[which].push_back({cost, t});
-      }
+    if (v[0].size() >= FEW_TILES) break;
   }
   for (int w = 0; w < 2; ++w)
     std::stable_sort(v[w].begin(), v[w].end(), [](const auto& a, const auto& b) { return a.first > b.first; });

@@ -99,7 +99,8 @@ struct GProb {
 };
 struct GTask {
   int prob;
-  short ti, tj;
+  int r0, c0;  // first row and column of the tile
+  int shape;   // tile_shape(rows, columns)
 };
 
 constexpr int NBUF = 7;
