@@ -688,15 +688,22 @@ int build_programs(qd_layout* L) {
       b.seg(BB, L->o_fpp, mp, N_, P_FPP, BA, L->o_fph, mp, N_, P_FPH, mp, -1.0);
     }
   }
-  // ---- construct_cc_ints as Z = XCC - YCC = hB P - hA P^T, P = X_A X_B^T ----
+  // ---- construct_cc_ints: Z = XCC - YCC = hB P - hA P^T, P = X_A X_B^T ----
+  // The re-coupling adds Z of block q at [(u,x),(y,v)] to Z of the opposite
+  // block qr at [(v,y),(x,u)], the reversed pairs.  With qr's rows in q's order
+  // that sum is W + s W^T, W = hB X_A X_B^T of q - hA X_A X_B^T of qr: one
+  // problem of q's size with both blocks' columns as its K, half the outputs
+  // and half the reads of the re-coupling.  In the block of no transfer both
+  // sit in the same block in different order: Z itself is stored.
   {
     GemmProgram& P = L->prog_pandya;
     Builder b(P);
     for (int q = 0; q < L->ncc; ++q) {
-      const int r = L->ccdim[q].x, nb = L->ccdim[q].y;
-      if (r == 0) continue;
+      const int r = L->ccdim[q].x, nb = L->ccdim[q].y, qr = L->ncc - 1 - q;
+      if (r == 0 || q < qr) continue;
       b.prob(r, r, L->cczoff[q], r, GM_SET_PAIR, BZ, -1.0, 1, 1);  // nb == 0 writes zeros
       if (nb > 0) b.seg(BXA, L->ccxoff[q], r, N_, -1, BXB, L->ccxoff[q], r, T_, -1, nb, 1.0, 0, 1);
+      if (q > qr) b.seg(BXA, L->ccxoff[qr], r, N_, -1, BXB, L->ccxoff[qr], r, T_, -1, L->ccdim[qr].y, -1.0, 1, 0);
     }
   }
   // upload

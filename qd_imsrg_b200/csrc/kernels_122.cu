@@ -123,10 +123,6 @@ __device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem) : "memory");
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-// wait until at most N committed groups of this thread are still in flight
-template <int N>
-__device__ __forceinline__ void cp_async_wait_group() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
 // q = a / b and r = a % b for 0 <= a < 2^22 - 1 and b >= 1, through one
 // single-precision reciprocal instead of an integer division: the exact value
@@ -1147,58 +1143,57 @@ __global__ void __launch_bounds__(GL_T, 2) k_gen_ladder(DevLayout L, const int4*
 //   1  (g', h)       (g, h')          (l1,k2; k1,l2)
 //   2  (h', h)       (g, g')          (l2,k2; k1,l1)
 //   3  (h', g)       (h, g')          (l2,k1; k2,l1)
+// Terms 0 and 2, and 1 and 3, lie in blocks of opposite transfer, whose sum
+// prog_pandya stores in the upper one: a tile reads the terms whose block is
+// the upper of its pair (two of the four, more where a transfer is zero).
 // Modes (per launch bucket, by the tile's size):
-//   PD_ALL4   the four sub-matrices staged at once (one wait), one pass over
-//             the stored cells adds the four elements into C;
-//   PD_PAIRS  two buffers: terms 0,1 in flight, then term t+2 is copied
-//             while term t is added into a shared accumulator per cell;
-//   PD_SINGLE one buffer and the accumulator, the terms one after another;
-//   PD_DIRECT no staging: each cell reads its four elements from global
-//             memory (tiles too large for the others).
-// Every cell adds the four terms in the order 0, 1, 2, 3 in all modes.
+//   PD_ALL    the sub-matrices of all its terms staged at once (one wait), one
+//             pass over the stored cells adds their elements into C;
+//   PD_SINGLE one buffer and an accumulator, the terms one after another;
+//   PD_DIRECT no staging: each cell reads its elements from global memory.
+// Every cell adds its terms in the order of t in all modes.  Bound: HBM and
+// L2 traffic of Z and C.
 constexpr int TPD = 256;
-enum { PD_DIRECT = 0, PD_ALL4 = 1, PD_PAIRS = 2, PD_SINGLE = 3 };
+enum { PD_DIRECT = 0, PD_ALL = 1, PD_SINGLE = 2 };
+constexpr size_t PD_SMEM = SMEM_MAX_122 - 1024;  // beside the term list
 
-struct PdTerm {  // geometry of one term's sub-matrix
+// One term's sub-matrix, and the position of a cell's element in it: row =
+// sk k + sl l over the term's row states, column likewise.
+struct PdTerm {
   const double* zb;  // element (0, 0)
-  i64 ldz;           // leading dimension of the cc block
-  int nrow, ncol, m2, m4;
+  int ldz;           // leading dimension of the cc block
+  int nrow, ncol;
+  int r[4], c[4];    // row and column strides of k1, k2, l1, l2
+  double sgn;
 };
 
-__device__ __forceinline__ PdTerm pd_term(int t, const DevLayout& L, const int2* __restrict__ zrow, int ng,
-                                          const double* __restrict__ Z, int2 gb, int2 gk, int n1, int n2, int n3,
-                                          int n4) {
-  int G1, G2, G3, G4, m1, m3;
-  PdTerm d;
-  if (t == 0) {
-    G1 = gk.x; G2 = gb.x; G3 = gb.y; G4 = gk.y; m1 = n3; d.m2 = n1; m3 = n2; d.m4 = n4;
-  } else if (t == 1) {
-    G1 = gk.x; G2 = gb.y; G3 = gb.x; G4 = gk.y; m1 = n3; d.m2 = n2; m3 = n1; d.m4 = n4;
-  } else if (t == 2) {
-    G1 = gk.y; G2 = gb.y; G3 = gb.x; G4 = gk.x; m1 = n4; d.m2 = n2; m3 = n1; d.m4 = n3;
-  } else {
-    G1 = gk.y; G2 = gb.x; G3 = gb.y; G4 = gk.x; m1 = n4; d.m2 = n1; m3 = n2; d.m4 = n3;
+// Terms of a tile into d (at most four), in the order of t.
+__device__ __forceinline__ int pd_terms(const DevLayout& L, const int2* __restrict__ zrow, int ng,
+                                        const double* __restrict__ Z, int2 gb, int2 gk, int n1, int n2, int n3, int n4,
+                                        PdTerm* d) {
+  int nt = 0;
+  for (int t = 0; t < 4; ++t) {
+    const bool lo = t < 2, same = t == 0 || t == 3;  // rows by l1 or l2; by k1 or k2
+    const int G1 = lo ? gk.x : gk.y, G2 = same ? gb.x : gb.y, G3 = same ? gb.y : gb.x, G4 = lo ? gk.y : gk.x;
+    const int2 zr = __ldg(&zrow[G1 * ng + G2]);
+    if (zr.x < L.ncc - 1 - zr.x) continue;  // summed into the opposite block
+    const int m2 = same ? n1 : n2, m3 = same ? n2 : n1, m1 = lo ? n3 : n4, m4 = lo ? n4 : n3;
+    PdTerm& p = d[nt++];
+    p.ldz = __ldg(&L.ccdim[zr.x]).x;
+    p.zb = Z + __ldg(&L.cczoff[zr.x]) + zr.y + (i64)__ldg(&zrow[G3 * ng + G4]).y * p.ldz;
+    p.nrow = m1 * m2;
+    p.ncol = m3 * m4;
+    p.r[0] = same ? 1 : 0;
+    p.r[1] = same ? 0 : 1;
+    p.r[2] = lo ? m2 : 0;
+    p.r[3] = lo ? 0 : m2;
+    p.c[0] = same ? 0 : m4;
+    p.c[1] = same ? m4 : 0;
+    p.c[2] = lo ? 0 : 1;
+    p.c[3] = lo ? 1 : 0;
+    p.sgn = t & 1 ? -1.0 : 1.0;
   }
-  const int2 zr = __ldg(&zrow[G1 * ng + G2]);
-  const int cs = __ldg(&zrow[G3 * ng + G4]).y;
-  d.ldz = __ldg(&L.ccdim[zr.x]).x;
-  d.zb = Z + __ldg(&L.cczoff[zr.x]) + zr.y + (i64)cs * d.ldz;
-  d.nrow = m1 * d.m2;
-  d.ncol = m3 * d.m4;
-  return d;
-}
-
-// (row, column) of the cell's element in term t's sub-matrix
-__device__ __forceinline__ int2 pd_rc(int t, const PdTerm& d, int k1, int k2, int l1, int l2) {
-  if (t == 0) return make_int2(l1 * d.m2 + k1, k2 * d.m4 + l2);
-  if (t == 1) return make_int2(l1 * d.m2 + k2, k1 * d.m4 + l2);
-  if (t == 2) return make_int2(l2 * d.m2 + k2, k1 * d.m4 + l1);
-  return make_int2(l2 * d.m2 + k1, k2 * d.m4 + l1);
-}
-// its position in the staged copy (column-major, nrow rows)
-__device__ __forceinline__ int pd_index(int t, const PdTerm& d, int k1, int k2, int l1, int l2) {
-  const int2 ij = pd_rc(t, d, k1, k2, l1, l2);
-  return ij.x + ij.y * d.nrow;
+  return nt;
 }
 
 // copy term d's sub-matrix into dst (runs of nrow doubles, coalesced)
@@ -1224,57 +1219,44 @@ __global__ void __launch_bounds__(TPD) k_pandya_tile(DevLayout L, const int* __r
                                                      const int2* __restrict__ zrow, int ng,
                                                      const double* __restrict__ Z, double* __restrict__ C) {
   extern __shared__ __align__(16) double smp[];
+  __shared__ PdTerm d[4];
+  __shared__ int snt;
   const int2 tl = __ldg(&tiles[__ldg(&tasks[blockIdx.x])]);
   const GpDesc da = load_gp(gpd, tl.x), db = load_gp(gpd, tl.y);
-  const int2 gb = __ldg(&gpg[tl.x]), gk = __ldg(&gpg[tl.y]);  // (g, h), (g', h')
   const int n1 = da.n1, n2 = da.n2, n3 = db.n1, n4 = db.n2;
   const int cells = n1 * n2 * n3 * n4;
   const int pa = da.cnt(0) + da.cnt(1) + da.cnt(2), pb = db.cnt(0) + db.cnt(1) + db.cnt(2);
   const int q = da.q;
   const int4 bd = __ldg(&L.blk[q]);
   const i64* boff = L.boff + 6 * q;
+  const int tid = threadIdx.x;
+  if (tid == 0) snt = pd_terms(L, zrow, ng, Z, __ldg(&gpg[tl.x]), __ldg(&gpg[tl.y]), n1, n2, n3, n4, d);
+  __syncthreads();
+  const int nt = snt;
   int nst = 0;  // stored cells: regions c1 >= c2
 #pragma unroll 1
   for (int c1 = 0; c1 < 3; ++c1)
     for (int c2 = 0; c2 <= c1; ++c2) nst += da.cnt(c1) * db.cnt(c2);
   // shared memory: sub-matrix buffers | accumulator | row, column pairs
-  constexpr int NBUF = MODE == PD_ALL4 ? 4 : (MODE == PD_PAIRS ? 2 : (MODE == PD_SINGLE ? 1 : 0));
-  constexpr bool ACCUM = MODE == PD_PAIRS || MODE == PD_SINGLE;
   double* Zs = smp;
-  double* Y = smp + NBUF * cells;
-  int2* pr = reinterpret_cast<int2*>(Y + (ACCUM ? nst : 0));
+  double* Y = smp + (MODE == PD_ALL ? nt * cells : (MODE == PD_SINGLE ? cells : 0));
+  int2* pr = reinterpret_cast<int2*>(Y + (MODE == PD_SINGLE ? nst : 0));
   int2* pc = pr + pa;
-  const int tid = threadIdx.x;
   for (int i = tid; i < pa; i += TPD) pr[i] = __ldg(&gpp[da.pstart + i]);
   for (int i = tid; i < pb; i += TPD) pc[i] = __ldg(&gpp[db.pstart + i]);
-  PdTerm d[4];
-#pragma unroll
-  for (int t = 0; t < 4; ++t) d[t] = pd_term(t, L, zrow, ng, Z, gb, gk, n1, n2, n3, n4);
-  if (MODE == PD_ALL4) {
-#pragma unroll
-    for (int t = 0; t < 4; ++t) pd_stage(d[t], Zs + t * cells, tid);
-    cp_async_wait_all();
-  } else if (MODE == PD_PAIRS) {
-    pd_stage(d[0], Zs, tid);
-    cp_async_commit();
-    pd_stage(d[1], Zs + cells, tid);
-    cp_async_commit();
-    cp_async_wait_group<1>();
-  } else if (MODE == PD_SINGLE) {
-    pd_stage(d[0], Zs, tid);
-    cp_async_wait_all();
-  }
-  __syncthreads();
-
-  // passes over the stored cells: ALL4 and DIRECT one (all terms), PAIRS and
-  // SINGLE one per term
-  constexpr int NPASS = ACCUM ? 4 : 1;
+  const int npass = MODE == PD_SINGLE ? nt : 1;
 #pragma unroll 1
-  for (int pass = 0; pass < NPASS; ++pass) {
-    const double* buf = Zs + (MODE == PD_PAIRS ? (pass & 1) * cells : 0);
-    // this pass's term geometry (recomputed: an array indexed by the pass
-    // would live in local memory)
-    const PdTerm dp = ACCUM ? pd_term(pass, L, zrow, ng, Z, gb, gk, n1, n2, n3, n4) : d[0];
+  for (int pass = 0; pass < npass; ++pass) {
+    if (MODE == PD_SINGLE) {
+      if (pass > 0) __syncthreads();  // the buffer is free again
+      pd_stage(d[pass], Zs, tid);
+      cp_async_wait_all();
+    } else if (MODE == PD_ALL) {
+#pragma unroll 1
+      for (int t = 0; t < nt; ++t) pd_stage(d[t], Zs + t * cells, tid);
+      cp_async_wait_all();
+    }
+    __syncthreads();
     int j0 = 0;  // first accumulator slot of the region
 #pragma unroll 1
     for (int rg = 0; rg < 6; ++rg) {
@@ -1286,6 +1268,7 @@ __global__ void __launch_bounds__(TPD) k_pandya_tile(DevLayout L, const int* __r
       const i64 ldc = cnt_of(c1, bd);
       const int2 i0 = divmod_small(tid, r1), di = divmod_small(TPD, r1);
       int p = i0.y, u = i0.x;
+#pragma unroll 2
       for (int e = tid; e < r1 * r2; e += TPD) {
         const int2 P = pr[o1 + p], Q = pc[o2 + u];
         p += di.y;
@@ -1294,51 +1277,29 @@ __global__ void __launch_bounds__(TPD) k_pandya_tile(DevLayout L, const int* __r
           p -= r1;
           ++u;
         }
+        double* out = C + base + P.x + (i64)Q.x * ldc;
+        const bool last = MODE != PD_SINGLE || pass == npass - 1;
+        const double old = last ? *out : 0.0;
         const int k1 = (P.y >> 17) & 15, k2 = (P.y >> 21) & 15;
         const int l1 = (Q.y >> 17) & 15, l2 = (Q.y >> 21) & 15;
-        double y;
-        bool last = true;
-        if (MODE == PD_ALL4) {
-          y = Zs[pd_index(0, d[0], k1, k2, l1, l2)];
-          y -= Zs[cells + pd_index(1, d[1], k1, k2, l1, l2)];
-          y += Zs[2 * cells + pd_index(2, d[2], k1, k2, l1, l2)];
-          y -= Zs[3 * cells + pd_index(3, d[3], k1, k2, l1, l2)];
-        } else if (MODE == PD_DIRECT) {
-          double z[4];
-#pragma unroll
-          for (int t = 0; t < 4; ++t) {
-            const int2 ij = pd_rc(t, d[t], k1, k2, l1, l2);
-            z[t] = __ldg(d[t].zb + ij.x + (i64)ij.y * d[t].ldz);
-          }
-          y = z[0] - z[1] + z[2] - z[3];
-        } else {
-          const double z = buf[pd_index(pass, dp, k1, k2, l1, l2)];
-          y = (pass == 0 ? 0.0 : Y[j0 + e]) + ((pass & 1) ? -z : z);
-          last = pass == 3;
-          if (!last) Y[j0 + e] = y;
+        double y = MODE == PD_SINGLE && pass > 0 ? Y[j0 + e] : 0.0;
+#pragma unroll 1
+        for (int t = MODE == PD_SINGLE ? pass : 0; t < (MODE == PD_SINGLE ? pass + 1 : nt); ++t) {
+          const PdTerm& D = d[t];
+          const int row = k1 * D.r[0] + k2 * D.r[1] + l1 * D.r[2] + l2 * D.r[3];
+          const int col = k1 * D.c[0] + k2 * D.c[1] + l1 * D.c[2] + l2 * D.c[3];
+          const double z = MODE == PD_DIRECT ? __ldg(D.zb + row + (i64)col * D.ldz)
+                                             : Zs[(MODE == PD_ALL ? t * cells : 0) + row + col * D.nrow];
+          y += D.sgn * z;
         }
-        if (last) {
+        if (!last) {
+          Y[j0 + e] = y;
+        } else {
           if ((P.y ^ Q.y) & (1 << 16)) y = -y;
-          C[base + P.x + (i64)Q.x * ldc] += y;
+          *out = old + y;
         }
       }
       j0 += r1 * r2;
-    }
-    if (MODE == PD_PAIRS && pass < 3) {
-      __syncthreads();  // buffer (pass & 1) is free again
-      if (pass < 2) {   // term pass + 2 into it, while term pass + 1 lands
-        pd_stage(pd_term(pass + 2, L, zrow, ng, Z, gb, gk, n1, n2, n3, n4), Zs + (pass & 1) * cells, tid);
-        cp_async_commit();
-        cp_async_wait_group<1>();
-      } else {
-        cp_async_wait_group<0>();
-      }
-      __syncthreads();
-    } else if (MODE == PD_SINGLE && pass < 3) {
-      __syncthreads();
-      pd_stage(pd_term(pass + 1, L, zrow, ng, Z, gb, gk, n1, n2, n3, n4), Zs, tid);
-      cp_async_wait_all();
-      __syncthreads();
     }
   }
 }
@@ -1358,7 +1319,7 @@ struct TileInfo {
 struct PdBucket {  // one launch of the particle-hole tile kernel
   int first, count;
   size_t smem;
-  int mode;  // PD_ALL4, PD_PAIRS, PD_SINGLE or PD_DIRECT
+  int mode;  // PD_ALL, PD_SINGLE or PD_DIRECT
 };
 struct Bucket122 {
   int tw;       // doubles per staged cell
@@ -1831,9 +1792,8 @@ static int plan_122(qd_layout* L, Plan122** out) {
     for (int g2 = 0; g2 < ngroup; ++g2)
       zrow[(size_t)g1 * ngroup + g2] = L->ccmap[(size_t)L->gmem[L->gstart[g1]] * m + L->gmem[L->gstart[g2]]];
   {
-    // per tile the first mode that fits: all four terms staged, two buffers
-    // (each while at least three CTAs fit an SM), one buffer, none; buckets
-    // by mode, then by size interval, largest first
+    // per tile the first mode that fits: all its terms staged, one buffer,
+    // none; buckets by mode, then by size interval, largest first
     struct PdT {
       int mode;
       size_t sm;
@@ -1842,14 +1802,17 @@ static int plan_122(qd_layout* L, Plan122** out) {
     std::vector<PdT> lst;
     for (size_t i = 0; i < p.tiles.size(); ++i) {
       const TileInfo& t = p.tiles[i];
+      const int2 gb = gpg[t.a], gk = gpg[t.b];
+      int nt = 0;  // as pd_terms
+      for (int k = 0; k < 4; ++k) {
+        const int q = zrow[(size_t)(k < 2 ? gk.x : gk.y) * ngroup + (k == 0 || k == 3 ? gb.x : gb.y)].x;
+        nt += q >= L->ncc - 1 - q;
+      }
       const size_t c = (size_t)t.cells, ns = (size_t)t.nst, np = (size_t)t.npair;
-      const size_t s4 = 8 * (4 * c + np), s2 = 8 * (2 * c + ns + np), s1 = 8 * (c + ns + np);
-      const size_t third = SMEM_MAX_122 / 3;
-      if (s4 <= third)
-        lst.push_back({PD_ALL4, s4, (int)i});
-      else if (s2 <= third)
-        lst.push_back({PD_PAIRS, s2, (int)i});
-      else if (s1 <= SMEM_MAX_122)
+      const size_t sa = 8 * (nt * c + np), s1 = 8 * (c + ns + np);
+      if (sa <= PD_SMEM)
+        lst.push_back({PD_ALL, sa, (int)i});
+      else if (s1 <= PD_SMEM)
         lst.push_back({PD_SINGLE, s1, (int)i});
       else
         lst.push_back({PD_DIRECT, 8 * np, (int)i});
@@ -1882,7 +1845,7 @@ static int plan_122(qd_layout* L, Plan122** out) {
   for (const void* fn : {(const void*)k_122_tile<1, 64>, (const void*)k_122_tile<2, 64>,
                          (const void*)k_122_tile<1, 128>, (const void*)k_122_tile<2, 128>,
                          (const void*)k_122_tile<1, 256>, (const void*)k_122_tile<2, 256>,
-                         (const void*)k_pandya_tile<PD_ALL4>, (const void*)k_pandya_tile<PD_PAIRS>,
+                         (const void*)k_pandya_tile<PD_ALL>,
                          (const void*)k_pandya_tile<PD_SINGLE>, (const void*)k_pandya_tile<PD_DIRECT>,
                          (const void*)k_gen_pppp<false>, (const void*)k_gen_pppp<true>, (const void*)k_122_gen, (const void*)k_gen_phph}) {
     cudaFuncAttributes fa;
@@ -2291,8 +2254,7 @@ int launch_pandya_tiles(qd_layout* L, const double* Z, double* C) {
   k_pandya_tile<M><<<b.count, TPD, b.smem, L->stream>>>(L->dev, p->d_ptask + b.first, p->d_tiles, p->d_gpd, \
                                                         p->d_gpp, p->d_gpg, p->d_zrow, p->ng, Z, C)
     switch (b.mode) {
-      case PD_ALL4: QD_PD_LAUNCH(PD_ALL4); break;
-      case PD_PAIRS: QD_PD_LAUNCH(PD_PAIRS); break;
+      case PD_ALL: QD_PD_LAUNCH(PD_ALL); break;
       case PD_SINGLE: QD_PD_LAUNCH(PD_SINGLE); break;
       default: QD_PD_LAUNCH(PD_DIRECT); break;
     }

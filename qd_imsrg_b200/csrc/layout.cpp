@@ -184,43 +184,48 @@ int layout_build(qd_layout* L, int nbody, int emax, const double* eig) {
   L->cchp_base.assign(L->ncc + 1, 0);
   L->ccxoff.assign(L->ncc, 0);
   L->cczoff.assign(L->ncc, 0);
-  int cq = 0;
+  // Blocks of opposite transfer, q and ncc - 1 - q, hold the reversed pairs of
+  // one another.  The rows of the lower one follow the upper one's, reversed,
+  // so that the particle-hole channel can add both blocks' products in one
+  // GEMM (see prog_pandya); only q >= ncc - 1 - q has product storage.
+  std::vector<std::vector<int>> ref(L->ncc);  // pairs i * m + j of each block, in (i, j) loop order
+  auto block_of = [&](int i, int j) {
+    return (L->qn[3 * i + 1] - L->qn[3 * j + 1] + L->mlmax) * 5 + (L->qn[3 * i + 2] - L->qn[3 * j + 2] + 2);
+  };
+  for (int i = 0; i < m; ++i)
+    for (int j = 0; j < m; ++j) ref[block_of(i, j)].push_back(i * m + j);
+  std::vector<int> refpos((size_t)m * m, -1);
+  std::vector<std::vector<int2>> rowsof(L->ncc);
+  for (int q = 0; q < L->ncc; ++q)
+    for (size_t t = 0; t < ref[q].size(); ++t) refpos[ref[q][t]] = (int)t;
+  for (size_t g = 0; g < keys.size(); ++g)
+    for (int i : mem[g])
+      for (int j = 0; j < m; ++j) rowsof[block_of(i, j)].push_back(int2{i, j});
+  for (int q = 0; q < L->ncc - 1 - q; ++q) {
+    rowsof[q].clear();
+    for (const int2& p : rowsof[L->ncc - 1 - q]) rowsof[q].push_back(int2{p.y, p.x});
+  }
   i64 xo = 0, zo = 0;
-  for (int ML = -L->mlmax; ML <= L->mlmax; ++ML)
-    for (int MS = -2; MS <= 2; ++MS, ++cq) {
-      L->ccab_base[cq] = (int)L->ccab.size();
-      L->cchp_base[cq] = (int)L->cchp.size();
-      int r = 0, nb = 0;
-      // reference row of (i, j): position in the (i, j) loop order
-      std::vector<int> refrow;
-      for (int i = 0; i < m; ++i)
-        for (int j = 0; j < m; ++j) {
-          if (L->qn[3 * i + 1] - L->qn[3 * j + 1] != ML) continue;
-          if (L->qn[3 * i + 2] - L->qn[3 * j + 2] != MS) continue;
-          refrow.push_back(i * m + j);
-          if (i < n && j >= n) {
-            L->cchp.push_back(int2{i, j});
-            ++nb;
-          }
-        }
-      std::vector<int> refpos((size_t)m * m, -1);
-      for (size_t t = 0; t < refrow.size(); ++t) refpos[refrow[t]] = (int)t;
-      for (size_t g = 0; g < keys.size(); ++g)
-        for (int i : mem[g])
-          for (int j = 0; j < m; ++j) {
-            if (L->qn[3 * i + 1] - L->qn[3 * j + 1] != ML) continue;
-            if (L->qn[3 * i + 2] - L->qn[3 * j + 2] != MS) continue;
-            L->ccmap[(size_t)i * m + j] = int2{cq, r};
-            L->ccab.push_back(int2{i, j});
-            L->ccref.push_back(refpos[(size_t)i * m + j]);
-            ++r;
-          }
-      L->ccdim[cq] = int2{r, nb};
-      L->ccxoff[cq] = xo;
-      L->cczoff[cq] = zo;
-      xo += (i64)r * nb;
-      zo += (i64)r * r;
+  for (int cq = 0; cq < L->ncc; ++cq) {
+    L->ccab_base[cq] = (int)L->ccab.size();
+    L->cchp_base[cq] = (int)L->cchp.size();
+    int r = 0, nb = 0;
+    for (int e : ref[cq])
+      if (e / m < n && e % m >= n) {
+        L->cchp.push_back(int2{e / m, e % m});
+        ++nb;
+      }
+    for (const int2& p : rowsof[cq]) {
+      L->ccmap[(size_t)p.x * m + p.y] = int2{cq, r++};
+      L->ccab.push_back(p);
+      L->ccref.push_back(refpos[(size_t)p.x * m + p.y]);
     }
+    L->ccdim[cq] = int2{r, nb};
+    L->ccxoff[cq] = xo;
+    L->cczoff[cq] = zo;
+    xo += (i64)r * nb;
+    if (cq >= L->ncc - 1 - cq) zo += (i64)r * r;
+  }
   L->ccab_base[L->ncc] = (int)L->ccab.size();
   L->cchp_base[L->ncc] = (int)L->cchp.size();
   L->xsize = xo;

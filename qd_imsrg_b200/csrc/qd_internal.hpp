@@ -63,7 +63,7 @@ struct DevLayout {
   const int2* ccmap;      // m*m: (cc block, row), 0-based
   const int2* ccdim;      // r, nb per cc block
   const i64* ccxoff;      // offset of X(r,nb) per cc block
-  const i64* cczoff;      // offset of the r x r product per cc block
+  const i64* cczoff;      // offset of the r x r product per cc block q >= ncc - 1 - q
   const int2* ccab;       // concatenated (i,j) row pairs of the cc blocks
   const int* ccab_base;
   const int2* cchp;       // concatenated (hole, particle) column pairs
@@ -152,7 +152,8 @@ struct qd_layout {
   std::vector<int2> ccmap, ccdim, ccab, cchp;
   std::vector<int> ccab_base, cchp_base;
   // Rows of a cc block are ordered by the (ml,ms) group of their first state,
-  // then (i, j): the rows (i in G1, j in G2) form one run.  ccref maps each
+  // then (i, j): the rows (i in G1, j in G2) form one run; below the block of
+  // no transfer, as the reversed pairs of the opposite block.  ccref maps each
   // row (indexed like ccab) to its row in the reference's (i, j) loop order.
   std::vector<int> ccref;
   std::vector<qd::i64> ccxoff, cczoff;
