@@ -1153,9 +1153,9 @@ __global__ void __launch_bounds__(GL_T, 2) k_gen_ladder(DevLayout L, const int4*
 //   PD_DIRECT no staging: each cell reads its elements from global memory.
 // Every cell adds its terms in the order of t in all modes.  Bound: HBM and
 // L2 traffic of Z and C.
-constexpr int TPD = 256;
 enum { PD_DIRECT = 0, PD_ALL = 1, PD_SINGLE = 2 };
 constexpr size_t PD_SMEM = SMEM_MAX_122 - 1024;  // beside the term list
+constexpr size_t PD_SMALL = 6 * 1024, PD_MEDIUM = 20 * 1024;
 
 // One term's sub-matrix, and the position of a cell's element in it: row =
 // sk k + sl l over the term's row states, column likewise.
@@ -1167,41 +1167,44 @@ struct PdTerm {
   double sgn;
 };
 
-// Terms of a tile into d (at most four), in the order of t.
-__device__ __forceinline__ int pd_terms(const DevLayout& L, const int2* __restrict__ zrow, int ng,
-                                        const double* __restrict__ Z, int2 gb, int2 gk, int n1, int n2, int n3, int n4,
-                                        PdTerm* d) {
-  int nt = 0;
-  for (int t = 0; t < 4; ++t) {
-    const bool lo = t < 2, same = t == 0 || t == 3;  // rows by l1 or l2; by k1 or k2
-    const int G1 = lo ? gk.x : gk.y, G2 = same ? gb.x : gb.y, G3 = same ? gb.y : gb.x, G4 = lo ? gk.y : gk.x;
-    const int2 zr = __ldg(&zrow[G1 * ng + G2]);
-    if (zr.x < L.ncc - 1 - zr.x) continue;  // summed into the opposite block
-    const int m2 = same ? n1 : n2, m3 = same ? n2 : n1, m1 = lo ? n3 : n4, m4 = lo ? n4 : n3;
-    PdTerm& p = d[nt++];
-    p.ldz = __ldg(&L.ccdim[zr.x]).x;
-    p.zb = Z + __ldg(&L.cczoff[zr.x]) + zr.y + (i64)__ldg(&zrow[G3 * ng + G4]).y * p.ldz;
-    p.nrow = m1 * m2;
-    p.ncol = m3 * m4;
-    p.r[0] = same ? 1 : 0;
-    p.r[1] = same ? 0 : 1;
-    p.r[2] = lo ? m2 : 0;
-    p.r[3] = lo ? 0 : m2;
-    p.c[0] = same ? 0 : m4;
-    p.c[1] = same ? m4 : 0;
-    p.c[2] = lo ? 0 : 1;
-    p.c[3] = lo ? 1 : 0;
-    p.sgn = t & 1 ? -1.0 : 1.0;
-  }
-  return nt;
+// The tile's terms into d (at most four, in the order of t), by lanes 0 to 3
+// of the first warp.
+__device__ __forceinline__ void pd_terms(const DevLayout& L, const int2* __restrict__ zrow, int ng,
+                                         const double* __restrict__ Z, int2 gb, int2 gk, int n1, int n2, int n3, int n4,
+                                         PdTerm* d, int* nt) {
+  const int t = threadIdx.x & 3;
+  const bool lo = t < 2, same = t == 0 || t == 3;  // rows by l1 or l2; by k1 or k2
+  const int G1 = lo ? gk.x : gk.y, G2 = same ? gb.x : gb.y, G3 = same ? gb.y : gb.x, G4 = lo ? gk.y : gk.x;
+  const int2 zr = __ldg(&zrow[G1 * ng + G2]);
+  const int zc = __ldg(&zrow[G3 * ng + G4]).y;
+  const bool on = zr.x >= L.ncc - 1 - zr.x;  // else summed into the opposite block
+  const unsigned act = __ballot_sync(0xffffffffu, on && threadIdx.x < 4);
+  if (threadIdx.x == 0) *nt = __popc(act);
+  if (!on || threadIdx.x >= 4) return;
+  const int m2 = same ? n1 : n2, m3 = same ? n2 : n1, m1 = lo ? n3 : n4, m4 = lo ? n4 : n3;
+  PdTerm& p = d[__popc(act & ((1u << t) - 1))];
+  p.ldz = __ldg(&L.ccdim[zr.x]).x;
+  p.zb = Z + __ldg(&L.cczoff[zr.x]) + zr.y + (i64)zc * p.ldz;
+  p.nrow = m1 * m2;
+  p.ncol = m3 * m4;
+  p.r[0] = same ? 1 : 0;
+  p.r[1] = same ? 0 : 1;
+  p.r[2] = lo ? m2 : 0;
+  p.r[3] = lo ? 0 : m2;
+  p.c[0] = same ? 0 : m4;
+  p.c[1] = same ? m4 : 0;
+  p.c[2] = lo ? 0 : 1;
+  p.c[3] = lo ? 1 : 0;
+  p.sgn = t & 1 ? -1.0 : 1.0;
 }
 
 // copy term d's sub-matrix into dst (runs of nrow doubles, coalesced)
+template <int T>
 __device__ __forceinline__ void pd_stage(const PdTerm& d, double* dst, int tid) {
   const int total = d.nrow * d.ncol;
-  const int2 i0 = divmod_small(tid, d.nrow), di = divmod_small(TPD, d.nrow);
+  const int2 i0 = divmod_small(tid, d.nrow), di = divmod_small(T, d.nrow);
   int fr = i0.y, fc = i0.x;
-  for (int e = tid; e < total; e += TPD) {
+  for (int e = tid; e < total; e += T) {
     cp_async8(&dst[e], d.zb + fr + (i64)fc * d.ldz);
     fr += di.y;
     fc += di.x;
@@ -1212,8 +1215,8 @@ __device__ __forceinline__ void pd_stage(const PdTerm& d, double* dst, int tid) 
   }
 }
 
-template <int MODE>
-__global__ void __launch_bounds__(TPD) k_pandya_tile(DevLayout L, const int* __restrict__ tasks,
+template <int MODE, int T>
+__global__ void __launch_bounds__(T) k_pandya_tile(DevLayout L, const int* __restrict__ tasks,
                                                      const int2* __restrict__ tiles, const int4* __restrict__ gpd,
                                                      const int2* __restrict__ gpp, const int2* __restrict__ gpg,
                                                      const int2* __restrict__ zrow, int ng,
@@ -1230,7 +1233,7 @@ __global__ void __launch_bounds__(TPD) k_pandya_tile(DevLayout L, const int* __r
   const int4 bd = __ldg(&L.blk[q]);
   const i64* boff = L.boff + 6 * q;
   const int tid = threadIdx.x;
-  if (tid == 0) snt = pd_terms(L, zrow, ng, Z, __ldg(&gpg[tl.x]), __ldg(&gpg[tl.y]), n1, n2, n3, n4, d);
+  if (tid < 32) pd_terms(L, zrow, ng, Z, __ldg(&gpg[tl.x]), __ldg(&gpg[tl.y]), n1, n2, n3, n4, d, &snt);
   __syncthreads();
   const int nt = snt;
   int nst = 0;  // stored cells: regions c1 >= c2
@@ -1242,18 +1245,18 @@ __global__ void __launch_bounds__(TPD) k_pandya_tile(DevLayout L, const int* __r
   double* Y = smp + (MODE == PD_ALL ? nt * cells : (MODE == PD_SINGLE ? cells : 0));
   int2* pr = reinterpret_cast<int2*>(Y + (MODE == PD_SINGLE ? nst : 0));
   int2* pc = pr + pa;
-  for (int i = tid; i < pa; i += TPD) pr[i] = __ldg(&gpp[da.pstart + i]);
-  for (int i = tid; i < pb; i += TPD) pc[i] = __ldg(&gpp[db.pstart + i]);
+  for (int i = tid; i < pa; i += T) pr[i] = __ldg(&gpp[da.pstart + i]);
+  for (int i = tid; i < pb; i += T) pc[i] = __ldg(&gpp[db.pstart + i]);
   const int npass = MODE == PD_SINGLE ? nt : 1;
 #pragma unroll 1
   for (int pass = 0; pass < npass; ++pass) {
     if (MODE == PD_SINGLE) {
       if (pass > 0) __syncthreads();  // the buffer is free again
-      pd_stage(d[pass], Zs, tid);
+      pd_stage<T>(d[pass], Zs, tid);
       cp_async_wait_all();
     } else if (MODE == PD_ALL) {
 #pragma unroll 1
-      for (int t = 0; t < nt; ++t) pd_stage(d[t], Zs + t * cells, tid);
+      for (int t = 0; t < nt; ++t) pd_stage<T>(d[t], Zs + t * cells, tid);
       cp_async_wait_all();
     }
     __syncthreads();
@@ -1266,10 +1269,10 @@ __global__ void __launch_bounds__(TPD) k_pandya_tile(DevLayout L, const int* __r
       const int o1 = da.off(c1), o2 = db.off(c2);
       const i64 base = __ldg(boff + slot_of(c1, c2));
       const i64 ldc = cnt_of(c1, bd);
-      const int2 i0 = divmod_small(tid, r1), di = divmod_small(TPD, r1);
+      const int2 i0 = divmod_small(tid, r1), di = divmod_small(T, r1);
       int p = i0.y, u = i0.x;
 #pragma unroll 2
-      for (int e = tid; e < r1 * r2; e += TPD) {
+      for (int e = tid; e < r1 * r2; e += T) {
         const int2 P = pr[o1 + p], Q = pc[o2 + u];
         p += di.y;
         u += di.x;
@@ -1817,10 +1820,10 @@ static int plan_122(qd_layout* L, Plan122** out) {
       else
         lst.push_back({PD_DIRECT, 8 * np, (int)i});
     }
-    const size_t bounds[4] = {24 * 1024, 56 * 1024, 112 * 1024, SMEM_MAX_122};
+    const size_t bounds[5] = {PD_SMALL, PD_MEDIUM, 48 * 1024, 112 * 1024, SMEM_MAX_122};
     auto interval = [&](size_t sm) {
       int l = 0;
-      while (l < 3 && sm > bounds[l]) ++l;
+      while (l < 4 && sm > bounds[l]) ++l;
       return l;
     };
     std::stable_sort(lst.begin(), lst.end(), [&](const PdT& x, const PdT& y) {
@@ -1845,8 +1848,9 @@ static int plan_122(qd_layout* L, Plan122** out) {
   for (const void* fn : {(const void*)k_122_tile<1, 64>, (const void*)k_122_tile<2, 64>,
                          (const void*)k_122_tile<1, 128>, (const void*)k_122_tile<2, 128>,
                          (const void*)k_122_tile<1, 256>, (const void*)k_122_tile<2, 256>,
-                         (const void*)k_pandya_tile<PD_ALL>,
-                         (const void*)k_pandya_tile<PD_SINGLE>, (const void*)k_pandya_tile<PD_DIRECT>,
+                         (const void*)k_pandya_tile<PD_ALL, 64>, (const void*)k_pandya_tile<PD_ALL, 128>,
+                         (const void*)k_pandya_tile<PD_ALL, 256>,
+                         (const void*)k_pandya_tile<PD_SINGLE, 256>, (const void*)k_pandya_tile<PD_DIRECT, 256>,
                          (const void*)k_gen_pppp<false>, (const void*)k_gen_pppp<true>, (const void*)k_122_gen, (const void*)k_gen_phph}) {
     cudaFuncAttributes fa;
     QD_CUDA(cudaFuncGetAttributes(&fa, fn));
@@ -2250,14 +2254,20 @@ int launch_pandya_tiles(qd_layout* L, const double* Z, double* C) {
   if (rc) return rc;
   for (const PdBucket& b : p->pbuckets) {
     if (b.count == 0) continue;
-#define QD_PD_LAUNCH(M)                                                                                       \
-  k_pandya_tile<M><<<b.count, TPD, b.smem, L->stream>>>(L->dev, p->d_ptask + b.first, p->d_tiles, p->d_gpd, \
-                                                        p->d_gpp, p->d_gpg, p->d_zrow, p->ng, Z, C)
-    switch (b.mode) {
-      case PD_ALL: QD_PD_LAUNCH(PD_ALL); break;
-      case PD_SINGLE: QD_PD_LAUNCH(PD_SINGLE); break;
-      default: QD_PD_LAUNCH(PD_DIRECT); break;
-    }
+#define QD_PD_LAUNCH(M, T)                                                                                  \
+  k_pandya_tile<M, T><<<b.count, T, b.smem, L->stream>>>(L->dev, p->d_ptask + b.first, p->d_tiles, p->d_gpd, \
+                                                         p->d_gpp, p->d_gpg, p->d_zrow, p->ng, Z, C)
+    // small tiles: few cells a thread, so the fixed part of a CTA weighs less
+    if (b.mode == PD_SINGLE)
+      QD_PD_LAUNCH(PD_SINGLE, 256);
+    else if (b.mode == PD_DIRECT)
+      QD_PD_LAUNCH(PD_DIRECT, 256);
+    else if (b.smem <= PD_SMALL)
+      QD_PD_LAUNCH(PD_ALL, 64);
+    else if (b.smem <= PD_MEDIUM)
+      QD_PD_LAUNCH(PD_ALL, 128);
+    else
+      QD_PD_LAUNCH(PD_ALL, 256);
 #undef QD_PD_LAUNCH
     ++L->nlaunch;
   }
