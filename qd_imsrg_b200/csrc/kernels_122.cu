@@ -72,6 +72,7 @@ __device__ __forceinline__ int cnt_of(int c, int4 bd) { return c == 0 ? bd.x : (
 //    k1 << 17 | k2 << 21}, the primary cell being (k1, k2) = k1 * n2 + k2
 struct GpDesc {
   int q, n1, n2, hg, hh, fg, fh, pstart, cntw;
+  bool same;  // g == h
   // pairs of class c (0 hh, 1 ph, 2 pp), decoded from the packed word (no local array)
   __device__ __forceinline__ int cnt(int c) const { return (cntw >> (10 * c)) & 0x3FF; }
   // pairs of the classes before c
@@ -83,6 +84,7 @@ __device__ __forceinline__ GpDesc load_gp(const int4* __restrict__ gpd, int u) {
   d.q = a.x;
   d.n1 = a.y & 0xFF;
   d.n2 = (a.y >> 8) & 0xFF;
+  d.same = (a.y >> 16) & 1;
   d.hg = a.z & 0xFF;
   d.hh = (a.z >> 8) & 0xFF;
   d.fg = a.w;
@@ -156,23 +158,16 @@ __host__ __device__ __forceinline__ bool leg_ok(int sparse, bool k_hole, bool t_
 // particles only, so every leg changes the class of the pair it acts on.
 constexpr unsigned LEG_SPARSE = 1u << 31;
 
-// Stored output regions (c1 >= c2) in the order of the output loop:
-// (0,0) (1,0) (1,1) (2,0) (2,1) (2,2) -> 0..5; bit r of an output mask.
-__host__ __device__ __forceinline__ int out_region(int c1, int c2) { return (c1 * (c1 + 1)) / 2 + c2; }
-constexpr unsigned OUT_ALL = 0x3Fu;
-// none: k_gen_pppp and k_122_gen write every part for a generator-like A
-constexpr unsigned OUT_NONE = 0u;
-
 // Regions (c1 * 3 + c2) of the staged operand that the legs of a tile read
 // when every leg changes the class of its pair by one: the four neighbours of
-// each stored output region (c1 >= c2) of the tile that the launch writes.
+// each stored output region (c1 >= c2) of the tile.
 // All regions otherwise.
-__device__ __forceinline__ unsigned regions_read(unsigned leg, const int ca[3], const int cb[3], unsigned outmask) {
+__device__ __forceinline__ unsigned regions_read(unsigned leg, const int ca[3], const int cb[3]) {
   if (!(leg & LEG_SPARSE)) return 0x1FFu;
   unsigned need = 0;
   for (int c1 = 0; c1 < 3; ++c1)
     for (int c2 = 0; c2 <= c1; ++c2) {
-      if (ca[c1] == 0 || cb[c2] == 0 || !((outmask >> out_region(c1, c2)) & 1u)) continue;
+      if (ca[c1] == 0 || cb[c2] == 0) continue;
       if (c1 > 0) need |= 1u << ((c1 - 1) * 3 + c2);
       if (c1 < 2) need |= 1u << ((c1 + 1) * 3 + c2);
       if (c2 > 0) need |= 1u << (c1 * 3 + c2 - 1);
@@ -205,7 +200,7 @@ __global__ void __launch_bounds__(T122, 1024 / T122) k_122_tile(DevLayout L, con
                                                    const double2* __restrict__ F, int nfent,
                                                    const double* __restrict__ A, double hA, unsigned zA, unsigned legA,
                                                    const double* __restrict__ B, double hB, unsigned zB, unsigned legB,
-                                                   double* __restrict__ C, unsigned outmask) {
+                                                   double* __restrict__ C) {
   extern __shared__ __align__(16) double sm122[];
   const int2 task = tasks[blockIdx.x];
   const int2 tl = __ldg(&tiles[task.x]);
@@ -262,7 +257,7 @@ __global__ void __launch_bounds__(T122, 1024 / T122) k_122_tile(DevLayout L, con
       const double* src = x == 0 ? A : B;
       const unsigned zm = x == 0 ? zA : zB;
       // the A term's legs carry FB (legA), the B term's FA (legB)
-      const unsigned need = regions_read(x == 0 ? legA : legB, ca, cb, outmask);
+      const unsigned need = regions_read(x == 0 ? legA : legB, ca, cb);
       const double hx = x == 0 ? hA : hB;
       const int xo = TW == 2 ? x : 0;
 #pragma unroll 1
@@ -315,7 +310,7 @@ __global__ void __launch_bounds__(T122, 1024 / T122) k_122_tile(DevLayout L, con
   for (int rg = 0; rg < 6; ++rg) {
     const int c1 = rg < 1 ? 0 : (rg < 3 ? 1 : 2), c2 = rg - (c1 * (c1 + 1)) / 2;  // (0,0) (1,0) (1,1) (2,0) (2,1) (2,2)
     const int r1 = da.cnt(c1), r2 = db.cnt(c2);
-    if (r1 == 0 || r2 == 0 || !((outmask >> rg) & 1u)) continue;
+    if (r1 == 0 || r2 == 0) continue;
     const int o1 = da.off(c1), o2 = db.off(c2);
     const i64 base = __ldg(boff + slot_of(c1, c2));
     const i64 ldc = cnt_of(c1, bd);
@@ -365,6 +360,231 @@ __global__ void __launch_bounds__(T122, 1024 / T122) k_122_tile(DevLayout L, con
       else
         *out = y;
     }
+  }
+}
+
+// ---- the same tiles with the legs from registers --------------------------
+// k_122_tile above sums each output cell's legs by itself: two shared-memory
+// reads per product.  k_122_full turns a leg into small matrix products: for
+// a fixed other index a thread loads the leg's n values of T once and forms
+// all n outputs from them, F read as a broadcast shared by the warp, and adds
+// them into a tile Y in shared memory.  Per leg and cell: one read of T, n / 2
+// broadcast reads and n products per operand, one read and write of Y.  Both
+// operands are staged together (24 bytes a cell, five barriers a tile) where
+// at least two such tiles fit an SM, else one after the other in the same
+// space (16 bytes a cell).  Bound: shared-memory bandwidth, the FP64 pipe, and
+// for small tiles the chain of barriers.  Legs known to vanish are not skipped
+// one by one: for an operand whose one-body part couples holes to particles
+// only, large bases keep k_122_tile (see use_full).  Measured on two dense
+// operators (us): N=20 R=20 4380 with k_122_tile, 3060 with this kernel (3290
+// and 3150 with both operands staged up to 30 and 48 KB, 3450 up to 112 KB);
+// N=6 R=10 81 and 71; N=2 R=3 37 and 14.
+// CTA sizes before tuning and launch buckets, by shared memory.
+constexpr size_t FULL_SMALL = 24 * 1024, FULL_BOTH = 72 * 1024;  // beyond FULL_BOTH one operand at a time
+constexpr size_t FULL_BOUNDS[6] = {6 * 1024, 12 * 1024, FULL_SMALL, FULL_BOTH, FULL_BOTH + 64 * 1024, FULL_BOTH + 112 * 1024};
+
+// Y[base + k st] (+)= sum over operands and t of F[k np + t] T[base + t st],
+// k, t < n = N, np = N rounded up to even: one leg for the item (its other
+// indices) at base.  BOTH: the second operand's T lies ts after the first's,
+// its F fs after.
+template <int N, bool BOTH>
+__device__ __forceinline__ void full_leg_n(const double* __restrict__ T, int ts, double* __restrict__ Y,
+                                           const double* __restrict__ F, int fs, int base, int st, bool first) {
+  constexpr int NP = (N + 1) & ~1;
+  double v[NP], u[BOTH ? NP : 1];
+#pragma unroll
+  for (int t = 0; t < N; ++t) {
+    v[t] = T[base + t * st];
+    if (BOTH) u[t] = T[ts + base + t * st];
+  }
+  if (NP > N) {
+    v[NP - 1] = 0.0;
+    if (BOTH) u[NP - 1] = 0.0;
+  }
+  const double2* f = reinterpret_cast<const double2*>(F);
+  const double2* h = reinterpret_cast<const double2*>(F + fs);
+#pragma unroll 2
+  for (int k = 0; k < N; ++k) {
+    double* y = Y + base + k * st;
+    double a = first ? 0.0 : *y, b = 0.0;
+#pragma unroll
+    for (int t = 0; t < NP / 2; ++t) {
+      const double2 w = f[k * (NP / 2) + t];
+      a += w.x * v[2 * t];
+      b += w.y * v[2 * t + 1];
+      if (BOTH) {
+        const double2 z = h[k * (NP / 2) + t];
+        a += z.x * u[2 * t];
+        b += z.y * u[2 * t + 1];
+      }
+    }
+    *y = a + b;
+  }
+}
+
+// All items of a leg: e = fast + nf * slow -> base = fast * sf + slow * ss.
+template <int N, int NT, bool BOTH>
+__device__ __forceinline__ void full_leg(const double* T, int ts, double* Y, const double* F, int fs, int nf, int ns,
+                                         int sf, int ss, int st, bool first) {
+  const int2 i0 = divmod_small(threadIdx.x, nf), di = divmod_small(NT, nf);
+  int fa = i0.y, sl = i0.x;
+  while (sl < ns) {
+    full_leg_n<N, BOTH>(T, ts, Y, F, fs, fa * sf + sl * ss, st, first);
+    fa += di.y;
+    sl += di.x;
+    if (fa >= nf) {
+      fa -= nf;
+      ++sl;
+    }
+  }
+}
+
+template <int NT, bool BOTH>
+__device__ __noinline__ void full_leg_any(int n, const double* T, int ts, double* Y, const double* F, int fs, int nf,
+                                          int ns, int sf, int ss, int st, bool first) {
+#define QD_LEG(N) \
+  case N: full_leg<N, NT, BOTH>(T, ts, Y, F, fs, nf, ns, sf, ss, st, first); break
+  switch (n) {
+    QD_LEG(1); QD_LEG(2); QD_LEG(3); QD_LEG(4); QD_LEG(5); QD_LEG(6); QD_LEG(7); QD_LEG(8);
+    QD_LEG(9); QD_LEG(10); QD_LEG(11); QD_LEG(12); QD_LEG(13); QD_LEG(14); QD_LEG(15); QD_LEG(16);
+  }
+#undef QD_LEG
+}
+
+__host__ __device__ __forceinline__ int full_fsz(int n) { return n * ((n + 1) & ~1); }
+
+template <int NT, bool BOTH>
+__global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1) k_122_full(DevLayout L, const int* __restrict__ tasks,
+                                                 const int2* __restrict__ tiles, const int4* __restrict__ gpd,
+                                                 const int2* __restrict__ gpp, const double2* __restrict__ F, int nfent,
+                                                 const double* __restrict__ A, double hA, unsigned zA,
+                                                 const double* __restrict__ B, double hB, unsigned zB,
+                                                 double* __restrict__ C) {
+  extern __shared__ __align__(16) double smf[];  // T (one or two) | Y | F1 F2 F3 F4 (one or two sets) | pairs
+  __shared__ i64 sboff[6];
+  const int2 tl = __ldg(&tiles[tasks[blockIdx.x]]);
+  const GpDesc da = load_gp(gpd, tl.x), db = load_gp(gpd, tl.y);
+  const int tid = threadIdx.x, q = da.q;
+  const int n1 = da.n1, n2 = da.n2, n3 = db.n1, n4 = db.n2;
+  const int nr = n1 * n2, nc = n3 * n4, ld = nc | 1, tsz = (nr * ld + 1) & ~1;
+  const int pa0 = da.cnt(0), pa1 = pa0 + da.cnt(1), pa = pa1 + da.cnt(2);
+  const int pb0 = db.cnt(0), pb1 = pb0 + db.cnt(1), pb = pb1 + db.cnt(2);
+  const int4 bd = __ldg(&L.blk[q]);
+  double* T = smf;
+  double* Y = T + (BOTH ? 2 : 1) * tsz;
+  double* F1 = Y + tsz;
+  double* F2 = F1 + full_fsz(n1);
+  double* F3 = F2 + full_fsz(n2);
+  double* F4 = F3 + full_fsz(n3);
+  const int fs = full_fsz(n1) + full_fsz(n2) + full_fsz(n3) + full_fsz(n4);  // one set
+  int2* pr = reinterpret_cast<int2*>(F1 + (BOTH ? 2 : 1) * fs);
+  int2* pc = pr + pa;
+  for (int i = tid; i < pa; i += NT) pr[i] = __ldg(&gpp[da.pstart + i]);
+  for (int i = tid; i < pb; i += NT) pc[i] = __ldg(&gpp[db.pstart + i]);
+  if (tid < 6) sboff[tid] = __ldg(L.boff + 6 * q + tid);
+  const unsigned one = (1u << P_FHH) | (1u << P_FPP) | (1u << P_FPH);
+  // an operand whose factor is zero counts as zero itself
+  const bool on[2] = {(zA & one) != one, (zB & one) != one};  // of the B term (factor FA) and the A term
+  const int2 e0 = divmod_small(tid, pa), de = divmod_small(NT, pa);
+  bool first = true;
+#pragma unroll 1
+  for (int pass = 0; pass < (BOTH ? 1 : 2); ++pass) {  // FA x TB, then -FB x TA
+    if (!BOTH && !on[pass]) continue;
+    if (!first) __syncthreads();  // T and the F matrices are free again
+    for (int g = 0; g < 4; ++g) {
+      const int n = g == 0 ? n1 : (g == 1 ? n2 : (g == 2 ? n3 : n4)), np = (n + 1) & ~1;
+      const double2* f = F + (g < 2 ? 0 : nfent) + (g == 0 ? da.fg : (g == 1 ? da.fh : (g == 2 ? db.fg : db.fh)));
+      double* d = g == 0 ? F1 : (g == 1 ? F2 : (g == 2 ? F3 : F4));
+      const double sg = g < 2 ? 1.0 : -1.0;
+      for (int i = tid; i < n * n; i += NT) {
+        const double2 v = __ldg(&f[i]);
+        const int k = i / n, t = i - k * n;
+        if (BOTH) {
+          d[k * np + t] = sg * v.x;
+          d[fs + k * np + t] = -sg * v.y;
+        } else {
+          d[k * np + t] = pass ? -sg * v.y : sg * v.x;
+        }
+      }
+      if (np > n)
+        for (int k = tid; k < n; k += NT) {
+          d[k * np + n] = 0.0;
+          if (BOTH) d[fs + k * np + n] = 0.0;
+        }
+    }
+    if (da.same || db.same) {  // the cells (t,t) hold no pair
+      for (int i = 2 * tid; i < (BOTH ? 2 : 1) * tsz; i += 2 * NT)
+        *reinterpret_cast<double2*>(T + i) = make_double2(0.0, 0.0);
+      __syncthreads();
+    } else if (first) {
+      __syncthreads();  // the pair lists
+    }
+    // gather: the stored element (P1,P2) of part (c1,c2) when c1 >= c2, else
+    // herm times (P2,P1) of part (c2,c1), on its cell with the orientation
+    // signs and on the mirror cells (g = h) with the opposite ones
+    {
+      int p = e0.y, u = e0.x;
+#pragma unroll 4
+      for (int e = tid; e < pa * pb; e += NT) {
+        const int c1 = (p >= pa0) + (p >= pa1), c2 = (u >= pb0) + (u >= pb1);
+        const bool lower = c1 >= c2;
+        const int part = lower ? slot_of(c1, c2) : slot_of(c2, c1);
+        const int2 P = pr[p], Q = pc[u];
+        p += de.y;
+        u += de.x;
+        if (p >= pa) {
+          p -= pa;
+          ++u;
+        }
+        const int ldv = cnt_of(lower ? c1 : c2, bd);
+        const i64 addr = sboff[part] + (lower ? P.x + (i64)Q.x * ldv : Q.x + (i64)P.x * ldv);
+        const int r = P.y & 0xFF, rm = ((P.y >> 8) & 0xFF) - 1;
+        const int c = Q.y & 0xFF, cm = ((Q.y >> 8) & 0xFF) - 1;
+        const bool neg = (P.y ^ Q.y) & (1 << 16);
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+          if (!BOTH && x != pass) continue;
+          const unsigned zm = x ? zA : zB;
+          double v = !on[x] || ((zm >> (P_HHHH + part)) & 1u) ? 0.0 : __ldg((x ? A : B) + addr);
+          if (!lower) v *= x ? hA : hB;
+          if (neg) v = -v;
+          double* t = T + (BOTH ? x * tsz : 0);
+          t[r * ld + c] = v;
+          if (rm >= 0) t[rm * ld + c] = -v;
+          if (cm >= 0) {
+            t[r * ld + cm] = -v;
+            if (rm >= 0) t[rm * ld + cm] = v;
+          }
+        }
+      }
+    }
+    __syncthreads();
+    full_leg_any<NT, BOTH>(n1, T, tsz, Y, F1, fs, nc, n2, 1, ld, n2 * ld, first);  // items (s; k2), t = k1
+    __syncthreads();
+    full_leg_any<NT, BOTH>(n2, T, tsz, Y, F2, fs, nc, n1, 1, n2 * ld, ld, false);  // items (s; k1), t = k2
+    __syncthreads();
+    full_leg_any<NT, BOTH>(n3, T, tsz, Y, F3, fs, nr, n4, ld, 1, n4, false);       // items (r; l2), t = l1
+    __syncthreads();
+    full_leg_any<NT, BOTH>(n4, T, tsz, Y, F4, fs, nr, n3, ld, n4, 1, false);       // items (r; l1), t = l2
+    first = false;
+  }
+  __syncthreads();
+  // stored output cells: c1 >= c2, rows of S_a fastest
+  int p = e0.y, u = e0.x;
+#pragma unroll 4
+  for (int e = tid; e < pa * pb; e += NT) {
+    const int c1 = (p >= pa0) + (p >= pa1), c2 = (u >= pb0) + (u >= pb1);
+    const int2 P = pr[p], Q = pc[u];
+    p += de.y;
+    u += de.x;
+    if (p >= pa) {
+      p -= pa;
+      ++u;
+    }
+    if (c1 < c2) continue;
+    double y = first ? 0.0 : Y[(P.y & 0xFF) * ld + (Q.y & 0xFF)];
+    if ((P.y ^ Q.y) & (1 << 16)) y = -y;
+    C[sboff[slot_of(c1, c2)] + P.x + (i64)Q.x * cnt_of(c1, bd)] = y;
   }
 }
 
@@ -1317,7 +1537,6 @@ struct TileInfo {
   unsigned parts;    // two-body parts the tile touches (bit = vectorize slot)
   int nst;           // stored output cells
   bool holefree;     // none of the four (m_l, m_s) groups holds a hole
-  unsigned outs;     // stored output regions of the tile (bit out_region(c1, c2))
 };
 struct PdBucket {  // one launch of the particle-hole tile kernel
   int first, count;
@@ -1337,7 +1556,6 @@ struct TaskSet {
   int2* d_task = nullptr;
   std::vector<Bucket122> buckets;
   bool tuned = false;
-  unsigned outmask = OUT_ALL;  // output regions the tiles write (OUT_NONE: A generator-like)
   int bounds_id = 0;           // which bucketing (see kBounds) the tuner kept
   float ms_total = 0.f;        // tuned time of this bucketing
   std::vector<TaskSet> alts;   // the other bucketings, until tuned
@@ -1369,6 +1587,16 @@ struct Plan122 {
   int4* d_cterm = nullptr;
   int gen_rso[6] = {0}, gen_cso[6] = {0};
   int4* d_sptask = nullptr;  // C_pppp tile pairs, then the k_122_gen tiles, then the C_phph tile pairs
+  int* d_ftask = nullptr;  // k_122_full: tile indices, by CTA size, largest first
+  struct FullBucket {
+    int first, count, threads;
+    size_t smem;
+    bool both;                // both operands staged together
+    float ms[3] = {0, 0, 0};  // measured with 64, 128 and 256 threads
+  };
+  std::vector<FullBucket> fbuckets;
+  bool full_fits = true;  // every tile fits k_122_full's shared memory
+  bool full_tuned = false;
   int4* d_ltask = nullptr;   // k_gen_ladder: {block, role, first row}, longest first
   int nsp_ladder = 0;
   int nsp_pppp = 0, nsp_gen = 0;
@@ -1388,6 +1616,11 @@ size_t tile_smem(const TileInfo& t, int tw) {
   const size_t ld = (size_t)(t.nc | 1);
   const size_t tsz = ((size_t)t.nr * ld * tw + 1) & ~(size_t)1;
   return 8 * tsz + 16 * (size_t)t.nf + 8 * (size_t)t.npair;
+}
+size_t full_smem(const TileInfo& t, int n1, int n2, int n3, int n4, bool both) {
+  const size_t tsz = ((size_t)t.nr * (t.nc | 1) + 1) & ~(size_t)1;
+  return 8 * ((both ? 3 : 2) * tsz + (both ? 2 : 1) * (size_t)(full_fsz(n1) + full_fsz(n2) + full_fsz(n3) + full_fsz(n4))) +
+         8 * (size_t)t.npair;
 }
 // a task that only writes zeros keeps just the two pair lists
 size_t zero_smem(const TileInfo& t) { return 8 * (size_t)t.npair; }
@@ -1510,10 +1743,6 @@ static int plan_122(qd_layout* L, Plan122** out) {
             }
         if (!out) continue;
         TileInfo t;
-        t.outs = 0;
-        for (int c1 = 0; c1 < 3; ++c1)
-          for (int c2 = 0; c2 <= c1; ++c2)
-            if (A.cnt[c1] > 0 && B.cnt[c2] > 0) t.outs |= 1u << out_region(c1, c2);
         t.a = u0 + (int)a;
         t.b = u0 + (int)b;
         t.nr = A.n1 * A.n2;
@@ -1788,6 +2017,38 @@ static int plan_122(qd_layout* L, Plan122** out) {
         (rc = upload_vec(L, all, &p.d_sptask)))
       return rc;
   }
+  {  // k_122_full: buckets by shared memory, small tiles with fewer threads
+    std::vector<std::pair<size_t, int>> v;
+    for (size_t i = 0; i < p.tiles.size(); ++i) {
+      const TileInfo& t = p.tiles[i];
+      const int2 gb = gpg[t.a], gk = gpg[t.b];
+      const size_t two = full_smem(t, gsz[gb.x], gsz[gb.y], gsz[gk.x], gsz[gk.y], true);
+      v.push_back({two <= FULL_BOTH ? two : FULL_BOTH + full_smem(t, gsz[gb.x], gsz[gb.y], gsz[gk.x], gsz[gk.y], false),
+                   (int)i});  // beyond FULL_BOTH: one operand at a time
+    }
+    std::stable_sort(v.begin(), v.end(), [](const auto& x, const auto& y) { return x.first > y.first; });
+    p.full_fits = v.empty() || v[0].first <= FULL_BOTH + SMEM_MAX_122 - 1024;
+    std::vector<int> tasks;
+    size_t i = 0;
+    while (i < v.size()) {
+      size_t lower = 0;
+      for (size_t b : FULL_BOUNDS)
+        if (b < v[i].first) lower = std::max(lower, b);
+      Plan122::FullBucket b;
+      b.first = (int)tasks.size();
+      b.both = v[i].first <= FULL_BOTH;
+      b.smem = b.both ? v[i].first : v[i].first - FULL_BOTH;
+      b.threads = !b.both ? 256 : (b.smem <= FULL_SMALL ? 64 : 128);
+      while (i < v.size() && v[i].first > lower) tasks.push_back(v[i++].second);
+      b.count = (int)tasks.size() - b.first;
+      // column strips together (see build_variant)
+      std::stable_sort(tasks.begin() + b.first, tasks.end(), [&](int x, int y) {
+        return p.tiles[x].b != p.tiles[y].b ? p.tiles[x].b < p.tiles[y].b : p.tiles[x].a < p.tiles[y].a;
+      });
+      p.fbuckets.push_back(b);
+    }
+    if ((rc = upload_vec(L, tasks, &p.d_ftask))) return rc;
+  }
   // particle-hole channel: first cc row of each (G1, G2) and the launches
   p.ng = ngroup;
   std::vector<int2> zrow((size_t)ngroup * ngroup);
@@ -1848,6 +2109,8 @@ static int plan_122(qd_layout* L, Plan122** out) {
   for (const void* fn : {(const void*)k_122_tile<1, 64>, (const void*)k_122_tile<2, 64>,
                          (const void*)k_122_tile<1, 128>, (const void*)k_122_tile<2, 128>,
                          (const void*)k_122_tile<1, 256>, (const void*)k_122_tile<2, 256>,
+                         (const void*)k_122_full<64, true>, (const void*)k_122_full<128, true>, (const void*)k_122_full<256, true>,
+                         (const void*)k_122_full<64, false>, (const void*)k_122_full<128, false>, (const void*)k_122_full<256, false>,
                          (const void*)k_pandya_tile<PD_ALL, 64>, (const void*)k_pandya_tile<PD_ALL, 128>,
                          (const void*)k_pandya_tile<PD_ALL, 256>,
                          (const void*)k_pandya_tile<PD_SINGLE, 256>, (const void*)k_pandya_tile<PD_DIRECT, 256>,
@@ -1934,10 +2197,8 @@ static int task_set(qd_layout* L, Plan122* p, unsigned zA, unsigned zB, TaskSet*
   const unsigned za2 = (zA >> P_HHHH) & 63u, zb2 = (zB >> P_HHHH) & 63u;
   // lists: 0 one operand (set), 1 both operands (set), 2 one operand (accumulate)
   std::vector<std::pair<size_t, int2>> lst[3];
-  const unsigned outmask = gen_like(zA) ? OUT_NONE : OUT_ALL;
   for (size_t i = 0; i < p->tiles.size(); ++i) {
     const TileInfo& t = p->tiles[i];
-    if (!(t.outs & outmask)) continue;  // every output of the tile comes from k_gen_pppp / k_122_gen
     const bool nb = !fa0 && (t.parts & ~zb2) && !(spa && t.holefree);
     const bool na = !fb0 && (t.parts & ~za2) && !(spb && t.holefree);
     const int op = (nb ? 1 : 0) | (na ? 2 : 0);
@@ -1955,7 +2216,6 @@ static int task_set(qd_layout* L, Plan122* p, unsigned zA, unsigned zB, TaskSet*
   TaskSet ts;
   for (int bid = 0; bid < kNumBounds; ++bid) {
     TaskSet& v = bid == 0 ? ts : (ts.alts.emplace_back(), ts.alts.back());
-    v.outmask = outmask;
     int rc = build_variant(L, p, lst, bid, v);
     if (rc) return rc;
   }
@@ -1970,7 +2230,7 @@ void drop_122_plan(const qd_layout* L) {
   if (it == plans().end()) return;
   Plan122& p = it->second;
   for (void* ptr : {(void*)p.d_gpd, (void*)p.d_gpp, (void*)p.d_tiles, (void*)p.d_sbase,
-                    (void*)p.d_ftab, (void*)p.d_ltask, (void*)p.d_gpg, (void*)p.d_zrow, (void*)p.d_ptask, (void*)p.d_ppbase,
+                    (void*)p.d_ftab, (void*)p.d_ltask, (void*)p.d_ftask, (void*)p.d_gpg, (void*)p.d_zrow, (void*)p.d_ptask, (void*)p.d_ppbase,
                     (void*)p.d_ppstart, (void*)p.d_ppterm, (void*)p.d_gbase, (void*)p.d_rstart,
                     (void*)p.d_cstart, (void*)p.d_rterm, (void*)p.d_cterm, (void*)p.d_sptask})
     if (ptr) cudaFree(ptr);
@@ -2015,7 +2275,7 @@ static int launch_bucket(qd_layout* L, const Plan122* p, const TaskSet* ts, cons
   k_122_tile<TW, NT><<<b.count, NT, b.smem, L->stream>>>(L->dev, ts->d_task + b.first, p->d_tiles, p->d_gpd,   \
                                                          p->d_gpp, p->d_ftab, p->nfent, A->d,                   \
                                                          (double)A->herm, A->zero_mask, legA, B->d,             \
-                                                         (double)B->herm, B->zero_mask, legB, C, ts->outmask)
+                                                         (double)B->herm, B->zero_mask, legB, C)
   if (b.tw == 2) {
     if (threads == 64) QD_122_LAUNCH(2, 64); else if (threads == 128) QD_122_LAUNCH(2, 128); else QD_122_LAUNCH(2, 256);
   } else {
@@ -2111,12 +2371,75 @@ static int tune_122(qd_layout* L, Plan122* p, TaskSet* ts, const qd_op* A, const
 }
 
 // Text summary of the autotuned buckets of every task set of the layout.
+static int launch_full(qd_layout* L, const Plan122* p, const Plan122::FullBucket& b, int threads, const qd_op* A,
+                       const qd_op* B, double* C) {
+#define QD_FULL_LAUNCH(NT, BOTH)                                                                                    \
+  k_122_full<NT, BOTH><<<b.count, NT, b.smem, L->stream>>>(L->dev, p->d_ftask + b.first, p->d_tiles, p->d_gpd, p->d_gpp, \
+                                                           p->d_ftab, p->nfent, A->d, (double)A->herm, A->zero_mask, \
+                                                           B->d, (double)B->herm, B->zero_mask, C)
+  if (b.both) {
+    if (threads == 64) QD_FULL_LAUNCH(64, true); else if (threads == 128) QD_FULL_LAUNCH(128, true); else QD_FULL_LAUNCH(256, true);
+  } else {
+    if (threads == 64) QD_FULL_LAUNCH(64, false); else if (threads == 128) QD_FULL_LAUNCH(128, false); else QD_FULL_LAUNCH(256, false);
+  }
+#undef QD_FULL_LAUNCH
+  ++L->nlaunch;
+  QD_CUDA(cudaGetLastError());
+  return QD_OK;
+}
+
+// The CTA size of each bucket of k_122_full, once per layout: best of two
+// runs on the real operands into a workspace operator (results do not depend
+// on it).  The F tables of A and B are in place.
+static int tune_full(qd_layout* L, Plan122* p, const qd_op* A, const qd_op* B) {
+  double* scratch = scratch_operator(L);
+  if (!scratch) return QD_OK;
+  cudaEvent_t e0, e1;
+  QD_CUDA(cudaEventCreate(&e0));
+  QD_CUDA(cudaEventCreate(&e1));
+  const long long n0 = L->nlaunch;
+  const int nts[3] = {64, 128, 256};
+  for (Plan122::FullBucket& b : p->fbuckets) {
+    int best = 0;
+    for (int k = 0; k < 3; ++k) {
+      b.ms[k] = 1e30f;
+      for (int rep = 0; rep < 2; ++rep) {
+        QD_CUDA(cudaEventRecord(e0, L->stream));
+        TRY(launch_full(L, p, b, nts[k], A, B, scratch));
+        QD_CUDA(cudaEventRecord(e1, L->stream));
+        QD_CUDA(cudaEventSynchronize(e1));
+        float ms = 0.f;
+        QD_CUDA(cudaEventElapsedTime(&ms, e0, e1));
+        b.ms[k] = std::min(b.ms[k], ms);
+      }
+      if (b.ms[k] < b.ms[best]) best = k;
+    }
+    b.threads = nts[best];
+  }
+  cudaEventDestroy(e0);
+  cudaEventDestroy(e1);
+  L->nlaunch = n0;  // tuning launches are not the caller's work
+  p->full_tuned = true;
+  return QD_OK;
+}
+
 std::string tuning_report_122(const qd_layout* L) {
   std::lock_guard<std::mutex> lock(g_plan_mutex);
   auto it = plans().find(L);
   if (it == plans().end()) return "";
   std::string out;
   char line[256];
+  if (it->second.full_tuned) {
+    float sum = 0.f;
+    for (const auto& b : it->second.fbuckets) sum += std::min(b.ms[0], std::min(b.ms[1], b.ms[2]));
+    snprintf(line, sizeof(line), "commutator_122, legs from registers: bucketing 0 kept (%.4f ms)\n", sum);
+    out += line;
+    for (const auto& b : it->second.fbuckets) {
+      snprintf(line, sizeof(line), "  tiles %6d smem %6zu B: 64 thr %.4f ms, 128 thr %.4f ms, 256 thr %.4f ms -> %d\n",
+               b.count, b.smem, b.ms[0], b.ms[1], b.ms[2], b.threads);
+      out += line;
+    }
+  }
   for (const auto& kv : it->second.sets) {
     const TaskSet& ts = kv.second;
     snprintf(line, sizeof(line), "commutator_122 masks A=0x%03x B=0x%03x: bucketing %d kept (%.4f ms)",
@@ -2147,6 +2470,14 @@ static int spars(const qd_op* X) {
   return (X->zero_mask & hp) == hp;
 }
 
+// Whether the tiles run through k_122_full: not where a one-body factor
+// couples holes to particles only and the basis is large (k_122_tile then
+// skips most of the legs and tiles), nor where a tile is too large for it.
+constexpr i64 FULL_SPARSE_ENTRIES = 1000000;
+static bool use_full(const qd_layout* L, const Plan122* p, const qd_op* A, const qd_op* B) {
+  return p->full_fits && ((!spars(A) && !spars(B)) || L->neq < FULL_SPARSE_ENTRIES);
+}
+
 // Build (and autotune on A, B) the plan and the task set of a pair of
 // zero-part masks ahead of a stream capture, which must neither allocate
 // nor synchronise.  A and B may be views with the masks zA, zB.
@@ -2154,15 +2485,21 @@ int prepare_122(qd_layout* L, const qd_op* A, const qd_op* B) {
   Plan122* p;
   int rc = plan_122(L, &p);
   if (rc) return rc;
-  TaskSet* ts;
-  if ((rc = task_set(L, p, A->zero_mask, B->zero_mask, &ts))) return rc;
-  if (!ts->tuned && !ts->buckets.empty() && !L->prof.on && !capturing(L->stream)) {
+  if (gen_like(A->zero_mask)) return QD_OK;  // no tiles
+  const bool tune = !L->prof.on && !capturing(L->stream);
+  TaskSet* ts = nullptr;
+  const bool full = use_full(L, p, A, B);
+  if (!full && (rc = task_set(L, p, A->zero_mask, B->zero_mask, &ts))) return rc;
+  if (tune && (full ? !p->full_tuned : !ts->tuned && !ts->buckets.empty())) {
     // the F tables of these operands first: the timed launches read them
     const int nf = L->m * p->gmax;
     k_ftab<<<(nf + 127) / 128, 128, 0, L->stream>>>(L->dev, p->d_sbase, A->d, (double)A->herm, B->d,
                                                     (double)B->herm, p->d_ftab, p->gmax, p->nfent);
     QD_CUDA(cudaGetLastError());
-    TRY(tune_122(L, p, ts, A, B, spars(A), spars(B)));
+    if (full)
+      TRY(tune_full(L, p, A, B));
+    else
+      TRY(tune_122(L, p, ts, A, B, spars(A), spars(B)));
   }
   return QD_OK;
 }
@@ -2228,15 +2565,20 @@ int launch_122(qd_layout* L, const qd_op* A, const qd_op* B, double* C, bool lad
   int rc = plan_122(L, &p);
   if (rc) return rc;
   if (p->tiles.empty()) return QD_OK;
-  TaskSet* ts;
-  if ((rc = task_set(L, p, A->zero_mask, B->zero_mask, &ts))) return rc;
+  if (gen_like(A->zero_mask)) return launch_122_gen(L, p, A, B, C, ladder, L->stream, st2 ? st2 : L->stream, upd);
   const int spA = spars(A), spB = spars(B);
-  if (ts->outmask != OUT_ALL) TRY(launch_122_gen(L, p, A, B, C, ladder, L->stream, st2 ? st2 : L->stream, upd));
-  if (ts->buckets.empty()) return QD_OK;  // no group-pair tiles: their F tables are not needed
+  const bool full = use_full(L, p, A, B);
+  TaskSet* ts = nullptr;
+  if (!full && (rc = task_set(L, p, A->zero_mask, B->zero_mask, &ts))) return rc;
   const int nf = L->m * p->gmax;
   k_ftab<<<(nf + 127) / 128, 128, 0, L->stream>>>(L->dev, p->d_sbase, A->d, (double)A->herm, B->d,
                                                   (double)B->herm, p->d_ftab, p->gmax, p->nfent);
   ++L->nlaunch;
+  if (full) {
+    if (!p->full_tuned && !L->prof.on && !capturing(L->stream)) TRY(tune_full(L, p, A, B));
+    for (const Plan122::FullBucket& b : p->fbuckets) TRY(launch_full(L, p, b, b.threads, A, B, C));
+    return QD_OK;
+  }
   if (!ts->tuned && !L->prof.on && !capturing(L->stream)) TRY(tune_122(L, p, ts, A, B, spA, spB));
   for (const Bucket122& b : ts->buckets) TRY(launch_bucket(L, p, ts, b, b.threads, A, B, spA, spB, C));
   QD_CUDA(cudaGetLastError());
