@@ -27,7 +27,6 @@ namespace {
 constexpr int NI = 16, NH = 256;
 constexpr i64 O_W1 = 0, O_B1 = O_W1 + NH * NI, O_W2 = O_B1 + NH, O_B2 = O_W2 + NH * NH, O_W3 = O_B2 + NH,
               O_B3 = O_W3 + NH, NPARAM = O_B3 + 1;
-constexpr int RED_CHUNKS = 64;  // row chunks of the batch reductions
 
 __device__ __forceinline__ float gelu(float z) { return 0.5f * z * (1.0f + erff(z * 0.70710678118654752f)); }
 __device__ __forceinline__ float gelu_d(float z) {
@@ -45,14 +44,23 @@ __device__ __forceinline__ void mma_bf16(float* d, const unsigned* a, const unsi
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
 
+// 16 bytes into shared memory, zeros where !ok
+__device__ __forceinline__ void cp16(void* smem, const void* g, bool ok) {
+  const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(sa), "l"(g), "r"(ok ? 16 : 0) : "memory");
+}
+
 // K and kchunk multiples of GBK; lda, ldb multiples of 8 (16-byte rows).
 // Slice z = blockIdx.z covers k in [z*kchunk, min(K, (z+1)*kchunk)) and
-// writes C + z * cstride.
+// writes C + z * cstride.  Bound: the latency of a slab's loads; three slabs
+// are in flight (one at a time: 300 us a gradient of 8,192 rows with the
+// reductions below as they were; now see mlp_grad).
+constexpr int GST = 3;
 __global__ void __launch_bounds__(128) k_gemm_nt_bf16(const bf16* __restrict__ A, int lda, const bf16* __restrict__ B,
                                                       int ldb, float* __restrict__ C, int ldc, i64 cstride, int M,
                                                       int N, int K, int kchunk) {
-  __shared__ __align__(16) bf16 As[GBM][GLD];
-  __shared__ __align__(16) bf16 Bs[GBN][GLD];
+  __shared__ __align__(16) bf16 As[GST][GBM][GLD];
+  __shared__ __align__(16) bf16 Bs[GST][GBN][GLD];
   const int m0 = blockIdx.y * GBM, n0 = blockIdx.x * GBN;
   const int kb = blockIdx.z * kchunk, ke = min(K, kb + kchunk);
   C += (i64)blockIdx.z * cstride;
@@ -65,40 +73,49 @@ __global__ void __launch_bounds__(128) k_gemm_nt_bf16(const bf16* __restrict__ A
     for (int j = 0; j < 4; ++j)
 #pragma unroll
       for (int r = 0; r < 4; ++r) acc[i][j][r] = 0.f;
-  for (int k0 = kb; k0 < ke; k0 += GBK) {
+  auto load = [&](int k0, int st) {
 #pragma unroll
     for (int it = 0; it < 2; ++it) {  // 64 rows x 4 vectors of 8 per operand
       const int v = tid + it * 128, r = v >> 2, seg = (v & 3) * 8;
-      uint4 va = make_uint4(0, 0, 0, 0), vb = make_uint4(0, 0, 0, 0);
-      if (m0 + r < M) va = *reinterpret_cast<const uint4*>(A + (i64)(m0 + r) * lda + k0 + seg);
-      if (n0 + r < N) vb = *reinterpret_cast<const uint4*>(B + (i64)(n0 + r) * ldb + k0 + seg);
-      *reinterpret_cast<uint4*>(&As[r][seg]) = va;
-      *reinterpret_cast<uint4*>(&Bs[r][seg]) = vb;
+      const bool oa = m0 + r < M, ob = n0 + r < N;
+      cp16(&As[st][r][seg], oa ? A + (i64)(m0 + r) * lda + k0 + seg : A, oa);
+      cp16(&Bs[st][r][seg], ob ? B + (i64)(n0 + r) * ldb + k0 + seg : B, ob);
     }
-    __syncthreads();
+  };
+#pragma unroll
+  for (int st = 0; st < GST - 1; ++st) {
+    if (kb + st * GBK < ke) load(kb + st * GBK, st);
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  }
+  int st = 0;
+  for (int k0 = kb; k0 < ke; k0 += GBK) {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(GST - 2) : "memory");
+    __syncthreads();  // slab st is here, slab st - 1 is read by nobody any more
+    if (k0 + (GST - 1) * GBK < ke) load(k0 + (GST - 1) * GBK, (st + GST - 1) % GST);
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
 #pragma unroll
     for (int kk = 0; kk < GBK; kk += 16) {
       unsigned af[2][4], bfr[4][2];
 #pragma unroll
       for (int mi = 0; mi < 2; ++mi) {
         const int rb = wm * 32 + mi * 16;
-        af[mi][0] = *reinterpret_cast<const unsigned*>(&As[rb + g][kk + 2 * t]);
-        af[mi][1] = *reinterpret_cast<const unsigned*>(&As[rb + g + 8][kk + 2 * t]);
-        af[mi][2] = *reinterpret_cast<const unsigned*>(&As[rb + g][kk + 2 * t + 8]);
-        af[mi][3] = *reinterpret_cast<const unsigned*>(&As[rb + g + 8][kk + 2 * t + 8]);
+        af[mi][0] = *reinterpret_cast<const unsigned*>(&As[st][rb + g][kk + 2 * t]);
+        af[mi][1] = *reinterpret_cast<const unsigned*>(&As[st][rb + g + 8][kk + 2 * t]);
+        af[mi][2] = *reinterpret_cast<const unsigned*>(&As[st][rb + g][kk + 2 * t + 8]);
+        af[mi][3] = *reinterpret_cast<const unsigned*>(&As[st][rb + g + 8][kk + 2 * t + 8]);
       }
 #pragma unroll
       for (int ni = 0; ni < 4; ++ni) {
         const int cb = wn * 32 + ni * 8;
-        bfr[ni][0] = *reinterpret_cast<const unsigned*>(&Bs[cb + g][kk + 2 * t]);
-        bfr[ni][1] = *reinterpret_cast<const unsigned*>(&Bs[cb + g][kk + 2 * t + 8]);
+        bfr[ni][0] = *reinterpret_cast<const unsigned*>(&Bs[st][cb + g][kk + 2 * t]);
+        bfr[ni][1] = *reinterpret_cast<const unsigned*>(&Bs[st][cb + g][kk + 2 * t + 8]);
       }
 #pragma unroll
       for (int mi = 0; mi < 2; ++mi)
 #pragma unroll
         for (int ni = 0; ni < 4; ++ni) mma_bf16(acc[mi][ni], af[mi], bfr[ni]);
     }
-    __syncthreads();
+    st = (st + 1) % GST;
   }
 #pragma unroll
   for (int mi = 0; mi < 2; ++mi)
@@ -115,32 +132,53 @@ __global__ void __launch_bounds__(128) k_gemm_nt_bf16(const bf16* __restrict__ A
     }
 }
 
-// out[i] = sum over the nz slices of part[z][i], fixed order
-__global__ void k_sum_slices(const float* __restrict__ part, int nz, i64 n, float* __restrict__ out) {
-  const i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  float s = 0.f;
-  for (int z = 0; z < nz; ++z) s += part[(i64)z * n + i];
-  out[i] = s;
+// ---- layer 1: Z1 = X W1^T + b1, H1 = GELU(Z1) -> bf16 row-major (and
+// transposed).  One CTA per RB rows, thread j = unit j: its weights stay in
+// registers, the transposed copy goes through shared memory in 16-byte runs.
+constexpr int RB = 32;
+// the RB x NH tile t[row][unit] as columns of out (leading dimension ld), rows r0..
+__device__ __forceinline__ void write_transposed(const bf16 (*t)[NH + 8], bf16* __restrict__ out, i64 ld, i64 r0,
+                                                 int rows) {
+  if (rows == RB && (ld & 7) == 0) {
+    for (int e = threadIdx.x; e < NH * (RB / 8); e += blockDim.x) {
+      const int j = e / (RB / 8), seg = (e % (RB / 8)) * 8;
+      __align__(16) bf16 v[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[k] = t[seg + k][j];
+      *reinterpret_cast<uint4*>(out + (i64)j * ld + r0 + seg) = *reinterpret_cast<const uint4*>(v);
+    }
+  } else {
+    for (int e = threadIdx.x; e < NH * rows; e += blockDim.x) out[(i64)(e / rows) * ld + r0 + e % rows] = t[e % rows][e / rows];
+  }
 }
 
-// ---- layer 1: Z1 = X W1^T + b1, H1 = GELU(Z1) -> bf16 row-major (and transposed)
-__global__ void k_layer1(const float* __restrict__ X, const float* __restrict__ P, float* __restrict__ Z1,
-                         bf16* __restrict__ H1, bf16* __restrict__ H1t, i64 n) {
-  const i64 i = blockIdx.x;
-  const int j = threadIdx.x;  // NH threads
-  if (i >= n) return;
-  __shared__ float x[NI];
-  if (j < NI) x[j] = X[i * NI + j];
-  __syncthreads();
-  float z = P[O_B1 + j];
-  const float* w = P + O_W1 + j * NI;
+__global__ void __launch_bounds__(NH) k_layer1(const float* __restrict__ X, const float* __restrict__ P,
+                                               float* __restrict__ Z1, bf16* __restrict__ H1, bf16* __restrict__ H1t,
+                                               i64 n) {
+  __shared__ __align__(16) float x[RB * NI];
+  __shared__ bf16 tt[RB][NH + 8];
+  const i64 r0 = (i64)blockIdx.x * RB;
+  const int rows = (int)min((i64)RB, n - r0), j = threadIdx.x;
+  for (int e = j; e < rows * NI; e += NH) x[e] = X[r0 * NI + e];
+  float w[NI];
 #pragma unroll
-  for (int c = 0; c < NI; ++c) z += x[c] * w[c];
-  if (Z1) Z1[i * NH + j] = z;
-  const bf16 h = __float2bfloat16_rn(gelu(z));
-  H1[i * NH + j] = h;
-  if (H1t) H1t[(i64)j * n + i] = h;
+  for (int c = 0; c < NI; ++c) w[c] = P[O_W1 + j * NI + c];
+  const float b = P[O_B1 + j];
+  __syncthreads();
+#pragma unroll 4
+  for (int r = 0; r < rows; ++r) {
+    float z = b;
+#pragma unroll
+    for (int c = 0; c < NI; ++c) z += x[r * NI + c] * w[c];
+    const bf16 h = __float2bfloat16_rn(gelu(z));
+    const i64 o = (r0 + r) * NH + j;
+    if (Z1) Z1[o] = z;
+    H1[o] = h;
+    if (H1t) tt[r][j] = h;
+  }
+  if (!H1t) return;
+  __syncthreads();
+  write_transposed(tt, H1t, n, r0, rows);
 }
 
 // ---- layer 2 epilogue and layer 3: Z2 += b2, H2 = GELU(Z2), y = H2 w3 + b3 (warp per row)
@@ -158,68 +196,84 @@ __global__ void k_layer23(float* __restrict__ Z2, const float* __restrict__ P, f
   if (lane == 0) y[i] = s + P[O_B3];
 }
 
-// ---- backward
-// dy = 2 (y - t) / n; per-chunk partial sums of (y - t)^2
-__global__ void k_loss(const float* __restrict__ y, const float* __restrict__ tg, float* __restrict__ dy, i64 n,
-                       float* __restrict__ lpart) {
-  __shared__ double sh[8];
-  double s = 0.0;
-  for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) {
-    const float d = y[i] - tg[i];
-    dy[i] = 2.0f * d / (float)n;
-    s += (double)d * d;
+// ---- the same with the loss and the last layer's backward: per chunk of RB
+// rows Z2 += b2, y = GELU(Z2) w3 + b3, dy = 2 (y - t) / n, the sum of
+// (y - t)^2, dZ2 = dy (x) w3 * GELU'(Z2) as bf16 (row-major and transposed),
+// and the chunk's db2, dw3, db3.  Z2 is read once and never written back.
+__global__ void __launch_bounds__(NH) k_tail(const float* __restrict__ Z2, const float* __restrict__ P,
+                                             const float* __restrict__ tg, i64 n, bf16* __restrict__ dZ2,
+                                             bf16* __restrict__ dZ2t, float* __restrict__ part,
+                                             float* __restrict__ lpart) {
+  extern __shared__ __align__(16) float zs[];  // [RB][NH]
+  __shared__ bf16 tt[RB][NH + 8];
+  __shared__ float dys[RB];
+  __shared__ double sq[RB];
+  const i64 r0 = (i64)blockIdx.x * RB;
+  const int rows = (int)min((i64)RB, n - r0), tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  for (int r = w; r < RB; r += NH / 32) {  // a warp per row, as k_layer23
+    if (r >= rows) {
+      if (lane == 0) sq[r] = 0.0;
+      continue;
+    }
+    float s = 0.f;
+#pragma unroll
+    for (int k = 0; k < NH / 32; ++k) {
+      const int j = lane + 32 * k;
+      const float z = Z2[(r0 + r) * NH + j] + P[O_B2 + j];
+      zs[r * NH + j] = z;
+      s += gelu(z) * P[O_W3 + j];
+    }
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if (lane == 0) {
+      const float d = s + P[O_B3] - tg[r0 + r];
+      dys[r] = 2.0f * d / (float)n;
+      sq[r] = (double)d * d;
+    }
   }
-  s = block_sum<256>(s, sh);
-  if (threadIdx.x == 0) lpart[blockIdx.x] = (float)s;
-}
-
-// dZ2 = dy (x) w3 * GELU'(Z2), bf16, row-major and transposed
-__global__ void k_dz2(const float* __restrict__ dy, const float* __restrict__ Z2, const float* __restrict__ P,
-                      bf16* __restrict__ dZ2, bf16* __restrict__ dZ2t, i64 n) {
-  const i64 i = blockIdx.x;
-  const int j = threadIdx.x;
-  if (i >= n) return;
-  const bf16 v = __float2bfloat16_rn(dy[i] * P[O_W3 + j] * gelu_d(Z2[i * NH + j]));
-  dZ2[i * NH + j] = v;
-  dZ2t[(i64)j * n + i] = v;
-}
-
-// per row chunk: db2[j] += dy_i w3_j g'(Z2_ij); dw3[j] += dy_i GELU(Z2_ij); db3 += dy_i
-__global__ void k_red23(const float* __restrict__ dy, const float* __restrict__ Z2, const float* __restrict__ P,
-                        i64 n, float* __restrict__ part) {
-  const int j = threadIdx.x;
-  const i64 r0 = n * blockIdx.x / gridDim.x, r1 = n * (blockIdx.x + 1) / gridDim.x;
-  float db2 = 0.f, dw3 = 0.f, db3 = 0.f;
+  __syncthreads();
+  const int j = tid;
   const float w3 = P[O_W3 + j];
-  for (i64 i = r0; i < r1; ++i) {
-    const float z = Z2[i * NH + j], d = dy[i];
-    db2 += d * w3 * gelu_d(z);
+  float db2 = 0.f, dw3 = 0.f, db3 = 0.f;
+#pragma unroll 2
+  for (int r = 0; r < rows; ++r) {
+    const float z = zs[r * NH + j], d = dys[r], v = d * w3 * gelu_d(z);
+    const bf16 q = __float2bfloat16_rn(v);
+    dZ2[(r0 + r) * NH + j] = q;
+    tt[r][j] = q;
+    db2 += v;
     dw3 += d * gelu(z);
     db3 += d;
   }
   float* o = part + (i64)blockIdx.x * (2 * NH + 1);
   o[j] = db2;
   o[NH + j] = dw3;
-  if (j == 0) o[2 * NH] = db3;
+  if (j == 0) {
+    o[2 * NH] = db3;
+    double s = 0.0;
+    for (int r = 0; r < RB; ++r) s += sq[r];
+    lpart[blockIdx.x] = (float)s;
+  }
+  __syncthreads();
+  write_transposed(tt, dZ2t, n, r0, rows);
 }
 
-// per row chunk: dZ1 = dH1 * GELU'(Z1); db1[j] += dZ1_ij; dW1[j][c] += dZ1_ij X_ic
-__global__ void k_red1(const float* __restrict__ dH1, const float* __restrict__ Z1, const float* __restrict__ X, i64 n,
-                       float* __restrict__ part) {
-  const int j = threadIdx.x;
-  const i64 r0 = n * blockIdx.x / gridDim.x, r1 = n * (blockIdx.x + 1) / gridDim.x;
+// per chunk of RB rows: dZ1 = dH1 * GELU'(Z1); db1[j] += dZ1_ij; dW1[j][c] += dZ1_ij X_ic
+__global__ void __launch_bounds__(NH) k_red1(const float* __restrict__ dH1, const float* __restrict__ Z1,
+                                             const float* __restrict__ X, i64 n, float* __restrict__ part) {
+  __shared__ __align__(16) float x[RB * NI];
+  const i64 r0 = (i64)blockIdx.x * RB;
+  const int rows = (int)min((i64)RB, n - r0), j = threadIdx.x;
+  for (int e = j; e < rows * NI; e += NH) x[e] = X[r0 * NI + e];
   float db1 = 0.f, dw[NI];
 #pragma unroll
   for (int c = 0; c < NI; ++c) dw[c] = 0.f;
-  __shared__ float xs[NI];
-  for (i64 i = r0; i < r1; ++i) {
-    __syncthreads();
-    if (j < NI) xs[j] = X[i * NI + j];
-    __syncthreads();
-    const float d = dH1[i * NH + j] * gelu_d(Z1[i * NH + j]);
+  __syncthreads();
+#pragma unroll 4
+  for (int r = 0; r < rows; ++r) {
+    const float d = dH1[(r0 + r) * NH + j] * gelu_d(Z1[(r0 + r) * NH + j]);
     db1 += d;
 #pragma unroll
-    for (int c = 0; c < NI; ++c) dw[c] += d * xs[c];
+    for (int c = 0; c < NI; ++c) dw[c] += d * x[r * NI + c];
   }
   float* o = part + (i64)blockIdx.x * (NH + NH * NI);
   o[j] = db1;
@@ -227,24 +281,43 @@ __global__ void k_red1(const float* __restrict__ dH1, const float* __restrict__ 
   for (int c = 0; c < NI; ++c) o[NH + j * NI + c] = dw[c];
 }
 
-// gradient vector G from the chunk partials (fixed order) and the dW2 product
-__global__ void k_grad_collect(const float* __restrict__ p23, const float* __restrict__ p1, int nch,
-                               const float* __restrict__ dW2, float* __restrict__ G) {
+// out[e] = sum over chunks z of part[z * ld + e], e < ne: CS_P threads per
+// entry take every CS_P-th chunk and add up in a fixed order
+constexpr int CS_E = 32, CS_P = 8;
+__global__ void __launch_bounds__(CS_E * CS_P) k_sum_chunks(const float* __restrict__ part, i64 nch, int ld, int ne,
+                                                            float* __restrict__ out) {
+  __shared__ float sh[CS_P][CS_E];
+  const int l = threadIdx.x % CS_E, p = threadIdx.x / CS_E, e = blockIdx.x * CS_E + l;
+  float s = 0.f;
+  if (e < ne) {
+#pragma unroll 8
+    for (i64 z = p; z < nch; z += CS_P) s += part[z * ld + e];
+  }
+  sh[p][l] = s;
+  __syncthreads();
+  if (p || e >= ne) return;
+  s = 0.f;
+#pragma unroll
+  for (int k = 0; k < CS_P; ++k) s += sh[k][l];
+  out[e] = s;
+}
+
+// gradient vector G from the sums of the chunk partials (s23: db2, dw3, db3;
+// s1: db1, dW1) and the slices of the dW2 product, all in fixed order
+__global__ void k_grad_collect(const float* __restrict__ s23, const float* __restrict__ s1,
+                               const float* __restrict__ kpart, int nz, float* __restrict__ G) {
   const i64 e = (i64)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= NPARAM) return;
   float s = 0.f;
   if (e < O_B1) {  // W1[j][c]
-    for (int z = 0; z < nch; ++z) s += p1[(i64)z * (NH + NH * NI) + NH + e];
+    s = s1[NH + e];
   } else if (e < O_W2) {  // b1
-    for (int z = 0; z < nch; ++z) s += p1[(i64)z * (NH + NH * NI) + (e - O_B1)];
-  } else if (e < O_B2) {  // W2[j][l] = dW2[j][l]
-    s = dW2[e - O_W2];
-  } else if (e < O_W3) {  // b2
-    for (int z = 0; z < nch; ++z) s += p23[(i64)z * (2 * NH + 1) + (e - O_B2)];
-  } else if (e < O_B3) {  // w3
-    for (int z = 0; z < nch; ++z) s += p23[(i64)z * (2 * NH + 1) + NH + (e - O_W3)];
-  } else {
-    for (int z = 0; z < nch; ++z) s += p23[(i64)z * (2 * NH + 1) + 2 * NH];
+    s = s1[e - O_B1];
+  } else if (e < O_B2) {  // W2[j][l]
+#pragma unroll 8
+    for (int z = 0; z < nz; ++z) s += kpart[(i64)z * NH * NH + (e - O_W2)];
+  } else {  // b2, w3, b3
+    s = s23[e - O_B2];
   }
   G[e] = s;
 }
@@ -280,9 +353,10 @@ struct qd_mlp {
   long long step = 0;
   // activations for up to cap rows
   qd::i64 cap = 0;
-  float *Z1 = nullptr, *Z2 = nullptr, *y = nullptr, *dy = nullptr, *dH1 = nullptr;
+  float *Z1 = nullptr, *Z2 = nullptr, *dH1 = nullptr;
   bf16 *H1 = nullptr, *H1t = nullptr, *dZ2 = nullptr, *dZ2t = nullptr;
-  float *p23 = nullptr, *p1 = nullptr, *lpart = nullptr, *dW2 = nullptr, *kpart = nullptr;
+  float *p23 = nullptr, *p1 = nullptr, *lpart = nullptr, *kpart = nullptr;  // partials per RB rows, dW2 slices
+  float *s23 = nullptr, *s1 = nullptr, *h_loss = nullptr;                    // their sums; pinned copy of lpart
   int kslices = 0;
 };
 
@@ -290,10 +364,11 @@ using namespace qd;
 
 namespace {
 void mlp_free_acts(qd_mlp* m) {
-  for (void* p : {(void*)m->Z1, (void*)m->Z2, (void*)m->y, (void*)m->dy, (void*)m->dH1, (void*)m->H1, (void*)m->H1t,
-                  (void*)m->dZ2, (void*)m->dZ2t, (void*)m->kpart})
+  for (void* p : {(void*)m->Z1, (void*)m->Z2, (void*)m->dH1, (void*)m->H1, (void*)m->H1t, (void*)m->dZ2,
+                  (void*)m->dZ2t, (void*)m->kpart, (void*)m->p23, (void*)m->p1, (void*)m->lpart})
     if (p) cudaFree(p);
-  m->Z1 = m->Z2 = m->y = m->dy = m->dH1 = m->kpart = nullptr;
+  if (m->h_loss) cudaFreeHost(m->h_loss);
+  m->Z1 = m->Z2 = m->dH1 = m->kpart = m->p23 = m->p1 = m->lpart = m->h_loss = nullptr;
   m->H1 = m->H1t = m->dZ2 = m->dZ2t = nullptr;
   m->cap = 0;
 }
@@ -305,8 +380,11 @@ int mlp_ensure(qd_mlp* m, i64 n) {
   QD_CUDA(cudaMalloc(&m->Z1, sizeof(float) * c * NH));
   QD_CUDA(cudaMalloc(&m->Z2, sizeof(float) * c * NH));
   QD_CUDA(cudaMalloc(&m->dH1, sizeof(float) * c * NH));
-  QD_CUDA(cudaMalloc(&m->y, sizeof(float) * c));
-  QD_CUDA(cudaMalloc(&m->dy, sizeof(float) * c));
+  const i64 nch = c / RB;
+  QD_CUDA(cudaMalloc(&m->p23, sizeof(float) * nch * (2 * NH + 1)));
+  QD_CUDA(cudaMalloc(&m->p1, sizeof(float) * nch * (NH + NH * NI)));
+  QD_CUDA(cudaMalloc(&m->lpart, sizeof(float) * nch));
+  QD_CUDA(cudaMallocHost(&m->h_loss, sizeof(float) * nch));
   QD_CUDA(cudaMalloc(&m->H1, sizeof(bf16) * c * NH));
   QD_CUDA(cudaMalloc(&m->H1t, sizeof(bf16) * c * NH));
   QD_CUDA(cudaMalloc(&m->dZ2, sizeof(bf16) * c * NH));
@@ -317,65 +395,73 @@ int mlp_ensure(qd_mlp* m, i64 n) {
   return QD_OK;
 }
 
-int gemm_nt(const bf16* A, int lda, const bf16* B, int ldb, float* C, int ldc, int M, int N, int K, int slices,
-            float* part, cudaStream_t st) {
+// C = A B^T, or with *slices > 1 the K slices' partial products one after
+// another in C (*slices: how many)
+int gemm_nt(const bf16* A, int lda, const bf16* B, int ldb, float* C, int ldc, int M, int N, int K, int* slices,
+            cudaStream_t st) {
   if (K % GBK) {
     set_error("mlp: inner dimension %d is not a multiple of %d", K, GBK);
     return QD_ERR_ARG;
   }
-  int kchunk = ((K + slices - 1) / slices + GBK - 1) / GBK * GBK;
-  slices = (K + kchunk - 1) / kchunk;
-  dim3 grid((N + GBN - 1) / GBN, (M + GBM - 1) / GBM, slices);
-  if (slices == 1) {
-    k_gemm_nt_bf16<<<grid, 128, 0, st>>>(A, lda, B, ldb, C, ldc, 0, M, N, K, kchunk);
-  } else {
-    k_gemm_nt_bf16<<<grid, 128, 0, st>>>(A, lda, B, ldb, part, ldc, (i64)M * ldc, M, N, K, kchunk);
-    const i64 nn = (i64)M * ldc;
-    k_sum_slices<<<(unsigned)((nn + 255) / 256), 256, 0, st>>>(part, slices, nn, C);
-  }
+  const int want = slices ? *slices : 1;
+  const int kchunk = ((K + want - 1) / want + GBK - 1) / GBK * GBK, nz = (K + kchunk - 1) / kchunk;
+  dim3 grid((N + GBN - 1) / GBN, (M + GBM - 1) / GBM, nz);
+  k_gemm_nt_bf16<<<grid, 128, 0, st>>>(A, lda, B, ldb, C, ldc, (i64)M * ldc, M, N, K, kchunk);
+  if (slices) *slices = nz;
   QD_CUDA(cudaGetLastError());
   return QD_OK;
 }
 
-// forward of rows [0, n) of X into m->y (keeps Z1, H1, H1t, Z2 when train)
-int mlp_forward(qd_mlp* m, const float* X, i64 n, bool train, cudaStream_t st) {
+// layers 1 and 2 of rows [0, n) of X: Z2 without its bias (keeps Z1, H1, H1t when train)
+int mlp_hidden(qd_mlp* m, const float* X, i64 n, bool train, cudaStream_t st) {
   int rc = mlp_ensure(m, n);
   if (rc) return rc;
-  k_layer1<<<(unsigned)n, NH, 0, st>>>(X, m->P, train ? m->Z1 : nullptr, m->H1, train ? m->H1t : nullptr, n);
-  if ((rc = gemm_nt(m->H1, NH, m->W2b, NH, m->Z2, NH, (int)n, NH, NH, 1, nullptr, st))) return rc;
-  k_layer23<<<(unsigned)((n + 7) / 8), 256, 0, st>>>(m->Z2, m->P, m->y, n);
+  k_layer1<<<(unsigned)((n + RB - 1) / RB), NH, 0, st>>>(X, m->P, train ? m->Z1 : nullptr, m->H1,
+                                                        train ? m->H1t : nullptr, n);
+  return gemm_nt(m->H1, NH, m->W2b, NH, m->Z2, NH, (int)n, NH, NH, nullptr, st);
+}
+
+// forward of rows [0, n) of X into y
+int mlp_forward(qd_mlp* m, const float* X, i64 n, float* y, cudaStream_t st) {
+  int rc = mlp_hidden(m, X, n, false, st);
+  if (rc) return rc;
+  k_layer23<<<(unsigned)((n + 7) / 8), 256, 0, st>>>(m->Z2, m->P, y, n);
   QD_CUDA(cudaGetLastError());
   return QD_OK;
 }
 
-// gradient of mean((y - t)^2) into m->G; loss into *loss (host) if given
-int mlp_grad(qd_mlp* m, const float* X, const float* T, i64 n, float* loss, cudaStream_t st) {
+// gradient of mean((y - t)^2) into G; with want_loss the chunks' sums of
+// squares on their way to m->h_loss (mlp_loss, after a synchronisation).
+// Bound: latency of nine launches.  A batch of 8,192 rows, with the earlier
+// reductions (64 CTAs for all rows, a barrier per row) and now: 302 and 112 us.
+int mlp_grad(qd_mlp* m, const float* X, const float* T, i64 n, float* G, bool want_loss, cudaStream_t st) {
   if (n <= 0 || n % GBK) {
     set_error("qd_mlp: the batch (%lld rows) must be a positive multiple of %d", (long long)n, GBK);
     return QD_ERR_ARG;
   }
-  int rc = mlp_forward(m, X, n, true, st);
+  int rc = mlp_hidden(m, X, n, true, st);
   if (rc) return rc;
-  k_loss<<<RED_CHUNKS, 256, 0, st>>>(m->y, T, m->dy, n, m->lpart);
-  k_dz2<<<(unsigned)n, NH, 0, st>>>(m->dy, m->Z2, m->P, m->dZ2, m->dZ2t, n);
-  k_red23<<<RED_CHUNKS, NH, 0, st>>>(m->dy, m->Z2, m->P, n, m->p23);
+  const i64 nch = (n + RB - 1) / RB;
+  k_tail<<<(unsigned)nch, NH, sizeof(float) * RB * NH, st>>>(m->Z2, m->P, T, n, m->dZ2, m->dZ2t, m->p23, m->lpart);
+  if (want_loss)
+    QD_CUDA(cudaMemcpyAsync(m->h_loss, m->lpart, sizeof(float) * nch, cudaMemcpyDeviceToHost, st));
   // dW2[j][l] = sum_i dZ2[i][j] H1[i][l]: A = dZ2^T (256 x n), B = H1^T (256 x n), K = n
-  if ((rc = gemm_nt(m->dZ2t, (int)n, m->H1t, (int)n, m->dW2, NH, NH, NH, (int)n, m->kslices, m->kpart, st)))
-    return rc;
+  int nz = m->kslices;
+  if ((rc = gemm_nt(m->dZ2t, (int)n, m->H1t, (int)n, m->kpart, NH, NH, NH, (int)n, &nz, st))) return rc;
   // dH1 = dZ2 W2: A = dZ2 (n x 256), B = W2^T (256 x 256)
-  if ((rc = gemm_nt(m->dZ2, NH, m->W2tb, NH, m->dH1, NH, (int)n, NH, NH, 1, nullptr, st))) return rc;
-  k_red1<<<RED_CHUNKS, NH, 0, st>>>(m->dH1, m->Z1, X, n, m->p1);
-  k_grad_collect<<<(unsigned)((NPARAM + 255) / 256), 256, 0, st>>>(m->p23, m->p1, RED_CHUNKS, m->dW2, m->G);
+  if ((rc = gemm_nt(m->dZ2, NH, m->W2tb, NH, m->dH1, NH, (int)n, NH, NH, nullptr, st))) return rc;
+  k_red1<<<(unsigned)nch, NH, 0, st>>>(m->dH1, m->Z1, X, n, m->p1);
+  k_sum_chunks<<<(2 * NH + 1 + CS_E - 1) / CS_E, CS_E * CS_P, 0, st>>>(m->p23, nch, 2 * NH + 1, 2 * NH + 1, m->s23);
+  k_sum_chunks<<<(NH + NH * NI + CS_E - 1) / CS_E, CS_E * CS_P, 0, st>>>(m->p1, nch, NH + NH * NI, NH + NH * NI, m->s1);
+  k_grad_collect<<<(unsigned)((NPARAM + 255) / 256), 256, 0, st>>>(m->s23, m->s1, m->kpart, nz, G);
   QD_CUDA(cudaGetLastError());
-  if (loss) {
-    float lp[RED_CHUNKS];
-    QD_CUDA(cudaMemcpyAsync(lp, m->lpart, sizeof(lp), cudaMemcpyDeviceToHost, st));
-    QD_CUDA(cudaStreamSynchronize(st));
-    double s = 0.0;
-    for (int z = 0; z < RED_CHUNKS; ++z) s += lp[z];
-    *loss = (float)(s / (double)n);
-  }
   return QD_OK;
+}
+
+float mlp_loss(const qd_mlp* m, i64 n) {
+  double s = 0.0;
+  for (i64 z = 0; z < (n + RB - 1) / RB; ++z) s += m->h_loss[z];
+  return (float)(s / (double)n);
 }
 }  // namespace
 
@@ -415,10 +501,8 @@ int qd_mlp_create(int device, uint64_t seed, qd_mlp** out) {
   al((void**)&m->G, sizeof(float) * NPARAM);
   al((void**)&m->W2b, sizeof(bf16) * NH * NH);
   al((void**)&m->W2tb, sizeof(bf16) * NH * NH);
-  al((void**)&m->p23, sizeof(float) * RED_CHUNKS * (2 * NH + 1));
-  al((void**)&m->p1, sizeof(float) * RED_CHUNKS * (NH + NH * NI));
-  al((void**)&m->lpart, sizeof(float) * RED_CHUNKS);
-  al((void**)&m->dW2, sizeof(float) * NH * NH);
+  al((void**)&m->s23, sizeof(float) * (2 * NH + 1));
+  al((void**)&m->s1, sizeof(float) * (NH + NH * NI));
   if (rc) {
     delete m;
     return rc;
@@ -426,6 +510,7 @@ int qd_mlp_create(int device, uint64_t seed, qd_mlp** out) {
   QD_CUDA(cudaMemcpy(m->P, p.data(), sizeof(float) * NPARAM, cudaMemcpyHostToDevice));
   QD_CUDA(cudaMemset(m->M, 0, sizeof(float) * NPARAM));
   QD_CUDA(cudaMemset(m->V, 0, sizeof(float) * NPARAM));
+  QD_CUDA(cudaFuncSetAttribute(k_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(sizeof(float) * RB * NH)));
   k_w2_bf16<<<NH * NH / 256, 256>>>(m->P, m->W2b, m->W2tb);
   QD_CUDA(cudaDeviceSynchronize());
   *out = m;
@@ -437,8 +522,8 @@ int qd_mlp_destroy(qd_mlp* m) {
   cudaSetDevice(m->device);
   cudaDeviceSynchronize();
   mlp_free_acts(m);
-  for (void* p : {(void*)m->P, (void*)m->M, (void*)m->V, (void*)m->G, (void*)m->W2b, (void*)m->W2tb, (void*)m->p23,
-                  (void*)m->p1, (void*)m->lpart, (void*)m->dW2})
+  for (void* p : {(void*)m->P, (void*)m->M, (void*)m->V, (void*)m->G, (void*)m->W2b, (void*)m->W2tb, (void*)m->s23,
+                  (void*)m->s1})
     if (p) cudaFree(p);
   (void)cudaGetLastError();
   delete m;
@@ -480,9 +565,8 @@ int qd_mlp_forward(qd_mlp* m, const float* d_X, float* d_y, int64_t n, void* str
   const i64 chunk = 1 << 18;  // bounded activation workspace
   for (i64 r = 0; r < n; r += chunk) {
     const i64 k = std::min<i64>(chunk, n - r);
-    int rc = mlp_forward(m, d_X + r * NI, k, false, st);
+    int rc = mlp_forward(m, d_X + r * NI, k, d_y + r, st);
     if (rc) return rc;
-    QD_CUDA(cudaMemcpyAsync(d_y + r, m->y, sizeof(float) * k, cudaMemcpyDeviceToDevice, st));
   }
   return QD_OK;
 }
@@ -494,10 +578,10 @@ int qd_mlp_grad(qd_mlp* m, const float* d_X, const float* d_T, int64_t n, float*
   }
   QD_CUDA(cudaSetDevice(m->device));
   cudaStream_t st = (cudaStream_t)stream;
-  int rc = mlp_grad(m, d_X, d_T, n, loss, st);
+  int rc = mlp_grad(m, d_X, d_T, n, d_grad, loss != nullptr, st);
   if (rc) return rc;
-  QD_CUDA(cudaMemcpyAsync(d_grad, m->G, sizeof(float) * NPARAM, cudaMemcpyDeviceToDevice, st));
   QD_CUDA(cudaStreamSynchronize(st));
+  if (loss) *loss = mlp_loss(m, n);
   return QD_OK;
 }
 
@@ -509,8 +593,12 @@ int qd_mlp_train_step(qd_mlp* m, const float* d_X, const float* d_T, int64_t n, 
   }
   QD_CUDA(cudaSetDevice(m->device));
   cudaStream_t st = (cudaStream_t)stream;
-  int rc = mlp_grad(m, d_X, d_T, n, loss, st);
+  int rc = mlp_grad(m, d_X, d_T, n, m->G, loss != nullptr, st);
   if (rc) return rc;
+  if (loss) {
+    QD_CUDA(cudaStreamSynchronize(st));
+    *loss = mlp_loss(m, n);
+  }
   m->step += 1;
   const float c1 = 1.0f - std::pow(0.9f, (float)m->step), c2 = 1.0f - std::pow(0.999f, (float)m->step);
   k_adam<<<(unsigned)((NPARAM + 255) / 256), 256, 0, st>>>(m->P, m->G, m->M, m->V, lr, c1, c2);
