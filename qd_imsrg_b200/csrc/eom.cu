@@ -19,7 +19,7 @@
 //   grouped GEMM  Wb[q] = Vpppp[q] Qb[q] + Qb[q] Vhhhh[q'] on the DMMA pipe:
 //                 the c<d and k<l sums of HQ_comm_2b
 //   k_eom_2b      w(2p2h) = Wb + the one-body, three-leg and particle-hole
-//                 sums of HQ_comm_2b, one thread per entry
+//                 sums of HQ_comm_2b, one warp per entry
 //   k_eom_1b      w(1p1h) = HQ_comm_1b, one CTA per entry
 // Every sum runs only over the states where its factors can be non-zero:
 // Q carries the target, V conserves (M_L, M_S), so each one-body index and
@@ -112,96 +112,97 @@ __global__ void k_eom_unwrap(const double* __restrict__ v, i64 n1, i64 n2, const
   }
 }
 
+// Element H(a,b,c,d) and Q_elem of pair-table entries already read (without a
+// branch, so that a thread's reads overlap).
+__device__ __forceinline__ double eom_v(const DevLayout& L, const double* __restrict__ H, double hh, int a, int b,
+                                        int c, int d) {
+  return dv_at(dv_pos(L, __ldg(&L.ptab[a * L.m + b]), __ldg(&L.ptab[c * L.m + d])), H, hh);
+}
+
 // HQ_comm_2b(a, b, i, j) (src/commutators.f90:1214-1272) minus its two ladder
 // sums, plus those sums from Wb.  a < b particles, i < j holes (0-based).
-__global__ void __launch_bounds__(128, 4) k_eom_2b(DevLayout L, EomDev E, const double* __restrict__ H, double hh,
-                                                const int4* __restrict__ out2, const int* __restrict__ pos2, i64 n2,
-                                                const double* __restrict__ wb, double* __restrict__ w) {
-  const i64 e = (i64)blockIdx.x * blockDim.x + threadIdx.x;
+// One warp per entry: the particle-hole part has four terms for each hole k,
+// the others are eight short sums over one group each; the lanes take the
+// 4 n + 8 sums in turn, one shuffle tree adds them.  Bound: the chain of table
+// and element reads of a sum (with one thread per entry all 4 n + 8 followed
+// one another: 215 us for the 2p2h part at N=12, R=10).
+constexpr int EOM2_THREADS = 128;
+__global__ void __launch_bounds__(EOM2_THREADS) k_eom_2b(DevLayout L, EomDev E, const double* __restrict__ H,
+                                                         double hh, const int4* __restrict__ out2,
+                                                         const int* __restrict__ pos2, i64 n2,
+                                                         const double* __restrict__ wb, double* __restrict__ w) {
+  const i64 e = (i64)blockIdx.x * (EOM2_THREADS / 32) + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
   if (e >= n2) return;
   const int4 o = out2[e];
   const int a = o.x, b = o.y, i = o.z, j = o.w;
-  const int la = __ldg(&E.ml[a]), lb = __ldg(&E.ml[b]), li = __ldg(&E.ml[i]), lj = __ldg(&E.ml[j]);
-  const int sa = __ldg(&E.ms[a]), sb = __ldg(&E.ms[b]), si = __ldg(&E.ms[i]), sj = __ldg(&E.ms[j]);
   const int n = L.n;
   double sm = 0.0;
-  int gb, ge;
-  // 12 -> 2: f(a,c) Q(c,b,i,j) - f(b,c) Q(c,a,i,j), c particle
-  grp_range(L, eom_grp(E, E.tml + li + lj - lb, E.tms + si + sj - sb), &gb, &ge);
-  for (int t = gb; t < ge; ++t) {
-    const int c = __ldg(&L.gmem[t]);
-    if (c >= n) sm += eom_f(L, H, hh, a, c) * eom_q(L, E, c, b, i, j);
-  }
-  grp_range(L, eom_grp(E, E.tml + li + lj - la, E.tms + si + sj - sa), &gb, &ge);
-  for (int t = gb; t < ge; ++t) {
-    const int c = __ldg(&L.gmem[t]);
-    if (c >= n) sm -= eom_f(L, H, hh, b, c) * eom_q(L, E, c, a, i, j);
-  }
-  //        Qf(c,i) V(a,b,c,j) - Qf(c,j) V(a,b,c,i)
-  grp_range(L, eom_grp(E, li + E.tml, si + E.tms), &gb, &ge);
-  for (int t = gb; t < ge; ++t) {
-    const int c = __ldg(&L.gmem[t]);
-    if (c >= n) sm += eom_qf(L, E, c, i) * dv_elem(L, H, hh, a, b, c, j);
-  }
-  grp_range(L, eom_grp(E, lj + E.tml, sj + E.tms), &gb, &ge);
-  for (int t = gb; t < ge; ++t) {
-    const int c = __ldg(&L.gmem[t]);
-    if (c >= n) sm -= eom_qf(L, E, c, j) * dv_elem(L, H, hh, a, b, c, i);
-  }
-  //        -Q(a,b,k,j) f(k,i) + Q(a,b,k,i) f(k,j), k hole
-  grp_range(L, eom_grp(E, la + lb - E.tml - lj, sa + sb - E.tms - sj), &gb, &ge);
-  for (int t = gb; t < ge; ++t) {
-    const int k = __ldg(&L.gmem[t]);
-    if (k < n) sm -= eom_q(L, E, a, b, k, j) * eom_f(L, H, hh, k, i);
-  }
-  grp_range(L, eom_grp(E, la + lb - E.tml - li, sa + sb - E.tms - si), &gb, &ge);
-  for (int t = gb; t < ge; ++t) {
-    const int k = __ldg(&L.gmem[t]);
-    if (k < n) sm += eom_q(L, E, a, b, k, i) * eom_f(L, H, hh, k, j);
-  }
-  //        -V(b,k,j,i) Qf(a,k) + V(a,k,j,i) Qf(b,k)
-  grp_range(L, eom_grp(E, la - E.tml, sa - E.tms), &gb, &ge);
-  for (int t = gb; t < ge; ++t) {
-    const int k = __ldg(&L.gmem[t]);
-    if (k < n) sm -= dv_elem(L, H, hh, b, k, j, i) * eom_qf(L, E, a, k);
-  }
-  grp_range(L, eom_grp(E, lb - E.tml, sb - E.tms), &gb, &ge);
-  for (int t = gb; t < ge; ++t) {
-    const int k = __ldg(&L.gmem[t]);
-    if (k < n) sm += dv_elem(L, H, hh, a, k, j, i) * eom_qf(L, E, b, k);
-  }
-  // 22 -> 2, particle-hole: for each hole k the particle c of each term lies
-  // in the group fixed by V's conservation
-  for (int k = 0; k < n; ++k) {
-    const int lk = __ldg(&E.ml[k]), sk = __ldg(&E.ms[k]);
-    grp_range(L, eom_grp(E, lb + lk - li, sb + sk - si), &gb, &ge);
-    for (int t = gb; t < ge; ++t) {
-      const int c = __ldg(&L.gmem[t]);
-      if (c >= n) sm -= dv_elem(L, H, hh, b, k, c, i) * eom_q(L, E, a, c, k, j);
+  for (int u = lane; u < 4 * n + 8; u += 32) {
+    int gb, ge;
+    if (u < 4 * n) {
+      // 22 -> 2, particle-hole: for hole k and term t the particle c lies in the
+      // group fixed by V's conservation: -+ V(p,k,c,h) Q(q,c,k,g), (p, q) = (b, a)
+      // or (a, b), (h, g) = (i, j) or (j, i)
+      const int k = u >> 2, t = u & 3;
+      const int p = t & 1 ? a : b, q = t & 1 ? b : a, h = t & 2 ? j : i, g = t & 2 ? i : j;
+      grp_range(L, eom_grp(E, __ldg(&E.ml[p]) + __ldg(&E.ml[k]) - __ldg(&E.ml[h]),
+                           __ldg(&E.ms[p]) + __ldg(&E.ms[k]) - __ldg(&E.ms[h])), &gb, &ge);
+      double s = 0.0;
+#pragma unroll 4
+      for (int x = gb; x < ge; ++x) {
+        const int c = __ldg(&L.gmem[x]);
+        if (c >= n) s += eom_v(L, H, hh, p, k, c, h) * eom_q(L, E, q, c, k, g);
+      }
+      sm += t == 0 || t == 3 ? -s : s;
+      continue;
     }
-    grp_range(L, eom_grp(E, la + lk - li, sa + sk - si), &gb, &ge);
-    for (int t = gb; t < ge; ++t) {
-      const int c = __ldg(&L.gmem[t]);
-      if (c >= n) sm += dv_elem(L, H, hh, a, k, c, i) * eom_q(L, E, b, c, k, j);
-    }
-    grp_range(L, eom_grp(E, lb + lk - lj, sb + sk - sj), &gb, &ge);
-    for (int t = gb; t < ge; ++t) {
-      const int c = __ldg(&L.gmem[t]);
-      if (c >= n) sm += dv_elem(L, H, hh, b, k, c, j) * eom_q(L, E, a, c, k, i);
-    }
-    grp_range(L, eom_grp(E, la + lk - lj, sa + sk - sj), &gb, &ge);
-    for (int t = gb; t < ge; ++t) {
-      const int c = __ldg(&L.gmem[t]);
-      if (c >= n) sm -= dv_elem(L, H, hh, a, k, c, j) * eom_q(L, E, b, c, k, i);
+    const int t = (u - 4 * n) & 7, half = t & 1;
+    double s = 0.0;
+    if (t < 2) {  // 12 -> 2: f(a,c) Q(c,b,i,j) - f(b,c) Q(c,a,i,j), c particle
+      const int p = half ? b : a, q = half ? a : b;
+      grp_range(L, eom_grp(E, E.tml + __ldg(&E.ml[i]) + __ldg(&E.ml[j]) - __ldg(&E.ml[q]),
+                           E.tms + __ldg(&E.ms[i]) + __ldg(&E.ms[j]) - __ldg(&E.ms[q])), &gb, &ge);
+      for (int x = gb; x < ge; ++x) {
+        const int c = __ldg(&L.gmem[x]);
+        if (c >= n) s += eom_f(L, H, hh, p, c) * eom_q(L, E, c, q, i, j);
+      }
+      sm += half ? -s : s;
+    } else if (t < 4) {  // Qf(c,i) V(a,b,c,j) - Qf(c,j) V(a,b,c,i)
+      const int h = half ? j : i, g = half ? i : j;
+      grp_range(L, eom_grp(E, __ldg(&E.ml[h]) + E.tml, __ldg(&E.ms[h]) + E.tms), &gb, &ge);
+      for (int x = gb; x < ge; ++x) {
+        const int c = __ldg(&L.gmem[x]);
+        if (c >= n) s += eom_qf(L, E, c, h) * eom_v(L, H, hh, a, b, c, g);
+      }
+      sm += half ? -s : s;
+    } else if (t < 6) {  // -Q(a,b,k,j) f(k,i) + Q(a,b,k,i) f(k,j), k hole
+      const int h = half ? j : i, g = half ? i : j;
+      grp_range(L, eom_grp(E, __ldg(&E.ml[a]) + __ldg(&E.ml[b]) - E.tml - __ldg(&E.ml[g]),
+                           __ldg(&E.ms[a]) + __ldg(&E.ms[b]) - E.tms - __ldg(&E.ms[g])), &gb, &ge);
+      for (int x = gb; x < ge; ++x) {
+        const int k = __ldg(&L.gmem[x]);
+        if (k < n) s += eom_q(L, E, a, b, k, g) * eom_f(L, H, hh, k, h);
+      }
+      sm += half ? s : -s;
+    } else {  // -V(b,k,j,i) Qf(a,k) + V(a,k,j,i) Qf(b,k)
+      const int p = half ? a : b, q = half ? b : a;
+      grp_range(L, eom_grp(E, __ldg(&E.ml[q]) - E.tml, __ldg(&E.ms[q]) - E.tms), &gb, &ge);
+      for (int x = gb; x < ge; ++x) {
+        const int k = __ldg(&L.gmem[x]);
+        if (k < n) s += eom_v(L, H, hh, p, k, j, i) * eom_qf(L, E, q, k);
+      }
+      sm += half ? s : -s;
     }
   }
-  w[e] = wb[pos2[e]] + sm;
+  for (int d = 16; d > 0; d >>= 1) sm += __shfl_down_sync(0xffffffffu, sm, d);
+  if (lane == 0) w[e] = wb[pos2[e]] + sm;
 }
 
-constexpr int EOM1_THREADS = 128;
+constexpr int EOM1_THREADS = 256;
 
 // HQ_comm_1b(a, i) (src/commutators.f90:1162-1211), one CTA per entry.
-__global__ void __launch_bounds__(EOM1_THREADS, 4) k_eom_1b(DevLayout L, EomDev E, const double* __restrict__ H,
+__global__ void __launch_bounds__(EOM1_THREADS, 2) k_eom_1b(DevLayout L, EomDev E, const double* __restrict__ H,
                                                          double hh, const int2* __restrict__ out1,
                                                          double* __restrict__ w) {
   __shared__ double red[EOM1_THREADS / 32];
@@ -237,27 +238,28 @@ __global__ void __launch_bounds__(EOM1_THREADS, 4) k_eom_1b(DevLayout L, EomDev 
       if (b >= n) sm += eom_qf(L, E, b, j) * dv_elem(L, H, hh, a, j, i, b);
     }
   }
-  // 22 -> 1: sum over b < c particles and holes j of Q(c,b,i,j) V(a,j,c,b);
-  // V is non-zero only for the particle pairs of the block of (a, j)
-  for (int j = 0; j < n; ++j) {
+  // 22 -> 1: sum over b < c particles and holes j of Q(c,b,i,j) V(a,j,c,b); V
+  // is non-zero only for the particle pairs of the block of (a, j).  A warp
+  // per hole, its lanes along the pairs.
+  const int lane = tid & 31, wp = tid >> 5;
+  for (int j = wp; j < n; j += EOM1_THREADS / 32) {
     const int ep = __ldg(&L.ptab[a * L.m + j]);
     const int q = pt_blk(ep);
     const int npp = __ldg(&L.blk[q]).z;
-    for (int k = tid; k < npp; k += EOM1_THREADS) {
+#pragma unroll 4
+    for (int k = lane; k < npp; k += 32) {
       const int2 bc = block_pair(L, q, 2, k);  // b < c
-      sm += eom_q(L, E, bc.y, bc.x, i, j) * dv_elem(L, H, hh, a, j, bc.y, bc.x);
+      sm += eom_q(L, E, bc.y, bc.x, i, j) * dv_at(dv_pos(L, ep, __ldg(&L.ptab[bc.y * L.m + bc.x])), H, hh);
     }
   }
   //          minus the sum over particles b and holes k < j of Q(a,b,k,j) V(k,j,i,b)
-  for (int k = tid; k < n; k += EOM1_THREADS) {
-    const int lk = __ldg(&E.ml[k]), sk = __ldg(&E.ms[k]);
-    for (int j = k + 1; j < n; ++j) {
-      const int lj = __ldg(&E.ml[j]), sj = __ldg(&E.ms[j]);
-      grp_range(L, eom_grp(E, lk + lj - li, sk + sj - si), &gb, &ge);
-      for (int t = gb; t < ge; ++t) {
-        const int b = __ldg(&L.gmem[t]);
-        if (b >= n) sm -= eom_q(L, E, a, b, k, j) * dv_elem(L, H, hh, k, j, i, b);
-      }
+  for (int kj = tid; kj < n * n; kj += EOM1_THREADS) {
+    const int k = kj / n, j = kj - k * n;
+    if (j <= k) continue;
+    grp_range(L, eom_grp(E, __ldg(&E.ml[k]) + __ldg(&E.ml[j]) - li, __ldg(&E.ms[k]) + __ldg(&E.ms[j]) - si), &gb, &ge);
+    for (int t = gb; t < ge; ++t) {
+      const int b = __ldg(&L.gmem[t]);
+      if (b >= n) sm -= eom_q(L, E, a, b, k, j) * eom_v(L, H, hh, k, j, i, b);
     }
   }
   sm = block_sum<EOM1_THREADS>(sm, red);
@@ -488,8 +490,9 @@ extern "C" int qd_eom_matvec_target(const qd_op* H, int ml, int ms, const double
   if (p->n2 > 0) {
     const double* bufs[NBUF] = {H->d, p->d_qb, nullptr, nullptr, p->d_wb, nullptr, nullptr};
     EOM_TRY(run_program_f64(L, p->prog, bufs, 1.0, 1.0, H->zero_mask, 0u));
-    k_eom_2b<<<(unsigned)((p->n2 + 127) / 128), 128, 0, s>>>(L->dev, E, H->d, hh, p->d_out2, p->d_pos2, p->n2,
-                                                             p->d_wb, d_w + p->n1);
+    constexpr int W = EOM2_THREADS / 32;
+    k_eom_2b<<<(unsigned)((p->n2 + W - 1) / W), EOM2_THREADS, 0, s>>>(L->dev, E, H->d, hh, p->d_out2, p->d_pos2, p->n2,
+                                                                    p->d_wb, d_w + p->n1);
     ++L->nlaunch;
   }
   if (p->n1 > 0) {
