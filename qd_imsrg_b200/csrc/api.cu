@@ -369,11 +369,13 @@ struct Branches {
     }
     return QD_OK;
   }
-  int join() {
+  // wait for one branch, or for all (which ends the branches)
+  int join(int one = -1) {
     if (!on) return QD_OK;
-    on = false;
+    on = one >= 0;
     for (int k = 0; k < qd_layout::NSIDE; ++k) {
-      if (!((used >> k) & 1)) continue;
+      if (!((used >> k) & 1) || (one >= 0 && k != one)) continue;
+      used &= ~(1 << k);
       QD_CUDA(cudaEventRecord(L->ev_side[k], L->side[k]));
       QD_CUDA(cudaStreamWaitEvent(L->stream, L->ev_side[k], 0));
     }
@@ -441,12 +443,12 @@ int commutator_seq(qd_layout* L, const qd_op* A, const qd_op* B, qd_op* C, qd_op
     TRY(stage_one_body(L, A, B, C));
   }
   {
-    if (gen) TRY(br.side(1, &side));
+    TRY(br.side(1, &side));
     StageTimer tm(L, S_122);
-    TRY(launch_122(L, A, B, C->d, ladder_in_122(L, A), gen ? side : nullptr, upd));
+    TRY(launch_122(L, A, B, C->d, ladder_in_122(L, A), side, upd));
   }
   GemmProgram& ladders = ladder_program(L, A);
-  if (gen) TRY(br.join());  // the branches write parts that the rest adds to
+  TRY(br.join(1));  // the rest adds to the two-body parts
   if (!ladders.probs.empty()) TRY(stage_ladders(L, A, B, C, ladders));
   TRY(br.join());
   if (ph_short) {

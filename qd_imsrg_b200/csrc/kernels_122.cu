@@ -2372,9 +2372,9 @@ static int tune_122(qd_layout* L, Plan122* p, TaskSet* ts, const qd_op* A, const
 
 // Text summary of the autotuned buckets of every task set of the layout.
 static int launch_full(qd_layout* L, const Plan122* p, const Plan122::FullBucket& b, int threads, const qd_op* A,
-                       const qd_op* B, double* C) {
+                       const qd_op* B, double* C, cudaStream_t st) {
 #define QD_FULL_LAUNCH(NT, BOTH)                                                                                    \
-  k_122_full<NT, BOTH><<<b.count, NT, b.smem, L->stream>>>(L->dev, p->d_ftask + b.first, p->d_tiles, p->d_gpd, p->d_gpp, \
+  k_122_full<NT, BOTH><<<b.count, NT, b.smem, st>>>(L->dev, p->d_ftask + b.first, p->d_tiles, p->d_gpd, p->d_gpp, \
                                                            p->d_ftab, p->nfent, A->d, (double)A->herm, A->zero_mask, \
                                                            B->d, (double)B->herm, B->zero_mask, C)
   if (b.both) {
@@ -2405,7 +2405,7 @@ static int tune_full(qd_layout* L, Plan122* p, const qd_op* A, const qd_op* B) {
       b.ms[k] = 1e30f;
       for (int rep = 0; rep < 2; ++rep) {
         QD_CUDA(cudaEventRecord(e0, L->stream));
-        TRY(launch_full(L, p, b, nts[k], A, B, scratch));
+        TRY(launch_full(L, p, b, nts[k], A, B, scratch, L->stream));
         QD_CUDA(cudaEventRecord(e1, L->stream));
         QD_CUDA(cudaEventSynchronize(e1));
         float ms = 0.f;
@@ -2576,7 +2576,19 @@ int launch_122(qd_layout* L, const qd_op* A, const qd_op* B, double* C, bool lad
   ++L->nlaunch;
   if (full) {
     if (!p->full_tuned && !L->prof.on && !capturing(L->stream)) TRY(tune_full(L, p, A, B));
-    for (const Plan122::FullBucket& b : p->fbuckets) TRY(launch_full(L, p, b, b.threads, A, B, C));
+    // The buckets write different tiles: every other one on the second stream,
+    // after the F tables.  One after the other they leave most of a small
+    // basis's chip idle (two dense operators at N=6, R=10: 154 us in one
+    // stream, 146 with two); where the tiles fill the chip the caller gives
+    // no second stream.
+    if (st2 && st2 != L->stream && p->fbuckets.size() > 1) {
+      QD_CUDA(cudaEventRecord(L->ev_side[1], L->stream));
+      QD_CUDA(cudaStreamWaitEvent(st2, L->ev_side[1], 0));
+    } else {
+      st2 = L->stream;
+    }
+    for (size_t k = 0; k < p->fbuckets.size(); ++k)
+      TRY(launch_full(L, p, p->fbuckets[k], p->fbuckets[k].threads, A, B, C, k & 1 ? st2 : L->stream));
     return QD_OK;
   }
   if (!ts->tuned && !L->prof.on && !capturing(L->stream)) TRY(tune_122(L, p, ts, A, B, spA, spB));

@@ -300,8 +300,9 @@ int launch_221_fused(qd_layout* L, const qd_op* A, const qd_op* B, double* C);
 int gen_pppp_ctas(qd_layout* L, int* n);
 // ladder: for a generator-like A also the ladders of the blocks for which
 // gen_ladder_fused holds (the caller then runs prog_ladder_gen, not prog_ladder)
-// st2: stream for the parts other than C_pppp of a generator-like A (null:
-// the layout's); upd: update HS with C_pppp (generator-like A only)
+// st2: second stream: the parts other than C_pppp of a generator-like A,
+// every other launch of the tiles otherwise (null: the layout's); upd: update
+// HS with C_pppp (generator-like A only)
 int launch_122(qd_layout* L, const qd_op* A, const qd_op* B, double* C, bool ladder, cudaStream_t st2 = nullptr,
                const HsUpdate* upd = nullptr);
 bool gen_ladder_fused(const qd_layout* L, int q);
