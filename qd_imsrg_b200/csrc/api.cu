@@ -351,6 +351,9 @@ struct Branches {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     QD_CUDA(cudaStreamIsCapturing(L->stream, &cs));
     const bool cap = cs != cudaStreamCaptureStatusNone;
+    // the split form's programs share one set of slices and accumulators on
+    // the layout (run_program_split): they have to run one after the other
+    if (L->split_slices > 0) return QD_OK;
     if (L->prof.on || (!gen_like(A->zero_mask) && L->neq >= FORK_ENTRIES)) return QD_OK;
     if (!L->ev_fork) {
       if (cap) return QD_OK;  // no stream or event is created inside a capture
