@@ -388,14 +388,6 @@ struct Branches {
   ~Branches() {
     if (on) join();
   }
-  static int make_branches(qd_layout* L) {
-    for (int k = 0; k < qd_layout::NSIDE; ++k) {
-      QD_CUDA(cudaStreamCreateWithFlags(&L->side[k], cudaStreamNonBlocking));
-      QD_CUDA(cudaEventCreateWithFlags(&L->ev_side[k], cudaEventDisableTiming));
-    }
-    QD_CUDA(cudaEventCreateWithFlags(&L->ev_fork, cudaEventDisableTiming));
-    return QD_OK;
-  }
 };
 
 // The layout's launches go to another stream while this lives.
@@ -496,6 +488,16 @@ void drop_ws(const qd_layout* L) {
 }
 
 }  // namespace
+
+int qd::make_branches(qd_layout* L) {
+  if (L->ev_fork) return QD_OK;
+  for (int k = 0; k < qd_layout::NSIDE; ++k) {
+    QD_CUDA(cudaStreamCreateWithFlags(&L->side[k], cudaStreamNonBlocking));
+    QD_CUDA(cudaEventCreateWithFlags(&L->ev_side[k], cudaEventDisableTiming));
+  }
+  QD_CUDA(cudaEventCreateWithFlags(&L->ev_fork, cudaEventDisableTiming));
+  return QD_OK;
+}
 
 // A workspace operator of the layout that the full commutator never reads
 // or writes (the reference's w1/w2, which the fused 221 replaces), for the
@@ -1345,7 +1347,7 @@ int bch_step_launch(qd_layout* L, qd_op* HS, const qd_op* G, const qd_op* H, qd_
     TRY(prepare_program(L, L->prog_pandya, 0u, 0u));
     TRY(prepare_onebody(L));
     TRY(prepare_hs_update(L));
-    if (!L->ev_fork) TRY(Branches::make_branches(L));
+    if (!L->ev_fork) TRY(make_branches(L));
     TRY(prepare_122(L, G, &full));
     TRY(prepare_program(L, ladder_program(L, G), G->zero_mask, H->zero_mask));
     TRY(prepare_program(L, L->prog_111, G->zero_mask, H->zero_mask));

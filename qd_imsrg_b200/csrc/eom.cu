@@ -124,8 +124,9 @@ __device__ __forceinline__ double eom_v(const DevLayout& L, const double* __rest
 // One warp per entry: the particle-hole part has four terms for each hole k,
 // the others are eight short sums over one group each; the lanes take the
 // 4 n + 8 sums in turn, one shuffle tree adds them.  Bound: the chain of table
-// and element reads of a sum (with one thread per entry all 4 n + 8 followed
-// one another: 215 us for the 2p2h part at N=12, R=10).
+// and element reads of a sum.  With one thread per entry all 4 n + 8 followed
+// one another: at N=12, R=10 a whole product took 296 us, and 97 in this form
+// (of them this kernel 42).
 constexpr int EOM2_THREADS = 128;
 __global__ void __launch_bounds__(EOM2_THREADS) k_eom_2b(DevLayout L, EomDev E, const double* __restrict__ H,
                                                          double hh, const int4* __restrict__ out2,
@@ -436,6 +437,23 @@ void drop_eom_plans(const qd_layout* L) {
 
 using namespace qd;
 
+namespace {
+// the main stream s waits for branch 0 of the layout, on an error path too
+struct SideJoin {
+  qd_layout* L;
+  cudaStream_t s;
+  bool on = false;
+  int wait() {
+    if (!on) return QD_OK;
+    on = false;
+    QD_CUDA(cudaEventRecord(L->ev_side[0], L->side[0]));
+    QD_CUDA(cudaStreamWaitEvent(s, L->ev_side[0], 0));
+    return QD_OK;
+  }
+  ~SideJoin() { wait(); }
+};
+}  // namespace
+
 extern "C" int qd_eom_dim(const qd_layout* L, int ml, int ms, int64_t* n1, int64_t* n2) {
   if (!L || !n1 || !n2) {
     set_error("qd_eom_dim: null argument");
@@ -487,6 +505,23 @@ extern "C" int qd_eom_matvec_target(const qd_op* H, int ml, int ms, const double
   E.qf = p->d_qf;
   E.qb = p->d_qb;
   const double hh = (double)H->herm;
+  // the 1p1h part beside the GEMM and k_eom_2b, which write other entries
+  // (a product at N=12, R=10: 97 us when it followed them, 85 beside them)
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  QD_CUDA(cudaStreamIsCapturing(s, &cs));
+  if (cs == cudaStreamCaptureStatusNone) EOM_TRY(make_branches(L));  // nothing is created inside a capture
+  const bool side = p->n1 > 0 && p->n2 > 0 && L->ev_fork;
+  SideJoin join{L, s};  // waits on every way out: d_w is the caller's
+  if (side) {
+    QD_CUDA(cudaEventRecord(L->ev_fork, s));
+    QD_CUDA(cudaStreamWaitEvent(L->side[0], L->ev_fork, 0));
+    join.on = true;
+  }
+  if (p->n1 > 0) {
+    k_eom_1b<<<(unsigned)p->n1, EOM1_THREADS, 0, side ? L->side[0] : s>>>(L->dev, E, H->d, hh, p->d_out1, d_w);
+    ++L->nlaunch;
+    QD_CUDA(cudaGetLastError());
+  }
   if (p->n2 > 0) {
     const double* bufs[NBUF] = {H->d, p->d_qb, nullptr, nullptr, p->d_wb, nullptr, nullptr};
     EOM_TRY(run_program_f64(L, p->prog, bufs, 1.0, 1.0, H->zero_mask, 0u));
@@ -495,10 +530,6 @@ extern "C" int qd_eom_matvec_target(const qd_op* H, int ml, int ms, const double
                                                                     p->d_wb, d_w + p->n1);
     ++L->nlaunch;
   }
-  if (p->n1 > 0) {
-    k_eom_1b<<<(unsigned)p->n1, EOM1_THREADS, 0, s>>>(L->dev, E, H->d, hh, p->d_out1, d_w);
-    ++L->nlaunch;
-  }
   QD_CUDA(cudaGetLastError());
-  return QD_OK;
+  return join.wait();
 }

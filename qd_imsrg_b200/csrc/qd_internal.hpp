@@ -307,6 +307,7 @@ int launch_122(qd_layout* L, const qd_op* A, const qd_op* B, double* C, bool lad
                const HsUpdate* upd = nullptr);
 bool gen_ladder_fused(const qd_layout* L, int q);
 int launch_calc_cc(qd_layout* L, const qd_op* H, double* X);
+int make_branches(qd_layout* L);  // the side streams and events of a layout (api.cu)
 // Particle-hole channel (commutators.f90:716-980): C += the four re-coupled
 // Z terms, over the commutator_122 tiles (kernels_122.cu).
 int launch_pandya_tiles(qd_layout* L, const double* Z, double* C);
