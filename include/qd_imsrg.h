@@ -107,8 +107,8 @@ int qd_layout_profile_read(qd_layout* L, double* ms, int64_t* counts, int nstage
 /* number of kernels this library has launched for the layout so far        */
 int qd_layout_launches(const qd_layout* L, int64_t* n);
 /* The autotuner's choices so far, as text: the first commutator_122 launch
- * for each pair of zero-part masks times every launch bucket with 128- and
- * 256-thread CTAs and keeps the faster (results do not depend on it).
+ * for each pair of zero-part masks times every launch bucket with 64-, 128-
+ * and 256-thread CTAs and keeps the fastest (results do not depend on it).
  * Writes at most len bytes (NUL-terminated) into buf; *needed = full size.
  * No reference counterpart.                                                 */
 int qd_layout_tuning(const qd_layout* L, char* buf, int64_t len, int64_t* needed);
@@ -327,11 +327,10 @@ int qd_flow_omega(const qd_flow* flow, qd_op** G);
 int qd_flow_state(const qd_flow* flow, qd_flow_result* result);
 int qd_flow_destroy(qd_flow* flow);
 /* Several independent flows (e.g. a grid of (N, hbar-omega, emax)), one per
- * layout.  Default: the instances advance in lockstep on one stream, and each
- * BCH term's commutator_122 tiles and ladder GEMM tasks of every instance
- * whose series is still running go into one launch per kernel (uneven blocks
- * of all instances in one task list, longest first); the small stages run
- * per instance.  flags | QD_BATCH_STREAMS instead runs one host thread per
+ * layout.  Default: the instances advance in lockstep, each on its own
+ * layout's stream; the BCH steps (graphs) of every instance not yet converged
+ * are launched before the host waits for any, so that the instances' kernels
+ * fill the chip together.  flags | QD_BATCH_STREAMS instead runs one host thread per
  * instance on its own layout's stream (each flow as qd_magnus_flow, BCH steps
  * as graphs).  Results equal the separate flows'.  No reference counterpart
  * (the reference runs one flow per process).  status[i] is instance i's

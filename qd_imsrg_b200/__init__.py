@@ -463,9 +463,9 @@ class DeviceView:
 def magnus_flow_batch(pairs, pandya: bool = False, max_iter: int = 500, raise_on_error: bool = True,
                       streams: bool = False):
     """Run several independent flows: pairs = [(HAM, HS), ...], each pair on
-    its own layout.  Default: lockstep, each BCH term's 122 tiles and ladder
-    tasks of all instances in one launch per kernel; streams=True: one host
-    thread and stream per instance.  Returns ([FlowResult], [status]); with
+    its own layout.  Default: lockstep, each on its own layout's
+    stream, the steps of all launched before any is waited for; streams=True:
+    one host thread and stream per instance.  Returns ([FlowResult], [status]); with
     raise_on_error, raises QDError for the first failing instance."""
     n = len(pairs)
     hams = (C.c_void_p * n)(*[h.h.value for h, _ in pairs])

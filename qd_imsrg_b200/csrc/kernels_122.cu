@@ -643,7 +643,8 @@ constexpr int MULT_MASK = 0x3FFFFFFF;
 // a CTA's chain of dependent table reads (~4 us) is the same for any size:
 // the 32 x 32 tiles used before paid it four times as often, and the ladder
 // as a separate read-modify-write of C_pppp moved its half that has hh pairs
-// twice more.  Times of both forms stand at launch_122_gen.
+// twice more (a commutator [Omega, X] at N=20, R=20: 875 us with these, 750
+// with this kernel).
 constexpr int GP_B = 64, GP_LD = GP_B + 1, GP_T = 256, GP_KMAX = 16;
 
 // A warp takes one column at a time, its lanes the rows l and l + 32: a staged

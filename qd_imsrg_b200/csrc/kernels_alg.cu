@@ -268,8 +268,8 @@ constexpr int AXN_BLOCKS = 4 * 148, AXN_THREADS = 256;
 // coefficient index is *kidx, continue while |INT2| cof / |INT1| >= conv and
 // fewer than 11 terms ran; the answer sets the graph's loop condition (and,
 // for the first term of a two-term loop body, the condition of the second),
-// and *kidx advances by one.  (As two more launches, a final sum and the
-// test, a term of a small flow took 6 us more.)  Every CTA calls this after
+// and *kidx advances by one, without the two more launches that a final sum
+// and the test would be.  Every CTA calls this after
 // its partial sums are written; count returns to zero for the next launch.
 __device__ __forceinline__ void axn_finish(const double2* partial, int np, unsigned* count, double* out, int* kidx,
                                            const BchDecide& D) {
