@@ -370,7 +370,7 @@ int eom_upload(EomPlan& p, T** dst, const T* src, size_t count) {
   if (count == 0) return QD_OK;
   QD_CUDA(cudaMalloc((void**)dst, count * sizeof(T)));
   p.allocs.push_back(*dst);
-  if (src) QD_CUDA(cudaMemcpy(*dst, src, count * sizeof(T), cudaMemcpyHostToDevice));
+  if (src) QD_CUDA(copy_table(*dst, src, count * sizeof(T)));
   return QD_OK;
 }
 

@@ -713,9 +713,9 @@ int build_programs(qd_layout* L) {
     QD_CUDA(cudaMalloc(&P->d_probs, pb));
     QD_CUDA(cudaMalloc(&P->d_segs, sb));
     if (!P->probs.empty())
-      QD_CUDA(cudaMemcpy(P->d_probs, P->probs.data(), P->probs.size() * sizeof(GProb), cudaMemcpyHostToDevice));
+      QD_CUDA(copy_table(P->d_probs, P->probs.data(), P->probs.size() * sizeof(GProb)));
     if (!P->segs.empty())
-      QD_CUDA(cudaMemcpy(P->d_segs, P->segs.data(), P->segs.size() * sizeof(GSeg), cudaMemcpyHostToDevice));
+      QD_CUDA(copy_table(P->d_segs, P->segs.data(), P->segs.size() * sizeof(GSeg)));
   }
   QD_CUDA(cudaFuncSetAttribute(k_grouped_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMM_SMEM));
   QD_CUDA(cudaFuncSetAttribute(k_gemm_kshort, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)KS_SMEM));
@@ -729,9 +729,9 @@ static int upload_program(GemmProgram& P) {
   QD_CUDA(cudaMalloc(&P.d_probs, pb));
   QD_CUDA(cudaMalloc(&P.d_segs, sb));
   if (!P.probs.empty())
-    QD_CUDA(cudaMemcpy(P.d_probs, P.probs.data(), P.probs.size() * sizeof(GProb), cudaMemcpyHostToDevice));
+    QD_CUDA(copy_table(P.d_probs, P.probs.data(), P.probs.size() * sizeof(GProb)));
   if (!P.segs.empty())
-    QD_CUDA(cudaMemcpy(P.d_segs, P.segs.data(), P.segs.size() * sizeof(GSeg), cudaMemcpyHostToDevice));
+    QD_CUDA(copy_table(P.d_segs, P.segs.data(), P.segs.size() * sizeof(GSeg)));
   return QD_OK;
 }
 
@@ -856,7 +856,7 @@ static int get_tasks(qd_layout* L, GemmProgram& P, unsigned mA, unsigned mB, GTa
     for (size_t i = 0; i < v[w].size(); ++i) h[i] = v[w][i].second;
     if (!h.empty()) {
       QD_CUDA(cudaMalloc(&d[w], h.size() * sizeof(GTask)));
-      QD_CUDA(cudaMemcpy(d[w], h.data(), h.size() * sizeof(GTask), cudaMemcpyHostToDevice));
+      QD_CUDA(copy_table(d[w], h.data(), h.size() * sizeof(GTask)));
     }
   }
   P.tasks[key] = std::make_pair(d[0], (int)v[0].size());

@@ -1629,7 +1629,7 @@ size_t zero_smem(const TileInfo& t) { return 8 * (size_t)t.npair; }
 template <class T>
 int upload_vec(qd_layout* L, const std::vector<T>& vec, T** dptr) {
   QD_CUDA(cudaMalloc(dptr, std::max<size_t>(1, vec.size()) * sizeof(T)));
-  if (!vec.empty()) QD_CUDA(cudaMemcpy(*dptr, vec.data(), vec.size() * sizeof(T), cudaMemcpyHostToDevice));
+  if (!vec.empty()) QD_CUDA(copy_table(*dptr, vec.data(), vec.size() * sizeof(T)));
   L->ws_bytes += (i64)(vec.size() * sizeof(T));
   return QD_OK;
 }

@@ -421,7 +421,7 @@ int prepare_hs_update(qd_layout* L) {
   void* p = nullptr;
   QD_CUDA(cudaMalloc(&p, sizeof(longlong2) * std::max<size_t>(1, v.size())));
   L->dev_allocs.push_back(p);
-  QD_CUDA(cudaMemcpy(p, v.data(), sizeof(longlong2) * v.size(), cudaMemcpyHostToDevice));
+  QD_CUDA(copy_table(p, v.data(), sizeof(longlong2) * v.size()));
   L->d_axrest = (const longlong2*)p;
   L->naxrest = (int)v.size();
   const size_t bytes = sizeof(double) * 2 * (size_t)std::max(1, L->naxp + L->naxrest);
@@ -548,7 +548,7 @@ int launch_calc_cc(qd_layout* L, const qd_op* H, double* X) {
     void* p = nullptr;
     QD_CUDA(cudaMalloc(&p, sizeof(int4) * std::max<size_t>(1, v.size())));
     L->dev_allocs.push_back(p);
-    QD_CUDA(cudaMemcpy(p, v.data(), sizeof(int4) * v.size(), cudaMemcpyHostToDevice));
+    QD_CUDA(copy_table(p, v.data(), sizeof(int4) * v.size()));
     L->ncctask = (int)v.size();
     L->d_cctask = (const int4*)p;
   }

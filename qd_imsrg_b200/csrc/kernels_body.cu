@@ -459,7 +459,7 @@ int launch_221_fused(qd_layout* L, const qd_op* A, const qd_op* B, double* C) {
     void* p = nullptr;
     QD_CUDA(cudaMalloc(&p, sizeof(int) * std::max<size_t>(1, tg.size())));
     L->dev_allocs.push_back(p);
-    if (!tg.empty()) QD_CUDA(cudaMemcpy(p, tg.data(), sizeof(int) * tg.size(), cudaMemcpyHostToDevice));
+    if (!tg.empty()) QD_CUDA(copy_table(p, tg.data(), sizeof(int) * tg.size()));
     L->d_tgt221 = (const int*)p;
     L->ntgt221 = (int)tg.size();
   }

@@ -261,7 +261,7 @@ static int up(qd_layout* L, const std::vector<T>& v, const T** out) {
   void* p = nullptr;
   QD_CUDA(cudaMalloc(&p, bytes));
   L->dev_allocs.push_back(p);
-  if (!v.empty()) QD_CUDA(cudaMemcpy(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));
+  if (!v.empty()) QD_CUDA(copy_table(p, v.data(), v.size() * sizeof(T)));
   *out = (const T*)p;
   return QD_OK;
 }

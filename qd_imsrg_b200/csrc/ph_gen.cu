@@ -103,7 +103,7 @@ int pg_up(qd_layout* L, const std::vector<V>& v, const V** out) {
   QD_CUDA(cudaMalloc(&p, std::max<size_t>(1, v.size()) * sizeof(V)));
   L->dev_allocs.push_back(p);
   L->ws_bytes += (i64)(v.size() * sizeof(V));
-  if (!v.empty()) QD_CUDA(cudaMemcpy(p, v.data(), v.size() * sizeof(V), cudaMemcpyHostToDevice));
+  if (!v.empty()) QD_CUDA(copy_table(p, v.data(), v.size() * sizeof(V)));
   *out = (const V*)p;
   return QD_OK;
 }

@@ -226,6 +226,15 @@ int cuda_fail(cudaError_t e, const char* what);
     if (e_ != cudaSuccess) return qd::cuda_fail(e_, #call); \
   } while (0)
 
+// A plan's table from host memory, at its place when this returns.  A copy
+// from pageable memory may return before it has arrived, and the layouts'
+// streams do not wait for the legacy stream: a kernel launched next could
+// read what the (recycled) memory held before.
+inline cudaError_t copy_table(void* dst, const void* src, size_t bytes) {
+  const cudaError_t e = cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice);
+  return e != cudaSuccess ? e : cudaStreamSynchronize(cudaStreamLegacy);
+}
+
 int layout_build(qd_layout* L, int nbody, int emax, const double* eig);
 int layout_upload(qd_layout* L);
 void layout_free_device(qd_layout* L);

@@ -526,7 +526,7 @@ struct SplitState {
 template <class T>
 int upload(const std::vector<T>& h, T** d) {
   QD_CUDA(cudaMalloc((void**)d, std::max<size_t>(1, h.size()) * sizeof(T)));
-  if (!h.empty()) QD_CUDA(cudaMemcpy(*d, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice));
+  if (!h.empty()) QD_CUDA(copy_table(*d, h.data(), h.size() * sizeof(T)));
   return QD_OK;
 }
 

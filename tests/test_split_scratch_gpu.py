@@ -39,3 +39,23 @@ def test_split_programs_share_no_scratch(gen):
         assert np.array_equal(got, first)
     for X in (A, B, C):
         X.close()
+
+
+def test_new_layouts_in_recycled_memory():
+    """A layout's tables are in place before its first kernels read them, also
+    in memory that an earlier layout's tables left: every new layout's first
+    commutator is bitwise that of the first one, in both forms."""
+    first = {}
+    for k in range(8):
+        n, R = ((6, 8), (12, 7))[k % 2]
+        P = qd.Layout(n, R)
+        A, B, C = qd.random_operator(P, -1, 5), qd.random_operator(P, 1, 6), qd.FullHam(P, 1)
+        A, B = qd.FullHam(P, -1, A), qd.FullHam(P, 1, B)
+        for slices in (3, 0):
+            P.split = slices
+            qd.commutator(A, B, C, True)
+            out = C.download()
+            assert np.array_equal(out, first.setdefault((n, slices), out))
+        for X in (A, B, C):
+            X.close()
+        P.close()
