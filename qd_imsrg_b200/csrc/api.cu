@@ -314,13 +314,14 @@ int white(qd_op* gen, const qd_op* H) {
 // E0 and the one-body part of C = [A, B] (110, 220, 111, 121, 221): two
 // launches when both operands conserve (m_l, m_s), piece by piece otherwise.
 int stage_one_body(qd_layout* L, const qd_op* A, const qd_op* B, qd_op* C) {
-  bool done = false;
-  {
+  // the split form keeps the pieces: its 111 is a product of slices
+  if (L->split_slices == 0) {
+    bool done = false;
     StageTimer tm(L, S_221);
     TRY(launch_onebody(L, A, B, C->d, &done));
-    if (!done) tm.cancel();
+    if (done) return QD_OK;
+    tm.cancel();
   }
-  if (done) return QD_OK;
   TRY(stage_e0(L, A, B, C->d, 0.0));
   TRY(stage_111(L, A, B, C));
   {

@@ -1,11 +1,11 @@
 """The split form's programs of one commutator, which share a workspace of the
-layout, against the FP64 form and against themselves."""
+layout, against the FP64 form, against themselves and against the pieces."""
 import numpy as np
 import pytest
 
 import oracle
 import qd_imsrg_b200 as qd
-from helpers import compare_parts, part_slices
+from helpers import compare_parts, numpy_random_op, part_slices
 
 pytestmark = pytest.mark.gpu
 
@@ -39,6 +39,30 @@ def test_split_programs_share_no_scratch(gen):
         assert np.array_equal(got, first)
     for X in (A, B, C):
         X.close()
+
+
+@pytest.mark.parametrize("n,R", [(2, 4), (6, 8)])
+@pytest.mark.parametrize("slices", [3, 6])
+def test_split_one_body_is_the_sliced_111(n, R, slices):
+    """The one-body part of a commutator in the split form is the sliced 111
+    plus the FP64 121 and 221, to the bar of the plain form (1e-12 per part);
+    a 111 in FP64 would differ by the slices' truncation (1e-8 with three)."""
+    P, O = qd.Layout(n, R), oracle.Layout(n, R)
+    rng = np.random.default_rng(n + R)
+    a, b = (numpy_random_op(O, h, rng, conserve=True) for h in (-1, 1))
+    A, B = qd.FullHam(P, -1, a), qd.FullHam(P, 1, b)
+    C, D, w1, w2 = (qd.FullHam(P, 1) for _ in range(4))
+    P.split = slices
+    qd.commutator(A, B, C, True)
+    qd.set_to_zero(D)
+    qd.commutator_111(A, B, D)
+    P.split = 0
+    qd.commutator_121(A, B, D)
+    qd.commutator_221(A, B, D, w1, w2)
+    got, want = C.download(), D.download()
+    for name, s in dict(part_slices(O)).items():
+        if name in ("fhh", "fpp", "fph"):
+            assert np.abs(got[s] - want[s]).max() <= 1e-12 * np.abs(want[s]).max(), name
 
 
 def test_new_layouts_in_recycled_memory():
