@@ -347,14 +347,12 @@ struct Branches {
   qd_layout* L = nullptr;
   bool on = false;
   int used = 0;  // bit k: branch k has work
+  int open = 0;  // bit k: branch k may have work
   int fork(qd_layout* l, const qd_op* A) {
     L = l;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     QD_CUDA(cudaStreamIsCapturing(L->stream, &cs));
     const bool cap = cs != cudaStreamCaptureStatusNone;
-    // the split form's programs share one set of slices and accumulators on
-    // the layout (run_program_split): they have to run one after the other
-    if (L->split_slices > 0) return QD_OK;
     if (L->prof.on || (!gen_like(A->zero_mask) && L->neq >= FORK_ENTRIES)) return QD_OK;
     if (!L->ev_fork) {
       if (cap) return QD_OK;  // no stream or event is created inside a capture
@@ -362,12 +360,20 @@ struct Branches {
     }
     QD_CUDA(cudaEventRecord(L->ev_fork, L->stream));
     on = true;
+    // The split form's programs (111, the products, the ladders) share one set
+    // of slices and accumulators on the layout (run_program_split): they stay
+    // in order on the main stream, and only 122, which uses none of these,
+    // runs beside them (all in one stream and 122 beside: [Omega, X] with three
+    // slices at N=6, R=15 328 and 276 us, two dense operators with three at
+    // N=6, R=10 364 and 347 us).
+    open = L->split_slices > 0 ? 1 << 1 : (1 << qd_layout::NSIDE) - 1;
     return QD_OK;
   }
   // stream of branch k (the main one without branches)
   int side(int k, cudaStream_t* st) {
-    *st = on ? L->side[k] : L->stream;
-    if (on && !((used >> k) & 1)) {
+    const bool go = on && ((open >> k) & 1);
+    *st = go ? L->side[k] : L->stream;
+    if (go && !((used >> k) & 1)) {
       QD_CUDA(cudaStreamWaitEvent(*st, L->ev_fork, 0));
       used |= 1 << k;
     }
