@@ -139,8 +139,9 @@ int same_layout(const qd_op* a, const qd_op* b) {
   CHECK(a && b, QD_ERR_ARG, "null operator handle");
   CHECK(a->L == b->L, QD_ERR_ARG, "operators belong to different layouts");
   // an operand whose raw pointer the caller holds may have been written since
+  // its mask was set (by an upload, a copy, a result): nothing is known zero
   for (const qd_op* o : {a, b})
-    if (o->exposed) const_cast<qd_op*>(o)->zero_mask &= ~CONSERVES;
+    if (o->exposed) const_cast<qd_op*>(o)->zero_mask = 0;
   return QD_OK;
 }
 
@@ -820,7 +821,7 @@ int qd_add_arrays(const qd_op* r1, double s1, const qd_op* r2, double s2, qd_op*
   qd_layout* L = r1->L;
   TRY(use_device(L));
   // two generators into one that already holds zeros elsewhere (euler_step)
-  if (std::isfinite(s1) && std::isfinite(s2) && gen_like(r1->zero_mask & r2->zero_mask & r3->zero_mask) && !r1->exposed && !r2->exposed && !r3->exposed)
+  if (std::isfinite(s1) && std::isfinite(s2) && gen_like(r1->zero_mask & r2->zero_mask & r3->zero_mask))
     TRY(launch_axpy_gen(L, r1->d, s1, r2->d, s2, r3->d));
   else
     TRY(launch_axpy(L, r1->d, s1, r2->d, s2, r3->d, L->neq));

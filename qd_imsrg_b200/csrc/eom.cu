@@ -524,7 +524,7 @@ extern "C" int qd_eom_matvec_target(const qd_op* H, int ml, int ms, const double
   }
   if (p->n2 > 0) {
     const double* bufs[NBUF] = {H->d, p->d_qb, nullptr, nullptr, p->d_wb, nullptr, nullptr};
-    EOM_TRY(run_program_f64(L, p->prog, bufs, 1.0, 1.0, H->zero_mask, 0u));
+    EOM_TRY(run_program_f64(L, p->prog, bufs, 1.0, 1.0, H->exposed ? 0u : H->zero_mask, 0u));
     constexpr int W = EOM2_THREADS / 32;
     k_eom_2b<<<(unsigned)((p->n2 + W - 1) / W), EOM2_THREADS, 0, s>>>(L->dev, E, H->d, hh, p->d_out2, p->d_pos2, p->n2,
                                                                     p->d_wb, d_w + p->n1);
