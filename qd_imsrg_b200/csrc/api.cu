@@ -1500,8 +1500,9 @@ int flow_eta_norm(qd_flow* f, const qd_op* op, double* out) { return qd_mat_2_no
 int flow_home_hs(qd_flow* f) {
   if (f->HS->d == f->hs_home) return QD_OK;
   QD_CUDA(cudaMemcpyAsync(f->hs_home, f->HS->d, sizeof(double) * f->L->neq, cudaMemcpyDeviceToDevice, f->L->stream));
+  const unsigned zero = f->HS->zero_mask;
   swap_ops(f->HS, f->HS0);  // HS0 held hs_home: after the swap HS->d == hs_home again
-  f->HS0->zero_mask = f->HS->zero_mask;
+  f->HS->zero_mask = f->HS0->zero_mask = zero;  // both buffers hold HS now
   return QD_OK;
 }
 

@@ -1,11 +1,12 @@
 """What the library knows to be zero in an operator is never trusted where
-that may have changed: after a caller's write through a raw pointer."""
+that may have changed: after a caller's write through a raw pointer, and in
+the result of a flow, whose buffers change places."""
 import numpy as np
 import pytest
 
 import oracle
 import qd_imsrg_b200 as qd
-from helpers import compare_parts, numpy_random_op
+from helpers import compare_parts, numpy_random_op, part_slices, synth_hamiltonian
 
 pytestmark = pytest.mark.gpu
 
@@ -69,3 +70,28 @@ def test_eom_product_of_a_written_hamiltonian(gpu):
     got = np.asarray(qd.eom_matvec_target(H, 1, 0, v))
     want = np.asarray(qd.eom_matvec_target(ref, 1, 0, v))
     assert np.linalg.norm(got - want) <= 1e-13 * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("steps", [1, 2])
+def test_result_of_a_short_flow(gpu, steps):
+    n, R = 6, 5
+    O = oracle.Layout(n, R)
+    rng = np.random.default_rng(23)
+    h, b = synth_hamiltonian(O, rng), numpy_random_op(O, -1, rng)
+    for name, ix in part_slices(O):
+        if name in ("Vppph", "Vphhh"):
+            h[ix] = 0.0  # in H, but not in the evolved operator
+    P = qd.Layout(n, R)
+    H, HS = qd.FullHam(P, 1, h), qd.FullHam(P, 1)
+    f = qd.Flow(H, HS)
+    for _ in range(steps):
+        assert f.step().accepted
+    f.close()  # HS is the caller's again
+    hs = HS.download()
+    ix = dict(part_slices(O))["Vppph"]
+    assert np.abs(hs[ix]).max() > 1e-6
+    B, C = qd.FullHam(P, -1, b), qd.FullHam(P, 1)
+    qd.commutator(HS, B, C, pandya=True)
+    oA, oB, oC = oracle.Op(O, 1, hs), oracle.Op(O, -1, b), oracle.Op(O, 1)
+    oracle.commutator(oA, oB, oC, True)
+    compare_parts(O, C.download(), oC.get(), rtol=1e-12, atol=1e-13)
