@@ -28,6 +28,7 @@ void set_error(const char* fmt, ...) {
 
 int cuda_fail(cudaError_t e, const char* what) {
   set_error("CUDA error %d (%s) in %s", (int)e, cudaGetErrorString(e), what);
+  (void)cudaGetLastError();  // reported here: not again by the next launch's check
   return e == cudaErrorMemoryAllocation ? QD_ERR_OOM : QD_ERR_CUDA;
 }
 
@@ -300,6 +301,35 @@ int layout_upload(qd_layout* L) {
   if ((rc = up(L, L->pcum, &D.pcum))) return rc;
   D.ns2 = (int)L->s2off.size();
   D.o2 = L->o_fph + (i64)L->mp * L->n;
+  return QD_OK;
+}
+
+int PlanMemory::commit(qd_layout* L) {
+  const auto place = [](size_t* at, size_t bytes) {  // 256-byte boundaries, as cudaMalloc gives
+    const size_t o = *at;
+    *at += (bytes + 255) / 256 * 256;
+    return o;
+  };
+  size_t end = 0;
+  std::vector<size_t> to, ro;
+  for (const Piece& p : tables_) to.push_back(place(&end, p.bytes));
+  std::vector<unsigned char> host(end);
+  for (size_t k = 0; k < tables_.size(); ++k)
+    if (tables_[k].bytes) std::memcpy(host.data() + to[k], tables_[k].src, tables_[k].bytes);
+  for (const Piece& p : rooms_) ro.push_back(place(&end, p.bytes));
+  unsigned char* d = nullptr;
+  QD_CUDA(cudaMalloc((void**)&d, std::max<size_t>(1, end)));
+  if (!host.empty()) {
+    const cudaError_t e = copy_table(d, host.data(), host.size());
+    if (e != cudaSuccess) {
+      cudaFree(d);
+      return cuda_fail(e, "copy of a plan's tables");
+    }
+  }
+  L->dev_allocs.push_back(d);
+  L->ws_bytes += (i64)end;
+  for (size_t k = 0; k < tables_.size(); ++k) *tables_[k].out = d + to[k];
+  for (size_t k = 0; k < rooms_.size(); ++k) *rooms_[k].out = d + ro[k];
   return QD_OK;
 }
 

@@ -17,6 +17,7 @@
 // products 0.34 ms and re-coupling 0.33 ms in the general form, 0.083 ms for
 // all three kernels of this one.
 #include <algorithm>
+#include <memory>
 #include <vector>
 
 #include "dev_common.cuh"
@@ -97,17 +98,6 @@ __global__ void __launch_bounds__(PG_T) k_ph_gen(DevLayout L, PhTab T, const dou
   }
 }
 
-template <class V>
-int pg_up(qd_layout* L, const std::vector<V>& v, const V** out) {
-  void* p = nullptr;
-  QD_CUDA(cudaMalloc(&p, std::max<size_t>(1, v.size()) * sizeof(V)));
-  L->dev_allocs.push_back(p);
-  L->ws_bytes += (i64)(v.size() * sizeof(V));
-  if (!v.empty()) QD_CUDA(copy_table(p, v.data(), v.size() * sizeof(V)));
-  *out = (const V*)p;
-  return QD_OK;
-}
-
 }  // namespace
 
 struct PhGen {
@@ -129,8 +119,7 @@ void ph_gen_free(qd_layout* L) {
 // capture, which must not allocate).
 int prepare_ph_gen(qd_layout* L) {
   if (L->ph_gen) return QD_OK;
-  PhGen* p = new PhGen();
-  L->ph_gen = p;
+  std::unique_ptr<PhGen> p(new PhGen());  // the layout's when complete: a failure leaves no plan
   const int n = L->n, mp = L->mp, m = L->m;
   std::vector<i64> phbase((size_t)std::max(1, mp * n), 0), xoff(std::max(1, L->ncc), 0), yoff(std::max(1, L->ncc), 0);
   std::vector<int4> xtask, task;
@@ -162,21 +151,24 @@ int prepare_ph_gen(qd_layout* L) {
       for (int i = 0; i * PG_R < rows[slot]; ++i)
         for (int j = 0; j * PG_C < cols[slot]; ++j) task.push_back(int4{q, slot, i, j});
   }
-  int rc;
-  if ((rc = pg_up(L, task, &p->tab.task)) || (rc = pg_up(L, phbase, &p->tab.phbase)) ||
-      (rc = pg_up(L, xtask, &p->tab.xtask)) || (rc = pg_up(L, xoff, &p->tab.xoff)))
-    return rc;
   p->ntask = (int)task.size();
   p->nxtask = (int)xtask.size();
-  for (auto b : {std::make_pair(&p->d_xa, xa), std::make_pair(&p->d_y, ys)}) {
-    void* d = nullptr;
-    QD_CUDA(cudaMalloc(&d, sizeof(double) * std::max<i64>(1, b.second)));
-    L->dev_allocs.push_back(d);
-    L->ws_bytes += (i64)sizeof(double) * b.second;
-    *b.first = (double*)d;
+  PlanMemory mem;
+  mem.add(task, &p->tab.task);
+  mem.add(phbase, &p->tab.phbase);
+  mem.add(xtask, &p->tab.xtask);
+  mem.add(xoff, &p->tab.xoff);
+  mem.room(xa, &p->d_xa);
+  mem.room(ys, &p->d_y);
+  int rc = build_ph_products(L, prod, p->prog);
+  if (!rc) rc = prepare_program(L, p->prog, 0u, 0u);
+  if (!rc) rc = mem.commit(L);
+  if (rc) {
+    p->prog.clear_device();
+    return rc;
   }
-  if ((rc = build_ph_products(L, prod, p->prog))) return rc;
-  return prepare_program(L, p->prog, 0u, 0u);
+  L->ph_gen = p.release();
+  return QD_OK;
 }
 
 // The products of the particle-hole channel of [A, B] for a generator-like A,

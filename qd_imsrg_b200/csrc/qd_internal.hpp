@@ -235,6 +235,31 @@ inline cudaError_t copy_table(void* dst, const void* src, size_t bytes) {
   return e != cudaSuccess ? e : cudaStreamSynchronize(cudaStreamLegacy);
 }
 
+// Device memory of one plan, tables and scratch together in one allocation
+// that belongs to the layout, the tables brought there by one copy.  commit()
+// sets every pointer, or on failure none and keeps nothing.  The vectors given
+// to add() must live until then.
+class PlanMemory {
+ public:
+  template <class T>
+  void add(const std::vector<T>& v, const T** out) {
+    tables_.push_back(Piece{v.data(), v.size() * sizeof(T), (const void**)out});
+  }
+  template <class T>
+  void room(i64 n, T** out) {  // not initialised
+    rooms_.push_back(Piece{nullptr, (size_t)n * sizeof(T), (const void**)out});
+  }
+  int commit(qd_layout* L);
+
+ private:
+  struct Piece {
+    const void* src;
+    size_t bytes;
+    const void** out;
+  };
+  std::vector<Piece> tables_, rooms_;
+};
+
 int layout_build(qd_layout* L, int nbody, int emax, const double* eig);
 int layout_upload(qd_layout* L);
 void layout_free_device(qd_layout* L);
