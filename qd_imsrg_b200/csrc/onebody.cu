@@ -21,6 +21,7 @@
 // columns of every product from L2, about |g| times the traffic, and the
 // pieces ran as eleven launches; the times of both stand at launch_onebody).
 #include <algorithm>
+#include <memory>
 #include <vector>
 
 #include "dev_common.cuh"
@@ -357,17 +358,6 @@ __global__ void __launch_bounds__(OB_T) k_one_final(DevLayout L, OneTab T, const
   if (lane == 0) C[L.o_fhh + tg.x] = s;
 }
 
-template <class V>
-int ob_up(qd_layout* L, const std::vector<V>& v, const V** out) {
-  void* p = nullptr;
-  QD_CUDA(cudaMalloc(&p, std::max<size_t>(1, v.size()) * sizeof(V)));
-  L->dev_allocs.push_back(p);
-  L->ws_bytes += (i64)(v.size() * sizeof(V));
-  if (!v.empty()) QD_CUDA(copy_table(p, v.data(), v.size() * sizeof(V)));
-  *out = (const V*)p;
-  return QD_OK;
-}
-
 }  // namespace
 
 // Tables and buffers of one layout, built on first use.
@@ -387,8 +377,7 @@ void onebody_free(qd_layout* L) {
 
 static int onebody_plan(qd_layout* L) {
   if (L->onebody) return QD_OK;
-  OneBody* p = new OneBody();
-  L->onebody = p;
+  std::unique_ptr<OneBody> p(new OneBody());  // the layout's when complete: a failure leaves no plan
   const int m = L->m, n = L->n, mp = L->mp, ng = (int)L->gstart.size() - 1;
   std::vector<int> gslot(ng + 1, 0), ghole(ng, 0), kpos(m, 0);
   for (int g = 0; g < ng; ++g) {
@@ -405,7 +394,10 @@ static int onebody_plan(qd_layout* L) {
     }
   }
   if (m > 0x7FFF || m == 0) p->usable = false;
-  if (!p->usable) return QD_OK;
+  if (!p->usable) {
+    L->onebody = p.release();
+    return QD_OK;
+  }
   // hole units first: they are the longer ones
   std::vector<int4> unit;
   const int npu = (mp + OB_U - 1) / OB_U;
@@ -443,22 +435,22 @@ static int onebody_plan(qd_layout* L) {
   T.nslot = gslot[ng];
   T.nrow = nrow;
   T.q0 = L->ccmap[0].x;  // (0, 0): no transfer
-  int rc;
-  if ((rc = ob_up(L, unit, &T.unit)) || (rc = ob_up(L, piece, &T.piece)) || (rc = ob_up(L, gslot, &T.gslot)) ||
-      (rc = ob_up(L, ghole, &T.ghole)) || (rc = ob_up(L, target, &T.target)))
-    return rc;
-  std::vector<double> zp((size_t)nrow * T.nslot, 0.0), ze(std::max<size_t>(1, piece.size()), 0.0);
-  std::vector<int> zf(1, 0);
-  const double *dp, *de;
-  const int* df;
-  if ((rc = ob_up(L, zp, &dp)) || (rc = ob_up(L, ze, &de)) || (rc = ob_up(L, zf, &df))) return rc;
-  p->d_partial = const_cast<double*>(dp);
-  p->d_epart = const_cast<double*>(de);
-  p->d_flag = const_cast<int*>(df);
   const i64 n1 = nhh + npp + (i64)mp * n;
   p->grid1 = T.nunit + T.npiece + 1;
   p->grid2 = (T.ntarget + OB_T / 32 - 1) / (OB_T / 32) + (int)((n1 + OB_FILL - 1) / OB_FILL) + 1;
-  return QD_OK;
+  PlanMemory mem;
+  mem.add(unit, &T.unit);
+  mem.add(piece, &T.piece);
+  mem.add(gslot, &T.gslot);
+  mem.add(ghole, &T.ghole);
+  mem.add(target, &T.target);
+  // k_one_part writes every partial sum, dot and the flag before k_one_final reads them
+  mem.room((i64)nrow * T.nslot, &p->d_partial);
+  mem.room(T.npiece, &p->d_epart);
+  mem.room(1, &p->d_flag);
+  const int rc = mem.commit(L);
+  if (!rc) L->onebody = p.release();
+  return rc;
 }
 
 // Tables and buffers of the layout for onebody (ahead of a stream capture,

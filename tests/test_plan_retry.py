@@ -20,7 +20,8 @@ int main(int argc, char** argv) {
   for (int call = 0; call < 3; ++call) {
     int rc = -1;
     if (!strcmp(argv[1], "ph_gen")) rc = qd::prepare_ph_gen(L);
-    printf("%d %d %zu\n", rc != QD_OK, L->ph_gen != nullptr, L->dev_allocs.size());
+    if (!strcmp(argv[1], "onebody")) rc = qd::prepare_onebody(L);
+    printf("%d %d %zu\n", rc != QD_OK, L->ph_gen || L->onebody, L->dev_allocs.size());
   }
   return 0;
 }
@@ -46,6 +47,7 @@ def calls(program, what):
     return [tuple(int(x) for x in line.split()) for line in out.stdout.splitlines()]
 
 
-def test_particle_hole_plan(program):
+@pytest.mark.parametrize("plan", ["ph_gen", "onebody"])
+def test_failed_plan_is_not_kept(program, plan):
     # every call fails, no plan and no memory is kept
-    assert calls(program, "ph_gen") == [(1, 0, 0)] * 3
+    assert calls(program, plan) == [(1, 0, 0)] * 3
