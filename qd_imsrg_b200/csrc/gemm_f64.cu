@@ -570,8 +570,19 @@ const bool N_ = false, T_ = true;
 
 }  // namespace
 
-int build_programs(qd_layout* L) {
-  if (L->programs_built) return QD_OK;
+static int upload_program(GemmProgram& P) {
+  size_t pb = std::max<size_t>(1, P.probs.size()) * sizeof(GProb);
+  size_t sb = std::max<size_t>(1, P.segs.size()) * sizeof(GSeg);
+  QD_CUDA(cudaMalloc(&P.d_probs, pb));
+  QD_CUDA(cudaMalloc(&P.d_segs, sb));
+  if (!P.probs.empty())
+    QD_CUDA(copy_table(P.d_probs, P.probs.data(), P.probs.size() * sizeof(GProb)));
+  if (!P.segs.empty())
+    QD_CUDA(copy_table(P.d_segs, P.segs.data(), P.segs.size() * sizeof(GSeg)));
+  return QD_OK;
+}
+
+static int make_programs(qd_layout* L) {
   const int n = L->n, mp = L->mp;
   // ---- matrix_mult222 ladders (ACC into C) ----
   for (int gen = 0; gen < 2; ++gen) {
@@ -706,33 +717,29 @@ int build_programs(qd_layout* L) {
       if (q > qr) b.seg(BXA, L->ccxoff[qr], r, N_, -1, BXB, L->ccxoff[qr], r, T_, -1, L->ccdim[qr].y, -1.0, 1, 0);
     }
   }
-  // upload
   for (GemmProgram* P : {&L->prog_ladder, &L->prog_ladder_gen, &L->prog_221, &L->prog_111, &L->prog_pandya}) {
-    size_t pb = std::max<size_t>(1, P->probs.size()) * sizeof(GProb);
-    size_t sb = std::max<size_t>(1, P->segs.size()) * sizeof(GSeg);
-    QD_CUDA(cudaMalloc(&P->d_probs, pb));
-    QD_CUDA(cudaMalloc(&P->d_segs, sb));
-    if (!P->probs.empty())
-      QD_CUDA(copy_table(P->d_probs, P->probs.data(), P->probs.size() * sizeof(GProb)));
-    if (!P->segs.empty())
-      QD_CUDA(copy_table(P->d_segs, P->segs.data(), P->segs.size() * sizeof(GSeg)));
+    const int rc = upload_program(*P);
+    if (rc) return rc;
   }
   QD_CUDA(cudaFuncSetAttribute(k_grouped_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMM_SMEM));
   QD_CUDA(cudaFuncSetAttribute(k_gemm_kshort, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)KS_SMEM));
-  L->programs_built = true;
   return QD_OK;
 }
 
-static int upload_program(GemmProgram& P) {
-  size_t pb = std::max<size_t>(1, P.probs.size()) * sizeof(GProb);
-  size_t sb = std::max<size_t>(1, P.segs.size()) * sizeof(GSeg);
-  QD_CUDA(cudaMalloc(&P.d_probs, pb));
-  QD_CUDA(cudaMalloc(&P.d_segs, sb));
-  if (!P.probs.empty())
-    QD_CUDA(copy_table(P.d_probs, P.probs.data(), P.probs.size() * sizeof(GProb)));
-  if (!P.segs.empty())
-    QD_CUDA(copy_table(P.d_segs, P.segs.data(), P.segs.size() * sizeof(GSeg)));
-  return QD_OK;
+// All programs of the layout or, on failure, none: the next call starts anew.
+int build_programs(qd_layout* L) {
+  if (L->programs_built) return QD_OK;
+  const int rc = make_programs(L);
+  if (!rc) {
+    L->programs_built = true;
+    return QD_OK;
+  }
+  for (GemmProgram* P : {&L->prog_ladder, &L->prog_ladder_gen, &L->prog_221, &L->prog_111, &L->prog_pandya}) {
+    P->clear_device();
+    P->probs.clear();
+    P->segs.clear();
+  }
+  return rc;
 }
 
 // The products of the particle-hole channel of a generator-like A (ph_gen.cu)
@@ -854,9 +861,13 @@ static int get_tasks(qd_layout* L, GemmProgram& P, unsigned mA, unsigned mB, GTa
   for (int w = 0; w < 2; ++w) {
     std::vector<GTask> h(v[w].size());
     for (size_t i = 0; i < v[w].size(); ++i) h[i] = v[w][i].second;
-    if (!h.empty()) {
-      QD_CUDA(cudaMalloc(&d[w], h.size() * sizeof(GTask)));
-      QD_CUDA(copy_table(d[w], h.data(), h.size() * sizeof(GTask)));
+    if (h.empty()) continue;
+    cudaError_t e = cudaMalloc(&d[w], h.size() * sizeof(GTask));
+    if (e == cudaSuccess) e = copy_table(d[w], h.data(), h.size() * sizeof(GTask));
+    if (e != cudaSuccess) {
+      for (GTask* p : d)
+        if (p) cudaFree(p);
+      return cuda_fail(e, "task lists");
     }
   }
   P.tasks[key] = std::make_pair(d[0], (int)v[0].size());

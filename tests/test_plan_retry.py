@@ -11,6 +11,7 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 PROGRAM = r"""
 #include <cstdio>
 #include <cstring>
+#include <initializer_list>
 
 #include "qd_internal.hpp"
 
@@ -21,6 +22,14 @@ int main(int argc, char** argv) {
     int rc = -1;
     if (!strcmp(argv[1], "ph_gen")) rc = qd::prepare_ph_gen(L);
     if (!strcmp(argv[1], "onebody")) rc = qd::prepare_onebody(L);
+    if (!strcmp(argv[1], "programs")) {
+      rc = qd::build_programs(L);
+      size_t n = 0;
+      for (qd::GemmProgram* P : {&L->prog_ladder, &L->prog_ladder_gen, &L->prog_221, &L->prog_111, &L->prog_pandya})
+        n += P->probs.size() + P->segs.size() + (P->d_probs || P->d_segs);
+      printf("%d %d %zu\n", rc != QD_OK, (int)L->programs_built, n);
+      continue;
+    }
     printf("%d %d %zu\n", rc != QD_OK, L->ph_gen || L->onebody, L->dev_allocs.size());
   }
   return 0;
@@ -47,7 +56,7 @@ def calls(program, what):
     return [tuple(int(x) for x in line.split()) for line in out.stdout.splitlines()]
 
 
-@pytest.mark.parametrize("plan", ["ph_gen", "onebody"])
+@pytest.mark.parametrize("plan", ["ph_gen", "onebody", "programs"])
 def test_failed_plan_is_not_kept(program, plan):
     # every call fails, no plan and no memory is kept
     assert calls(program, plan) == [(1, 0, 0)] * 3
