@@ -499,9 +499,9 @@ void drop_ws(const qd_layout* L) {
 
 int qd::make_branches(qd_layout* L) {
   if (L->ev_fork) return QD_OK;
-  for (int k = 0; k < qd_layout::NSIDE; ++k) {
-    QD_CUDA(cudaStreamCreateWithFlags(&L->side[k], cudaStreamNonBlocking));
-    QD_CUDA(cudaEventCreateWithFlags(&L->ev_side[k], cudaEventDisableTiming));
+  for (int k = 0; k < qd_layout::NSIDE; ++k) {  // a call after a failed one makes what is missing
+    if (!L->side[k]) QD_CUDA(cudaStreamCreateWithFlags(&L->side[k], cudaStreamNonBlocking));
+    if (!L->ev_side[k]) QD_CUDA(cudaEventCreateWithFlags(&L->ev_side[k], cudaEventDisableTiming));
   }
   QD_CUDA(cudaEventCreateWithFlags(&L->ev_fork, cudaEventDisableTiming));
   return QD_OK;

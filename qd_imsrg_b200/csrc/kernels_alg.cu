@@ -349,8 +349,14 @@ __global__ void __launch_bounds__(AXN_THREADS) k_axpy_norms(const double* a, dou
 static int ensure_axn(qd_layout* L) {
   if (L->d_axn) return QD_OK;
   const size_t bytes = sizeof(double2) * (AXN_BLOCKS + 1);
-  QD_CUDA(cudaMalloc(&L->d_axn, bytes));
-  QD_CUDA(cudaMemsetAsync(L->d_axn, 0, bytes, L->stream));
+  double* p = nullptr;
+  QD_CUDA(cudaMalloc(&p, bytes));
+  const cudaError_t e = cudaMemsetAsync(p, 0, bytes, L->stream);
+  if (e != cudaSuccess) {  // the counter has to be zero before the first update
+    cudaFree(p);
+    return cuda_fail(e, "cudaMemsetAsync(update sums)");
+  }
+  L->d_axn = p;
   L->ws_bytes += (i64)bytes;
   return QD_OK;
 }
@@ -418,16 +424,11 @@ int prepare_hs_update(qd_layout* L) {
     o = L->boff[6 * q + 2];
   }
   add(o, L->neq);
-  void* p = nullptr;
-  QD_CUDA(cudaMalloc(&p, sizeof(longlong2) * std::max<size_t>(1, v.size())));
-  L->dev_allocs.push_back(p);
-  QD_CUDA(copy_table(p, v.data(), sizeof(longlong2) * v.size()));
-  L->d_axrest = (const longlong2*)p;
+  PlanMemory mem;
+  mem.add(v, &L->d_axrest);
+  mem.room(2 * (i64)(L->naxp + (int)v.size()), &L->d_axp);
   L->naxrest = (int)v.size();
-  const size_t bytes = sizeof(double) * 2 * (size_t)std::max(1, L->naxp + L->naxrest);
-  QD_CUDA(cudaMalloc(&L->d_axp, bytes));
-  L->ws_bytes += (i64)(bytes + sizeof(longlong2) * v.size());
-  return QD_OK;
+  return mem.commit(L);
 }
 
 int hs_update_begin(qd_layout* L, const double* src, double* HS, double cof, int* kidx, HsUpdate* upd) {

@@ -361,9 +361,8 @@ void layout_free_device(qd_layout* L) {
   if (L->d_red) cudaFree(L->d_red);
   if (L->d_axn) cudaFree(L->d_axn);
   L->d_axn = nullptr;
-  if (L->d_axp) cudaFree(L->d_axp);
-  L->d_axp = nullptr;
-  L->d_axrest = nullptr;  // in dev_allocs
+  L->d_axp = nullptr;  // in dev_allocs, as d_axrest
+  L->d_axrest = nullptr;
   if (L->h_red) cudaFreeHost(L->h_red);
   L->d_z = nullptr;
   L->d_red = nullptr;
