@@ -351,10 +351,12 @@ struct qd_mlp {
   float *P = nullptr, *M = nullptr, *V = nullptr, *G = nullptr;
   bf16 *W2b = nullptr, *W2tb = nullptr;
   long long step = 0;
-  // activations for up to cap rows
-  qd::i64 cap = 0;
-  float *Z1 = nullptr, *Z2 = nullptr, *dH1 = nullptr;
-  bf16 *H1 = nullptr, *H1t = nullptr, *dZ2 = nullptr, *dZ2t = nullptr;
+  // activations of up to cap rows, and what a gradient needs beside them for up to gcap
+  qd::i64 cap = 0, gcap = 0;
+  bf16* H1 = nullptr;
+  float* Z2 = nullptr;
+  float *Z1 = nullptr, *dH1 = nullptr;
+  bf16 *H1t = nullptr, *dZ2 = nullptr, *dZ2t = nullptr;
   float *p23 = nullptr, *p1 = nullptr, *lpart = nullptr, *kpart = nullptr;  // partials per RB rows, dW2 slices
   float *s23 = nullptr, *s1 = nullptr, *h_loss = nullptr;                    // their sums; pinned copy of lpart
   int kslices = 0;
@@ -364,34 +366,52 @@ using namespace qd;
 
 namespace {
 void mlp_free_acts(qd_mlp* m) {
-  for (void* p : {(void*)m->Z1, (void*)m->Z2, (void*)m->dH1, (void*)m->H1, (void*)m->H1t, (void*)m->dZ2,
-                  (void*)m->dZ2t, (void*)m->kpart, (void*)m->p23, (void*)m->p1, (void*)m->lpart})
+  for (void* p : {(void*)m->H1, (void*)m->Z2})
     if (p) cudaFree(p);
-  if (m->h_loss) cudaFreeHost(m->h_loss);
-  m->Z1 = m->Z2 = m->dH1 = m->kpart = m->p23 = m->p1 = m->lpart = m->h_loss = nullptr;
-  m->H1 = m->H1t = m->dZ2 = m->dZ2t = nullptr;
+  m->H1 = nullptr;
+  m->Z2 = nullptr;
   m->cap = 0;
 }
+void mlp_free_grad(qd_mlp* m) {
+  for (void* p : {(void*)m->Z1, (void*)m->dH1, (void*)m->H1t, (void*)m->dZ2, (void*)m->dZ2t, (void*)m->kpart,
+                  (void*)m->p23, (void*)m->p1, (void*)m->lpart})
+    if (p) cudaFree(p);
+  if (m->h_loss) cudaFreeHost(m->h_loss);
+  m->Z1 = m->dH1 = m->kpart = m->p23 = m->p1 = m->lpart = m->h_loss = nullptr;
+  m->H1t = m->dZ2 = m->dZ2t = nullptr;
+  m->gcap = 0;
+}
 
+i64 mlp_rows(i64 n) { return (n + 1023) / 1024 * 1024; }
+
+// a forward pass of n rows: 1.5 KB a row
 int mlp_ensure(qd_mlp* m, i64 n) {
   if (n <= m->cap) return QD_OK;
   mlp_free_acts(m);
-  const i64 c = ((n + 1023) / 1024) * 1024;
-  QD_CUDA(cudaMalloc(&m->Z1, sizeof(float) * c * NH));
+  const i64 c = mlp_rows(n);
+  QD_CUDA(cudaMalloc(&m->H1, sizeof(bf16) * c * NH));
   QD_CUDA(cudaMalloc(&m->Z2, sizeof(float) * c * NH));
+  m->cap = c;
+  return QD_OK;
+}
+
+// a gradient of n rows: further 4.1 KB a row
+int mlp_ensure_grad(qd_mlp* m, i64 n) {
+  if (n <= m->gcap) return QD_OK;
+  mlp_free_grad(m);
+  const i64 c = mlp_rows(n), nch = c / RB;
+  QD_CUDA(cudaMalloc(&m->Z1, sizeof(float) * c * NH));
   QD_CUDA(cudaMalloc(&m->dH1, sizeof(float) * c * NH));
-  const i64 nch = c / RB;
   QD_CUDA(cudaMalloc(&m->p23, sizeof(float) * nch * (2 * NH + 1)));
   QD_CUDA(cudaMalloc(&m->p1, sizeof(float) * nch * (NH + NH * NI)));
   QD_CUDA(cudaMalloc(&m->lpart, sizeof(float) * nch));
   QD_CUDA(cudaMallocHost(&m->h_loss, sizeof(float) * nch));
-  QD_CUDA(cudaMalloc(&m->H1, sizeof(bf16) * c * NH));
   QD_CUDA(cudaMalloc(&m->H1t, sizeof(bf16) * c * NH));
   QD_CUDA(cudaMalloc(&m->dZ2, sizeof(bf16) * c * NH));
   QD_CUDA(cudaMalloc(&m->dZ2t, sizeof(bf16) * c * NH));
   m->kslices = (int)std::max<i64>(1, std::min<i64>(64, c / 512));
   QD_CUDA(cudaMalloc(&m->kpart, sizeof(float) * (size_t)m->kslices * NH * NH));
-  m->cap = c;
+  m->gcap = c;
   return QD_OK;
 }
 
@@ -439,7 +459,8 @@ int mlp_grad(qd_mlp* m, const float* X, const float* T, i64 n, float* G, bool wa
     set_error("qd_mlp: the batch (%lld rows) must be a positive multiple of %d", (long long)n, GBK);
     return QD_ERR_ARG;
   }
-  int rc = mlp_hidden(m, X, n, true, st);
+  int rc = mlp_ensure_grad(m, n);
+  if (!rc) rc = mlp_hidden(m, X, n, true, st);
   if (rc) return rc;
   const i64 nch = (n + RB - 1) / RB;
   k_tail<<<(unsigned)nch, NH, sizeof(float) * RB * NH, st>>>(m->Z2, m->P, T, n, m->dZ2, m->dZ2t, m->p23, m->lpart);
@@ -522,6 +543,7 @@ int qd_mlp_destroy(qd_mlp* m) {
   cudaSetDevice(m->device);
   cudaDeviceSynchronize();
   mlp_free_acts(m);
+  mlp_free_grad(m);
   for (void* p : {(void*)m->P, (void*)m->M, (void*)m->V, (void*)m->G, (void*)m->W2b, (void*)m->W2tb, (void*)m->s23,
                   (void*)m->s1})
     if (p) cudaFree(p);
