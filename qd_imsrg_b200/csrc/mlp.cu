@@ -353,66 +353,77 @@ struct qd_mlp {
   long long step = 0;
   // activations of up to cap rows, and what a gradient needs beside them for up to gcap
   qd::i64 cap = 0, gcap = 0;
+  void *acts = nullptr, *grads = nullptr;  // their memory, one allocation each
   bf16* H1 = nullptr;
   float* Z2 = nullptr;
   float *Z1 = nullptr, *dH1 = nullptr;
   bf16 *H1t = nullptr, *dZ2 = nullptr, *dZ2t = nullptr;
   float *p23 = nullptr, *p1 = nullptr, *lpart = nullptr, *kpart = nullptr;  // partials per RB rows, dW2 slices
-  float *s23 = nullptr, *s1 = nullptr, *h_loss = nullptr;                    // their sums; pinned copy of lpart
+  float *s23 = nullptr, *s1 = nullptr;                                       // their sums
+  std::vector<float> h_loss;        // host copy of lpart
+  cudaStream_t loss_st = nullptr;   // brings it while the rest of the gradient runs
+  cudaEvent_t loss_ev = nullptr;
   int kslices = 0;
 };
 
 using namespace qd;
 
 namespace {
-void mlp_free_acts(qd_mlp* m) {
-  for (void* p : {(void*)m->H1, (void*)m->Z2})
-    if (p) cudaFree(p);
-  m->H1 = nullptr;
-  m->Z2 = nullptr;
-  m->cap = 0;
-}
-void mlp_free_grad(qd_mlp* m) {
-  for (void* p : {(void*)m->Z1, (void*)m->dH1, (void*)m->H1t, (void*)m->dZ2, (void*)m->dZ2t, (void*)m->kpart,
-                  (void*)m->p23, (void*)m->p1, (void*)m->lpart})
-    if (p) cudaFree(p);
-  if (m->h_loss) cudaFreeHost(m->h_loss);
-  m->Z1 = m->dH1 = m->kpart = m->p23 = m->p1 = m->lpart = m->h_loss = nullptr;
-  m->H1t = m->dZ2 = m->dZ2t = nullptr;
-  m->gcap = 0;
+// n elements of T at the end of a memory plan of *bytes so far
+template <class T>
+T* mlp_place(void* base, size_t* bytes, i64 n) {
+  T* p = base ? reinterpret_cast<T*>((char*)base + *bytes) : nullptr;
+  *bytes += ((size_t)n * sizeof(T) + 255) / 256 * 256;
+  return p;
 }
 
 i64 mlp_rows(i64 n) { return (n + 1023) / 1024 * 1024; }
 
+// (Re)allocates *mem for what plan(base) places (called without memory first,
+// for the size).  cudaMalloc takes about 0.4 ms for arrays of this size: with
+// eleven of them, and 2.8 ms for pinned memory for the loss, a network's first
+// gradient (8,192 rows) took 5.4 ms and its destruction 3.3; now 0.8 and 0.9.
+template <class F>
+int mlp_alloc(void** mem, i64* cap, i64 rows, F plan) {
+  if (*mem) cudaFree(*mem);
+  *mem = nullptr;
+  *cap = 0;
+  QD_CUDA(cudaMalloc(mem, plan(nullptr)));
+  plan(*mem);
+  *cap = rows;
+  return QD_OK;
+}
+
 // a forward pass of n rows: 1.5 KB a row
 int mlp_ensure(qd_mlp* m, i64 n) {
   if (n <= m->cap) return QD_OK;
-  mlp_free_acts(m);
   const i64 c = mlp_rows(n);
-  QD_CUDA(cudaMalloc(&m->H1, sizeof(bf16) * c * NH));
-  QD_CUDA(cudaMalloc(&m->Z2, sizeof(float) * c * NH));
-  m->cap = c;
-  return QD_OK;
+  return mlp_alloc(&m->acts, &m->cap, c, [&](void* b) {
+    size_t o = 0;
+    m->H1 = mlp_place<bf16>(b, &o, c * NH);
+    m->Z2 = mlp_place<float>(b, &o, c * NH);
+    return o;
+  });
 }
 
 // a gradient of n rows: further 4.1 KB a row
 int mlp_ensure_grad(qd_mlp* m, i64 n) {
   if (n <= m->gcap) return QD_OK;
-  mlp_free_grad(m);
   const i64 c = mlp_rows(n), nch = c / RB;
-  QD_CUDA(cudaMalloc(&m->Z1, sizeof(float) * c * NH));
-  QD_CUDA(cudaMalloc(&m->dH1, sizeof(float) * c * NH));
-  QD_CUDA(cudaMalloc(&m->p23, sizeof(float) * nch * (2 * NH + 1)));
-  QD_CUDA(cudaMalloc(&m->p1, sizeof(float) * nch * (NH + NH * NI)));
-  QD_CUDA(cudaMalloc(&m->lpart, sizeof(float) * nch));
-  QD_CUDA(cudaMallocHost(&m->h_loss, sizeof(float) * nch));
-  QD_CUDA(cudaMalloc(&m->H1t, sizeof(bf16) * c * NH));
-  QD_CUDA(cudaMalloc(&m->dZ2, sizeof(bf16) * c * NH));
-  QD_CUDA(cudaMalloc(&m->dZ2t, sizeof(bf16) * c * NH));
   m->kslices = (int)std::max<i64>(1, std::min<i64>(64, c / 512));
-  QD_CUDA(cudaMalloc(&m->kpart, sizeof(float) * (size_t)m->kslices * NH * NH));
-  m->gcap = c;
-  return QD_OK;
+  return mlp_alloc(&m->grads, &m->gcap, c, [&](void* b) {
+    size_t o = 0;
+    m->Z1 = mlp_place<float>(b, &o, c * NH);
+    m->dH1 = mlp_place<float>(b, &o, c * NH);
+    m->H1t = mlp_place<bf16>(b, &o, c * NH);
+    m->dZ2 = mlp_place<bf16>(b, &o, c * NH);
+    m->dZ2t = mlp_place<bf16>(b, &o, c * NH);
+    m->p23 = mlp_place<float>(b, &o, nch * (2 * NH + 1));
+    m->p1 = mlp_place<float>(b, &o, nch * (NH + NH * NI));
+    m->lpart = mlp_place<float>(b, &o, nch);
+    m->kpart = mlp_place<float>(b, &o, (i64)m->kslices * NH * NH);
+    return o;
+  });
 }
 
 // C = A B^T, or with *slices > 1 the K slices' partial products one after
@@ -450,10 +461,10 @@ int mlp_forward(qd_mlp* m, const float* X, i64 n, float* y, cudaStream_t st) {
   return QD_OK;
 }
 
-// gradient of mean((y - t)^2) into G; with want_loss the chunks' sums of
-// squares on their way to m->h_loss (mlp_loss, after a synchronisation).
+// gradient of mean((y - t)^2) into G; the chunks' sums of squares stay in
+// m->lpart (with want_loss, mlp_loss brings them).
 // Bound: latency of nine launches.  A batch of 8,192 rows, with the earlier
-// reductions (64 CTAs for all rows, a barrier per row) and now: 302 and 112 us.
+// reductions (64 CTAs for all rows, a barrier per row) and now: 302 and 104 us.
 int mlp_grad(qd_mlp* m, const float* X, const float* T, i64 n, float* G, bool want_loss, cudaStream_t st) {
   if (n <= 0 || n % GBK) {
     set_error("qd_mlp: the batch (%lld rows) must be a positive multiple of %d", (long long)n, GBK);
@@ -464,8 +475,11 @@ int mlp_grad(qd_mlp* m, const float* X, const float* T, i64 n, float* G, bool wa
   if (rc) return rc;
   const i64 nch = (n + RB - 1) / RB;
   k_tail<<<(unsigned)nch, NH, sizeof(float) * RB * NH, st>>>(m->Z2, m->P, T, n, m->dZ2, m->dZ2t, m->p23, m->lpart);
-  if (want_loss)
-    QD_CUDA(cudaMemcpyAsync(m->h_loss, m->lpart, sizeof(float) * nch, cudaMemcpyDeviceToHost, st));
+  if (want_loss) {
+    if (!m->loss_st) QD_CUDA(cudaStreamCreateWithFlags(&m->loss_st, cudaStreamNonBlocking));
+    if (!m->loss_ev) QD_CUDA(cudaEventCreateWithFlags(&m->loss_ev, cudaEventDisableTiming));
+    QD_CUDA(cudaEventRecord(m->loss_ev, st));
+  }
   // dW2[j][l] = sum_i dZ2[i][j] H1[i][l]: A = dZ2^T (256 x n), B = H1^T (256 x n), K = n
   int nz = m->kslices;
   if ((rc = gemm_nt(m->dZ2t, (int)n, m->H1t, (int)n, m->kpart, NH, NH, NH, (int)n, &nz, st))) return rc;
@@ -479,10 +493,21 @@ int mlp_grad(qd_mlp* m, const float* X, const float* T, i64 n, float* G, bool wa
   return QD_OK;
 }
 
-float mlp_loss(const qd_mlp* m, i64 n) {
+// The loss of the gradient just launched on st, and the end of that gradient:
+// a few KB to pageable memory, on a stream of its own, which holds up the host
+// but not the kernels after k_tail.  A gradient of 8,192 rows: copied on st to
+// pinned memory behind k_tail 110 us, at its end 112, this way 104.
+int mlp_loss(qd_mlp* m, i64 n, cudaStream_t st, float* loss) {
+  const i64 nch = (n + RB - 1) / RB;
+  m->h_loss.resize((size_t)nch);
+  QD_CUDA(cudaStreamWaitEvent(m->loss_st, m->loss_ev, 0));
+  QD_CUDA(cudaMemcpyAsync(m->h_loss.data(), m->lpart, sizeof(float) * nch, cudaMemcpyDeviceToHost, m->loss_st));
+  QD_CUDA(cudaStreamSynchronize(m->loss_st));
+  QD_CUDA(cudaStreamSynchronize(st));
   double s = 0.0;
-  for (i64 z = 0; z < (n + RB - 1) / RB; ++z) s += m->h_loss[z];
-  return (float)(s / (double)n);
+  for (float v : m->h_loss) s += v;
+  *loss = (float)(s / (double)n);
+  return QD_OK;
 }
 }  // namespace
 
@@ -542,9 +567,9 @@ int qd_mlp_destroy(qd_mlp* m) {
   if (!m) return QD_OK;
   cudaSetDevice(m->device);
   cudaDeviceSynchronize();
-  mlp_free_acts(m);
-  mlp_free_grad(m);
-  for (void* p : {(void*)m->P, (void*)m->M, (void*)m->V, (void*)m->G, (void*)m->W2b, (void*)m->W2tb, (void*)m->s23,
+  if (m->loss_st) cudaStreamDestroy(m->loss_st);
+  if (m->loss_ev) cudaEventDestroy(m->loss_ev);
+  for (void* p : {m->acts, m->grads, (void*)m->P, (void*)m->M, (void*)m->V, (void*)m->G, (void*)m->W2b, (void*)m->W2tb, (void*)m->s23,
                   (void*)m->s1})
     if (p) cudaFree(p);
   (void)cudaGetLastError();
@@ -602,8 +627,8 @@ int qd_mlp_grad(qd_mlp* m, const float* d_X, const float* d_T, int64_t n, float*
   cudaStream_t st = (cudaStream_t)stream;
   int rc = mlp_grad(m, d_X, d_T, n, d_grad, loss != nullptr, st);
   if (rc) return rc;
+  if (loss) return mlp_loss(m, n, st, loss);
   QD_CUDA(cudaStreamSynchronize(st));
-  if (loss) *loss = mlp_loss(m, n);
   return QD_OK;
 }
 
@@ -616,11 +641,8 @@ int qd_mlp_train_step(qd_mlp* m, const float* d_X, const float* d_T, int64_t n, 
   QD_CUDA(cudaSetDevice(m->device));
   cudaStream_t st = (cudaStream_t)stream;
   int rc = mlp_grad(m, d_X, d_T, n, m->G, loss != nullptr, st);
+  if (!rc && loss) rc = mlp_loss(m, n, st, loss);
   if (rc) return rc;
-  if (loss) {
-    QD_CUDA(cudaStreamSynchronize(st));
-    *loss = mlp_loss(m, n);
-  }
   m->step += 1;
   const float c1 = 1.0f - std::pow(0.9f, (float)m->step), c2 = 1.0f - std::pow(0.999f, (float)m->step);
   k_adam<<<(unsigned)((NPARAM + 255) / 256), 256, 0, st>>>(m->P, m->G, m->M, m->V, lr, c1, c2);
