@@ -1626,13 +1626,6 @@ size_t full_smem(const TileInfo& t, int n1, int n2, int n3, int n4, bool both) {
 // a task that only writes zeros keeps just the two pair lists
 size_t zero_smem(const TileInfo& t) { return 8 * (size_t)t.npair; }
 
-template <class T>
-int upload_vec(qd_layout* L, const std::vector<T>& vec, T** dptr) {
-  QD_CUDA(cudaMalloc(dptr, std::max<size_t>(1, vec.size()) * sizeof(T)));
-  if (!vec.empty()) QD_CUDA(copy_table(*dptr, vec.data(), vec.size() * sizeof(T)));
-  L->ws_bytes += (i64)(vec.size() * sizeof(T));
-  return QD_OK;
-}
 }  // namespace
 
 static int plan_122(qd_layout* L, Plan122** out) {
@@ -1674,11 +1667,11 @@ static int plan_122(qd_layout* L, Plan122** out) {
   struct GpHost {
     int n1, n2, cnt[3], nf, npair;
   };
+  std::vector<int> gpidx((size_t)ngroup * ngroup, -1);  // place of a group pair in `order`, within a block
   for (int q = 0; q < L->nblock; ++q) {
     const int nh = L->blk[q].x, nb = L->blk[q].y, ntot = L->blk[q].w, pb = L->pbase[q];
     // group pairs in order of first appearance; per group pair its pairs in
     // class order (pairs are enumerated [hh | ph | pp], each class by index)
-    std::map<std::pair<int, int>, int> idx;
     std::vector<std::pair<int, int>> order;
     std::vector<std::vector<int2>> plist;  // {w, packed cells}
     std::vector<GpHost> gh;
@@ -1688,13 +1681,14 @@ static int plan_122(qd_layout* L, Plan122** out) {
       const int w = P - (c == 0 ? 0 : (c == 1 ? nh : nh + nb));
       const int gi = L->gid[pr.x], gj = L->gid[pr.y];
       const int g = std::min(gi, gj), h = std::max(gi, gj);
-      auto ins = idx.emplace(std::make_pair(g, h), (int)order.size());
-      if (ins.second) {
+      int& at = gpidx[(size_t)g * ngroup + h];
+      if (at < 0) {
+        at = (int)order.size();
         order.push_back({g, h});
         plist.emplace_back();
         gh.push_back(GpHost{gsz[g], gsz[h], {0, 0, 0}, 0, 0});
       }
-      const int u = ins.first->second;
+      const int u = at;
       int t1, t2;
       if (g != h) {
         t1 = gi == g ? pr.x : pr.y;
@@ -1714,6 +1708,7 @@ static int plan_122(qd_layout* L, Plan122** out) {
       plist[u].push_back(int2{w, r | ((rm + 1) << 8) | (neg << 16) | (kpos[t1] << 17) | (kpos[t2] << 21)});
       gh[u].cnt[c] += 1;
     }
+    for (const auto& o : order) gpidx[(size_t)o.first * ngroup + o.second] = -1;
     const int u0 = (int)gpd.size() / 2;
     for (size_t u = 0; u < order.size(); ++u) {
       const int g = order[u].first, h = order[u].second;
@@ -1767,11 +1762,11 @@ static int plan_122(qd_layout* L, Plan122** out) {
     }
   std::vector<int2> th(p.tiles.size());
   for (size_t i = 0; i < p.tiles.size(); ++i) th[i] = int2{p.tiles[i].a, p.tiles[i].b};
-  int rc;
-  if ((rc = upload_vec(L, gpd, &p.d_gpd)) || (rc = upload_vec(L, gpp, &p.d_gpp)) ||
-      (rc = upload_vec(L, th, &p.d_tiles)) ||
-      (rc = upload_vec(L, sbase, &p.d_sbase)))
-    return rc;
+  PlanMemory mem;
+  mem.add(std::move(gpd), &p.d_gpd);
+  mem.add(std::move(gpp), &p.d_gpp);
+  mem.add(std::move(th), &p.d_tiles);
+  mem.add(std::move(sbase), &p.d_sbase);
   // generator-like A: the pp pairs' W terms (k_gen_pppp) and the row and
   // column terms of the other five parts (k_122_gen), per block
   {
@@ -1783,6 +1778,22 @@ static int plan_122(qd_layout* L, Plan122** out) {
     std::vector<int> rst[6], cst[6];
     std::vector<int4> rterm_s[6], cterm_s[6];
     std::vector<int4> ptask, gtask, htask;
+    // room for the most terms there can be (memory that is not touched costs
+    // nothing, growing the arrays copies them several times over)
+    {
+      size_t pairs[3] = {0, 0, 0};
+      for (int q = 0; q < L->nblock; ++q) {
+        pairs[0] += L->blk[q].x;
+        pairs[1] += L->blk[q].y;
+        pairs[2] += L->blk[q].z;
+      }
+      for (int slot : {0, 2, 3, 4, 5}) {
+        int cr, cc;
+        part_classes(P_HHHH + slot, cr, cc);
+        rterm_s[slot].reserve(pairs[cr] * 3 * p.gmax);
+        cterm_s[slot].reserve(pairs[cc] * 3 * p.gmax);
+      }
+    }
     int cnt[3] = {0, 0, 0};
     enum { NEG = 1, MA = 2, MB = 4, CB = 8 };
     auto fA = [&](int pt, int h) { return ofph + (pt - n) + h * mp; };  // A's or B's fph(p, h)
@@ -1795,10 +1806,12 @@ static int plan_122(qd_layout* L, Plan122** out) {
       cnt[0] += nh;
       cnt[1] += nb;
       cnt[2] += np;
-      std::map<std::pair<int, int>, int> ihh, iph, ipp;
-      for (int k = 0; k < nh; ++k) ihh[{L->pairs[pb + k].x, L->pairs[pb + k].y}] = k;
-      for (int k = 0; k < nb; ++k) iph[{L->pairs[pb + nh + k].x, L->pairs[pb + nh + k].y}] = k;
-      for (int k = 0; k < np; ++k) ipp[{L->pairs[pb + nh + nb + k].x, L->pairs[pb + nh + nb + k].y}] = k;
+      // index of the pair (u, v), u < v, among the pairs of class c of this block, or -1
+      auto at = [&](int c, int u, int v) {
+        if (u >= v) return -1;
+        const int e = L->ptab[(size_t)u * m + v];
+        return e >= 0 && pt_blk(e) == q && pt_cls(e) == c ? pt_idx(e) : -1;
+      };
       auto grp = [&](int x) { return std::make_pair(L->gstart[L->gid[x]], L->gstart[L->gid[x] + 1]); };
       // members t of G(x) that are holes (want_hole) or particles, excluding `skip`
       auto each = [&](int x, bool want_hole, int skip, auto fn) {
@@ -1808,13 +1821,11 @@ static int plan_122(qd_layout* L, Plan122** out) {
           if ((tt < n) == want_hole && tt != skip) fn(tt);
         }
       };
-      // index and ordering sign of the pair {u, v} in a class map
-      auto srt = [](const std::map<std::pair<int, int>, int>& m, int u, int v, int* idx, int* sg) {
-        auto f = m.find({std::min(u, v), std::max(u, v)});
-        if (f == m.end()) return false;
-        *idx = f->second;
+      // index and ordering sign of the pair {u, v}
+      auto srt = [&](int c, int u, int v, int* idx, int* sg) {
+        *idx = at(c, std::min(u, v), std::max(u, v));
         *sg = u < v ? 1 : -1;
-        return true;
+        return *idx >= 0;
       };
       const auto hhp = [&](int k) { return L->pairs[pb + k]; };
       const auto php = [&](int k) { return L->pairs[pb + nh + k]; };
@@ -1826,8 +1837,8 @@ static int plan_122(qd_layout* L, Plan122** out) {
         for (int side = 0; side < 2; ++side) {
           const int x = side ? y0 : x0, y = side ? x0 : y0;
           each(x, true, -1, [&](int t) {
-            auto f = iph.find({t, y});
-            if (f != iph.end()) ppterm.push_back(int2{f->second, (t) | ((x - n) << 8) | ((side ? 1 : 0) << 20)});
+            const int f = at(1, t, y);
+            if (f >= 0) ppterm.push_back(int2{f, (t) | ((x - n) << 8) | ((side ? 1 : 0) << 20)});
           });
         }
         ppstart.push_back((int)ppterm.size());
@@ -1840,19 +1851,19 @@ static int plan_122(qd_layout* L, Plan122** out) {
           for (int side = 0; side < 2; ++side) {
             const int x = side ? y0 : x0, y = side ? x0 : y0;
             each(x, true, -1, [&](int t) {
-              auto f = iph.find({t, y});
-              if (f != iph.end()) T.push_back(int4{f->second, fA(x, t), side ? NEG : 0, src(1, slot == 4 ? 3 : 5, 0)});
+              const int f = at(1, t, y);
+              if (f >= 0) T.push_back(int4{f, fA(x, t), side ? NEG : 0, src(1, slot == 4 ? 3 : 5, 0)});
             });
             if (slot == 2)  // -s hB fppB(t, x) A_pphh((t,y)) over particles t in G(x)
               each(x, false, y, [&](int t) {
-                if (srt(ipp, side ? y : t, side ? t : y, &idx, &sg))
+                if (srt(2, side ? y : t, side ? t : y, &idx, &sg))
                   T.push_back(int4{idx, fpp(t, x), MB | CB | (sg > 0 ? NEG : 0), src(0, 2, 0)});
               });
           }
         } else if (slot == 5 || slot == 3) {  // rows ph (h, p)
           const int h = php(k).x, pt = php(k).y;
           each(h, false, pt, [&](int t) {
-            if (!srt(ipp, t, pt, &idx, &sg)) return;
+            if (!srt(2, t, pt, &idx, &sg)) return;
             if (slot == 5) {
               T.push_back(int4{idx, fA(t, h), MA | (sg < 0 ? NEG : 0), src(1, 2, 0)});
               T.push_back(int4{idx, fA(t, h), MB | CB | (sg > 0 ? NEG : 0), src(0, 2, 0)});
@@ -1861,7 +1872,7 @@ static int plan_122(qd_layout* L, Plan122** out) {
             }
           });
           each(pt, true, h, [&](int t) {
-            if (!srt(ihh, h, t, &idx, &sg)) return;
+            if (!srt(0, h, t, &idx, &sg)) return;
             if (slot == 5)
               T.push_back(int4{idx, fA(pt, t), sg < 0 ? NEG : 0, src(1, 0, 0)});
             else
@@ -1870,12 +1881,12 @@ static int plan_122(qd_layout* L, Plan122** out) {
         } else {  // slot 0, rows hh (b1, b2)
           const int b1 = hhp(k).x, b2 = hhp(k).y;
           each(b1, false, -1, [&](int t) {
-            auto f = iph.find({b2, t});
-            if (f != iph.end()) T.push_back(int4{f->second, fA(t, b1), MA | NEG, src(1, 5, 0)});
+            const int f = at(1, b2, t);
+            if (f >= 0) T.push_back(int4{f, fA(t, b1), MA | NEG, src(1, 5, 0)});
           });
           each(b2, false, -1, [&](int t) {
-            auto f = iph.find({b1, t});
-            if (f != iph.end()) T.push_back(int4{f->second, fA(t, b2), MA, src(1, 5, 0)});
+            const int f = at(1, b1, t);
+            if (f >= 0) T.push_back(int4{f, fA(t, b2), MA, src(1, 5, 0)});
           });
         }
       };
@@ -1884,10 +1895,10 @@ static int plan_122(qd_layout* L, Plan122** out) {
         if (slot == 4) {  // columns ph (h, p)
           const int h = php(k).x, pt = php(k).y;
           each(h, false, pt, [&](int t) {
-            if (srt(ipp, t, pt, &idx, &sg)) T.push_back(int4{idx, fA(t, h), sg > 0 ? NEG : 0, src(1, 1, 0)});
+            if (srt(2, t, pt, &idx, &sg)) T.push_back(int4{idx, fA(t, h), sg > 0 ? NEG : 0, src(1, 1, 0)});
           });
           each(pt, true, h, [&](int t) {
-            if (!srt(ihh, h, t, &idx, &sg)) return;
+            if (!srt(0, h, t, &idx, &sg)) return;
             T.push_back(int4{idx, fA(pt, t), MA | (sg > 0 ? NEG : 0), src(1, 2, 0)});
             T.push_back(int4{idx, fA(pt, t), MB | CB | (sg < 0 ? NEG : 0), src(0, 2, 0)});
           });
@@ -1897,16 +1908,16 @@ static int plan_122(qd_layout* L, Plan122** out) {
           for (int side = 0; side < 2; ++side) {
             const int kk = side ? k2 : k1, ko = side ? k1 : k2;
             each(kk, false, -1, [&](int t) {
-              auto f = iph.find({ko, t});
-              if (f == iph.end()) return;
+              const int f = at(1, ko, t);
+              if (f < 0) return;
               const int ng = side ? NEG : 0;
-              if (slot == 2) T.push_back(int4{f->second, fA(t, kk), ng, src(1, 4, 0)});
-              else if (slot == 5) T.push_back(int4{f->second, fA(t, kk), ng, src(1, 3, 0)});
-              else T.push_back(int4{f->second, fA(t, kk), MB | ng, src(1, 5, 1)});
+              if (slot == 2) T.push_back(int4{f, fA(t, kk), ng, src(1, 4, 0)});
+              else if (slot == 5) T.push_back(int4{f, fA(t, kk), ng, src(1, 3, 0)});
+              else T.push_back(int4{f, fA(t, kk), MB | ng, src(1, 5, 1)});
             });
             if (slot == 2)  // +s hB fhhB(kk, t) A_pphh(., (t,ko)) over holes t in G(kk)
               each(kk, true, ko, [&](int t) {
-                if (srt(ihh, side ? ko : t, side ? t : ko, &idx, &sg))
+                if (srt(0, side ? ko : t, side ? t : ko, &idx, &sg))
                   T.push_back(int4{idx, fhh(kk, t), MB | CB | (sg < 0 ? NEG : 0), src(0, 2, 0)});
               });
           }
@@ -1938,17 +1949,20 @@ static int plan_122(qd_layout* L, Plan122** out) {
     // concatenated: per slot a start 0 then the pairs' ends, shifted by the
     // slot's first term in the joint term arrays
     std::vector<int> rall, call;
-    std::vector<int4> rterm, cterm;
+    int r0 = 0, c0 = 0;
+    const auto next = [](int at, size_t n) {  // where PlanMemory places the terms of the next slot
+      constexpr int A = (int)(PlanMemory::ALIGN / sizeof(int4));
+      return at + ((int)n + A - 1) / A * A;
+    };
     for (int slot = 0; slot < 6; ++slot) {
       p.gen_rso[slot] = (int)rall.size();
       p.gen_cso[slot] = (int)call.size();
-      const int r0 = (int)rterm.size(), c0 = (int)cterm.size();
       rall.push_back(r0);
       for (int e : rst[slot]) rall.push_back(r0 + e);
       call.push_back(c0);
       for (int e : cst[slot]) call.push_back(c0 + e);
-      rterm.insert(rterm.end(), rterm_s[slot].begin(), rterm_s[slot].end());
-      cterm.insert(cterm.end(), cterm_s[slot].begin(), cterm_s[slot].end());
+      r0 = next(r0, rterm_s[slot].size());
+      c0 = next(c0, cterm_s[slot].size());
     }
     p.nsp_pppp = (int)ptask.size();
     p.nsp_gen = (int)gtask.size();
@@ -2008,15 +2022,18 @@ static int plan_122(qd_layout* L, Plan122** out) {
     std::vector<int4> ltask;
     for (const auto& x : lt) ltask.push_back(x.second);
     p.nsp_ladder = (int)ltask.size();
-    if ((rc = upload_vec(L, ltask, &p.d_ltask))) return rc;
+    mem.add(std::move(ltask), &p.d_ltask);
     std::vector<int> ppbase(L->nblock);
     for (int q = 0; q < L->nblock; ++q) ppbase[q] = gbase[2 * L->nblock + q];
-    if ((rc = upload_vec(L, ppbase, &p.d_ppbase)) || (rc = upload_vec(L, ppstart, &p.d_ppstart)) ||
-        (rc = upload_vec(L, ppterm, &p.d_ppterm)) || (rc = upload_vec(L, gbase, &p.d_gbase)) ||
-        (rc = upload_vec(L, rall, &p.d_rstart)) || (rc = upload_vec(L, call, &p.d_cstart)) ||
-        (rc = upload_vec(L, rterm, &p.d_rterm)) || (rc = upload_vec(L, cterm, &p.d_cterm)) ||
-        (rc = upload_vec(L, all, &p.d_sptask)))
-      return rc;
+    mem.add(std::move(ppbase), &p.d_ppbase);
+    mem.add(std::move(ppstart), &p.d_ppstart);
+    mem.add(std::move(ppterm), &p.d_ppterm);
+    mem.add(std::move(gbase), &p.d_gbase);
+    mem.add(std::move(rall), &p.d_rstart);
+    mem.add(std::move(call), &p.d_cstart);
+    for (int slot = 0; slot < 6; ++slot) mem.add(std::move(rterm_s[slot]), slot ? (int4**)nullptr : &p.d_rterm);
+    for (int slot = 0; slot < 6; ++slot) mem.add(std::move(cterm_s[slot]), slot ? (int4**)nullptr : &p.d_cterm);
+    mem.add(std::move(all), &p.d_sptask);
   }
   {  // k_122_full: buckets by shared memory, small tiles with fewer threads
     std::vector<std::pair<size_t, int>> v;
@@ -2048,7 +2065,7 @@ static int plan_122(qd_layout* L, Plan122** out) {
       });
       p.fbuckets.push_back(b);
     }
-    if ((rc = upload_vec(L, tasks, &p.d_ftask))) return rc;
+    mem.add(std::move(tasks), &p.d_ftask);
   }
   // particle-hole channel: first cc row of each (G1, G2) and the launches
   p.ng = ngroup;
@@ -2100,13 +2117,11 @@ static int plan_122(qd_layout* L, Plan122** out) {
       b.count = (int)tasks.size() - b.first;
       p.pbuckets.push_back(b);
     }
-    int rc2;
-    if ((rc2 = upload_vec(L, gpg, &p.d_gpg)) || (rc2 = upload_vec(L, zrow, &p.d_zrow)) ||
-        (rc2 = upload_vec(L, tasks, &p.d_ptask)))
-      return rc2;
+    mem.add(std::move(gpg), &p.d_gpg);
+    mem.add(std::move(zrow), &p.d_zrow);
+    mem.add(std::move(tasks), &p.d_ptask);
   }
-  QD_CUDA(cudaMalloc(&p.d_ftab, sizeof(double2) * 2 * (size_t)std::max(1, p.nfent)));
-  L->ws_bytes += (i64)sizeof(double2) * 2 * p.nfent;
+  mem.room(2 * (i64)p.nfent, &p.d_ftab);
   for (const void* fn : {(const void*)k_122_tile<1, 64>, (const void*)k_122_tile<2, 64>,
                          (const void*)k_122_tile<1, 128>, (const void*)k_122_tile<2, 128>,
                          (const void*)k_122_tile<1, 256>, (const void*)k_122_tile<2, 256>,
@@ -2121,8 +2136,11 @@ static int plan_122(qd_layout* L, Plan122** out) {
     QD_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)SMEM_MAX_122 - (int)fa.sharedSizeBytes));
   }
-  plans()[L] = p;
-  *out = &plans()[L];
+  const int rc = mem.commit(L);
+  if (rc) return rc;
+  Plan122& kept = plans()[L];
+  kept = std::move(p);
+  *out = &kept;
   return QD_OK;
 }
 
@@ -2175,8 +2193,9 @@ static int build_variant(qd_layout* L, const Plan122* p, std::vector<std::pair<s
       const TileInfo &tx = p->tiles[x.x], &ty = p->tiles[y.x];
       return tx.b != ty.b ? tx.b < ty.b : tx.a < ty.a;
     });
-  int rc = upload_vec(L, all, &ts.d_task);
-  if (rc) return rc;
+  QD_CUDA(cudaMalloc(&ts.d_task, std::max<size_t>(1, all.size()) * sizeof(int2)));
+  if (!all.empty()) QD_CUDA(copy_table(ts.d_task, all.data(), all.size() * sizeof(int2)));
+  L->ws_bytes += (i64)(all.size() * sizeof(int2));
   return QD_OK;
 }
 
@@ -2230,11 +2249,6 @@ void drop_122_plan(const qd_layout* L) {
   auto it = plans().find(L);
   if (it == plans().end()) return;
   Plan122& p = it->second;
-  for (void* ptr : {(void*)p.d_gpd, (void*)p.d_gpp, (void*)p.d_tiles, (void*)p.d_sbase,
-                    (void*)p.d_ftab, (void*)p.d_ltask, (void*)p.d_ftask, (void*)p.d_gpg, (void*)p.d_zrow, (void*)p.d_ptask, (void*)p.d_ppbase,
-                    (void*)p.d_ppstart, (void*)p.d_ppterm, (void*)p.d_gbase, (void*)p.d_rstart,
-                    (void*)p.d_cstart, (void*)p.d_rterm, (void*)p.d_cterm, (void*)p.d_sptask})
-    if (ptr) cudaFree(ptr);
   for (auto& kv : p.sets) {
     if (kv.second.d_task) cudaFree(kv.second.d_task);
     for (TaskSet& t : kv.second.alts)

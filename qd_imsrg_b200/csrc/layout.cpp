@@ -305,31 +305,29 @@ int layout_upload(qd_layout* L) {
 }
 
 int PlanMemory::commit(qd_layout* L) {
-  const auto place = [](size_t* at, size_t bytes) {  // 256-byte boundaries, as cudaMalloc gives
-    const size_t o = *at;
-    *at += (bytes + 255) / 256 * 256;
-    return o;
-  };
-  size_t end = 0;
-  std::vector<size_t> to, ro;
-  for (const Piece& p : tables_) to.push_back(place(&end, p.bytes));
-  std::vector<unsigned char> host(end);
-  for (size_t k = 0; k < tables_.size(); ++k)
-    if (tables_[k].bytes) std::memcpy(host.data() + to[k], tables_[k].src, tables_[k].bytes);
-  for (const Piece& p : rooms_) ro.push_back(place(&end, p.bytes));
+  size_t bytes = 0;
+  std::vector<size_t> at;
+  for (const Piece& p : pieces_) {
+    at.push_back(bytes);
+    bytes += (p.bytes + ALIGN - 1) / ALIGN * ALIGN;
+  }
   unsigned char* d = nullptr;
-  QD_CUDA(cudaMalloc((void**)&d, std::max<size_t>(1, end)));
-  if (!host.empty()) {
-    const cudaError_t e = copy_table(d, host.data(), host.size());
-    if (e != cudaSuccess) {
-      cudaFree(d);
-      return cuda_fail(e, "copy of a plan's tables");
-    }
+  QD_CUDA(cudaMalloc((void**)&d, std::max<size_t>(1, bytes)));
+  cudaError_t e = cudaSuccess;
+  for (size_t k = 0; k < pieces_.size() && e == cudaSuccess; ++k)
+    if (pieces_[k].src && pieces_[k].bytes)
+      e = cudaMemcpyAsync(d + at[k], pieces_[k].src, pieces_[k].bytes, cudaMemcpyHostToDevice, cudaStreamLegacy);
+  // in place before this returns, as copy_table
+  const cudaError_t w = cudaStreamSynchronize(cudaStreamLegacy);
+  if (e == cudaSuccess) e = w;
+  if (e != cudaSuccess) {
+    cudaFree(d);
+    return cuda_fail(e, "copy of a plan's tables");
   }
   L->dev_allocs.push_back(d);
-  L->ws_bytes += (i64)end;
-  for (size_t k = 0; k < tables_.size(); ++k) *tables_[k].out = d + to[k];
-  for (size_t k = 0; k < rooms_.size(); ++k) *rooms_[k].out = d + ro[k];
+  L->ws_bytes += (i64)bytes;
+  for (size_t k = 0; k < pieces_.size(); ++k)
+    if (pieces_[k].out) *pieces_[k].out = d + at[k];
   return QD_OK;
 }
 

@@ -18,6 +18,8 @@
 #include <map>
 #include <memory>
 #include <string>
+#include <memory>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/qd_imsrg.h"
@@ -236,18 +238,22 @@ inline cudaError_t copy_table(void* dst, const void* src, size_t bytes) {
 }
 
 // Device memory of one plan, tables and scratch together in one allocation
-// that belongs to the layout, the tables brought there by one copy.  commit()
-// sets every pointer, or on failure none and keeps nothing.  The vectors given
-// to add() must live until then.
+// that belongs to the layout.  The tables lie in the order of add(), each on
+// the next multiple of ALIGN bytes.  commit() brings them to the device and
+// sets every pointer, or on failure none and keeps nothing.
 class PlanMemory {
  public:
-  template <class T>
-  void add(const std::vector<T>& v, const T** out) {
-    tables_.push_back(Piece{v.data(), v.size() * sizeof(T), (const void**)out});
+  static constexpr size_t ALIGN = 256;
+  template <class T, class P>
+  void add(std::vector<T> v, P** out) {
+    static_assert(std::is_same<typename std::remove_const<P>::type, T>::value, "pointer of another type");
+    auto kept = std::make_shared<std::vector<T>>(std::move(v));
+    pieces_.push_back(Piece{kept->data(), kept->size() * sizeof(T), (const void**)out});
+    kept_.push_back(kept);
   }
   template <class T>
   void room(i64 n, T** out) {  // not initialised
-    rooms_.push_back(Piece{nullptr, (size_t)n * sizeof(T), (const void**)out});
+    pieces_.push_back(Piece{nullptr, (size_t)n * sizeof(T), (const void**)out});
   }
   int commit(qd_layout* L);
 
@@ -255,9 +261,10 @@ class PlanMemory {
   struct Piece {
     const void* src;
     size_t bytes;
-    const void** out;
+    const void** out;  // may be null
   };
-  std::vector<Piece> tables_, rooms_;
+  std::vector<Piece> pieces_;
+  std::vector<std::shared_ptr<void>> kept_;
 };
 
 int layout_build(qd_layout* L, int nbody, int emax, const double* eig);
