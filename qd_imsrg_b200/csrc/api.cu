@@ -351,14 +351,10 @@ struct Branches {
   int open = 0;  // bit k: branch k may have work
   int fork(qd_layout* l, const qd_op* A) {
     L = l;
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    QD_CUDA(cudaStreamIsCapturing(L->stream, &cs));
-    const bool cap = cs != cudaStreamCaptureStatusNone;
     if (L->prof.on || (!gen_like(A->zero_mask) && L->neq >= FORK_ENTRIES)) return QD_OK;
-    if (!L->ev_fork) {
-      if (cap) return QD_OK;  // no stream or event is created inside a capture
-      TRY(make_branches(L));
-    }
+    bool use;
+    TRY(use_branches(L, &use));
+    if (!use) return QD_OK;
     QD_CUDA(cudaEventRecord(L->ev_fork, L->stream));
     on = true;
     // The split form's programs (111, the products, the ladders) share one set
@@ -504,6 +500,25 @@ int qd::make_branches(qd_layout* L) {
     if (!L->ev_side[k]) QD_CUDA(cudaEventCreateWithFlags(&L->ev_side[k], cudaEventDisableTiming));
   }
   QD_CUDA(cudaEventCreateWithFlags(&L->ev_fork, cudaEventDisableTiming));
+  return QD_OK;
+}
+
+// Whether the calling launch may use the side streams.  Making them takes
+// about 200 us; a call without them takes 10 to 40 us longer.  So the first
+// calls go without: a layout that is used once or twice, as in a scan over
+// dots, never pays for them (first commutator at N=2, R=3 780 and 580 us, first
+// EOM product at N=12, R=10 1280 and 1100).  A step graph makes them for its
+// capture, since it is replayed.
+int qd::use_branches(qd_layout* L, bool* use) {
+  constexpr int SERIAL_CALLS = 2;
+  *use = L->ev_fork != nullptr;
+  if (*use) return QD_OK;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  QD_CUDA(cudaStreamIsCapturing(L->stream, &cs));
+  if (cs != cudaStreamCaptureStatusNone) return QD_OK;  // no stream or event is created inside a capture
+  if (L->serial_calls++ < SERIAL_CALLS) return QD_OK;
+  TRY(make_branches(L));
+  *use = true;
   return QD_OK;
 }
 

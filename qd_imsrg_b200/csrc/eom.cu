@@ -507,10 +507,8 @@ extern "C" int qd_eom_matvec_target(const qd_op* H, int ml, int ms, const double
   const double hh = (double)H->herm;
   // the 1p1h part beside the GEMM and k_eom_2b, which write other entries
   // (a product at N=12, R=10: 97 us when it followed them, 85 beside them)
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  QD_CUDA(cudaStreamIsCapturing(s, &cs));
-  if (cs == cudaStreamCaptureStatusNone) EOM_TRY(make_branches(L));  // nothing is created inside a capture
-  const bool side = p->n1 > 0 && p->n2 > 0 && L->ev_fork;
+  bool side = false;
+  if (p->n1 > 0 && p->n2 > 0) EOM_TRY(use_branches(L, &side));
   SideJoin join{L, s};  // waits on every way out: d_w is the caller's
   if (side) {
     QD_CUDA(cudaEventRecord(L->ev_fork, s));

@@ -186,6 +186,7 @@ struct qd_layout {
   static constexpr int NSIDE = 3;
   cudaStream_t side[NSIDE] = {nullptr};
   cudaEvent_t ev_fork = nullptr, ev_side[NSIDE] = {nullptr};
+  int serial_calls = 0;  // calls that went without them
   qd::i64 ws_bytes = 0;
   // GEMM programs
   qd::GemmProgram prog_ladder, prog_221, prog_111, prog_pandya;
@@ -349,6 +350,7 @@ int launch_122(qd_layout* L, const qd_op* A, const qd_op* B, double* C, bool lad
 bool gen_ladder_fused(const qd_layout* L, int q);
 int launch_calc_cc(qd_layout* L, const qd_op* H, double* X);
 int make_branches(qd_layout* L);  // the side streams and events of a layout (api.cu)
+int use_branches(qd_layout* L, bool* use);
 // Particle-hole channel (commutators.f90:716-980): C += the four re-coupled
 // Z terms, over the commutator_122 tiles (kernels_122.cu).
 int launch_pandya_tiles(qd_layout* L, const double* Z, double* C);
