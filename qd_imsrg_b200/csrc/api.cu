@@ -266,8 +266,10 @@ GemmProgram& ladder_program(qd_layout* L, const qd_op* A) {
 
 // From here on a BCH term's update of HS runs where C_pppp is made: reading
 // C_pppp back then costs more than the slower kernel does.  Whole flows with
-// the update split and in one pass (ms): N=12 R=12 6.7 and 6.3, N=12 R=14
-// (5.4 M entries) 10.9 and 10.6, N=20 R=16 (13 M) 19.0 and 19.5.
+// the update in one pass and split (ms, medians of 24, three runs within 0.3%):
+// N=20 R=12 (1.7 M entries) 6.90 and 7.33, N=12 R=14 (5.4 M) 10.63 and 10.88,
+// N=12 R=15 (8.7 M) 14.49 and 14.55, N=20 R=16 (13 M) 19.48 and 19.05, N=6 R=16
+// (14 M) 14.41 and 13.70, N=20 R=20 (62 M) 61.1 and 57.9: equal near 9 M.
 constexpr i64 SPLIT_UPDATE_ENTRIES = 8000000;
 // Whether a BCH term's update of HS runs where C_pppp is made: C_pppp must be
 // final there (no ladder left to the grouped GEMM; the particle-hole channel
