@@ -236,19 +236,34 @@ def stage_roofline(prof: dict, flops: dict, neq2b: int, dgemm_peak: float, hbm_p
             "unit": "GB/s", "peak_source": hbm_source(), "algorithmic_per_launch": byts}
 
 
-# DRAM bytes per launch (dram__bytes_read.sum + dram__bytes_write.sum) of the
-# engine's stages, from one ncu capture of the N=20, R=17 case (19,841,598
-# entries per operator, inputs above L2).  GEMM and gather traffic is operand
-# and output traffic, so it is scaled to the benchmarked basis by the number
-# of entries per operator.
-NCU_NEQ = 19841598
-NCU_TRAFFIC = {"ladder_gemm": 794.761728e6 + 162.643712e6, "pandya_gemm": 200.469760e6 + 676.389888e6,
-               "pandya_gather": 2126.409e6 + 154.573824e6}
-# commutator_122 of one flow commutator [Omega, X] in its earlier form (32 x 32
-# C_pppp tiles and k_122_gen, without the ladders), from the N=20, R=18 capture (29,618,726 entries per
-# operator): scaled to the flow's basis by entries per operator
-NCU_FLOW_NEQ = 29618726
-NCU_FLOW_TRAFFIC = {"c122": (29.3e6 + 139.6e6) + (179.3e6 + 51.9e6)}
+# DRAM bytes per commutator (dram__bytes_read.sum + dram__bytes_write.sum, one
+# pass, cold caches) of the engine's stages at N=20, R=20: two dense operators
+# with the particle-hole channel, and one term of the flow's series (its 122
+# stage holds the ladders and the update of HS for C_pppp).
+NCU_BASIS = (20, 20)
+NCU_SOURCE = "ncu dram bytes at N=20 R=20 (profiles/dram_bytes_N20R20.md)"
+NCU_TRAFFIC = {"ladder_gemm": 5.301e9, "pandya_gemm": 1.605e9, "c122": 2.760e9, "pandya_gather": 3.513e9}
+NCU_FLOW_TRAFFIC = {"c122": 1.959e9}
+
+
+def stage_traffic(table: dict, stage: str, nbody: int, emax: int) -> dict:
+    known = stage in table and (nbody, emax) == NCU_BASIS
+    return {"traffic": table[stage] if known else None, "traffic_source": NCU_SOURCE if known else None}
+
+
+# entries from which a term's update of HS runs in the 122 stage (csrc/api.cu)
+SPLIT_UPDATE_ENTRIES = 8000000
+
+
+def flow_c122_bytes(dims: np.ndarray, neq: int, neq2b: int, split: int) -> float:
+    """Bytes that the 122 stage of one flow commutator cannot do without: B's
+    two-body parts and Omega's Vpphh read, C's written, and where the stage
+    also updates HS its Vpppp read and written."""
+    nh, npp = dims[:, 0].astype(np.int64), dims[:, 2].astype(np.int64)
+    entries = 2 * neq2b + int((nh * npp).sum())
+    if neq >= SPLIT_UPDATE_ENTRIES and not split and nh.max() <= 16:
+        entries += 2 * int((npp * npp).sum())
+    return 8.0 * entries
 
 
 def _peaks_present() -> bool:
@@ -567,14 +582,14 @@ def run_flow(args, world, rank, local):
     neq2b = P.neq - (1 + n * n + mp * mp + mp * n)
     name, (ms, cnt) = max(prof.items(), key=lambda kv: kv[1][0])
     per = (ms / max(cnt, 1)) / 1e3
-    byts = 3.0 * 8 * neq2b
+    gen = name == "c122"
+    byts = flow_c122_bytes(P.dims, P.neq, neq2b, args.split) if gen else 3.0 * 8 * neq2b
     roof = {"kernel": name, "bound": "hbm", "achieved": byts / per / 1e9, "peak": hbm_peak_gbs(), "unit": "GB/s",
             "peak_source": hbm_source(), "algorithmic_per_launch": byts,
-            "note": "stage with the most device time, per launch = per commutator; bytes = read A, B and "
-                    "write C two-body parts once",
-            "traffic": NCU_FLOW_TRAFFIC[name] * P.neq / NCU_FLOW_NEQ if name in NCU_FLOW_TRAFFIC else None,
-            "traffic_source": "ncu dram bytes of an earlier form (without ladders and update) of one commutator at N=20 R=18, "
-                              "scaled by entries per operator" if name in NCU_FLOW_TRAFFIC else None}
+            "note": "stage with the most device time, per launch = per commutator; bytes = " +
+                    ("read B's two-body parts and Omega's Vpphh, write C's, read and write HS's Vpppp where the stage "
+                     "updates it" if gen else "read A, B and write C two-body parts once")}
+    roof.update(stage_traffic({} if args.split or args.pandya else NCU_FLOW_TRAFFIC, name, args.nbody, args.emax))
     roof["frac"] = roof["achieved"] / roof["peak"]
     cpu = None
     if rank == 0 and world == 1 and not args.no_cpu_baseline:
@@ -615,8 +630,9 @@ BATCH_GRID = [(nb, hw) for nb in (6, 12, 20, 30) for hw in (0.1, 0.28, 0.5, 1.0)
 
 def run_batch(args, world, rank, local):
     """16 independent flows (the N x hbar-omega grid) run concurrently by
-    qd_magnus_flow_batch (one host thread and stream per instance) against
-    the same flows one after another; per-instance E_gs must agree."""
+    qd_magnus_flow_batch (in lockstep, and with one host thread and stream per
+    instance) against the same flows one after another; per-instance E_gs must
+    agree."""
     import torch
 
     import qd_imsrg_b200 as qd
@@ -969,9 +985,7 @@ def main():
     roof = stage_roofline(prof, fl, neq2b, dgemm_peak, hbm_peak_gbs(), args.split)
     roof["frac"] = roof["achieved"] / roof["peak"]
     stage = max(prof.items(), key=lambda kv: kv[1][0])[0]
-    roof["traffic"] = NCU_TRAFFIC[stage] * neq / NCU_NEQ if stage in NCU_TRAFFIC else None
-    roof["traffic_source"] = ("ncu dram bytes of the N=20 R=17 capture, scaled by entries per operator"
-                              if roof["traffic"] is not None else None)
+    roof.update(stage_traffic({} if args.split else NCU_TRAFFIC, stage, args.nbody, args.emax))
 
     cpu = None
     if rank == 0 and world == 1 and not args.no_cpu_baseline and args.nbody == NBODY and args.emax == EMAX:

@@ -106,9 +106,13 @@ int qd_layout_profile(qd_layout* L, int enable);
 int qd_layout_profile_read(qd_layout* L, double* ms, int64_t* counts, int nstage);
 /* number of kernels this library has launched for the layout so far        */
 int qd_layout_launches(const qd_layout* L, int64_t* n);
-/* The autotuner's choices so far, as text: the first commutator_122 launch
- * for each pair of zero-part masks times every launch bucket with 64-, 128-
- * and 256-thread CTAs and keeps the fastest (results do not depend on it).
+/* The autotuner's choices so far, as text.  commutator_122 of two dense
+ * operators, on its first launch on a layout, times every launch bucket with
+ * 64-, 128- and 256-thread CTAs and keeps the fastest; from a million entries
+ * on, where one operand's one-body part couples holes to particles only, the
+ * first launch for each pair of zero-part masks does the same for each of four
+ * bucketings.  A left operand that holds only fph and Vpphh needs no tuning.
+ * Results do not depend on the choices.
  * Writes at most len bytes (NUL-terminated) into buf; *needed = full size.
  * No reference counterpart.                                                 */
 int qd_layout_tuning(const qd_layout* L, char* buf, int64_t len, int64_t* needed);

@@ -936,9 +936,8 @@ __global__ void __launch_bounds__(GP_T, UPD ? 3 : 4) k_gen_pppp(DevLayout L, con
 // GEMM, whose read-modify-write of C is then a smaller part of the work.
 bool gen_ladder_fused(const qd_layout* L, int q) { return L->blk[q].x > 0 && L->blk[q].x <= GP_KMAX; }
 
-// one term more than any tile stages: an empty last column reads (and drops) it
-size_t gp_smem(int terms) { return sizeof(double) * GP_B * GP_LD + sizeof(StagedTerm) * (size_t)(terms + 1); }
-size_t gen_smem(int terms) { return sizeof(StagedTerm) * (size_t)(terms + 1); }
+size_t gp_smem(int terms) { return sizeof(double) * GP_B * GP_LD + sizeof(StagedTerm) * (size_t)terms; }
+size_t gen_smem(int terms) { return sizeof(StagedTerm) * (size_t)terms; }
 static_assert(4 * GP_KMAX * GP_B <= GP_B * GP_LD, "the panels share the tile's shared memory");
 
 // The other five parts of a block for a generator-like A, one 64 x 64 tile
@@ -2302,11 +2301,7 @@ static int launch_bucket(qd_layout* L, const Plan122* p, const TaskSet* ts, cons
   return QD_OK;
 }
 
-// Autotuner: the first launch of a task set times every bucket with 64-, 128-
-// and 256-thread CTAs (CUDA events, best of two runs each) on the real operands,
-// writing into a scratch operator of the layout, and keeps the fastest size
-// per bucket.  Every output cell is summed by one thread in a fixed order
-// whatever the CTA size, so the choice never changes a result.
+// The CTA size of each bucket of one bucketing (see tune_122).
 static int tune_variant(qd_layout* L, Plan122* p, TaskSet* ts, const qd_op* A, const qd_op* B, int spA, int spB,
                         double* scratch, cudaEvent_t e0, cudaEvent_t e1) {
   ts->ms_total = 0.f;
@@ -2385,7 +2380,7 @@ static int tune_122(qd_layout* L, Plan122* p, TaskSet* ts, const qd_op* A, const
   return QD_OK;
 }
 
-// Text summary of the autotuned buckets of every task set of the layout.
+// One bucket of k_122_full on stream st.
 static int launch_full(qd_layout* L, const Plan122* p, const Plan122::FullBucket& b, int threads, const qd_op* A,
                        const qd_op* B, double* C, cudaStream_t st) {
 #define QD_FULL_LAUNCH(NT, BOTH)                                                                                    \
@@ -2438,6 +2433,7 @@ static int tune_full(qd_layout* L, Plan122* p, const qd_op* A, const qd_op* B) {
   return QD_OK;
 }
 
+// Text summary of the autotuned buckets: k_122_full's, then every task set's.
 std::string tuning_report_122(const qd_layout* L) {
   std::lock_guard<std::mutex> lock(g_plan_mutex);
   auto it = plans().find(L);

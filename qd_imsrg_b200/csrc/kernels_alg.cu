@@ -1,7 +1,7 @@
 // kernels_alg.cu -- bandwidth-bound kernels of the commutator engine:
 // axpy (add_arrays), deterministic FP64 reductions (commutator_110/220 traces,
-// mat_2_norm, MBPT2, HF_E2), the White generator, the Pandya re-coupling
-// (calc_cc) and the particle-hole gather of commutator_222.
+// mat_2_norm, MBPT2, HF_E2), the White generator, the BCH term's update with
+// its norms and exit test, and the Pandya transform of an operator (calc_cc).
 #include <algorithm>
 #include <vector>
 
