@@ -353,7 +353,7 @@ struct qd_mlp {
   long long step = 0;
   // activations of up to cap rows, and what a gradient needs beside them for up to gcap
   qd::i64 cap = 0, gcap = 0;
-  void *acts = nullptr, *grads = nullptr;  // their memory, one allocation each
+  void *params = nullptr, *acts = nullptr, *grads = nullptr;  // all memory, one allocation each
   bf16* H1 = nullptr;
   float* Z2 = nullptr;
   float *Z1 = nullptr, *dH1 = nullptr;
@@ -538,17 +538,19 @@ int qd_mlp_create(int device, uint64_t seed, qd_mlp** out) {
   for (i64 e = O_W2; e < O_B2; ++e) p[e] = nd(rng) * std::sqrt(2.0f / NH);
   for (i64 e = O_W3; e < O_B3; ++e) p[e] = nd(rng) * std::sqrt(1.0f / NH);
   int rc = QD_OK;
-  auto al = [&](void** ptr, size_t b) {
-    if (!rc && cudaMalloc(ptr, b) != cudaSuccess) rc = cuda_fail(cudaErrorMemoryAllocation, "qd_mlp_create");
-  };
-  al((void**)&m->P, sizeof(float) * NPARAM);
-  al((void**)&m->M, sizeof(float) * NPARAM);
-  al((void**)&m->V, sizeof(float) * NPARAM);
-  al((void**)&m->G, sizeof(float) * NPARAM);
-  al((void**)&m->W2b, sizeof(bf16) * NH * NH);
-  al((void**)&m->W2tb, sizeof(bf16) * NH * NH);
-  al((void**)&m->s23, sizeof(float) * (2 * NH + 1));
-  al((void**)&m->s1, sizeof(float) * (NH + NH * NI));
+  i64 one = 0;
+  rc = mlp_alloc(&m->params, &one, 1, [&](void* b) {
+    size_t o = 0;
+    m->P = mlp_place<float>(b, &o, NPARAM);
+    m->M = mlp_place<float>(b, &o, NPARAM);
+    m->V = mlp_place<float>(b, &o, NPARAM);
+    m->G = mlp_place<float>(b, &o, NPARAM);
+    m->W2b = mlp_place<bf16>(b, &o, NH * NH);
+    m->W2tb = mlp_place<bf16>(b, &o, NH * NH);
+    m->s23 = mlp_place<float>(b, &o, 2 * NH + 1);
+    m->s1 = mlp_place<float>(b, &o, NH + NH * NI);
+    return o;
+  });
   if (rc) {
     delete m;
     return rc;
@@ -569,8 +571,7 @@ int qd_mlp_destroy(qd_mlp* m) {
   cudaDeviceSynchronize();
   if (m->loss_st) cudaStreamDestroy(m->loss_st);
   if (m->loss_ev) cudaEventDestroy(m->loss_ev);
-  for (void* p : {m->acts, m->grads, (void*)m->P, (void*)m->M, (void*)m->V, (void*)m->G, (void*)m->W2b, (void*)m->W2tb, (void*)m->s23,
-                  (void*)m->s1})
+  for (void* p : {m->params, m->acts, m->grads})
     if (p) cudaFree(p);
   (void)cudaGetLastError();
   delete m;
