@@ -241,7 +241,7 @@ def stage_roofline(prof: dict, flops: dict, neq2b: int, dgemm_peak: float, hbm_p
 # with the particle-hole channel, and one term of the flow's series (its 122
 # stage holds the ladders and the update of HS for C_pppp).
 NCU_BASIS = (20, 20)
-NCU_SOURCE = "ncu dram bytes at N=20 R=20 (profiles/dram_bytes_N20R20.md)"
+NCU_SOURCE = "ncu dram bytes of these kernels at N=20 R=20, launch by launch under profiles/"
 NCU_TRAFFIC = {"ladder_gemm": 5.301e9, "pandya_gemm": 1.605e9, "c122": 2.760e9, "pandya_gather": 3.513e9}
 NCU_FLOW_TRAFFIC = {"c122": 1.959e9}
 
